@@ -160,6 +160,8 @@ struct mfd_handle {
   static constexpr int kSide = 4;
   cudaStream_t sst[kSide] = {};
   cudaEvent_t ev_lvl = nullptr, ev_side[kSide] = {};
+  cudaStream_t sinv = nullptr;                      // inverted diagonal blocks, off the panel chain
+  cudaEvent_t ev_inv = nullptr;
 
   // systems
   std::vector<Symbolic> sys;
@@ -203,6 +205,7 @@ struct mfd_handle {
   void* d_panel = nullptr;
   void* d_upool = nullptr;
   void* d_diag = nullptr;
+  double* d_packed = nullptr;                       // the current panel step's packed diagonal blocks, one per list slot
   float* d_q = nullptr;                             // FP32: packed update operands, two step parities
   DBuf<double> d_a, d_b, d_xp, d_bp, d_r, d_norms, d_cnorms, d_xt;
   void* d_X = nullptr;   // T, n_total x nrhs
@@ -242,7 +245,7 @@ struct mfd_handle {
     for (auto& kv : g_solve) cudaGraphExecDestroy(kv.second);
     for (auto& kv : g_ir) cudaGraphExecDestroy(kv.second);
     if (bst) cudaStreamDestroy(bst);
-    for (void* p : {d_panel, d_upool, d_diag, d_X, d_V, d_S, static_cast<void*>(d_q), d_bwpart})
+    for (void* p : {d_panel, d_upool, d_diag, d_X, d_V, d_S, static_cast<void*>(d_q), static_cast<void*>(d_packed), d_bwpart})
       if (p) cudaFree(p);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
@@ -251,6 +254,8 @@ struct mfd_handle {
     for (cudaEvent_t e : ev_part)
       if (e) cudaEventDestroy(e);
     if (ev_lvl) cudaEventDestroy(ev_lvl);
+    if (ev_inv) cudaEventDestroy(ev_inv);
+    if (sinv) cudaStreamDestroy(sinv);
     for (int b = 0; b < kSide; ++b) {
       if (ev_side[b]) cudaEventDestroy(ev_side[b]);
       if (sst[b]) cudaStreamDestroy(sst[b]);
@@ -763,6 +768,7 @@ int upload_plan(mfd_handle* h) {
   CK(cudaMalloc(&h->d_panel, (std::max<int64_t>(h->panel_elems, 1) + 32) * esz));
   CK(cudaMalloc(&h->d_upool, std::max<int64_t>(h->upool_elems, 1) * esz));
   CK(cudaMalloc(&h->d_diag, (size_t)std::max<int64_t>(h->dinv_elems, 1) * esz));
+  CK(cudaMalloc(&h->d_packed, (size_t)std::max(1, h->max_large_count) * kPackedPanelElems * sizeof(double)));
   CK(cudaMalloc(&h->d_bwpart, (size_t)std::max<int64_t>(h->bw_part_elems, 1) * esz));
   if (h->fp32 && h->q_elems > 0) {
     CK(cudaMalloc(&h->d_q, (size_t)(2 * h->q_elems) * sizeof(float)));
@@ -892,6 +898,7 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
   // 1 FFMA tiles, 2 tcgen05 1xTF32 (FP32), 3 FP64 DMMA in whole 128 x 128 tiles, one CTA per SM
   const int kind = h->opt.reserved[0];
   const bool side = side_streams(h);
+  bool inverting = false;                   // launches on h->sinv to wait for
   for (const LevelPlan& L : h->levels) {
     // the level's small-front bins and its large fronts are independent (their
     // children are on lower levels; their update matrices are distinct blocks)
@@ -966,9 +973,9 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
         if (!prof) continue;
         double c0 = (double)s * kFactB, wd = std::min<double>(kFactB, f.nc - c0);
         double nrem = f.nc + f.nr - c0 - wd;
-        pf += wd * wd * wd / 3 + wd * wd * wd / 3;            // POTRF + triangular inverse
-        pb += w * wd * wd * 2;
-        tf += 2.0 * nrem * wd * wd;                          // X = A Li^T
+        pf += wd * wd * wd / 3;
+        pb += w * wd * (wd + 1);
+        tf += nrem * wd * wd;                                // X = A L11^{-T}
         tb += w * (2.0 * nrem * wd + wd * wd);
       }
       // algorithmic work of an update launch over a band (update_k_range's rules)
@@ -995,12 +1002,12 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
              [&] {
                // many fronts: one launch per sub-block class (narrow blocks fit many CTAs per SM);
                // a few: one launch (measured: the extra launches on the panel chain cost more)
-               launch_potrf<T>(F, lists + p.off, p.count, (int)s, panel, diag, h->d_info.p, st, pdl, 0,
+               launch_potrf<T>(F, lists + p.off, p.count, (int)s, panel, h->d_packed, h->d_info.p, st, pdl, 0,
                                h->d_info.p + 3, p.count > kPotrfSplitMin ? L.potrf_cls[s].data() : nullptr);
              });
       record(h, st, MFD_K_TRSM, tf, tb, [&] {
-        launch_trsm<T>(F, lists + p.off, p.count, (int)s, p.param, panel, diag, kind == 1 ? 1 : 0, st, pdl,
-                       tcq ? h->d_q + (s & 1) * h->q_elems : nullptr);
+        launch_trsm<T>(F, lists + p.off, p.count, (int)s, p.param, std::min(kFactB, L.large.param2 - (int)s * kFactB),
+                       panel, h->d_packed, st, pdl, tcq ? h->d_q + (s & 1) * h->q_elems : nullptr);
       });
       n += 2;
       auto update = [&](cudaStream_t us, UpdBand band) {
@@ -1054,7 +1061,31 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
         pend = (int)s;
       }
     }
+    // the inverted diagonal blocks serve the solves only: next to the rest of the factorization
+    cudaStream_t si = side ? h->sinv : st;
+    if (side) {
+      cudaEventRecord(h->ev_inv, st);
+      cudaStreamWaitEvent(si, h->ev_inv, 0);
+      inverting = true;
+    }
+    double vf = 0, vb = 0;
+    if (prof)
+      for (int i = 0; i < L.large.count; ++i)
+        for (int c = 0, nc = h->fronts[hl[L.large.off + i]].nc; c < nc; c += kFactB) {
+          const double wd = std::min(kFactB, nc - c);
+          vf += wd * wd * wd / 3;
+          vb += w * wd * (wd + 1);
+        }
+    record(h, si, MFD_K_PANEL, vf, vb, [&] {
+      launch_invert<T>(F, lists + L.large.off, L.large.count, (int)L.steps.size(), std::min(kFactB, L.large.param2),
+                       panel, diag, si);
+    });
+    ++n;
     if (nside) side_join(h, st, nside);
+  }
+  if (inverting) {
+    cudaEventRecord(h->ev_inv, h->sinv);
+    cudaStreamWaitEvent(st, h->ev_inv, 0);
   }
   // values of the permuted full matrix for residuals
   record(h, st, MFD_K_OTHER, 0, 0, [&] {
@@ -1496,6 +1527,8 @@ int create_common(mfd_handle** out, std::vector<Symbolic>&& syms, const mfd_opti
   h->defer = h->opt.reserved[5] > 0 ? std::min(h->opt.reserved[5], mfd_handle::kMaxDefer)
                                      : (h->opt.precision == MFD_PREC_FP32_IR ? kDeferDefaultFp32 : kDeferDefaultFp64);
   CK(cudaEventCreateWithFlags(&h->ev_lvl, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&h->ev_inv, cudaEventDisableTiming));
+  CK(cudaStreamCreateWithPriority(&h->sinv, cudaStreamNonBlocking, prio_lo));
   for (int b = 0; b < mfd_handle::kSide; ++b) {
     CK(cudaStreamCreateWithPriority(&h->sst[b], cudaStreamNonBlocking, prio_lo));
     CK(cudaEventCreateWithFlags(&h->ev_side[b], cudaEventDisableTiming));

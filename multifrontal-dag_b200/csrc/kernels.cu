@@ -22,6 +22,7 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "chol_smem.cuh"
 #include "kernels.cuh"
 
 namespace mfd {
@@ -301,12 +302,6 @@ __global__ void k_bli_fill(DevFronts F, const int32_t* fronts, int count, int nb
 // factorization
 // ============================================================================
 
-__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
-
 constexpr int kSfW = 8;   // panel width of the small-front elimination
 
 // Fused small front: zero, assemble A, extend-add the children in order, partial
@@ -566,399 +561,11 @@ __global__ void __launch_bounds__(256) k_extend_add_ilp(DevFronts F, const int32
   }
 }
 
-// ---- blocked large-front factorization: per panel step s (columns c0 = s*128) ----
-//   k_potrf : one CTA per front: Cholesky of the w x w diagonal block in shared
-//             memory, written back as L11, then inverted in place (lower
-//             triangular) and stored as L11^{-1} in per-front scratch
-//   k_trsm  : the rows below, X <- A L11^{-T} = A (L11^{-1})^T, a GEMM with K = w
-//   k_update: trailing C(lower) -= P P^T with P the solved panel rows
-
-// Diagonal-block POTRF + inverse, one CTA (8 warps) per front, w <= 128.  The
-// block lives in shared memory in FP64 whatever the storage type.  FP64
-// factorization: every step in FP64.  FP32 factorization: the serial pivot
-// chain of each 32 x 32 diagonal sub-block (and its inverse) runs in FP32,
-// with a fallback to the FP64 chain when a pivot is small (warp_chol32_f32;
-// the `fallbacks` counter counts them); the sub-panel TRSM, the trailing SYRK
-// and the block inverse stay on FP64 DMMA.
-//
-// The block (zero-padded to wp = 32 * ceil(w / 32), identity on the padded
-// diagonal) sits in shared memory S, column-major, ld kPLd.  Right-looking
-// over 32-wide sub-blocks b:
-//   1. warp 0: Cholesky of the 32 x 32 diagonal sub-block, one row per lane,
-//      pivots by shuffle, 1/sqrt by rsqrt (no division), the next column
-//      updated ahead of the rest (one shuffle) so the next pivot's 1/sqrt
-//      overlaps the rank-1 update, whose column broadcast goes through a
-//      double-buffered shared vector; then the sub-block's inverse D_b by
-//      forward substitution, one column per lane;
-//   2. sub-panel below: L_ib = A_ib D_b^T, one 32-row tile per warp (DMMA);
-//   3. trailing update S_ij -= L_ib L_jb^T, 32 x 32 lower tiles over the warps
-//      (DMMA).
-// Then the full inverse X = L^{-1}: X_bb = D_b and, per block row r,
-// X_rc = -D_r (sum_{k=c}^{r-1} L_rk X_kc), two warps per block column c; the
-// off-diagonal X blocks are kept in the strict upper part of S (block (c, r) holds X_rc).
-// L goes to the panel, X (column-major, ld 128, zero outside the lower w x w;
-// persistent blocks are zeroed at allocation and written on that part only)
-// to linv.  A non-positive pivot records its 1-based column in info (atomic
-// min) and continues with pivot 1.
-constexpr int kPSub = 32;
-constexpr int kPLd = kFactB + 4;   // 132: ld = 4 mod 16 doubles keeps DMMA fragment loads conflict-free
-constexpr int kDLd = kPSub + 4;    // 36
-// The kernel is instantiated per number of 32-wide sub-blocks NSB (the block
-// width w <= 32 NSB): shared memory for 32 NSB columns of S (ld kPLd), NSB
-// inverse blocks and NSB - 1 scratch blocks; 32 x {1, 2, 4, 8} threads, the
-// most any phase uses (sub-panel TRSM: NSB - 1 warps, trailing tiles, inverse:
-// 2 (NSB - 1) warps), so narrow panels fit many fronts per SM.
-// scratch blocks Yv: NSB - 1 for the inverse, at least one (the FP32 pivot chain's
-// 32 x 33 float copy of the sub-block lives there)
-template <int NSB>
-__host__ __device__ constexpr int potrf_yblocks() {
-  return NSB > 1 ? NSB - 1 : 1;
-}
-template <int NSB>
-__host__ __device__ constexpr size_t potrf_smem() {
-  return sizeof(double) * ((size_t)kPSub * NSB * kPLd + (size_t)NSB * kPSub * kDLd +
-                           (size_t)potrf_yblocks<NSB>() * kPSub * kDLd + kFactB + 2 * kPSub);
-}
-template <int NSB>
-__host__ __device__ constexpr int potrf_threads() {
-  return NSB == 1 ? 32 : NSB == 2 ? 64 : NSB == 3 ? 128 : 256;
-}
-
-
-// One warp: acc(8 MF x 32) += A(8 MF x K) B(K x 32), K a multiple of 4, operands
-// in shared memory addressed as A(i, k) = A[i * ai + k * ak] and
-// B(k, j) = B[k * bk + j * bj].  acc[m][n][e] holds C(8m + g, 8n + 2q + e)
-// with g = lane / 4, q = lane % 4 (the m8n8k4 accumulator layout).
-template <int MF>
-__device__ __forceinline__ void warp_mm32(double (&acc)[MF][4][2], const double* A, int ai, int ak, const double* B,
-                                          int bk, int bj, int K, int lane) {
-  const int g = lane >> 2, q = lane & 3;
-  for (int k = 0; k < K; k += 4) {
-    double a[MF], b[4];
-#pragma unroll
-    for (int m = 0; m < MF; ++m) a[m] = A[(8 * m + g) * ai + (k + q) * ak];
-#pragma unroll
-    for (int n = 0; n < 4; ++n) b[n] = B[(k + q) * bk + (8 * n + g) * bj];
-#pragma unroll
-    for (int m = 0; m < MF; ++m)
-#pragma unroll
-      for (int n = 0; n < 4; ++n) dmma(acc[m][n][0], acc[m][n][1], a[m], b[n]);
-  }
-}
-
-template <int MF>
-__device__ __forceinline__ void acc_zero(double (&acc)[MF][4][2]) {
-#pragma unroll
-  for (int m = 0; m < MF; ++m)
-#pragma unroll
-    for (int n = 0; n < 4; ++n) acc[m][n][0] = acc[m][n][1] = 0.0;
-}
-
-// store s * acc at C(i, j) = C[i * ci + j * cj]
-template <int MF>
-__device__ __forceinline__ void acc_store(const double (&acc)[MF][4][2], double* C, int ci, int cj, double s,
-                                          int lane) {
-  const int g = lane >> 2, q = lane & 3;
-#pragma unroll
-  for (int m = 0; m < MF; ++m)
-#pragma unroll
-    for (int n = 0; n < 4; ++n)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) C[(8 * m + g) * ci + (8 * n + 2 * q + e) * cj] = s * acc[m][n][e];
-}
-
-// warp 0 of the CTA: Cholesky of S(o:o+32, o:o+32) in place, rsqrt of the
-// pivots into rq[o..o+31], inverse of the factor into D (column-major, ld kDLd,
-// zero above the diagonal).  Returns the 1-based sub-block pivot that failed, or 0.
-__device__ int warp_chol32(double* S, int o, double* D, double* rq, double* cbuf, int lane) {
-  double a[kPSub];
-#pragma unroll
-  for (int j = 0; j < kPSub; ++j) a[j] = S[(o + lane) + (o + j) * kPLd];
-  int bad = 0;
-  // pivot k's scale y and column l = L(lane, k) are formed one step ahead: at
-  // step k the next column is updated first (one shuffle), so pivot k+1's
-  // 1/sqrt overlaps the rest of step k's rank-1 update
-  double d = __shfl_sync(0xffffffffu, a[0], 0);
-  if (!(d > 0.0)) { bad = 1; d = 1.0; }
-  double y = rsqrt(d);
-  double l = a[0] * y;
-#pragma unroll
-  for (int k = 0; k < kPSub; ++k) {
-    double* cb = cbuf + (k & 1) * kPSub;
-    cb[lane] = l;
-    if (lane == 0) rq[o + k] = y;
-    a[k] = lane == k ? d * y : l;
-    double dn = 1.0, yn = 1.0, ln = 0.0;
-    if (k + 1 < kPSub) {
-      a[k + 1] = fma(-l, __shfl_sync(0xffffffffu, l, k + 1), a[k + 1]);
-      dn = __shfl_sync(0xffffffffu, a[k + 1], k + 1);
-      if (!(dn > 0.0)) {               // uniform: every lane holds the same pivot
-        if (!bad) bad = k + 2;
-        dn = 1.0;
-      }
-      yn = rsqrt(dn);
-      ln = a[k + 1] * yn;
-    }
-    __syncwarp();
-#pragma unroll
-    for (int j = k + 2; j < kPSub; ++j) a[j] = fma(-l, cb[j], a[j]);
-    d = dn;
-    y = yn;
-    l = ln;
-  }
-#pragma unroll
-  for (int j = 0; j < kPSub; ++j)
-    if (j <= lane) S[(o + lane) + (o + j) * kPLd] = a[j];
-  __syncwarp();
-  // inverse: lane j owns column j of X = L^{-1}; forward substitution on e_j
-  double x[kPSub];
-#pragma unroll
-  for (int i = 0; i < kPSub; ++i) x[i] = i == lane ? 1.0 : 0.0;
-#pragma unroll
-  for (int k = 0; k < kPSub; ++k) {
-    x[k] *= rq[o + k];
-#pragma unroll
-    for (int i = k + 1; i < kPSub; ++i) x[i] = fma(-S[(o + i) + (o + k) * kPLd], x[k], x[i]);
-  }
-#pragma unroll
-  for (int i = 0; i < kPSub; ++i) D[i + lane * kDLd] = x[i];
-  return bad;
-}
-
-// The FP64 chain as the FP32 path's fallback, out of line so that its
-// registers do not add to the FP32 chain's.
-__device__ __noinline__ int warp_chol32_fallback(double* S, int o, double* D, double* rq, double* cbuf, int lane) {
-  return warp_chol32(S, o, D, rq, cbuf, lane);
-}
-
-// FP32 form of warp_chol32 for the FP32 factorization: the pivot chain runs
-// in FP32 (rsqrtf, FP32 FMAs) on the block's values as stored; the factor
-// goes back to S widened to FP64 and, as FP32, to Fb (32 x 33 floats), from
-// which the inverse is formed in FP32 and written to D in FP64.  A pivot is
-// "small" when it is not positive or below kSmallPivot times the diagonal
-// entry it started from (more than 12 of FP32's 24 significand bits
-// cancelled): the function then returns -1 before writing S or D, and the
-// caller redoes the sub-block with the FP64 warp_chol32 (the fallback).  The
-// test is uniform across the warp (the pivot comes from a shuffle, the
-// diagonal entry from shared memory).
-constexpr float kSmallPivot = 1.0f / 4096.0f;
-constexpr int kFbLd = kPSub + 1;
-__device__ int warp_chol32_f32(double* S, int o, double* D, double* rq, float* cbuf, float* Fb, int lane) {
-  float a[kPSub], dg[kPSub];
-#pragma unroll
-  for (int j = 0; j < kPSub; ++j) a[j] = (float)S[(o + lane) + (o + j) * kPLd];
-#pragma unroll
-  for (int j = 0; j < kPSub; ++j) dg[j] = __shfl_sync(0xffffffffu, a[j], j) * kSmallPivot;   // small-pivot bounds
-  float d = __shfl_sync(0xffffffffu, a[0], 0);
-  if (!(d > dg[0])) return -1;
-  float y = rsqrtf(d);
-  float l = a[0] * y;
-#pragma unroll
-  for (int k = 0; k < kPSub; ++k) {
-    float* cb = cbuf + (k & 1) * kPSub;
-    cb[lane] = l;
-    if (lane == 0) rq[o + k] = (double)y;              // the FP64 fallback rewrites rq if it runs
-    a[k] = lane == k ? d * y : l;
-    float dn = 1.0f, yn = 1.0f, ln = 0.0f;
-    if (k + 1 < kPSub) {
-      a[k + 1] = fmaf(-l, __shfl_sync(0xffffffffu, l, k + 1), a[k + 1]);
-      dn = __shfl_sync(0xffffffffu, a[k + 1], k + 1);
-      if (!(dn > dg[k + 1])) return -1;                  // uniform: small pivot, FP64 fallback
-      yn = rsqrtf(dn);
-      ln = a[k + 1] * yn;
-    }
-    __syncwarp();
-#pragma unroll
-    for (int j = k + 2; j < kPSub; ++j) a[j] = fmaf(-l, cb[j], a[j]);
-    d = dn;
-    y = yn;
-    l = ln;
-  }
-#pragma unroll
-  for (int j = 0; j < kPSub; ++j) {
-    Fb[lane + j * kFbLd] = a[j];
-    if (j <= lane) S[(o + lane) + (o + j) * kPLd] = (double)a[j];
-  }
-  __syncwarp();
-  // inverse: lane j owns column j of X = L^{-1}; forward substitution on e_j (FP32)
-  float x[kPSub];
-#pragma unroll
-  for (int i = 0; i < kPSub; ++i) x[i] = i == lane ? 1.0f : 0.0f;
-#pragma unroll
-  for (int k = 0; k < kPSub; ++k) {
-    x[k] *= (float)rq[o + k];
-#pragma unroll
-    for (int i = k + 1; i < kPSub; ++i) x[i] = fmaf(-Fb[i + k * kFbLd], x[k], x[i]);
-  }
-#pragma unroll
-  for (int i = 0; i < kPSub; ++i) D[i + lane * kDLd] = (double)x[i];
-  return 0;
-}
-
-// Inverted diagonal block of panel step `step` of front f: persistent per front
-// when the plan provides d_off (kept for the solves), else one slot per list
-// entry of the launch.
+// Inverted diagonal block of panel step `step` of front f (k_invert writes them).
 template <typename T>
-__device__ __forceinline__ T* inv_block(const DevFronts& F, T* linv, int f, int step, int slot) {
-  return F.d_off ? linv + F.d_off[f] + (size_t)step * kFactB * kFactB : linv + (size_t)slot * kFactB * kFactB;
+__device__ __forceinline__ T* inv_block(const DevFronts& F, T* linv, int f, int step) {
+  return linv + F.d_off[f] + (size_t)step * kFactB * kFactB;
 }
-
-// info_stride 0: every front reports into info[0]; 1: list slot i reports into info[i].
-// fallbacks (may be null): counts the FP32 sub-blocks redone in FP64.
-template <typename T, int NSB>
-__global__ void __launch_bounds__(potrf_threads<NSB>(), 1) k_potrf(DevFronts F, const int32_t* list, int step,
-                                                                   T* panel, T* linv, int32_t* info, int info_stride,
-                                                                   int32_t* fallbacks) {
-  constexpr int B = kPSub * NSB;                             // the block's capacity (w <= B)
-  constexpr int NT = potrf_threads<NSB>();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* S = reinterpret_cast<double*>(smem_raw);
-  double* Dv = S + (size_t)B * kPLd;                         // NSB blocks of kPSub x kDLd
-  double* Yv = Dv + (size_t)NSB * kPSub * kDLd;               // potrf_yblocks<NSB>() blocks
-  double* rq = Yv + (size_t)potrf_yblocks<NSB>() * kPSub * kDLd;   // kFactB
-  double* cbuf = rq + kFactB;                                 // 2 x kPSub
-  const int f = list[blockIdx.x];
-  const int nc = F.nc[f], nf = nc + F.nr[f];
-  const int c0 = step * kFactB;
-  if (c0 >= nc) return;
-  const int w = min(kFactB, nc - c0);                       // <= B by the launch's choice of NSB
-  const int nsb = (w + kPSub - 1) / kPSub, wp = nsb * kPSub;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  T* P = panel + F.panel_off[f];
-  pdl_wait();
-  pdl_trigger();          // after the wait: every kernel before this one has completed
-  // ---- load the lower w x w block, identity on the padding ----
-  if constexpr (sizeof(T) == 8) {
-    // asynchronous 8-byte copies, all in flight at once; out-of-block entries zero-filled
-    for (int e = tid; e < B * B; e += NT) {
-      const int i = e % B, j = e / B;
-      if (i < wp && j < wp) {
-        if (i == j && i >= w) {
-          S[i + j * kPLd] = 1.0;              // identity on the padded diagonal
-        } else {
-          const bool v = i < w && j < w && i >= j;
-          cp_async8(&S[i + j * kPLd], v ? (const void*)&P[(c0 + i) + (size_t)(c0 + j) * nf] : (const void*)P, v);
-        }
-      }
-    }
-    cp_async_commit();
-    cp_async_wait<0>();
-  } else {
-    // FP32 storage: 4-byte copies into a float staging block (the D / Y / rq /
-    // cbuf area, larger than B x B floats, is free until the first sub-block),
-    // then widened into S
-    float* Fs = reinterpret_cast<float*>(Dv);
-    for (int e = tid; e < B * B; e += NT) {
-      const int i = e % B, j = e / B;
-      if (i < w && j < w && i >= j) cp_async_t(&Fs[e], (const float*)&P[(c0 + i) + (size_t)(c0 + j) * nf], true);
-    }
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncthreads();
-    for (int e = tid; e < B * B; e += NT) {
-      const int i = e % B, j = e / B;
-      if (i < wp && j < wp) S[i + j * kPLd] = (i < w && j < w) ? (i >= j ? (double)Fs[e] : 0.0) : (i == j ? 1.0 : 0.0);
-    }
-  }
-  __syncthreads();
-  // ---- right-looking over 32-wide sub-blocks ----
-  for (int b = 0; b < nsb; ++b) {
-    const int o = b * kPSub;
-    double* Db = Dv + (size_t)b * kPSub * kDLd;
-    if (warp == 0) {
-      int bad;
-      if constexpr (sizeof(T) == 4) {
-        // Yv (the inverse phase's scratch) is free here: the sub-block's FP32 copy
-        bad = warp_chol32_f32(S, o, Db, rq, reinterpret_cast<float*>(cbuf), reinterpret_cast<float*>(Yv), lane);
-        if (bad < 0) {                                   // small pivot: the FP64 chain
-          if (lane == 0 && fallbacks) atomicAdd(fallbacks, 1);
-          bad = warp_chol32_fallback(S, o, Db, rq, cbuf, lane);
-        }
-      } else {
-        bad = warp_chol32(S, o, Db, rq, cbuf, lane);
-      }
-      if (bad && lane == 0 && o + bad <= w) atomicMin(info + (size_t)info_stride * blockIdx.x, F.first[f] + c0 + o + bad);
-    }
-    __syncthreads();
-    const int rt = nsb - b - 1;                 // 32-row tiles below the sub-block
-    if (rt == 0) break;
-    if (warp < rt) {                            // L_ib = A_ib D_b^T, in place
-      const int r0 = o + kPSub + warp * kPSub;
-      double acc[4][4][2];
-      acc_zero(acc);
-      warp_mm32(acc, S + r0 + o * kPLd, 1, kPLd, Db, kDLd, 1, kPSub, lane);
-      __syncwarp();
-      acc_store(acc, S + r0 + o * kPLd, 1, kPLd, 1.0, lane);
-    }
-    __syncthreads();
-    for (int t = warp; t < rt * (rt + 1) / 2; t += NT / 32) {   // trailing lower tiles
-      int ti = 0;
-      while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-      const int tj = t - ti * (ti + 1) / 2;
-      const int r0 = o + kPSub + ti * kPSub, q0 = o + kPSub + tj * kPSub;
-      double acc[4][4][2];
-      acc_zero(acc);
-      warp_mm32(acc, S + r0 + o * kPLd, 1, kPLd, S + q0 + o * kPLd, kPLd, 1, kPSub, lane);
-      const int g = lane >> 2, q = lane & 3;
-#pragma unroll
-      for (int m = 0; m < 4; ++m)
-#pragma unroll
-        for (int n = 0; n < 4; ++n)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) S[(r0 + 8 * m + g) + (q0 + 8 * n + 2 * q + e) * kPLd] -= acc[m][n][e];
-    }
-    __syncthreads();
-  }
-  // ---- inverse: X_rc = -D_r sum_{k=c}^{r-1} L_rk X_kc, X_rc(i, j) stored at S(32c + i, 32r + j) (the
-  //      free block above the diagonal, not transposed, so the write-out below reads it conflict-free);
-  //      two warps per block column c, 16 rows each ----
-  for (int r = 1; r < nsb; ++r) {
-    const int c = warp >> 1, h = warp & 1;
-    double* Y = Yv + (size_t)c * kPSub * kDLd;
-    if (c < r) {
-      double acc[2][4][2];
-      acc_zero(acc);
-      // k = c: X_cc = D_c, B(k', j) = D_c(k', j)
-      warp_mm32(acc, S + r * kPSub + 16 * h + c * kPSub * kPLd, 1, kPLd, Dv + (size_t)c * kPSub * kDLd, 1, kDLd,
-                kPSub, lane);
-      for (int k = c + 1; k < r; ++k)   // B(k', j) = X_kc(k', j) = S(32c + k', 32k + j)
-        warp_mm32(acc, S + r * kPSub + 16 * h + k * kPSub * kPLd, 1, kPLd, S + c * kPSub + k * kPSub * kPLd, 1,
-                  kPLd, kPSub, lane);
-      acc_store(acc, Y + 16 * h, 1, kDLd, 1.0, lane);
-    }
-    __syncthreads();
-    if (c < r) {
-      double acc[2][4][2];
-      acc_zero(acc);
-      warp_mm32(acc, Dv + (size_t)r * kPSub * kDLd + 16 * h, 1, kDLd, Y, 1, kDLd, kPSub, lane);
-      acc_store(acc, S + c * kPSub + 16 * h + r * kPSub * kPLd, 1, kPLd, -1.0, lane);
-    }
-    __syncthreads();
-  }
-  // ---- write L11 to the panel and X to linv ----
-  for (int e = tid; e < B * B; e += NT) {
-    const int i = e % B, j = e / B;
-    if (i < w && j < w && i >= j) P[(c0 + i) + (size_t)(c0 + j) * nf] = (T)S[i + j * kPLd];
-  }
-  // persistent blocks (d_off) were zeroed once: only their lower w x w part is written
-  T* Li = inv_block(F, linv, f, step, blockIdx.x);
-  const bool full = F.d_off == nullptr;                      // scratch blocks: the whole 128 x 128 block written
-  const int EB = full ? kFactB : B;
-  for (int e = tid; e < EB * EB; e += NT) {
-    const int i = e % EB, j = e / EB;
-    const bool in = i < w && j < w && i >= j;
-    if (!in && !full) continue;
-    double v = 0.0;
-    if (in) {
-      const int bi = i / kPSub, bj = j / kPSub;
-      v = bi == bj ? Dv[(size_t)bi * kPSub * kDLd + (i - bi * kPSub) + (j - bj * kPSub) * kDLd]
-                   : S[(bj * kPSub + i - bi * kPSub) + (bi * kPSub + j - bj * kPSub) * kPLd];
-    }
-    Li[i + (size_t)j * kFactB] = (T)v;
-  }
-}
-
-
 
 template <typename T>
 __device__ __forceinline__ T* trailing_addr(T* P, T* U, int nc, int nr, int nf, int gi, int gj) {
@@ -986,121 +593,6 @@ __device__ __forceinline__ void dmma16(double (&d)[4], const double (&a)[8], con
       : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
       : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]), "d"(b[0]),
         "d"(b[1]), "d"(b[2]), "d"(b[3]));
-}
-
-// Panel TRSM X = A Li^T (Li = L11^{-1}, lower): one CTA per 32 rows of X and
-// all its w <= 128 columns (the TRSM is in place, so a CTA must read its rows
-// of A before any CTA writes them: rows are never split across CTAs), so a
-// panel step of nrem rows runs on nrem / 32 CTAs.  Operands arrive by
-// cp.async (all in flight at once).  FP64: 8 warps as 2 x 4 of 16 x 32
-// (m16n8k16 DMMA); FP32: 256 threads of 2 rows x 8 columns (FFMA).
-constexpr int kTr2Rows = 32;
-constexpr int kTr2LdA = kTr2Rows + 4, kTr2LdB = kFactB + 4;   // = 4 mod 16 doubles
-template <typename T>
-constexpr size_t trsm2_smem() {
-  return ((size_t)kFactB * kTr2LdA + (size_t)kFactB * kTr2LdB) * sizeof(T);
-}
-
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_trsm2(DevFronts F, const int32_t* list, int step, T* panel, const T* linv,
-                                               float* q) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* As = reinterpret_cast<T*>(smem_raw);            // [k][row]
-  T* Bs = As + kFactB * kTr2LdA;                      // [k][n]: Li(n, k)
-  const int f = list[blockIdx.y];
-  const int nc = F.nc[f], nf = nc + F.nr[f];
-  const int c0 = step * kFactB;
-  if (c0 >= nc) return;
-  const int w = min(kFactB, nc - c0);
-  const int r0 = c0 + w + blockIdx.x * kTr2Rows;
-  if (r0 >= nf) return;
-  T* P = panel + F.panel_off[f];
-  const T* Li = inv_block(F, linv, f, step, blockIdx.y);
-  const int kp = (w + 15) & ~15;
-  // the rows below the diagonal block do not depend on the POTRF that precedes this kernel
-  // (no event wait sits between the two launches)
-  for (int e = threadIdx.x; e < kTr2Rows * kp; e += blockDim.x) {
-    const int k = e / kTr2Rows, r = e - k * kTr2Rows;
-    const bool v = k < w && r0 + r < nf;
-    cp_async_t(&As[k * kTr2LdA + r], v ? P + (r0 + r) + (size_t)(c0 + k) * nf : P, v);
-  }
-  pdl_wait();
-  pdl_trigger();
-  // Li in 16-byte copies: the block is 16-byte aligned, rows of 128 elements, and zero
-  // outside its lower w x w part (so the rows k < kp copy whole)
-  constexpr int kVec = 16 / (int)sizeof(T);
-  for (int e = threadIdx.x; e < kFactB / kVec * kp; e += blockDim.x) {
-    const int k = e / (kFactB / kVec), n = (e - k * (kFactB / kVec)) * kVec;
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(&Bs[k * kTr2LdB + n]);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(Li + n + (size_t)k * kFactB));
-  }
-  cp_async_commit();
-  cp_async_wait<0>();
-  __syncthreads();
-  if constexpr (sizeof(T) == 8) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wm = warp >> 2, wn = warp & 3;            // 16-row band, 32-column band
-    const int g = lane >> 2, q = lane & 3;
-    double acc[4][4] = {};
-    for (int kk = 0; kk < kp; kk += 16) {
-      double av[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) av[i] = As[(kk + q + 4 * (i >> 1)) * kTr2LdA + wm * 16 + g + 8 * (i & 1)];
-#pragma unroll
-      for (int ni = 0; ni < 4; ++ni) {
-        double bv[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) bv[i] = Bs[(kk + q + 4 * i) * kTr2LdB + wn * 32 + ni * 8 + g];
-        dmma16(acc[ni], av, bv);
-      }
-    }
-#pragma unroll
-    for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int gi = r0 + wm * 16 + g + 8 * (e >> 1);
-        const int n = wn * 32 + ni * 8 + 2 * q + (e & 1);
-        if (gi < nf && n < w) P[gi + (size_t)(c0 + n) * nf] = acc[ni][e];
-      }
-  } else {
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // columns tx + 16 m, rows ty + 16 l
-    T acc[2][8] = {};
-    for (int k = 0; k < w; ++k) {
-      T av[2], bv[8];
-#pragma unroll
-      for (int l = 0; l < 2; ++l) av[l] = As[k * kTr2LdA + ty + 16 * l];
-#pragma unroll
-      for (int m = 0; m < 8; ++m) bv[m] = Bs[k * kTr2LdB + tx + 16 * m];
-#pragma unroll
-      for (int l = 0; l < 2; ++l)
-#pragma unroll
-        for (int m = 0; m < 8; ++m) acc[l][m] = fmaf(av[l], bv[m], acc[l][m]);
-    }
-#pragma unroll
-    for (int l = 0; l < 2; ++l)
-#pragma unroll
-      for (int m = 0; m < 8; ++m) {
-        const int gi = r0 + ty + 16 * l, n = tx + 16 * m;
-        if (gi < nf && n < w) P[gi + (size_t)(c0 + n) * nf] = acc[l][m];
-      }
-    if (q != nullptr) {     // the same rows as packed TF32 hi / lo operands of the tensor-core update
-      float* Q = q + F.q_off[f];
-      const int rrel = blockIdx.x * kTr2Rows;                 // first row of the CTA relative to c0 + w
-#pragma unroll
-      for (int l = 0; l < 2; ++l)
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-          const int rr = rrel + ty + 16 * l, n = tx + 16 * m;
-          const float v = (r0 + ty + 16 * l < nf && n < w) ? (float)acc[l][m] : 0.0f;
-          uint32_t hb;
-          asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hb) : "f"(v));
-          const float hi = __uint_as_float(hb);
-          Q[packed_offset(rr, n, 0)] = hi;
-          Q[packed_offset(rr, n, 1)] = v - hi;
-        }
-    }
-  }
 }
 
 __global__ void __launch_bounds__(kUThreads, 1) k_update_dmma(DevFronts F, const int32_t* list, int step, double* panel,
@@ -1198,29 +690,38 @@ __global__ void __launch_bounds__(kUThreads, 1) k_update_dmma(DevFronts F, const
       }
 }
 
-// FP64 trailing update in 128 x 64 halves: CTA x computes columns
-// 64 h .. 64 h + 63 (h = x & 1) of square tile x >> 1 of the band (the same
-// tiles, bands and K ranges as k_update_dmma).  256 threads: 8 warps as 4
-// (rows) x 2 (columns) of 32 x 32, each 2 x 4 mma.m16n8k16.f64 per K step of
-// 16, so 128 registers and 102 KB of shared memory per CTA and two CTAs per
-// SM: one CTA's C loads and stores overlap the other's MMAs.  Operands come
-// in K chunks of 32 by cp.async (16-byte row pairs where aligned),
-// double-buffered; a diagonal tile's B is rows 64 h .. of its A.  C is loaded into the accumulators (the A fragments enter
-// negated) and stored back; tiles wholly inside the trailing matrix, below
-// the diagonal and inside the panel or the update matrix take an unchecked
-// path.  In a diagonal tile's right half the warps whose 32 rows all lie
-// above the diagonal skip the MMAs.
-constexpr int kU2Threads = 256;
-constexpr int kU2N = 64;
-constexpr int kU2LdB = kU2N + 4;                             // 68 = 4 mod 16 doubles: conflict-free fragments
-constexpr int kU2Stage = kUK * kULD + kUK * kU2LdB;           // doubles per pipeline stage
-constexpr size_t kU2Smem = 2 * (size_t)kU2Stage * sizeof(double);
+// FP64 trailing update in WM x WN warps of 32 x 32 outputs: a CTA computes one
+// (32 WM) x (32 WN) piece of a square tile of the band (the same tiles, bands
+// and K ranges as k_update_dmma), 2 x 4 mma.m16n8k16.f64 per warp and K step
+// of 16.  Two shapes:
+//   <4, 2>, 128 x 64: 128 registers and 102 KB of shared memory, two CTAs per
+//     SM: one CTA's C loads and stores overlap the other's MMAs;
+//   <2, 1>, 64 x 32: 54 KB, four CTAs per SM, for launches whose 128 x 64
+//     pieces would leave SMs idle (launch_update).
+// Operands come in K chunks of 32 by cp.async (16-byte row pairs where
+// aligned), double-buffered; a 128-row diagonal tile's B is in its A.  C is
+// loaded into the accumulators (the A fragments enter negated) and stored
+// back; pieces wholly inside the trailing matrix, below the diagonal and
+// inside the panel or the update matrix take an unchecked path.  Warps whose
+// 32 rows all lie above the diagonal skip the MMAs.  Every element sees the
+// same K sequence in either shape: the results are bitwise the same.
+template <int WM, int WN>
+struct UpdShape {
+  static constexpr int kThreads = 32 * WM * WN, kM = 32 * WM, kN = 32 * WN;
+  static constexpr int kLdA = kM + 4, kLdB = kN + 4;          // = 4 mod 16 doubles: conflict-free fragments
+  static constexpr int kStage = kUK * (kLdA + kLdB);          // doubles per pipeline stage
+  static constexpr size_t kSmem = 2 * (size_t)kStage * sizeof(double);
+  static constexpr int kPerTile = (kUT / kM) * (kUT / kN);    // pieces of a 128 x 128 tile
+};
 
-__global__ void __launch_bounds__(kU2Threads, 2) k_update_dmma2(DevFronts F, const int32_t* list, int step,
+template <int WM, int WN>
+__global__ void __launch_bounds__(32 * WM * WN, WM * WN == 8 ? 2 : 4) k_update_dmma2(DevFronts F, const int32_t* list, int step,
                                                               double* panel, double* upool, int blo, int bhi,
                                                               int defer) {
+  using Sh = UpdShape<WM, WN>;
+  constexpr int kM = Sh::kM, kN = Sh::kN;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* sm = reinterpret_cast<double*>(smem_raw);     // per stage: A [k][kULD] (128 rows), B [k][kU2LdB] (64 rows)
+  double* sm = reinterpret_cast<double*>(smem_raw);     // per stage: A [k][kLdA] (kM rows), B [k][kLdB] (kN rows)
   const int f = list[blockIdx.y];
   const int nc = F.nc[f], nr = F.nr[f], nf = nc + nr;
   const int c0 = step * kFactB;
@@ -1230,24 +731,25 @@ __global__ void __launch_bounds__(kU2Threads, 2) k_update_dmma2(DevFronts F, con
   const int nrem = nf - base;
   if (nrem <= 0) return;
   const int T = (nrem + kUT - 1) / kUT;
-  const int hf = blockIdx.x & 1;
+  const int piece = blockIdx.x % Sh::kPerTile, hf = piece % (kUT / kN), rf = piece / (kUT / kN);
   int ti, tj, kbeg, kend;
-  if (!select_tile(T, kUT, blo, bhi, blockIdx.x >> 1, ti, tj)) return;
+  if (!select_tile(T, kUT, blo, bhi, blockIdx.x / Sh::kPerTile, ti, tj)) return;
   if (!update_k_range(nc, step, defer, tj, kUT, kbeg, kend)) return;
-  const int i0 = base + ti * kUT, j0 = base + tj * kUT + hf * kU2N;
-  if (j0 >= nf) return;                                 // the right half lies beyond the matrix
+  const int i0 = base + ti * kUT + rf * kM, j0 = base + tj * kUT + hf * kN;
+  if (i0 >= nf || j0 >= nf || i0 + kM <= j0) return;    // beyond the matrix, or above the diagonal
   const int K = kend - kbeg;                            // panel columns [kbeg, kend) of the front
-  const bool diag = ti == tj;
+  const bool diag = kM == kUT && ti == tj;
   double* P = panel + F.panel_off[f];
   double* U = upool + F.u_off[f];
   const int nchunks = (K + kUK - 1) / kUK;
-  // Copies: thread t moves row pairs -- A rows i0 + 2 (t & 63) (+1) at columns
-  // (t >> 6) + 4 v, v < 8; B rows j0 + 2 (t & 31) (+1) at columns (t >> 5) +
-  // 8 v, v < 4 (a diagonal tile's B is in A) -- 16 bytes per copy when the
-  // pair's source is 16-byte aligned.  A thread's copies are 4 or 8 columns
-  // apart, so the alignment is the same for all of them (and, the lanes of a
-  // warp sharing the column, the same across the warp); otherwise two 8-byte
-  // copies.  Rows past the matrix and columns past K are zero-filled.
+  // Copies: thread t moves row pairs -- A rows i0 + 2 (t % (kM / 2)) (+1) at
+  // columns t / (kM / 2) + kStepA v; B rows and columns likewise -- 16 bytes
+  // per copy when the pair's source is 16-byte aligned.  A thread's copies are
+  // an even number of columns apart, so the alignment is the same for all of
+  // them; otherwise two 8-byte copies.  Rows past the matrix and columns past
+  // K are zero-filled.
+  constexpr int kStepA = Sh::kThreads / (kM / 2), kStepB = Sh::kThreads / (kN / 2);
+  static_assert(kStepA % 2 == 0 && kStepB % 2 == 0, "alignment per thread");
   auto copy = [&](double* d, const double* src, int bytes, bool al) {
     const unsigned sa = (unsigned)__cvta_generic_to_shared(d);
     if (al) {
@@ -1260,42 +762,42 @@ __global__ void __launch_bounds__(kU2Threads, 2) k_update_dmma2(DevFronts F, con
   };
   auto load = [&](int stage, int kc) {
     // the per-thread quantities are recomputed here (kept live they would spill)
-    const int pa = threadIdx.x & 63, ka = threadIdx.x >> 6;
+    const int pa = threadIdx.x % (kM / 2), ka = threadIdx.x / (kM / 2);
     const int ra = i0 + 2 * pa;
     const int na = ra < nf ? (ra + 1 < nf ? 16 : 8) : 0;          // bytes of the A pair inside the matrix
     const bool ala = ((ra + (long long)(kbeg + ka) * nf) & 1) == 0; // panel offsets are multiples of 32 elements
-    double* dst = sm + stage * kU2Stage;
+    double* dst = sm + stage * Sh::kStage;
     const int k0 = kc * kUK;
     const double* sa = P + ra + (size_t)(kbeg + k0 + ka) * nf;
-    double* da = dst + ka * kULD + 2 * pa;
+    double* da = dst + ka * Sh::kLdA + 2 * pa;
 #pragma unroll 1
-    for (int v = 0; v < 8; ++v) {                   // rolled: unrolled, the copies' addresses would be kept live
-      const int k = k0 + ka + 4 * v;
-      copy(da + v * 4 * kULD, sa + (size_t)(4 * v) * nf, k < K ? na : 0, ala);
+    for (int v = 0; v < kUK / kStepA; ++v) {        // rolled: unrolled, the copies' addresses would be kept live
+      const int k = k0 + ka + kStepA * v;
+      copy(da + v * kStepA * Sh::kLdA, sa + (size_t)(kStepA * v) * nf, k < K ? na : 0, ala);
     }
     if (diag) return;
-    const int pb = threadIdx.x & 31, kb = threadIdx.x >> 5;
+    const int pb = threadIdx.x % (kN / 2), kb = threadIdx.x / (kN / 2);
     const int rb = j0 + 2 * pb;
     const int nbb = rb < nf ? (rb + 1 < nf ? 16 : 8) : 0;
     const bool alb = ((rb + (long long)(kbeg + kb) * nf) & 1) == 0;
     const double* sb = P + rb + (size_t)(kbeg + k0 + kb) * nf;
-    double* db = dst + kUK * kULD + kb * kU2LdB + 2 * pb;
+    double* db = dst + kUK * Sh::kLdA + kb * Sh::kLdB + 2 * pb;
 #pragma unroll 1
-    for (int v = 0; v < 4; ++v) {
-      const int k = k0 + kb + 8 * v;
-      copy(db + v * 8 * kU2LdB, sb + (size_t)(8 * v) * nf, k < K ? nbb : 0, alb);
+    for (int v = 0; v < kUK / kStepB; ++v) {
+      const int k = k0 + kb + kStepB * v;
+      copy(db + v * kStepB * Sh::kLdB, sb + (size_t)(kStepB * v) * nf, k < K ? nbb : 0, alb);
     }
   };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wm = warp >> 1, wn = warp & 1;
+  const int wm = warp / WN, wn = warp % WN;
   const int g = lane >> 2, q = lane & 3;
   const int rbase = i0 + wm * 32 + g, cbase = j0 + wn * 32 + 2 * q;
-  // warps of a diagonal tile's right half whose rows all lie above the diagonal
+  // warps of a diagonal tile whose rows all lie above the diagonal
   const bool idle = i0 + wm * 32 + 31 < j0 + wn * 32;
   // unchecked path: the tile is inside the trailing matrix, wholly below the
   // diagonal and wholly in the panel or wholly in the update matrix (formed
   // again for the epilogue rather than kept live through the K loop)
-  auto full_tile = [&]() { return i0 + kUT <= nf && j0 + kU2N <= nf && i0 >= j0 + kU2N && (j0 + kU2N <= nc || j0 >= nc); };
+  auto full_tile = [&]() { return i0 + kM <= nf && j0 + kN <= nf && i0 >= j0 + kN && (j0 + kN <= nc || j0 >= nc); };
   auto c_base = [&]() { return j0 < nc ? P + (size_t)j0 * nf : U + (size_t)(j0 - nc) * nr - nc; };   // C(gi, gj) = Cb[gi + (gj - j0) ldc]
   pdl_wait();
   pdl_trigger();
@@ -1329,9 +831,9 @@ __global__ void __launch_bounds__(kU2Threads, 2) k_update_dmma2(DevFronts F, con
     }
     __syncthreads();
     if (!idle) {
-      const double* As = sm + (kc & 1) * kU2Stage;
-      const double* Bs = diag ? As + hf * kU2N : As + kUK * kULD;
-      const int ldb = diag ? kULD : kU2LdB;
+      const double* As = sm + (kc & 1) * Sh::kStage;
+      const double* Bs = diag ? As + hf * kN : As + kUK * Sh::kLdA;
+      const int ldb = diag ? Sh::kLdA : Sh::kLdB;
 #pragma unroll
       for (int kk = 0; kk < kUK; kk += 16) {
         double bv[4][4];
@@ -1343,7 +845,7 @@ __global__ void __launch_bounds__(kU2Threads, 2) k_update_dmma2(DevFronts F, con
         for (int mi = 0; mi < 2; ++mi) {
           double av[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) av[i] = -As[(kk + q + 4 * (i >> 1)) * kULD + wm * 32 + mi * 16 + g + 8 * (i & 1)];
+          for (int i = 0; i < 8; ++i) av[i] = -As[(kk + q + 4 * (i >> 1)) * Sh::kLdA + wm * 32 + mi * 16 + g + 8 * (i & 1)];
 #pragma unroll
           for (int ni = 0; ni < 4; ++ni) dmma16(acc[mi][ni], av, bv[ni]);
         }
@@ -1825,7 +1327,7 @@ __device__ void fwd_diag_cta(const DevFronts& F, int f, int step, int slot, cons
   const int nc = F.nc[f];
   const int c0 = step * kSolveB;
   const int w = min(kSolveB, nc - c0);
-  const T* Li = inv_block(F, dinv, f, step, slot);
+  const T* Li = inv_block(F, dinv, f, step);
   const int first = F.first[f];
   const int tid = threadIdx.x, i = tid & (kSolveB - 1), h = tid >> 7;
   for (int r0 = 0; r0 < nrhs; r0 += kRhsG) {
@@ -2093,7 +1595,7 @@ __global__ void __launch_bounds__(256) k_fwd_large_fused(DevFronts F, const int4
   }
   if (h == 0) ys[ri] = valid ? v : T(0);
   __syncthreads();
-  const T* Li = inv_block(F, dinv, f, code, 0);    // zero outside its w x w part
+  const T* Li = inv_block(F, dinv, f, code);    // zero outside its w x w part
   T y = T(0);
 #pragma unroll 16
   for (int k = 0; k < 64; ++k) y += Li[ri + (size_t)(64 * h + k) * kSolveB] * ys[64 * h + k];
@@ -2217,7 +1719,7 @@ __global__ void __launch_bounds__(256) k_bwd_large_fused(DevFronts F, const int4
   }
   __syncthreads();
   // x = Li^T t: column i of Li against t, lanes over k (coalesced), 16 columns per warp
-  const T* Li = inv_block(F, dinv, f, s, 0);
+  const T* Li = inv_block(F, dinv, f, s);
   T tv[kSolveB / 32];
 #pragma unroll
   for (int q = 0; q < kSolveB / 32; ++q) tv[q] = ts[lane + 32 * q];
@@ -2356,7 +1858,7 @@ __global__ void __launch_bounds__(256, 3) k_bwd_large_step(DevFronts F, const in
     __threadfence();
   }
   // finish: x_s = Li^T (v_s - sum of partials)
-  const T* Li = inv_block(F, dinv, f, step, blockIdx.y);
+  const T* Li = inv_block(F, dinv, f, step);
   const int first = F.first[f];
   for (int r = 0; r < nrhs; ++r) {
     __syncthreads();
@@ -2448,7 +1950,7 @@ __global__ void __launch_bounds__(256) k_mrhs_diag(DevFronts F, const int32_t* l
   const int r0 = blockIdx.x * kMT;
   if (r0 >= nrhs) return;
   const int rt = min(kMT, nrhs - r0);
-  const T* Li = inv_block(F, dinv, f, step, blockIdx.y);
+  const T* Li = inv_block(F, dinv, f, step);
   T* Vf = V + F.v_off[f] * nrhs;
   auto load = [&](int buf, int k0) {
     for (int e = threadIdx.x; e < KC * kSolveB; e += blockDim.x) {
@@ -2858,6 +2360,7 @@ __global__ void k_fill_int(int32_t* p, int32_t v, int64_t n) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) p[i] = v;
 }
 
+constexpr int kNumSms = 148;
 inline int grid_1d(int64_t n, int threads = 256) { return clamp_grid(ceil_div(n, threads), 148 * 16); }
 
 template <typename T>
@@ -2885,16 +2388,12 @@ cudaError_t prepare_kernels() {
   auto chk = [&](cudaError_t r) { if (r != cudaSuccess && e == cudaSuccess) e = r; };
   chk(opt_in(k_small_front<double, false>)); chk(opt_in(k_small_front<float, false>));
   chk(opt_in(k_small_front<double, true>)); chk(opt_in(k_small_front<float, true>));
-  chk(opt_in(k_trsm2<double>)); chk(opt_in(k_trsm2<float>));
   chk(opt_in(k_update_dmma));
-  chk(opt_in(k_potrf<double, 4>)); chk(opt_in(k_potrf<float, 4>));
-  chk(opt_in(k_potrf<double, 3>)); chk(opt_in(k_potrf<float, 3>));
-  chk(opt_in(k_potrf<double, 2>)); chk(opt_in(k_potrf<float, 2>));
-  chk(opt_in(k_potrf<double, 1>)); chk(opt_in(k_potrf<float, 1>));
+  chk(prepare_panel());
   chk(prepare_update_tc());
   chk(prepare_update_tcq());
   chk(opt_in(k_update_simt<double>)); chk(opt_in(k_update_simt<float>));
-  chk(opt_in(k_update_dmma2));
+  chk(opt_in(k_update_dmma2<4, 2>)); chk(opt_in(k_update_dmma2<2, 1>));
   return e;
 }
 
@@ -2960,39 +2459,6 @@ void launch_extend_add(const DevFronts& F, const int32_t* list, int count, int m
   dim3 grid(clamp_grid(ceil_div(max_nr, 8), 1024), count);
   k_extend_add<T><<<grid, 256, 0, st>>>(F, list, panel, upool);
 }
-template <typename T>
-void launch_potrf(const DevFronts& F, const int32_t* list, int count, int step, T* panel, T* linv, int32_t* info,
-                  cudaStream_t st, bool pdl, int info_stride, int32_t* fallbacks, const int32_t* cls) {
-  if (count <= 0) return;
-  if (cls == nullptr) {                   // one launch, any block width
-    launch_k(k_potrf<T, 4>, dim3(count), dim3(potrf_threads<4>()), potrf_smem<4>(), st, pdl, F, list, step, panel,
-             linv, info, info_stride, fallbacks);
-    return;
-  }
-  // cls[k]: fronts of the list (in order, block widths non-increasing) whose block needs 4 - k sub-blocks;
-  // the list slots of a launch are offset, so this form is for persistent inverse blocks (F.d_off)
-  int off = 0;
-  auto go = [&](auto kern, int nt, size_t smem, int cnt) {
-    if (cnt > 0)
-      launch_k(kern, dim3(cnt), dim3(nt), smem, st, pdl, F, list + off, step, panel, linv, info, info_stride,
-               fallbacks);
-    off += cnt;
-  };
-  go(k_potrf<T, 4>, potrf_threads<4>(), potrf_smem<4>(), cls[0]);
-  go(k_potrf<T, 3>, potrf_threads<3>(), potrf_smem<3>(), cls[1]);
-  go(k_potrf<T, 2>, potrf_threads<2>(), potrf_smem<2>(), cls[2]);
-  go(k_potrf<T, 1>, potrf_threads<1>(), potrf_smem<1>(), cls[3]);
-}
-template <typename T>
-void launch_trsm(const DevFronts& F, const int32_t* list, int count, int step, int row_blocks, T* panel,
-                 const T* linv, int kind, cudaStream_t st, bool pdl, float* q) {
-  if (count <= 0 || row_blocks <= 0) return;
-  (void)kind;
-  // row_blocks counts 64-row blocks
-  dim3 grid(row_blocks * 2, count);
-  launch_k(k_trsm2<T>, grid, dim3(256), trsm2_smem<T>(), st, pdl, F, list, step, panel, linv,
-           sizeof(T) == 4 ? q : nullptr);
-}
 int update_grid(int T, int tw, UpdBand band) {
   const int c1 = kFactB / tw, jlo = band.blo * c1;
   if (T <= 0 || jlo >= T) return 0;
@@ -3005,11 +2471,18 @@ int launch_update(const DevFronts& F, const int32_t* list, int count, int step, 
                   T* upool, int kind, cudaStream_t st, UpdBand band, int defer, bool pdl) {
   if (count <= 0) return 0;
   if constexpr (sizeof(T) == 8) {
-    if (kind == 0) {                                   // 128 x 64 halves, two CTAs per SM
+    if (kind == 0) {
       const int g = update_grid(T128, kUT, band);
       if (g <= 0) return 0;
-      launch_k(k_update_dmma2, dim3(2 * g, count), dim3(kU2Threads), kU2Smem, st, pdl, F, list, step,
-               reinterpret_cast<double*>(panel), reinterpret_cast<double*>(upool), band.blo, band.bhi, defer);
+      auto go = [&](auto kern, auto sh) {
+        using Sh = decltype(sh);
+        launch_k(kern, dim3(Sh::kPerTile * g, count), dim3(Sh::kThreads), Sh::kSmem, st, pdl, F, list, step,
+                 reinterpret_cast<double*>(panel), reinterpret_cast<double*>(upool), band.blo, band.bhi, defer);
+      };
+      // at most one 128 x 64 piece per SM: four 64 x 32 pieces in its place still fit one wave
+      // (four per SM) and take a fourth of its MMAs each
+      if ((int64_t)2 * g * count <= kNumSms) go(k_update_dmma2<2, 1>, UpdShape<2, 1>{});
+      else go(k_update_dmma2<4, 2>, UpdShape<4, 2>{});
       return 1;
     }
     if (kind == 3) {                                   // whole 128 x 128 tiles, one CTA per SM
@@ -3225,10 +2698,6 @@ void launch_remap_int(const int32_t* map, int32_t* a, int64_t n, cudaStream_t st
   template void launch_assemble_large<T>(const DevFronts&, const int32_t*, int, int, const double*, T*,             \
                                          cudaStream_t);                                                            \
   template void launch_extend_add<T>(const DevFronts&, const int32_t*, int, int, T*, T*, cudaStream_t);             \
-  template void launch_potrf<T>(const DevFronts&, const int32_t*, int, int, T*, T*, int32_t*, cudaStream_t, bool,  \
-                                int, int32_t*, const int32_t*);                                                    \
-  template void launch_trsm<T>(const DevFronts&, const int32_t*, int, int, int, T*, const T*, int, cudaStream_t,   \
-                               bool, float*);                                                                           \
   template int launch_update<T>(const DevFronts&, const int32_t*, int, int, int, int, T*, T*, int, cudaStream_t,    \
                                  UpdBand, int, bool);                                                              \
   template void launch_fwd_small<T>(const DevFronts&, const int32_t*, int, int, const T*, T*, int64_t, T*, int,    \

@@ -130,26 +130,31 @@ void launch_assemble_large(const DevFronts& F, const int32_t* list, int count, i
 template <typename T>
 void launch_extend_add(const DevFronts& F, const int32_t* list, int count, int max_nr, T* panel, T* upool,
                        cudaStream_t st);
-// Panel step s of the blocked large-front factorization (columns s*kFactB ..):
-//   potrf  : one CTA per front; L11 into the panel, L11^{-1} into linv (at DevFronts::d_off, or
-//            one 128 x 128 slot per list entry when d_off is null)
-//   trsm   : rows below the diagonal block, X <- X L11^{-T}   (kind 0: DMMA, 1: FMA)
-//   update : trailing lower triangle -= P P^T                  (kind 0: DMMA 128-tiles, 1: FMA 64-tiles)
+// Panel step s of the blocked large-front factorization (columns s*kFactB ..), panel.cu:
+//   potrf  : one CTA per front; L11 into the panel and, in packed 8 x 8 blocks with the diagonal
+//            ones inverted, into list slot i's kPackedPanelElems doubles of `packed`
+//   trsm   : rows below the diagonal block, X <- X L11^{-T}, from the packed slots
+//   invert : L11^{-1} of the first `steps` panel steps of every front into linv (DevFronts::d_off)
+//   update : trailing lower triangle -= P P^T
 // info_stride 0: the first bad pivot of any front goes to info[0] (atomic min); 1: list slot i's to info[i].
-// FP32: the diagonal sub-blocks' pivot chains run in FP32 with an FP64 fallback on a small pivot;
-// fallbacks (may be null) counts the sub-blocks redone in FP64.
-template <typename T>
+// fallbacks (may be null; FP32 storage): counts the 32-column groups with a small pivot.
 // cls (may be null: one launch): four counts splitting the list, in order, into fronts whose
-// block needs 4, 3, 2, 1 sub-blocks of 32 columns, each class launched with its own (smaller)
-// shared memory and thread count; only for persistent inverse blocks (F.d_off).
-void launch_potrf(const DevFronts& F, const int32_t* list, int count, int step, T* panel, T* linv, int32_t* info,
+// block needs 4, 3, 2, 1 groups of 32 columns, each class launched with its own (smaller)
+// shared memory and thread count.
+constexpr int kPackedPanelElems = 136 * 64;   // 16 x 17 / 2 blocks
+cudaError_t prepare_panel();
+template <typename T>
+void launch_potrf(const DevFronts& F, const int32_t* list, int count, int step, T* panel, double* packed, int32_t* info,
                   cudaStream_t st, bool pdl = false, int info_stride = 0, int32_t* fallbacks = nullptr,
                   const int32_t* cls = nullptr);
-// q (FP32 only, may be null): also write the solved rows as packed TF32 operands of the
-// tensor-core update (packed_offset below), at q + F.q_off[f].
+// max_w: the widest diagonal block of the step.  q (FP32 only, may be null): also write the solved
+// rows as packed TF32 operands of the tensor-core update (packed_offset below), at q + F.q_off[f].
 template <typename T>
-void launch_trsm(const DevFronts& F, const int32_t* list, int count, int step, int row_blocks, T* panel,
-                 const T* linv, int kind, cudaStream_t st, bool pdl = false, float* q = nullptr);
+void launch_trsm(const DevFronts& F, const int32_t* list, int count, int step, int row_blocks, int max_w, T* panel,
+                 const double* packed, cudaStream_t st, bool pdl = false, float* q = nullptr);
+template <typename T>
+void launch_invert(const DevFronts& F, const int32_t* list, int count, int steps, int max_w, const T* panel, T* linv,
+                   cudaStream_t st);
 // Trailing update of step `step` over the tile-column band [blo, bhi) (128-column blocks relative to
 // the trailing matrix, bhi < 0: to the end; see select_tile) with updates deferred over groups of
 // `defer` steps (update_k_range).  T128 / T64: the largest front's trailing tiles per side.

@@ -6,7 +6,7 @@
 // loop that must not take the CUDA allocator's lock or trigger its implicit
 // synchronisation.  mfd_factor_fronts_noalloc serves them: the caller passes
 // the fronts in one device buffer it already owns, and the only scratch the
-// blocked factorization needs -- one inverted 128x128 diagonal block per front
+// blocked factorization needs -- one factored 128x128 diagonal block per front
 // and the small front tables -- lives in the file-scope array below, which
 // every GPU that loads the library holds until the process exits.
 #include <cuda_runtime.h>
@@ -24,7 +24,8 @@ namespace mfd {
 namespace {
 
 constexpr int kMaxFronts = MFD_NOALLOC_MAX_FRONTS;
-constexpr size_t kInvElems = (size_t)kMaxFronts * kFactB * kFactB;      // L11^{-1} blocks (FP64)
+constexpr size_t kInvElems = (size_t)kMaxFronts * kFactB * kFactB;      // packed diagonal blocks (FP64)
+static_assert(kPackedPanelElems <= kFactB * kFactB, "one slot per front");
 constexpr size_t kTableWords = 8 * kMaxFronts + 8;                        // front tables, in 8-byte words
 constexpr size_t kScratchElems = kInvElems + kTableWords;
 
@@ -146,7 +147,8 @@ extern "C" __attribute__((visibility("default"))) int mfd_factor_fronts_noalloc(
     }
     // fronts whose columns are exhausted return at once inside the kernels
     launch_potrf<double>(F, list, count, s, fronts, scratch, dinfo, st, false, 1);
-    launch_trsm<double>(F, list, count, s, rows, fronts, scratch, 0, st);
+    launch_trsm<double>(F, list, count, s, rows, maxnc - s * kFactB < kFactB ? maxnc - s * kFactB : kFactB, fronts,
+                        scratch, st);
     launch_update<double>(F, list, count, s, tiles, 0, fronts, fronts, 0, st);
   }
   e = cudaGetLastError();
