@@ -190,7 +190,8 @@ struct mfd_handle {
   DBuf<int32_t> d_nc, d_nr, d_first, d_parent, d_child_ptr, d_child, d_lrow_off, d_lrow, d_local, d_a_beg, d_a_src,
       d_a_pos, d_sidx, d_lists, d_perm, d_info, d_cnt;
   // fused solve: the tasks, and [0] expiry flag, [1 + 2 l] / [2 + 2 l] level l's forward /
-  // backward tickets, then forward and backward step flags (zeroed before every solve)
+  // backward tickets, then forward flags, backward flags and backward update-row counters,
+  // one per front, panel step and RHS tile (zeroed before every solve)
   DBuf<int32_t> d_stasks, d_ssync;
   DBuf<int64_t> d_panel_off, d_u_off, d_v_off, d_s_off, d_d_off, d_q_off;
   DevFronts F{};
@@ -364,14 +365,14 @@ int build_plan(mfd_handle* h) {
     if (nf > sfm) h->dinv_elems += (int64_t)((fr.nc + kFactB - 1) / kFactB) * kFactB * kFactB;   // kept for the solves
   }
   // large-front solve partials: one region per level (levels solve one after
-  // another), kMrhsRows-row chunks (the single-RHS backward uses the same 64)
+  // another), kSolveRows-row chunks
   {
     std::vector<int64_t> used(nlev, 0);
     for (int32_t g = 0; g < nfr; ++g) {
       HostFront& fr = h->fronts[g];
       const int nf = fr.nc + fr.nr;
       fr.s_off = used[fr.level];
-      if (nf > sfm) used[fr.level] += (int64_t)((nf + kMrhsRows - 1) / kMrhsRows) * kSolveB;
+      if (nf > sfm) used[fr.level] += (int64_t)((nf + kSolveRows - 1) / kSolveRows) * kSolveB;
     }
     for (int64_t u : used) h->s_elems = std::max(h->s_elems, u);
   }
@@ -595,9 +596,6 @@ int upload_plan(mfd_handle* h) {
     h->solve_flags = 0;
   }
   if (!h->h_stasks.empty()) CK(h->d_stasks.upload(h->h_stasks, st));
-  // [0] expiry, 2 tickets per level, forward flags, backward flags, backward update-row counters
-  CK(h->d_ssync.alloc(1 + 2 * h->levels.size() + 3 * (size_t)h->solve_flags));
-  CK(cudaMemsetAsync(h->d_ssync.p, 0, sizeof(int32_t) * h->d_ssync.n, st));
   CK(h->d_a_src.alloc(h->nnz_total));
   CK(h->d_a_pos.alloc(h->nnz_total));
   CK(h->d_sidx.alloc(h->nnz_total));
@@ -769,7 +767,6 @@ int upload_plan(mfd_handle* h) {
   CK(cudaMalloc(&h->d_upool, std::max<int64_t>(h->upool_elems, 1) * esz));
   CK(cudaMalloc(&h->d_diag, (size_t)std::max<int64_t>(h->dinv_elems, 1) * esz));
   CK(cudaMalloc(&h->d_packed, (size_t)std::max(1, h->max_large_count) * kPackedPanelElems * sizeof(double)));
-  CK(cudaMalloc(&h->d_bwpart, (size_t)std::max<int64_t>(h->bw_part_elems, 1) * esz));
   if (h->fp32 && h->q_elems > 0) {
     CK(cudaMalloc(&h->d_q, (size_t)(2 * h->q_elems) * sizeof(float)));
     // rows past a front's last row are never written and only reach discarded outputs; zero keeps them finite
@@ -784,6 +781,16 @@ int upload_plan(mfd_handle* h) {
   return MFD_OK;
 }
 
+int64_t solve_sync_ints(const mfd_handle* h, int nrhs) {
+  return 1 + 2 * (int64_t)h->levels.size() + 3 * (int64_t)h->solve_flags * multi_tiles(nrhs);
+}
+// One launch per level and sweep for the large fronts' steps; the per-step sweeps where the
+// flags or the tasks of a level would leave 32-bit range.
+bool solve_fused(const mfd_handle* h, int nrhs) {
+  return h->opt.reserved[6] != 1 && !h->h_stasks.empty() && solve_sync_ints(h, nrhs) <= INT32_MAX &&
+         (int64_t)h->h_stasks.size() / 4 * multi_tiles(nrhs) <= INT32_MAX;
+}
+
 int ensure_rhs(mfd_handle* h, int nrhs) {
   if (nrhs <= h->nrhs_cap) return MFD_OK;
   for (auto& kv : h->g_solve) cudaGraphExecDestroy(kv.second);
@@ -791,8 +798,14 @@ int ensure_rhs(mfd_handle* h, int nrhs) {
   for (auto& kv : h->g_ir) cudaGraphExecDestroy(kv.second);
   h->g_ir.clear();
   size_t esz = h->fp32 ? sizeof(float) : sizeof(double);
-  for (void** p : {&h->d_X, &h->d_V, &h->d_S})
+  for (void** p : {&h->d_X, &h->d_V, &h->d_S, &h->d_bwpart})
     if (*p) { cudaFree(*p); *p = nullptr; }
+  int widest = nrhs;                        // the most right-hand sides up to nrhs that take the fused sweeps
+  while (widest > 1 && !solve_fused(h, widest)) --widest;
+  CK(h->d_ssync.alloc(solve_sync_ints(h, solve_fused(h, widest) ? widest : 1)));
+  CK(cudaMemsetAsync(h->d_ssync.p, 0, sizeof(int32_t) * h->d_ssync.n, h->st));
+  CK(cudaMalloc(&h->d_bwpart, (size_t)std::max<int64_t>(h->bw_part_elems, 1) * esz *
+                                  multi_part(widest)));
   CK(cudaMalloc(&h->d_X, (size_t)std::max<int64_t>(h->n_total, 1) * nrhs * esz));
   CK(cudaMalloc(&h->d_V, (size_t)std::max<int64_t>(h->v_elems, 1) * nrhs * esz));
   CK(cudaMalloc(&h->d_S, (size_t)std::max<int64_t>(h->s_elems, 1) * nrhs * esz));
@@ -1113,16 +1126,30 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
   // programmatic dependent launch between the large-front solve steps (on
   // unless reserved[3] = 1; the profiling schedule times kernels one by one)
   const bool solve_pdl = h->opt.reserved[3] != 1 && !prof;
-  // one launch per level and sweep for the large fronts' steps (single right-hand side)
-  const bool fused = nrhs == 1 && h->opt.reserved[6] != 1 && !h->h_stasks.empty();
+  const bool fused = solve_fused(h, nrhs);
   const int4* stasks = reinterpret_cast<const int4*>(h->d_stasks.p);
   int32_t* ssync = h->d_ssync.p;
   int32_t* fwd_flags = ssync + 1 + 2 * h->levels.size();
-  int32_t* bwd_flags = fwd_flags + h->solve_flags;
+  const int64_t nflags = h->solve_flags * multi_tiles(nrhs);
+  int32_t* bwd_flags = fwd_flags + nflags;
   if (fused) {                              // a kernel, not a memset node: this also runs in the refinement loop's body
-    launch_fill_int(ssync, 0, (int64_t)h->d_ssync.n, st);
+    launch_fill_int(ssync, 0, solve_sync_ints(h, nrhs), st);
     ++n;
   }
+  // a level's fused sweep
+  auto sweep = [&](const LevelPlan& L, bool backward) {
+    const LaunchList& tl = backward ? L.bwd_tasks : L.fwd_tasks;
+    int32_t* ticket = ssync + 1 + 2 * (&L - h->levels.data()) + (backward ? 1 : 0);
+    int32_t* flags = backward ? bwd_flags : fwd_flags;
+    T* part = static_cast<T*>(h->d_bwpart);
+    if (nrhs == 1)
+      launch_large_fused<T>(F, stasks + tl.off, tl.count, backward, ticket, flags, ssync, panel, dinv, X, V, st,
+                            h->d_info.p + 2, part, bwd_flags + nflags);
+    else
+      launch_large_multi<T>(F, stasks + tl.off, tl.count, backward, ticket, flags, ssync, panel, dinv, X, ldx, V, nrhs, st,
+                            h->d_info.p + 2, part, bwd_flags + nflags);
+    ++n;
+  };
   // algorithmic work of one sweep over a list: read the panel once, 2 flops per entry per RHS
   auto work = [&](const LaunchList& l, double& fl, double& by) {
     if (!prof) return;
@@ -1158,12 +1185,7 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
       record(h, st, MFD_K_SOLVE_LARGE, fl, by, [&] {
         launch_fwd_large<T>(F, lists + L.large.off, L.large.count, L.large.param2, L.large_max_nf, panel, dinv, X,
                             ldx, V, h->d_cnt.p, nrhs, st, &n, solve_pdl, fused);
-        if (fused) {
-          const size_t lv = &L - h->levels.data();
-          launch_large_fused<T>(F, stasks + L.fwd_tasks.off, L.fwd_tasks.count, false, ssync + 1 + 2 * lv, fwd_flags,
-                                ssync, panel, dinv, X, V, st, h->d_info.p + 2);
-          ++n;
-        }
+        if (fused) sweep(L, false);
       });
     }
     if (nside) side_join(h, st, nside);
@@ -1187,13 +1209,7 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
       record(h, st, MFD_K_SOLVE_LARGE, fl, by, [&] {
         launch_bwd_large<T>(F, lists + L.large.off, L.large.count, L.large.param2, L.large_max_nf, panel, dinv, X,
                             ldx, V, S, h->d_cnt.p, nrhs, st, &n, solve_pdl, fused);
-        if (fused) {
-          const size_t lv = &L - h->levels.data();
-          launch_large_fused<T>(F, stasks + L.bwd_tasks.off, L.bwd_tasks.count, true, ssync + 2 + 2 * lv, bwd_flags,
-                                ssync, panel, dinv, X, V, st, h->d_info.p + 2, static_cast<T*>(h->d_bwpart),
-                                bwd_flags + h->solve_flags);
-          ++n;
-        }
+        if (fused) sweep(L, true);
       });
     }
     if (nside) side_join(h, st, nside);
@@ -1485,8 +1501,8 @@ int do_solve(mfd_handle* h, double* b, int nrhs, int64_t ldb, mfd_report* rep) {
     CK(cudaMemcpy2DAsync(b, sizeof(double) * ldb, h->d_b.p, sizeof(double) * n, sizeof(double) * n, nrhs,
                          dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
   }
-  int32_t expired = 0;                      // a bounded wait of the single-RHS large-front sweeps gave up
-  if (nrhs == 1 && !h->h_stasks.empty()) CK(cudaMemcpyAsync(&expired, h->d_ssync.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+  int32_t expired = 0;                      // a bounded wait of the fused large-front sweeps gave up
+  if (solve_fused(h, nrhs)) CK(cudaMemcpyAsync(&expired, h->d_ssync.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   if (expired) return fail(MFD_E_TIMEOUT, "a device wait of the solve timed out");
   float ms = 0;

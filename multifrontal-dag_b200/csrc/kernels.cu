@@ -24,6 +24,7 @@
 
 #include "chol_smem.cuh"
 #include "kernels.cuh"
+#include "sweep_sync.cuh"
 
 namespace mfd {
 
@@ -957,6 +958,77 @@ constexpr int kWFLd = kWF + 1;
 constexpr int kWFWarps = 4;
 
 
+// Gathers of a level with many fronts and several right-hand sides: eight
+// right-hand sides per CTA, a warp each (no CTA-wide barrier between children),
+// eight rows per lane in flight.  With one CTA per front and right-hand side
+// these levels paid each CTA's chain of loads for a few hundred rows: 218 us
+// against this form's figure in launch_fwd_large for 928 fronts x 64.
+constexpr int kGatherRhs = 8;
+template <typename T>
+__global__ void __launch_bounds__(32 * kGatherRhs) k_fwd_gather_warp(DevFronts F, const int32_t* list, const T* X,
+                                                                     int64_t ldx, T* V, int nrhs) {
+  constexpr int U = 8;
+  const int f = list[blockIdx.x], lane = threadIdx.x & 31, r = blockIdx.y * kGatherRhs + (threadIdx.x >> 5);
+  if (r >= nrhs) return;
+  const int nc = F.nc[f], nf = nc + F.nr[f], first = F.first[f];
+  T* Vf = V + F.v_off[f] * nrhs + (int64_t)r * nf;
+  const T* Xr = X + first + r * ldx;
+  for (int i0 = lane; i0 < nf; i0 += 32 * U) {
+    T v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = i0 + 32 * u < nc ? Xr[i0 + 32 * u] : T(0);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i0 + 32 * u < nf) Vf[i0 + 32 * u] = v[u];
+  }
+  for (int t = F.child_ptr[f]; t < F.child_ptr[f + 1]; ++t) {
+    __syncwarp();
+    const int c = F.child[t];
+    const int ncc = F.nc[c], nrc = F.nr[c];
+    const T* Vc = V + F.v_off[c] * nrhs + (int64_t)r * (ncc + nrc) + ncc;
+    const int32_t* loc = F.local + F.lrow_off[c];
+    for (int i0 = lane; i0 < nrc; i0 += 32 * U) {
+      int li[U];
+      T cv[U], ov[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + 32 * u;
+        li[u] = i < nrc ? loc[i] - 1 : -1;
+        cv[u] = i < nrc ? Vc[i] : T(0);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) ov[u] = li[u] >= 0 ? Vf[li[u]] : T(0);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (li[u] >= 0) Vf[li[u]] = ov[u] + cv[u];
+    }
+  }
+}
+template <typename T>
+__global__ void __launch_bounds__(32 * kGatherRhs) k_bwd_gather_warp(DevFronts F, const int32_t* list, const T* X,
+                                                                     int64_t ldx, T* V, int nrhs) {
+  constexpr int U = 8;
+  const int f = list[blockIdx.x], lane = threadIdx.x & 31, r = blockIdx.y * kGatherRhs + (threadIdx.x >> 5);
+  if (r >= nrhs) return;
+  const int nc = F.nc[f], nf = nc + F.nr[f], first = F.first[f];
+  const int32_t* lr = F.lrow + F.lrow_off[f];
+  T* Vf = V + F.v_off[f] * nrhs + (int64_t)r * nf;
+  for (int i0 = lane; i0 < nf; i0 += 32 * U) {
+    int gi[U];
+    T v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + 32 * u;
+      gi[u] = i < nc ? first + i : (i < nf ? lr[i - nc] : -1);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = gi[u] >= 0 ? X[gi[u] + r * ldx] : T(0);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (gi[u] >= 0) Vf[i0 + 32 * u] = v[u];
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kWFWarps * 32) k_small_warp(DevFronts F, const int32_t* list, int count,
                                                               const double* __restrict__ a, T* __restrict__ panel,
@@ -1419,7 +1491,7 @@ __global__ void __launch_bounds__(256) k_fwd_large_gather(DevFronts F, const int
       __syncthreads();
     }
   }
-  if (nrhs >= kMrhsMin || gridDim.y > 1 || !diag0) return;   // the GEMM-shaped diagonal kernel (or the fused sweep) follows
+  if (!diag0) return;                                     // the fused sweep follows
   __threadfence_block();
   fwd_diag_cta(F, f, 0, blockIdx.x, dinv, X, ldx, Vbase, nf, nrhs, vs, hs);
 }
@@ -1506,42 +1578,6 @@ __global__ void __launch_bounds__(256) k_fwd_large_rest(DevFronts F, const int32
 // (the solve reports MFD_E_TIMEOUT).  Each task's sums have a fixed order, so
 // the sweep is deterministic.
 constexpr int kFuseRows = 128;                // rows of a forward rest task
-constexpr long long kSolveWaitLimit = 1ll << 31;
-
-__device__ __forceinline__ int ld_acquire_i32(const int32_t* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release_i32(int32_t* p, int v) {
-  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-constexpr long long kSolveProbeLimit = 1ll << 21;   // the test request's wait (~1 ms)
-// thread 0 waits for *flag >= need (bounded; gives up at once when another
-// CTA's wait expired); the result is the CTA's.  probe (a test request): the
-// wait is for a value no producer writes, with a ~1 ms limit, so it expires.
-__device__ __forceinline__ bool cta_wait_flag(const int32_t* flag, int32_t* expired, int* sh_ok, bool probe,
-                                              int need = 1) {
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    if (probe) need = INT_MAX;
-    const long long limit = probe ? kSolveProbeLimit : kSolveWaitLimit;
-    if (ld_acquire_i32(flag) < need) {
-      const long long t0 = clock64();
-      while (ld_acquire_i32(flag) < need) {
-        if (clock64() - t0 > limit || ld_acquire_i32(expired) != 0) {
-          ok = 0;
-          atomicExch(expired, 1);
-          break;
-        }
-        __nanosleep(32);
-      }
-    }
-    *sh_ok = ok;
-  }
-  __syncthreads();
-  return *sh_ok != 0;
-}
 
 // forward: thread (row r0 + (t mod 128), half t / 128) sums its half of each
 // step's 128 columns; the step's 64 panel entries are loaded before the wait on
@@ -1899,341 +1935,6 @@ __global__ void __launch_bounds__(256, 3) k_bwd_large_step(DevFronts F, const in
   if (nchunks > 0 && threadIdx.x == 0) cnt[blockIdx.y] = 0;
 }
 
-// ---- many right-hand sides (nrhs >= kMrhsMin): GEMM-shaped large-front steps --
-// V of a front is an nf x nrhs column-major block (ld nf).  GEMMs over 64-wide
-// RHS tiles, on m8n8k4 DMMA in FP64 (one 32 x 32 or 16 x 32 block per warp)
-// and register-tiled FFMA in FP32; operands stream through shared memory in
-// K chunks with cp.async double buffering (the next chunk's copies are in
-// flight while the current one is multiplied):
-//   forward step s : Y = Li V_s (k_mrhs_diag), V_rest -= L_rest,s Y (k_mrhs_fwd_rest)
-//   backward step s: partial(chunk) = L_chunk,s^T X_chunk (k_mrhs_bwd_part, 64-row chunks),
-//                    V_s -= sum of partials in chunk order (k_mrhs_bwd_reduce),
-//                    X_s = Li^T V_s (k_mrhs_diag, transposed)
-constexpr int kMT = 64;          // RHS tile
-constexpr int kMKc = 16;         // K chunk
-
-// FP64: one warp accumulates an (8 MF) x 32 block of C += A B over a K chunk
-// of KC (a multiple of 4) on m8n8k4 DMMA, operands in shared memory as
-// A(i, k) = As[k * lda + i], B(k, j) = Bs[k * ldb + j]; acc[m][n][e] holds
-// C(wr + 8m + g, wc + 8n + 2q + e), g = lane / 4, q = lane % 4
-template <int MF, int KC>
-__device__ __forceinline__ void warp_mma_chunk(double (&acc)[MF][4][2], const double* As, int lda, const double* Bs,
-                                               int ldb, int wr, int wc, int lane) {
-  const int g = lane >> 2, q = lane & 3;
-#pragma unroll
-  for (int k0 = 0; k0 < KC; k0 += 4) {
-    double a[MF], b[4];
-#pragma unroll
-    for (int m = 0; m < MF; ++m) a[m] = As[(k0 + q) * lda + wr + 8 * m + g];
-#pragma unroll
-    for (int n = 0; n < 4; ++n) b[n] = Bs[(k0 + q) * ldb + wc + 8 * n + g];
-#pragma unroll
-    for (int m = 0; m < MF; ++m)
-#pragma unroll
-      for (int n = 0; n < 4; ++n) dmma(acc[m][n][0], acc[m][n][1], a[m], b[n]);
-  }
-}
-
-// Y (128 x 64 RHS tile) = op(Li) V_s, op = identity or transpose; writes V_s and X
-template <typename T>
-__global__ void __launch_bounds__(256) k_mrhs_diag(DevFronts F, const int32_t* list, int step,
-                                                   const T* __restrict__ dinv, T* X, int64_t ldx, T* V, int nrhs,
-                                                   int transposed) {
-  constexpr int KC = sizeof(T) == 8 ? 8 : 16;   // K chunk: two 128-wide stages under 48 KB
-  __shared__ __align__(16) T As[2][KC][kSolveB + 4];   // op(Li)(i, k), [k][i]
-  __shared__ __align__(16) T Bs[2][KC][kMT + 4];       // V_s(k, r)
-  const int f = list[blockIdx.y];
-  const int nc = F.nc[f], nf = nc + F.nr[f];
-  const int c0 = step * kSolveB;
-  if (c0 >= nc) return;
-  const int w = min(kSolveB, nc - c0);
-  const int r0 = blockIdx.x * kMT;
-  if (r0 >= nrhs) return;
-  const int rt = min(kMT, nrhs - r0);
-  const T* Li = inv_block(F, dinv, f, step);
-  T* Vf = V + F.v_off[f] * nrhs;
-  auto load = [&](int buf, int k0) {
-    for (int e = threadIdx.x; e < KC * kSolveB; e += blockDim.x) {
-      int i, k;
-      if (transposed) { k = e % KC; i = e / KC; }   // Li(k0 + k, i): k contiguous in global
-      else { i = e % kSolveB; k = e / kSolveB; }         // Li(i, k0 + k): i contiguous
-      const bool v = k0 + k < w && i < w;
-      const T* src = transposed ? Li + (k0 + k) + (size_t)i * kSolveB : Li + i + (size_t)(k0 + k) * kSolveB;
-      cp_async_t(&As[buf][k][i], v ? src : Li, v);
-    }
-    for (int e = threadIdx.x; e < KC * kMT; e += blockDim.x) {
-      const int k = e % KC, r = e / KC;
-      const bool v = k0 + k < w && r < rt;
-      cp_async_t(&Bs[buf][k][r], v ? Vf + (int64_t)(r0 + r) * nf + c0 + k0 + k : Vf, v);
-    }
-    cp_async_commit();
-  };
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // rows ty + 16 m (8), RHS tx + 16 n (4)
-  T acc[8][4] = {};
-  // FP64: DMMA, warp (warp % 4, warp / 4) owns rows 32 (warp % 4) .. +32, RHS 32 (warp / 4) .. +32
-  double dacc[4][4][2] = {};
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wr = 32 * (warp & 3), wc = 32 * (warp >> 2);
-  const int nch = (w + KC - 1) / KC;
-  load(0, 0);
-  for (int c = 0; c < nch; ++c) {
-    if (c + 1 < nch) {
-      load((c + 1) & 1, (c + 1) * KC);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    const int b = c & 1;
-    if constexpr (std::is_same<T, double>::value) {
-      warp_mma_chunk<4, KC>(dacc, &As[b][0][0], kSolveB + 4, &Bs[b][0][0], kMT + 4, wr, wc, lane);
-    } else {
-#pragma unroll
-      for (int k = 0; k < KC; ++k) {
-        T a[8], bv[4];
-#pragma unroll
-        for (int m = 0; m < 8; ++m) a[m] = As[b][k][ty + 16 * m];
-#pragma unroll
-        for (int n = 0; n < 4; ++n) bv[n] = Bs[b][k][tx + 16 * n];
-#pragma unroll
-        for (int m = 0; m < 8; ++m)
-#pragma unroll
-          for (int n = 0; n < 4; ++n) acc[m][n] += a[m] * bv[n];
-      }
-    }
-    __syncthreads();
-  }
-  const int first = F.first[f];
-  if constexpr (std::is_same<T, double>::value) {
-    const int g = lane >> 2, q = lane & 3;
-#pragma unroll
-    for (int m = 0; m < 4; ++m)
-#pragma unroll
-      for (int n = 0; n < 4; ++n)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i = wr + 8 * m + g, r = wc + 8 * n + 2 * q + e;
-          if (i < w && r < rt) {
-            Vf[(int64_t)(r0 + r) * nf + c0 + i] = dacc[m][n][e];
-            X[first + c0 + i + (int64_t)(r0 + r) * ldx] = dacc[m][n][e];
-          }
-        }
-  } else {
-#pragma unroll
-    for (int m = 0; m < 8; ++m)
-#pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        const int i = ty + 16 * m, r = tx + 16 * n;
-        if (i < w && r < rt) {
-          Vf[(int64_t)(r0 + r) * nf + c0 + i] = acc[m][n];
-          X[first + c0 + i + (int64_t)(r0 + r) * ldx] = acc[m][n];
-        }
-      }
-  }
-}
-
-// V_rest(64-row tile, 64 RHS) -= L(rows, step columns) Y_s
-template <typename T>
-__global__ void __launch_bounds__(256) k_mrhs_fwd_rest(DevFronts F, const int32_t* list, int step,
-                                                       const T* __restrict__ panel, T* V, int nrhs) {
-  __shared__ __align__(16) T As[2][kMKc][kMT + 4];   // L(row, k), [k][row]
-  __shared__ __align__(16) T Bs[2][kMKc][kMT + 4];   // Y(k, r)
-  const int f = list[blockIdx.z];
-  const int nc = F.nc[f], nf = nc + F.nr[f];
-  const int c0 = step * kSolveB;
-  if (c0 >= nc) return;
-  const int w = min(kSolveB, nc - c0);
-  const int i0 = c0 + w + blockIdx.x * kMT;
-  if (i0 >= nf) return;
-  const int r0 = blockIdx.y * kMT;
-  if (r0 >= nrhs) return;
-  const int rt = min(kMT, nrhs - r0);
-  const T* P = panel + F.panel_off[f];
-  T* Vf = V + F.v_off[f] * nrhs;
-  auto load = [&](int buf, int k0) {
-    for (int e = threadIdx.x; e < kMKc * kMT; e += blockDim.x) {
-      const int i = e % kMT, k = e / kMT;
-      const bool v = i0 + i < nf && k0 + k < w;
-      cp_async_t(&As[buf][k][i], v ? P + (i0 + i) + (size_t)(c0 + k0 + k) * nf : P, v);
-    }
-    for (int e = threadIdx.x; e < kMKc * kMT; e += blockDim.x) {
-      const int k = e % kMKc, r = e / kMKc;
-      const bool v = k0 + k < w && r < rt;
-      cp_async_t(&Bs[buf][k][r], v ? Vf + (int64_t)(r0 + r) * nf + c0 + k0 + k : Vf, v);
-    }
-    cp_async_commit();
-  };
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // rows ty + 16 m (4), RHS tx + 16 n (4)
-  T acc[4][4] = {};
-  // FP64: DMMA, warp (warp % 4, warp / 4) owns rows 16 (warp % 4) .. +16, RHS 32 (warp / 4) .. +32
-  double dacc[2][4][2] = {};
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wr = 16 * (warp & 3), wc = 32 * (warp >> 2);
-  const int nch = (w + kMKc - 1) / kMKc;
-  load(0, 0);
-  for (int c = 0; c < nch; ++c) {
-    if (c + 1 < nch) {
-      load((c + 1) & 1, (c + 1) * kMKc);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    const int b = c & 1;
-    if constexpr (std::is_same<T, double>::value) {
-      warp_mma_chunk<2, kMKc>(dacc, &As[b][0][0], kMT + 4, &Bs[b][0][0], kMT + 4, wr, wc, lane);
-    } else {
-#pragma unroll
-      for (int k = 0; k < kMKc; ++k) {
-        T a[4], bv[4];
-#pragma unroll
-        for (int m = 0; m < 4; ++m) a[m] = As[b][k][ty + 16 * m];
-#pragma unroll
-        for (int n = 0; n < 4; ++n) bv[n] = Bs[b][k][tx + 16 * n];
-#pragma unroll
-        for (int m = 0; m < 4; ++m)
-#pragma unroll
-          for (int n = 0; n < 4; ++n) acc[m][n] += a[m] * bv[n];
-      }
-    }
-    __syncthreads();
-  }
-  if constexpr (std::is_same<T, double>::value) {
-    const int g = lane >> 2, q = lane & 3;
-#pragma unroll
-    for (int m = 0; m < 2; ++m)
-#pragma unroll
-      for (int n = 0; n < 4; ++n)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i = i0 + wr + 8 * m + g, r = wc + 8 * n + 2 * q + e;
-          if (i < nf && r < rt) Vf[(int64_t)(r0 + r) * nf + i] -= dacc[m][n][e];
-        }
-  } else {
-#pragma unroll
-    for (int m = 0; m < 4; ++m)
-#pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        const int i = i0 + ty + 16 * m, r = tx + 16 * n;
-        if (i < nf && r < rt) Vf[(int64_t)(r0 + r) * nf + i] -= acc[m][n];
-      }
-  }
-}
-
-// partial(chunk)(128 columns, 64 RHS) = L(chunk rows, step columns)^T X(chunk rows), 64-row chunks
-template <typename T>
-__global__ void __launch_bounds__(256) k_mrhs_bwd_part(DevFronts F, const int32_t* list, int step,
-                                                       const T* __restrict__ panel, const T* V, T* scratch,
-                                                       int nrhs) {
-  constexpr int KC = sizeof(T) == 8 ? 8 : 16;   // K chunk: two 128-wide stages under 48 KB
-  __shared__ __align__(16) T As[2][KC][kSolveB + 4];   // L(row, col), [row][col]
-  __shared__ __align__(16) T Bs[2][KC][kMT + 4];       // X(row, r)
-  const int f = list[blockIdx.z];
-  const int nc = F.nc[f], nf = nc + F.nr[f];
-  const int c0 = step * kSolveB;
-  if (c0 >= nc) return;
-  const int w = min(kSolveB, nc - c0);
-  const int rs0 = c0 + w;
-  const int rbase = rs0 + blockIdx.x * kMrhsRows;
-  if (rbase >= nf) return;
-  const int nchunks = (nf - rs0 + kMrhsRows - 1) / kMrhsRows;
-  const int r0 = blockIdx.y * kMT;
-  if (r0 >= nrhs) return;
-  const int rt = min(kMT, nrhs - r0);
-  const int rend = min(nf, rbase + kMrhsRows);
-  const T* P = panel + F.panel_off[f];
-  const T* Vf = V + F.v_off[f] * nrhs;
-  auto load = [&](int buf, int k0) {
-    for (int e = threadIdx.x; e < KC * kSolveB; e += blockDim.x) {
-      const int k = e % KC, col = e / KC;     // rows contiguous in global
-      const bool v = k0 + k < rend && col < w;
-      cp_async_t(&As[buf][k][col], v ? P + (k0 + k) + (size_t)(c0 + col) * nf : P, v);
-    }
-    for (int e = threadIdx.x; e < KC * kMT; e += blockDim.x) {
-      const int k = e % KC, r = e / KC;
-      const bool v = k0 + k < rend && r < rt;
-      cp_async_t(&Bs[buf][k][r], v ? Vf + (int64_t)(r0 + r) * nf + k0 + k : Vf, v);
-    }
-    cp_async_commit();
-  };
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // columns ty + 16 m (8), RHS tx + 16 n (4)
-  T acc[8][4] = {};
-  // FP64: DMMA, warp (warp % 4, warp / 4) owns rows 32 (warp % 4) .. +32, RHS 32 (warp / 4) .. +32
-  double dacc[4][4][2] = {};
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wr = 32 * (warp & 3), wc = 32 * (warp >> 2);
-  const int nch = (rend - rbase + KC - 1) / KC;
-  load(0, rbase);
-  for (int c = 0; c < nch; ++c) {
-    if (c + 1 < nch) {
-      load((c + 1) & 1, rbase + (c + 1) * KC);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    const int b = c & 1;
-    if constexpr (std::is_same<T, double>::value) {
-      warp_mma_chunk<4, KC>(dacc, &As[b][0][0], kSolveB + 4, &Bs[b][0][0], kMT + 4, wr, wc, lane);
-    } else {
-#pragma unroll
-      for (int k = 0; k < KC; ++k) {
-        T a[8], bv[4];
-#pragma unroll
-        for (int m = 0; m < 8; ++m) a[m] = As[b][k][ty + 16 * m];
-#pragma unroll
-        for (int n = 0; n < 4; ++n) bv[n] = Bs[b][k][tx + 16 * n];
-#pragma unroll
-        for (int m = 0; m < 8; ++m)
-#pragma unroll
-          for (int n = 0; n < 4; ++n) acc[m][n] += a[m] * bv[n];
-      }
-    }
-    __syncthreads();
-  }
-  if constexpr (std::is_same<T, double>::value) {
-    const int g = lane >> 2, q = lane & 3;
-#pragma unroll
-    for (int m = 0; m < 4; ++m)
-#pragma unroll
-      for (int n = 0; n < 4; ++n)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int col = wr + 8 * m + g, r = wc + 8 * n + 2 * q + e;
-          if (col < w && r < rt)
-            scratch[F.s_off[f] * nrhs + ((int64_t)(r0 + r) * nchunks + blockIdx.x) * kSolveB + col] = dacc[m][n][e];
-        }
-  } else {
-#pragma unroll
-    for (int m = 0; m < 8; ++m)
-#pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        const int col = ty + 16 * m, r = tx + 16 * n;
-        if (col < w && r < rt)
-          scratch[F.s_off[f] * nrhs + ((int64_t)(r0 + r) * nchunks + blockIdx.x) * kSolveB + col] = acc[m][n];
-      }
-  }
-}
-
-// V_s(k, r) -= sum over chunks of partial (chunk order), one thread per entry
-template <typename T>
-__global__ void __launch_bounds__(256) k_mrhs_bwd_reduce(DevFronts F, const int32_t* list, int step, T* V,
-                                                         const T* scratch, int nrhs) {
-  const int f = list[blockIdx.y];
-  const int nc = F.nc[f], nf = nc + F.nr[f];
-  const int c0 = step * kSolveB;
-  if (c0 >= nc) return;
-  const int w = min(kSolveB, nc - c0);
-  const int rs0 = c0 + w;
-  const int nchunks = nf > rs0 ? (nf - rs0 + kMrhsRows - 1) / kMrhsRows : 0;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = e % kSolveB, r = e / kSolveB;
-  if (nchunks == 0 || r >= nrhs || k >= w) return;
-  T s = V[F.v_off[f] * nrhs + (int64_t)r * nf + c0 + k];
-  for (int q = 0; q < nchunks; ++q) s -= scratch[F.s_off[f] * nrhs + ((int64_t)r * nchunks + q) * kSolveB + k];
-  V[F.v_off[f] * nrhs + (int64_t)r * nf + c0 + k] = s;
-}
-
 // ============================================================================
 // vectors
 // ============================================================================
@@ -2526,27 +2227,23 @@ void launch_bwd_small(const DevFronts& F, const int32_t* list, int count, int nf
     default: k_bwd_small<T, 4><<<grid, block, 0, st>>>(F, list, count, panel, X, ldx, nrhs); break;
   }
 }
+// a warp per right-hand side once the level's CTAs of eight still fill the chip (below, the
+// long fronts of a small level want a CTA each)
+bool gather_by_warp(int count, int nrhs) { return nrhs > 1 && (int64_t)count * ceil_div(nrhs, kGatherRhs) >= 2 * kNumSms; }
 template <typename T>
 void launch_fwd_large(const DevFronts& F, const int32_t* list, int count, int max_nc, int max_nf, const T* panel,
                       const T* dinv, T* X, int64_t ldx, T* V, int32_t* cnt, int nrhs, cudaStream_t st,
                       int64_t* launches, bool pdl, bool fused) {
   if (count <= 0) return;
-  k_fwd_large_gather<T><<<dim3(count, nrhs >= kMrhsMin ? nrhs : 1), 256, 0, st>>>(F, list, dinv, X, ldx, V, nrhs,
-                                                                                    fused ? 0 : 1);
-  if (fused) {                    // the level's steps as one launch (single right-hand side)
+  // fused: one right-hand side per CTA row, the steps follow as one launch
+  if (fused && gather_by_warp(count, nrhs))
+    k_fwd_gather_warp<T><<<dim3(count, ceil_div(nrhs, kGatherRhs)), 32 * kGatherRhs, 0, st>>>(F, list, X, ldx, V, nrhs);
+  else k_fwd_large_gather<T><<<dim3(count, fused ? nrhs : 1), 256, 0, st>>>(F, list, dinv, X, ldx, V, nrhs, fused ? 0 : 1);
+  if (fused) {
     if (launches) *launches += 1;
     return;
   }
   const int steps = ceil_div(max_nc, kSolveB);
-  if (nrhs >= kMrhsMin) {
-    const int rtiles = ceil_div(nrhs, kMT), rows = std::max(1, ceil_div(max_nf, kMT));
-    for (int s = 0; s < steps; ++s) {
-      k_mrhs_diag<T><<<dim3(rtiles, count), 256, 0, st>>>(F, list, s, dinv, X, ldx, V, nrhs, 0);
-      k_mrhs_fwd_rest<T><<<dim3(rows, rtiles, count), 256, 0, st>>>(F, list, s, panel, V, nrhs);
-    }
-    if (launches) *launches += 1 + 2 * steps;
-    return;
-  }
   const int chunks = std::max(1, ceil_div(max_nf, kFwdRows));
   for (int s = 0; s < steps; ++s)
     launch_k(k_fwd_large_rest<T>, dim3(chunks, count), dim3(256), 0, st, pdl, F, list, s, panel, dinv, X, ldx, V, cnt,
@@ -2558,25 +2255,15 @@ void launch_bwd_large(const DevFronts& F, const int32_t* list, int count, int ma
                       const T* dinv, T* X, int64_t ldx, T* V, T* scratch, int32_t* cnt, int nrhs, cudaStream_t st,
                       int64_t* launches, bool pdl, bool fused) {
   if (count <= 0) return;
-  k_bwd_large_gather<T><<<dim3(count, nrhs >= kMrhsMin ? nrhs : 1), 256, 0, st>>>(F, list, X, ldx, V, nrhs);
+  if (fused && gather_by_warp(count, nrhs))
+    k_bwd_gather_warp<T><<<dim3(count, ceil_div(nrhs, kGatherRhs)), 32 * kGatherRhs, 0, st>>>(F, list, X, ldx, V, nrhs);
+  else k_bwd_large_gather<T><<<dim3(count, fused ? nrhs : 1), 256, 0, st>>>(F, list, X, ldx, V, nrhs);
   if (fused) {
     if (launches) *launches += 1;
     return;
   }
   const int steps = ceil_div(max_nc, kSolveB);
   const int chunks = std::max(1, ceil_div(max_nf, kSolveRows));
-  if (nrhs >= kMrhsMin) {
-    const int rtiles = ceil_div(nrhs, kMT);
-    for (int s = steps - 1; s >= 0; --s) {
-      k_mrhs_bwd_part<T><<<dim3(std::max(1, ceil_div(max_nf, kMrhsRows)), rtiles, count), 256, 0, st>>>(
-          F, list, s, panel, V, scratch, nrhs);
-      k_mrhs_bwd_reduce<T><<<dim3(ceil_div((int64_t)kSolveB * nrhs, 256), count), 256, 0, st>>>(F, list, s, V, scratch,
-                                                                                                nrhs);
-      k_mrhs_diag<T><<<dim3(rtiles, count), 256, 0, st>>>(F, list, s, dinv, X, ldx, V, nrhs, 1);
-    }
-    if (launches) *launches += 1 + 3 * steps;
-    return;
-  }
   for (int s = steps - 1; s >= 0; --s)
     launch_k(k_bwd_large_step<T>, dim3(chunks, count), dim3(256), 0, st, pdl, F, list, s, panel, dinv, X, ldx, V,
              scratch, cnt, nrhs);

@@ -18,8 +18,10 @@ constexpr int kUpdTile = 128;        // trailing-update output tile (tensor path
 constexpr int kUpdTileSimt = 64;     // trailing-update output tile (FMA path)
 constexpr int kSolveB = kFactB;      // column step of the large-front solves (one inverted diagonal block)
 constexpr int kSolveRows = 64;       // rows per CTA of the backward large-front partial sums
-constexpr int kMrhsRows = 64;        // rows per CTA of the many-RHS backward partial sums
-static_assert(kSolveRows >= kMrhsRows, "solve scratch is sized for kMrhsRows-row chunks");
+// tiles of the several-RHS fused large-front sweeps: eight right-hand sides each (a level may take
+// them sixteen at a time, launch_large_multi)
+constexpr int multi_tiles(int nrhs) { return (nrhs + 7) / 8; }
+constexpr int multi_part(int nrhs) { return nrhs == 1 ? 1 : 16 * ((nrhs + 15) / 16); }
 
 // Trailing-update work of panel step s of a front (columns c0 = s * kFactB
 // .. c0 + w, base = c0 + w): the lower triangle of the trailing matrix (rows
@@ -230,7 +232,14 @@ template <typename T>
 void launch_large_fused(const DevFronts& F, const int4* tasks, int ntask, bool backward, int32_t* ticket,
                         int32_t* flags, int32_t* expired, const T* panel, const T* dinv, T* X, T* V, cudaStream_t st,
                         const int32_t* test_req, T* part = nullptr, int32_t* counters = nullptr);
-// pdl: the single-RHS step kernels go out with programmatic dependent launch
+// The same sweep for several right-hand sides (solve_multi.cu), each task split into
+// multi_tiles(nrhs) tiles: flags and counters hold as many entries per front and panel
+// step, part multi_part(nrhs) times the single-RHS size.
+template <typename T>
+void launch_large_multi(const DevFronts& F, const int4* tasks, int ntask, bool backward, int32_t* ticket, int32_t* flags,
+                        int32_t* expired, const T* panel, const T* dinv, T* X, int64_t ldx, T* V, int nrhs,
+                        cudaStream_t st, const int32_t* test_req, T* part = nullptr, int32_t* counters = nullptr);
+// pdl: the step kernels go out with programmatic dependent launch
 // (each waits for its predecessor before reading the sweep's vectors)
 
 // ---- vectors, residuals ---------------------------------------------------------

@@ -1,0 +1,100 @@
+"""Blocked large-front kernels at the sizes where their tiling can go wrong.
+
+* Panel step (POTRF on 8 x 8 blocks, block-substitution TRSM): dense fronts
+  whose column counts sit at the edges of 8, 32 and 128, with and without rows
+  below, against numpy.  A backward-stable factorization of a matrix with
+  condition number below 10 differs from another by a modest multiple of
+  n eps: 1e-12 relative is 8 n eps at the largest n here.
+* Several-right-hand-side sweeps (tiles of eight): counts at the tile's edges
+  against the per-step sweeps on the same factor.
+"""
+import numpy as np
+import pytest
+
+from mfdag import hppllt as H
+from mfdag import problems as P
+
+pytestmark = pytest.mark.gpu
+
+
+def _spd(n, seed):
+    """Symmetric, eigenvalues within [n / 2, 3 n / 2] or so."""
+    a = np.random.default_rng(seed).uniform(-1.0, 1.0, (n, n))
+    return (a + a.T) * (np.sqrt(n) / 8.0) + n * np.eye(n)
+
+
+@pytest.mark.parametrize("nf,nc", [(1, 1), (7, 7), (8, 8), (9, 9), (31, 31), (33, 33), (65, 64), (97, 96), (127, 127),
+                                   (128, 128), (129, 129), (130, 1), (136, 128), (137, 9), (200, 63), (257, 128),
+                                   (300, 129), (333, 250), (400, 136)])
+def test_dense_partial_factor(nf, nc):
+    import torch
+    a = _spd(nf, nf * 1000 + nc)
+    nr = nf - nc
+    panel = np.asfortranarray(np.tril(a)[:, :nc])
+    upd = np.asfortranarray(np.tril(a[nc:, nc:]))
+    off = (nf * nc + 31) // 32 * 32
+    buf = np.zeros(off + max(1, nr * nr))
+    buf[:nf * nc] = panel.ravel(order="F")
+    buf[off:off + nr * nr] = upd.ravel(order="F")
+    d = torch.from_numpy(buf).cuda()
+    assert H.factor_fronts_noalloc(d, [0], [off], [nf], [nc]) == 0
+    got = d.cpu().numpy()
+    L = np.linalg.cholesky(a[:nc, :nc])
+    X = np.linalg.solve(L, a[nc:, :nc].T).T
+    want = np.vstack([L, X])
+    P_ = np.tril(got[:nf * nc].reshape((nf, nc), order="F"))
+    assert np.abs(P_ - np.tril(want)).max() <= 1e-12 * np.abs(want).max()
+    if nr:
+        U = np.tril(got[off:off + nr * nr].reshape((nr, nr), order="F"))
+        S = np.tril(a[nc:, nc:] - X @ X.T)
+        assert np.abs(U - S).max() <= 1e-12 * np.abs(S).max()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("nrhs", [2, 7, 8, 9, 33])
+def test_several_rhs_sweeps_match_per_step(nrhs, precision):
+    """3D Laplacian 20^3 with fronts above 48 rows on the blocked path (panel
+    steps of full and partial width, update-row chunks of full and partial
+    height).  FP64: both sweeps are backward stable and the condition number is
+    below 300, so they agree within 1e-12; FP32 + refinement: backward error
+    1e-12 each.  A second solve gives the same bits."""
+    p = P.laplace3d(20)
+    B = np.asfortranarray(np.random.default_rng(nrhs).uniform(-1, 1, (p.n, nrhs)))
+    xs = []
+    for per_step in (0, 1):
+        s = H.Solver.analyze(p.n, p.col, p.row, p.order, max_zero=1000, small_front_max=48, precision=precision,
+                             reserved=(0, 0, 0, 0, 0, 0, per_step))
+        assert s.factorize(p.val) == 0
+        X = B.copy(order="F")
+        rep, rc = s.solve(X)
+        assert rc == 0
+        for r in range(nrhs):
+            assert P.backward_error(p.n, p.col, p.row, p.val, X[:, r], B[:, r]) <= (1e-14 if precision == 0 else 1e-12)
+        if per_step == 0:
+            Y = B.copy(order="F")
+            s.solve(Y)
+            assert np.array_equal(X, Y)
+            x1 = B[:, 0].copy()                          # fewer right-hand sides on the same handle afterwards
+            s.solve(x1)
+            assert P.backward_error(p.n, p.col, p.row, p.val, x1, B[:, 0]) <= 1e-12
+        xs.append(X)
+        s.close()
+    assert np.abs(xs[0] - xs[1]).max() <= (1e-12 if precision == 0 else 1e-9) * np.abs(xs[1]).max()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_several_rhs_expired_wait(precision):
+    """A sweep's flag wait that runs out ends the solve with MFD_E_TIMEOUT; the handle solves afterwards."""
+    p = P.laplace3d(16)
+    s = H.Solver.analyze(p.n, p.col, p.row, p.order, max_zero=1000, small_front_max=48, precision=precision)
+    assert s.factorize(p.val) == 0
+    B = np.asfortranarray(np.random.default_rng(0).uniform(-1, 1, (p.n, 10)))
+    s.test_expire_waits(True)
+    with pytest.raises(H.MfdError) as e:
+        s.solve(B.copy(order="F"))
+    assert e.value.code == -4
+    s.test_expire_waits(False)
+    X = B.copy(order="F")
+    rep, rc = s.solve(X)
+    assert rc == 0
+    assert P.backward_error(p.n, p.col, p.row, p.val, X[:, 9], B[:, 9]) <= 1e-12
