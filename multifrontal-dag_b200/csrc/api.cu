@@ -157,7 +157,7 @@ struct mfd_handle {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // a level's independent launches (small-front size bins) on side streams,
   // forked from st at the level's start and joined back at its end
-  static constexpr int kSide = 4;
+  static constexpr int kSide = 6;
   cudaStream_t sst[kSide] = {};
   cudaEvent_t ev_lvl = nullptr, ev_side[kSide] = {};
   cudaStream_t sinv = nullptr;                      // inverted diagonal blocks, off the panel chain
@@ -193,6 +193,8 @@ struct mfd_handle {
   // backward tickets, then forward flags, backward flags and backward update-row counters,
   // one per front, panel step and RHS tile (zeroed before every solve)
   DBuf<int32_t> d_stasks, d_ssync;
+  DBuf<FrontRec> d_rec;
+  DBuf<ChildRec> d_crec;
   DBuf<int64_t> d_panel_off, d_u_off, d_v_off, d_s_off, d_d_off, d_q_off;
   DevFronts F{};
 
@@ -395,7 +397,7 @@ int build_plan(mfd_handle* h) {
     h->upool_elems = std::max<int64_t>(ff.top, kAlign);
   }
   // level launch lists
-  h->small_bins = std::vector<int>{32, 64, 96, 128};
+  h->small_bins = std::vector<int>{16, 24, 32, 64, 96, 128};
   while (!h->small_bins.empty() && h->small_bins.back() > sfm) h->small_bins.pop_back();
   if (h->small_bins.empty() || h->small_bins.back() < sfm) h->small_bins.push_back(sfm);
   h->levels.assign(nlev, LevelPlan{});
@@ -426,7 +428,17 @@ int build_plan(mfd_handle* h) {
       ll.off = push_list(h, bins[b]);
       ll.count = (int32_t)bins[b].size();
       ll.param = h->small_bins[b];
+      for (int32_t g : bins[b])
+        ll.param2 = std::max(ll.param2, ((h->fronts[g].nc + h->fronts[g].nr) | 1) * h->fronts[g].nc);
       L.small.push_back(ll);
+      // the solve kernels take 32 rows at a time: the bins up to 32, next to each other in the list pool, as one
+      if (!L.small_solve.empty() && ll.param <= 32) {
+        L.small_solve.back().count += ll.count;
+        L.small_solve.back().param = ll.param;
+        L.small_solve.back().param2 = std::max(L.small_solve.back().param2, ll.param2);
+      } else {
+        L.small_solve.push_back(ll);
+      }
     }
     if (large.empty()) continue;
     std::stable_sort(large.begin(), large.end(),
@@ -612,6 +624,10 @@ int upload_plan(mfd_handle* h) {
   F.a_src = h->d_a_src.p; F.a_pos = h->d_a_pos.p; F.v_off = h->d_v_off.p; F.s_off = h->d_s_off.p;
   F.d_off = h->d_d_off.p;
   F.q_off = h->d_q_off.p;
+  CK(h->d_rec.alloc(h->h_lists.size()));
+  CK(h->d_crec.alloc(h->h_child.size()));
+  F.crec = h->d_crec.p;
+  launch_records(F, h->d_lists.p, (int)h->h_lists.size(), h->d_rec.p, (int)h->h_child.size(), h->d_crec.p, st);
 
   // permuted global A structure, value sources, front of every column
   std::vector<int32_t> acol(h->n_total + 1), arow(h->nnz_total), src(h->nnz_total), colf(h->n_total),
@@ -924,7 +940,7 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
       if (prof)
         for (int i = 0; i < s.count; ++i) small_work(h, hl[s.off + i], w, fl, by);
       record(h, sb, MFD_K_SMALL_FRONT, fl, by,
-             [&] { launch_small_fronts<T>(F, lists + s.off, s.count, s.param, a, panel, upool, h->d_info.p, sb); });
+             [&] { launch_small_fronts<T>(F, h->d_rec.p + s.off, s.count, s.param, a, panel, upool, h->d_info.p, sb); });
       ++n;
     }
     if (L.large.count == 0) {
@@ -1165,18 +1181,18 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
   // levels in the forward sweep and ancestors' X entries in the backward one)
   const bool side = side_streams(h);
   auto nside_of = [&](const LevelPlan& L) {
-    return side && (L.small.size() > 1 || L.large.count) ? (int)std::min<size_t>(L.small.size(), mfd_handle::kSide) : 0;
+    return side && (L.small_solve.size() > 1 || L.large.count) ? (int)std::min<size_t>(L.small_solve.size(), mfd_handle::kSide) : 0;
   };
   for (const LevelPlan& L : h->levels) {
     const int nside = nside_of(L);
     if (nside) side_fork(h, st, nside);
-    for (size_t b = 0; b < L.small.size(); ++b) {
-      const LaunchList& s = L.small[b];
+    for (size_t b = 0; b < L.small_solve.size(); ++b) {
+      const LaunchList& s = L.small_solve[b];
       cudaStream_t sb = (int)b < nside ? h->sst[b] : st;
       double fl = 0, by = 0;
       work(s, fl, by);
       record(h, sb, MFD_K_SOLVE_SMALL, fl, by,
-             [&] { launch_fwd_small<T>(F, lists + s.off, s.count, s.param, panel, X, ldx, V, nrhs, sb); });
+             [&] { launch_fwd_small<T>(F, h->d_rec.p + s.off, s.count, s.param, s.param2, panel, X, ldx, V, nrhs, sb); });
       ++n;
     }
     if (L.large.count) {
@@ -1194,13 +1210,13 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
     const LevelPlan& L = *it;
     const int nside = nside_of(L);
     if (nside) side_fork(h, st, nside);
-    for (size_t b = 0; b < L.small.size(); ++b) {
-      const LaunchList& s = L.small[b];
+    for (size_t b = 0; b < L.small_solve.size(); ++b) {
+      const LaunchList& s = L.small_solve[b];
       cudaStream_t sb = (int)b < nside ? h->sst[b] : st;
       double fl = 0, by = 0;
       work(s, fl, by);
       record(h, sb, MFD_K_SOLVE_SMALL, fl, by,
-             [&] { launch_bwd_small<T>(F, lists + s.off, s.count, s.param, panel, X, ldx, nrhs, sb); });
+             [&] { launch_bwd_small<T>(F, h->d_rec.p + s.off, s.count, s.param, s.param2, panel, X, ldx, nrhs, sb); });
       ++n;
     }
     if (L.large.count) {

@@ -24,6 +24,11 @@ constexpr int kBlkElems = 64;
 
 __device__ __forceinline__ int blk_index(int bi, int bj, int nb) { return bj * nb - bj * (bj - 1) / 2 + bi - bj; }
 __device__ __forceinline__ int blk_elem(int r, int c) { return r * 8 + ((((c >> 1) ^ (r >> 1)) & 3) << 1) + (c & 1); }
+// entry (i, j), i >= j (or both in one diagonal block), of an nb x nb block matrix
+__device__ __forceinline__ int blk_addr(int i, int j, int nb) {
+  const int bj = j >> 3;
+  return kBlkElems * (bj * nb - bj * (bj + 1) / 2) + 8 * i + ((((j >> 1) ^ (i >> 1)) & 3) << 1) + (j & 1);
+}
 // where lane (g, q) finds its 16 bytes of a block
 __device__ __forceinline__ int blk_frag(int lane) { return blk_elem(lane >> 2, 2 * (lane & 3)); }
 __host__ __device__ constexpr int blk_count(int nb) { return nb * (nb + 1) / 2; }
@@ -56,6 +61,42 @@ __device__ __forceinline__ void named_barrier(int threads) {
   asm volatile("bar.sync %0, %1;" ::"n"(ID), "r"(threads) : "memory");
 }
 
+// One warp's share (warp u of nu) of the rank-8 update of block columns js ..
+// nbt - 1 by panel p: block rows in a there-and-back order, so that two rows of
+// a warp have as many blocks as any other two.  row_done(i) follows block row i.
+template <typename RowDone>
+__device__ __forceinline__ void panel_update(double* S, int p, int js, int nbt, int u, int nu, int lane,
+                                             RowDone&& row_done) {
+  const int fo = blk_frag(lane);
+  const double* Lp = S + blk_index(p, p, nbt) * kBlkElems + fo;       // block (i, p) at Lp + 64 (i - p)
+  for (int m = 0; js + m < nbt; m += 2 * nu) {
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+      const int i = js + m + (hh ? 2 * nu - 1 - u : u);
+      if (i >= nbt) continue;
+      double2 a = *reinterpret_cast<const double2*>(Lp + (i - p) * kBlkElems);
+      a.x = -a.x;
+      a.y = -a.y;
+      for (int j0 = js; j0 <= i; j0 += 4) {
+        double2 b[4], c[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          if (j0 + v <= i) {
+            b[v] = *reinterpret_cast<const double2*>(Lp + (j0 + v - p) * kBlkElems);
+            c[v] = *reinterpret_cast<const double2*>(S + blk_index(i, j0 + v, nbt) * kBlkElems + fo);
+          }
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          if (j0 + v <= i) dmma8(c[v], a, b[v]);
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          if (j0 + v <= i) *reinterpret_cast<double2*>(S + blk_index(i, j0 + v, nbt) * kBlkElems + fo) = c[v];
+      }
+      row_done(i);
+    }
+  }
+}
+
 // Scratch of chol_panels in shared memory, in doubles: two staged diagonal
 // blocks and the pivots' reciprocal roots; with small-pivot tracking the
 // diagonal entries its test compares with.
@@ -73,6 +114,7 @@ __host__ __device__ constexpr int chol_scratch_elems(int max_rows, bool track) {
 //     then, with the finished panel visible, its row of the next block column;
 //   update warps: the panel's rank-8 update of the block columns after the
 //     next, on m8n8k4 DMMA, while the panel warps factor the next panel.
+// The last panel's update is shared by all warps.
 // Dinv (optional, nbp blocks): the inverses of the diagonal blocks.
 // track: dgs holds, per 32-column group, the diagonal as it stood when the
 // group was reached, and on_small() is called once per group with a pivot not
@@ -171,44 +213,24 @@ __device__ __forceinline__ void chol_panels(double* S, double* scratch, double* 
         }
         __syncwarp();
         named_barrier<1>(32 * PW);
+      } else {
+        panel_update(S, p, p + 1, nbt, warp, PW + UW, lane, [](int) {});
       }
     }
   } else {
-    const int u = warp - PW, fo = blk_frag(lane);
+    const int u = warp - PW;
     for (int p = 0; p < nbp; ++p) {
       named_barrier<0>(32 * (PW + UW));
-      const int js = p + 1 < nbp ? p + 2 : p + 1;        // the panel warps take block column p + 1
-      const double* Lp = S + blk_index(p, p, nbt) * kBlkElems + fo;   // block (i, p) at Lp + 64 (i - p)
-      // block rows in a there-and-back order: two rows of a warp have as many blocks as any other two
-      for (int m = 0; js + m < nbt; m += 2 * UW) {
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          const int i = js + m + (hh ? 2 * UW - 1 - u : u);
-          if (i >= nbt) continue;
-          double2 a = *reinterpret_cast<const double2*>(Lp + (i - p) * kBlkElems);
-          a.x = -a.x;
-          a.y = -a.y;
-          for (int j0 = js; j0 <= i; j0 += 4) {
-            double2 b[4], c[4];
-#pragma unroll
-            for (int v = 0; v < 4; ++v)
-              if (j0 + v <= i) {
-                b[v] = *reinterpret_cast<const double2*>(Lp + (j0 + v - p) * kBlkElems);
-                c[v] = *reinterpret_cast<const double2*>(S + blk_index(i, j0 + v, nbt) * kBlkElems + fo);
-              }
-#pragma unroll
-            for (int v = 0; v < 4; ++v)
-              if (j0 + v <= i) dmma8(c[v], a, b[v]);
-#pragma unroll
-            for (int v = 0; v < 4; ++v)
-              if (j0 + v <= i) *reinterpret_cast<double2*>(S + blk_index(i, j0 + v, nbt) * kBlkElems + fo) = c[v];
-          }
+      if (p + 1 < nbp) {                                 // the panel warps take block column p + 1
+        panel_update(S, p, p + 2, nbt, u, UW, lane, [&](int i) {
           if constexpr (kTrack)                          // the next group's reference diagonal (its first block: above)
-            if ((p & 3) == 3 && i <= p + 4 && i < nbp && i >= p + 2) {
+            if ((p & 3) == 3 && i <= p + 4 && i < nbp) {
               __syncwarp();
               if (lane < 8) dgs[8 * i + lane] = S[blk_index(i, i, nbt) * kBlkElems + blk_elem(lane, lane)];
             }
-        }
+        });
+      } else {
+        panel_update(S, p, p + 1, nbt, warp, PW + UW, lane, [](int) {});
       }
       if constexpr (kInv) {
         if (u == p % UW && lane < 8) {                   // column `lane` of the inverse of the diagonal block

@@ -40,13 +40,6 @@ __device__ __forceinline__ int lower_bound_dev(const int32_t* a, int n, int32_t 
 }
 
 
-template <typename T>
-__device__ __forceinline__ T rsqrt_t(T x);
-template <>
-__device__ __forceinline__ double rsqrt_t<double>(double x) { return rsqrt(x); }
-template <>
-__device__ __forceinline__ float rsqrt_t<float>(float x) { return rsqrtf(x); }
-
 inline int ceil_div(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
 __device__ __forceinline__ void cp_async8(void* smem_dst, const void* gsrc, bool valid) {
@@ -67,106 +60,6 @@ __device__ __forceinline__ void cp_async_t(T* dst, const T* src, bool valid) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(src), "r"(sz));
   else
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sa), "l"(src), "r"(sz));
-}
-
-// Extend-add of one child's lower update triangle into a front held in shared
-// memory by `nthreads` threads starting at t0 (a multiple of 32 threads):
-// thread (row lane tx, column group ty) takes columns ty, ty + ny, ... and in
-// each the rows i >= j of its lane (no division, lower triangle only; the
-// unrolled row loop keeps several loads in flight).  The child's local_index
-// is first staged in shared memory (sloc, nrc entries) by the caller.
-// local_index is injective, so no two entries of one child share a target.
-// Packed lower storage (ldS < 0, nf = -ldS): column j starts at
-// j nf - j (j + 1) / 2 and holds rows j .. nf-1.
-__device__ __forceinline__ int packed_col(int j, int nf) { return j * nf - j * (j + 1) / 2; }
-
-// S(local) += U for one child's update matrix U (nrc x nrc, lower triangle,
-// column-major) through its staged local_index sloc: lanes over rows, warps
-// over columns, CU columns x RI row passes of loads issued together per
-// chunk (predicated, no early exit), then the shared-memory adds.  ldS > 0:
-// S column-major with leading dimension ldS; ldS < 0: S packed (nf = -ldS).
-template <typename T, int RI, int CU>
-__device__ __forceinline__ void extend_add_chunk(T* S, int ldS, const T* __restrict__ U, const int* sloc, int nrc,
-                                                 int tx, int ty, int ny) {
-  for (int j0 = ty; j0 < nrc; j0 += CU * ny) {
-    T u[CU][RI];
-#pragma unroll
-    for (int c = 0; c < CU; ++c) {
-      const int j = j0 + c * ny;
-#pragma unroll
-      for (int v = 0; v < RI; ++v) {
-        const int i = j + tx + 32 * v;
-        u[c][v] = (j < nrc && i < nrc) ? U[(size_t)j * nrc + i] : T(0);
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < CU; ++c) {
-      const int j = j0 + c * ny;
-      if (j < nrc) {
-        const int lj = sloc[j] - 1;
-        const int base = ldS > 0 ? lj * ldS : packed_col(lj, -ldS);
-#pragma unroll
-        for (int v = 0; v < RI; ++v) {
-          const int i = j + tx + 32 * v;
-          if (i < nrc) S[base + sloc[i] - 1] += u[c][v];
-        }
-      }
-    }
-  }
-}
-// The same scatter with one column per warp step (lanes over rows): the
-// one-CTA-per-front kernel, whose 8 warps already keep 8 columns in flight.
-template <typename T>
-__device__ __forceinline__ void extend_add_cols(T* S, int ldS, const T* __restrict__ U, const int* sloc, int nrc,
-                                                int t0, int nthreads) {
-  const int tx = t0 & 31, ty = t0 >> 5, ny = nthreads >> 5;
-  for (int j = ty; j < nrc; j += ny) {
-    const int lj = sloc[j] - 1;
-    const int base = ldS > 0 ? lj * ldS : packed_col(lj, -ldS);
-    const T* Uc = U + (size_t)j * nrc;
-#pragma unroll 4
-    for (int i = j + tx; i < nrc; i += 32) S[base + sloc[i] - 1] += Uc[i];
-  }
-}
-// NB: loads in flight per thread and chunk (register budget)
-template <int NB, typename T>
-__device__ __forceinline__ void extend_add_smem(T* S, int ldS, const T* __restrict__ U, const int* sloc, int nrc,
-                                                int t0, int nthreads) {
-  const int tx = t0 & 31, ty = t0 >> 5, ny = nthreads >> 5;
-  switch ((nrc + 31) >> 5) {                 // row passes a column needs (nrc <= 128)
-    case 0: break;
-    case 1: extend_add_chunk<T, 1, NB>(S, ldS, U, sloc, nrc, tx, ty, ny); break;
-    case 2: extend_add_chunk<T, 2, (NB / 2 > 0 ? NB / 2 : 1)>(S, ldS, U, sloc, nrc, tx, ty, ny); break;
-    case 3: extend_add_chunk<T, 3, (NB / 3 > 0 ? NB / 3 : 1)>(S, ldS, U, sloc, nrc, tx, ty, ny); break;
-    default: extend_add_chunk<T, 4, (NB / 4 > 0 ? NB / 4 : 1)>(S, ldS, U, sloc, nrc, tx, ty, ny); break;
-  }
-}
-
-// A's entries of front f into its shared buffer (entry position pos = row +
-// col * nf, row >= col, placed at S[addr(row, col)]), U entries per thread
-// with their loads in flight together
-template <int UN, typename T, typename Addr>
-__device__ __forceinline__ void assemble_smem(const DevFronts& F, int f, int nf, const double* __restrict__ a, T* S,
-                                              Addr addr, int t0, int nthreads) {
-  const int a0 = F.a_beg[f], a1 = F.a_beg[f + 1];
-  for (int k0 = a0 + t0; k0 < a1; k0 += UN * nthreads) {
-    int pos[UN], src[UN];
-#pragma unroll
-    for (int u = 0; u < UN; ++u) {
-      const int k = k0 + u * nthreads;
-      pos[u] = k < a1 ? F.a_pos[k] : -1;
-      src[u] = k < a1 ? F.a_src[k] : 0;
-    }
-    double v[UN];
-#pragma unroll
-    for (int u = 0; u < UN; ++u) v[u] = pos[u] >= 0 ? a[src[u]] : 0.0;
-#pragma unroll
-    for (int u = 0; u < UN; ++u)
-      if (pos[u] >= 0) {
-        const int c = pos[u] / nf, r = pos[u] - c * nf;
-        S[addr(r, c)] = T(v[u]);
-      }
-  }
 }
 
 // Strided element loop (e = threadIdx.x, += blockDim.x, e < total) whose
@@ -247,6 +140,31 @@ __global__ void k_assembly_map(DevFronts F, const int32_t* col_front, const int3
   }
 }
 
+// What a small-front kernel needs of a front, one record per entry of the
+// launch lists, and of a child, one per entry of the children lists: two loads
+// deep where the tables above are six (list entry, front, child id, child).
+__global__ void k_front_records(DevFronts F, const int32_t* lists, int n, FrontRec* rec) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const int f = lists[k];
+  FrontRec r;
+  r.nc = F.nc[f]; r.nr = F.nr[f]; r.first = F.first[f]; r.lrow_off = F.lrow_off[f];
+  r.a_beg = F.a_beg[f]; r.a_end = F.a_beg[f + 1];
+  r.child_beg = F.child_ptr[f]; r.child_end = F.child_ptr[f + 1];
+  r.panel_off = F.panel_off[f]; r.u_off = F.u_off[f]; r.v_off = F.v_off[f];
+  r.pad = 0;
+  rec[k] = r;
+}
+__global__ void k_child_records(DevFronts F, int n, ChildRec* rec) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const int c = F.child[k];
+  ChildRec r;
+  r.nc = F.nc[c]; r.nr = F.nr[c]; r.lrow_off = F.lrow_off[c]; r.pad = 0;
+  r.u_off = F.u_off[c]; r.v_off = F.v_off[c];
+  rec[k] = r;
+}
+
 // block_local_index (block_local_index_creator_m.f90:13-122): a group is a
 // maximal run of a child's local index with constant (parent tile, child tile).
 __device__ __forceinline__ void bli_key(int loc, int i, int ncc, int nb, int& pt, int& ct) {
@@ -302,165 +220,6 @@ __global__ void k_bli_fill(DevFronts F, const int32_t* fronts, int count, int nb
 // ============================================================================
 // factorization
 // ============================================================================
-
-constexpr int kSfW = 8;   // panel width of the small-front elimination
-
-// Fused small front: zero, assemble A, extend-add the children in order, partial
-// Cholesky of the nc supernode columns and the Schur complement, all in shared
-// memory; writes the factor panel and the update matrix once.
-// Launched with 128 threads per front.  BIG (fronts of 65..128 rows, the
-// upper levels, few fronts per launch): up to 128 registers per thread and the
-// children's update columns loaded 16 at a time per thread; otherwise 32
-// registers (16 CTAs per SM by registers, shared memory binds first) and one
-// child column per warp step.
-template <typename T, bool BIG>
-__global__ void __launch_bounds__(128, BIG ? 4 : 16) k_small_front(DevFronts F, const int32_t* list, const double* __restrict__ a,
-                                                     T* __restrict__ panel, T* __restrict__ upool, int32_t* info) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* S = reinterpret_cast<T*>(smem_raw);     // the front's lower triangle, packed by columns
-  const int f = list[blockIdx.x];
-  const int nc = F.nc[f], nr = F.nr[f], nf = nc + nr;
-  const int tri = nf * (nf + 1) / 2;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-
-  // shared memory: the packed front (tri), kSfW pivot scales, a child's
-  // local_index (nf ints)
-  int* sloc = reinterpret_cast<int*>(S + tri + kSfW);
-  for (int i = tid; i < tri; i += nt) S[i] = T(0);
-  __syncthreads();
-  for (int k = F.a_beg[f] + tid; k < F.a_beg[f + 1]; k += nt) {
-    const int pos = F.a_pos[k];
-    const int c = pos / nf, r = pos - c * nf;          // r >= c: the lower part of A
-    S[packed_col(c, nf) + r] = T(a[F.a_src[k]]);
-  }
-  __syncthreads();
-  for (int t = F.child_ptr[f]; t < F.child_ptr[f + 1]; ++t) {
-    const int c = F.child[t];
-    const int nrc = F.nr[c];
-    const int32_t* loc = F.local + F.lrow_off[c];
-    for (int i = tid; i < nrc; i += nt) sloc[i] = loc[i];
-    __syncthreads();
-    if constexpr (BIG) extend_add_smem<16>(S, -nf, upool + F.u_off[c], sloc, nrc, tid, nt);
-    else extend_add_cols(S, -nf, upool + F.u_off[c], sloc, nrc, tid, nt);
-    __syncthreads();
-  }
-  // blocked right-looking elimination, panels of kSfW columns, three barriers
-  // per panel: (1) lanes 0..w-1 of warp 0 factor the w x w diagonal block in
-  // registers (lane = row, pivots by shuffles); (2) every thread solves rows
-  // of the block column below it, l_ip = (a_ip - sum_{p'<p} l_ip' L_pp') y_p;
-  // (3) the rank-w update S_ij -= sum_p L_ip L_jp of the trailing triangle
-  // (FP64: 8 x 8 tiles on m8n8k4 DMMA, one warp per tile; FP32: warps over
-  // columns, lanes over rows)
-  T* ys = S + tri;                           // the panel's pivot scales y_p = 1/sqrt(d_p)
-  for (int k0 = 0; k0 < nc; k0 += kSfW) {
-    const int w = min(kSfW, nc - k0);
-    int pc[kSfW];
-#pragma unroll
-    for (int p = 0; p < kSfW; ++p) pc[p] = packed_col(k0 + min(p, w - 1), nf);
-    if (warp == 0) {
-      T rv[kSfW];
-      const int r = k0 + lane;
-#pragma unroll
-      for (int p = 0; p < kSfW; ++p) rv[p] = (lane < w && p < w && p <= lane) ? S[pc[p] + r] : T(0);
-#pragma unroll
-      for (int p = 0; p < kSfW; ++p) {
-        if (p < w) {
-          T d = __shfl_sync(0xffffffffu, rv[p], p);
-          if (!(d > T(0))) {
-            if (lane == 0) atomicMin(info, F.first[f] + k0 + p + 1);
-            d = T(1);
-          }
-          const T y = rsqrt_t<T>(d);
-          if (lane > p) rv[p] *= y;
-          else if (lane == p) { rv[p] = d * y; ys[p] = y; }
-#pragma unroll
-          for (int p2 = p + 1; p2 < kSfW; ++p2) {
-            if (p2 < w) {
-              const T lj = __shfl_sync(0xffffffffu, rv[p], p2);
-              if (lane >= p2) rv[p2] -= rv[p] * lj;
-            }
-          }
-        }
-      }
-      if (lane < w) {
-#pragma unroll
-        for (int p = 0; p < kSfW; ++p)
-          if (p <= lane) S[pc[p] + r] = rv[p];
-      }
-    }
-    __syncthreads();
-    for (int i = k0 + w + tid; i < nf; i += nt) {
-      T x[kSfW];
-#pragma unroll
-      for (int p = 0; p < kSfW; ++p) x[p] = p < w ? S[pc[p] + i] : T(0);
-#pragma unroll
-      for (int p = 0; p < kSfW; ++p) {
-        if (p < w) {
-          T v = x[p];
-#pragma unroll
-          for (int q = 0; q < p; ++q) v -= x[q] * S[pc[q] + k0 + p];
-          x[p] = v * ys[p];
-        }
-      }
-#pragma unroll
-      for (int p = 0; p < kSfW; ++p)
-        if (p < w) S[pc[p] + i] = x[p];
-    }
-    __syncthreads();
-    const int kb = k0 + w;                   // the trailing triangle: rows and columns [kb, nf)
-    if constexpr (std::is_same<T, double>::value) {
-      const int t8 = (nf - kb + 7) >> 3, tiles = t8 * (t8 + 1) / 2;
-      const int g = lane >> 2, q = lane & 3;
-      for (int t = warp; t < tiles; t += nw) {
-        int ti = 0;                          // tile (ti, tj), ti >= tj, row-major over the lower triangle
-        while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-        const int tj = t - ti * (ti + 1) / 2;
-        const int i0 = kb + 8 * ti, j0 = kb + 8 * tj;
-        const int ia = i0 + g, jb = j0 + g;  // the row of A and the column of B this lane feeds
-        double c[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int j = j0 + 2 * q + e;
-          c[e] = (ia < nf && j < nf && ia >= j) ? S[packed_col(j, nf) + ia] : 0.0;
-        }
-#pragma unroll
-        for (int s4 = 0; s4 < kSfW; s4 += 4) {
-          const int p = s4 + q;
-          const double av = (p < w && ia < nf) ? -S[pc[p] + ia] : 0.0;
-          const double bv = (p < w && jb < nf) ? S[pc[p] + jb] : 0.0;
-          dmma(c[0], c[1], av, bv);
-        }
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int j = j0 + 2 * q + e;
-          if (ia < nf && j < nf && ia >= j) S[packed_col(j, nf) + ia] = c[e];
-        }
-      }
-    } else {
-      for (int j = kb + warp; j < nf; j += nw) {
-        T lj[kSfW];
-#pragma unroll
-        for (int p = 0; p < kSfW; ++p) lj[p] = p < w ? S[pc[p] + j] : T(0);
-        T* colj = S + packed_col(j, nf);
-        for (int i = j + lane; i < nf; i += 32) {
-          T acc = colj[i];
-#pragma unroll
-          for (int p = 0; p < kSfW; ++p)
-            if (p < w) acc -= S[pc[p] + i] * lj[p];
-          colj[i] = acc;
-        }
-      }
-    }
-    __syncthreads();
-  }
-  T* P = panel + F.panel_off[f];
-  for (int j = warp; j < nc; j += nw)
-    for (int i = j + lane; i < nf; i += 32) P[i + (size_t)j * nf] = S[packed_col(j, nf) + i];
-  T* U = upool + F.u_off[f];
-  for (int j = warp; j < nr; j += nw)
-    for (int i = j + lane; i < nr; i += 32) U[i + (size_t)j * nr] = S[packed_col(nc + j, nf) + nc + i];
-}
 
 // Zero the lower triangles of a large front's panel (nf x nc) and update
 // matrix (nr x nr): one warp per column, grid-stride over columns.
@@ -944,436 +703,6 @@ __global__ void __launch_bounds__(256) k_update_simt(DevFronts F, const int32_t*
 // solves
 // ============================================================================
 
-// ---- fronts with nf <= 32: one warp per front ---------------------------------
-// Four fronts per 128-thread CTA.  The front is assembled in a per-warp
-// shared buffer (A entries, then the children's update matrices through
-// local_index), loaded one row per lane into registers and partially
-// factored there (nc pivots: shuffle for the pivot, rsqrt, rank-1 update with
-// the column broadcast through a double-buffered shared vector); the panel
-// columns and the update matrix are written back one column per step, lanes
-// over rows (coalesced).  No CTA-wide barrier: many more fronts in flight per
-// SM than the one-CTA-per-front kernel.
-constexpr int kWF = 32;          // front capacity of a warp
-constexpr int kWFLd = kWF + 1;
-constexpr int kWFWarps = 4;
-
-
-// Gathers of a level with many fronts and several right-hand sides: eight
-// right-hand sides per CTA, a warp each (no CTA-wide barrier between children),
-// eight rows per lane in flight.  With one CTA per front and right-hand side
-// these levels paid each CTA's chain of loads for a few hundred rows: 218 us
-// against this form's figure in launch_fwd_large for 928 fronts x 64.
-constexpr int kGatherRhs = 8;
-template <typename T>
-__global__ void __launch_bounds__(32 * kGatherRhs) k_fwd_gather_warp(DevFronts F, const int32_t* list, const T* X,
-                                                                     int64_t ldx, T* V, int nrhs) {
-  constexpr int U = 8;
-  const int f = list[blockIdx.x], lane = threadIdx.x & 31, r = blockIdx.y * kGatherRhs + (threadIdx.x >> 5);
-  if (r >= nrhs) return;
-  const int nc = F.nc[f], nf = nc + F.nr[f], first = F.first[f];
-  T* Vf = V + F.v_off[f] * nrhs + (int64_t)r * nf;
-  const T* Xr = X + first + r * ldx;
-  for (int i0 = lane; i0 < nf; i0 += 32 * U) {
-    T v[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) v[u] = i0 + 32 * u < nc ? Xr[i0 + 32 * u] : T(0);
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (i0 + 32 * u < nf) Vf[i0 + 32 * u] = v[u];
-  }
-  for (int t = F.child_ptr[f]; t < F.child_ptr[f + 1]; ++t) {
-    __syncwarp();
-    const int c = F.child[t];
-    const int ncc = F.nc[c], nrc = F.nr[c];
-    const T* Vc = V + F.v_off[c] * nrhs + (int64_t)r * (ncc + nrc) + ncc;
-    const int32_t* loc = F.local + F.lrow_off[c];
-    for (int i0 = lane; i0 < nrc; i0 += 32 * U) {
-      int li[U];
-      T cv[U], ov[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int i = i0 + 32 * u;
-        li[u] = i < nrc ? loc[i] - 1 : -1;
-        cv[u] = i < nrc ? Vc[i] : T(0);
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) ov[u] = li[u] >= 0 ? Vf[li[u]] : T(0);
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (li[u] >= 0) Vf[li[u]] = ov[u] + cv[u];
-    }
-  }
-}
-template <typename T>
-__global__ void __launch_bounds__(32 * kGatherRhs) k_bwd_gather_warp(DevFronts F, const int32_t* list, const T* X,
-                                                                     int64_t ldx, T* V, int nrhs) {
-  constexpr int U = 8;
-  const int f = list[blockIdx.x], lane = threadIdx.x & 31, r = blockIdx.y * kGatherRhs + (threadIdx.x >> 5);
-  if (r >= nrhs) return;
-  const int nc = F.nc[f], nf = nc + F.nr[f], first = F.first[f];
-  const int32_t* lr = F.lrow + F.lrow_off[f];
-  T* Vf = V + F.v_off[f] * nrhs + (int64_t)r * nf;
-  for (int i0 = lane; i0 < nf; i0 += 32 * U) {
-    int gi[U];
-    T v[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int i = i0 + 32 * u;
-      gi[u] = i < nc ? first + i : (i < nf ? lr[i - nc] : -1);
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) v[u] = gi[u] >= 0 ? X[gi[u] + r * ldx] : T(0);
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (gi[u] >= 0) Vf[i0 + 32 * u] = v[u];
-  }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kWFWarps * 32) k_small_warp(DevFronts F, const int32_t* list, int count,
-                                                              const double* __restrict__ a, T* __restrict__ panel,
-                                                              T* __restrict__ upool, int32_t* info) {
-  __shared__ T sbuf[kWFWarps][kWF * kWFLd];
-  __shared__ T cbuf[kWFWarps][2][kWF];
-  __shared__ int slocbuf[kWFWarps][kWF];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int slot = blockIdx.x * kWFWarps + warp;
-  if (slot >= count) return;
-  const int f = list[slot];
-  const int nc = F.nc[f], nr = F.nr[f], nf = nc + nr;
-  T* S = sbuf[warp];
-  // children's metadata one per lane (broadcast by shuffles), loaded while
-  // the front is zeroed and assembled
-  const int cp0 = F.child_ptr[f], nch = F.child_ptr[f + 1] - cp0;
-  int cnr = 0, clo = 0;
-  long long cuo = 0;
-  if (lane < nch) {
-    const int c = F.child[cp0 + lane];
-    cnr = F.nr[c]; clo = F.lrow_off[c]; cuo = F.u_off[c];
-  }
-  for (int e = lane; e < kWF * kWFLd; e += 32) S[e] = T(0);
-  __syncwarp();
-  assemble_smem<4>(F, f, nf, a, S, [](int r, int c) { return r + c * kWFLd; }, lane, 32);
-  __syncwarp();
-  int* sloc = slocbuf[warp];
-  for (int cb = 0; cb < nch; cb += 32) {
-    if (cb > 0) {
-      cnr = 0; clo = 0; cuo = 0;
-      if (cb + lane < nch) {
-        const int c = F.child[cp0 + cb + lane];
-        cnr = F.nr[c]; clo = F.lrow_off[c]; cuo = F.u_off[c];
-      }
-    }
-    const int m = min(32, nch - cb);
-    for (int t = 0; t < m; ++t) {
-      const int nrc = __shfl_sync(0xffffffffu, cnr, t), lo = __shfl_sync(0xffffffffu, clo, t);
-      const long long uo = __shfl_sync(0xffffffffu, cuo, t);
-      if (lane < nrc) sloc[lane] = F.local[lo + lane];
-      __syncwarp();
-      extend_add_smem<8>(S, kWFLd, upool + uo, sloc, nrc, lane, 32);
-      __syncwarp();
-    }
-  }
-  T row[kWF];
-#pragma unroll
-  for (int j = 0; j < kWF; ++j) row[j] = S[lane + j * kWFLd];
-  int bad = 0;
-#pragma unroll
-  for (int k = 0; k < kWF; ++k) {
-    if (k >= nc) break;
-    T d = __shfl_sync(0xffffffffu, row[k], k);
-    if (!(d > T(0))) {                    // uniform across the warp
-      if (!bad) bad = k + 1;
-      d = T(1);
-    }
-    const T y = rsqrt_t<T>(d);
-    const T l = row[k] * y;
-    T* cb = cbuf[warp][k & 1];
-    cb[lane] = l;
-    __syncwarp();
-    row[k] = lane == k ? d * y : l;
-#pragma unroll
-    for (int j = k + 1; j < kWF; ++j) row[j] -= l * cb[j];
-  }
-  if (bad && lane == 0) atomicMin(info, F.first[f] + bad);
-  T* P = panel + F.panel_off[f];
-  T* Uf = upool + F.u_off[f];
-#pragma unroll
-  for (int j = 0; j < kWF; ++j) {
-    if (j >= nf) break;
-    if (lane >= j && lane < nf) {
-      if (j < nc) P[lane + (size_t)j * nf] = row[j];
-      else Uf[(lane - nc) + (size_t)(j - nc) * nr] = row[j];
-    }
-  }
-}
-
-// ---- small-front solves: one warp per front (nf <= 32 R) ----------------------
-// Four fronts per 128-thread CTA, no CTA-wide barrier, so many fronts are in
-// flight per SM and their panel reads overlap.  The front's solve vector is
-// staged in a per-warp shared vector (the children's update vectors are
-// scattered into it through local_index).
-//   forward : lane l holds rows l + 32 q (q < R); column k of the panel is
-//             read lanes over rows (coalesced), y_k = v_k / L_kk is formed by
-//             the lane holding row k and broadcast by a shuffle, and every row
-//             below k takes v_i -= L_ik y_k.
-//   backward: 32-column blocks from the last: the rows below the block's
-//             triangle give t_k -= sum_i L_ik x_i as per-lane partial sums
-//             over rows (coalesced) reduced through a transposing per-warp
-//             tile; the 32 x 32 triangle is read lanes over rows, transposed
-//             through the same tile (lane k then holds column k) and solved
-//             by shuffles.
-constexpr int kSWarps = 4;
-constexpr int kTileLd = 33;
-
-template <typename T, int R>
-__device__ __forceinline__ T pick(const T (&a)[R], int q) {
-  T r = a[0];
-#pragma unroll
-  for (int p = 1; p < R; ++p)
-    if (p == q) r = a[p];
-  return r;
-}
-template <typename T, int R>
-__device__ __forceinline__ void put(T (&a)[R], int q, T v) {
-#pragma unroll
-  for (int p = 0; p < R; ++p)
-    if (p == q) a[p] = v;
-}
-
-// v += the children's update vectors of front f (right-hand side r), child
-// metadata loaded one child per lane so the per-child chain is one load deep
-template <typename T, int R>
-__device__ __forceinline__ void gather_children(const DevFronts& F, int f, const T* V, int nrhs, int r, T* vs,
-                                                int lane) {
-  const int c0 = F.child_ptr[f], nch = F.child_ptr[f + 1] - c0;
-  for (int cb = 0; cb < nch; cb += 32) {
-    int cnc = 0, cnr = 0, clo = 0;
-    long long cvo = 0;
-    if (cb + lane < nch) {
-      const int c = F.child[c0 + cb + lane];
-      cnc = F.nc[c]; cnr = F.nr[c]; clo = F.lrow_off[c]; cvo = F.v_off[c];
-    }
-    const int m = min(32, nch - cb);
-    for (int t = 0; t < m; ++t) {
-      const int ncc = __shfl_sync(0xffffffffu, cnc, t), nrc = __shfl_sync(0xffffffffu, cnr, t);
-      const int lo = __shfl_sync(0xffffffffu, clo, t);
-      const long long vo = __shfl_sync(0xffffffffu, cvo, t);
-      const T* Vc = V + vo * nrhs + (int64_t)r * (ncc + nrc) + ncc;
-      const int32_t* loc = F.local + lo;
-      int li[R];
-      T vv[R];
-#pragma unroll
-      for (int q = 0; q < R; ++q) {
-        const int i = lane + 32 * q;
-        li[q] = i < nrc ? loc[i] - 1 : -1;
-        vv[q] = i < nrc ? Vc[i] : T(0);
-      }
-#pragma unroll
-      for (int q = 0; q < R; ++q)
-        if (li[q] >= 0) vs[li[q]] += vv[q];
-      __syncwarp();
-    }
-  }
-}
-
-// L2 prefetch of a front's panel (nf x nc, contiguous, 16-byte aligned; the
-// size is rounded up into the pool's alignment padding)
-template <typename T>
-__device__ __forceinline__ void prefetch_panel(const T* P, int nf, int nc) {
-  const unsigned bytes = ((unsigned)((size_t)nf * nc * sizeof(T)) + 15u) & ~15u;
-  if (bytes) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(P), "r"(bytes) : "memory");
-}
-
-template <typename T, int R>
-__device__ __forceinline__ void fwd_small_front(const DevFronts& F, int f, const T* __restrict__ panel, T* X,
-                                                int64_t ldx, T* V, int nrhs, T* vs, int lane) {
-  const int nc = F.nc[f], nf = nc + F.nr[f], first = F.first[f];
-  const T* P = panel + F.panel_off[f];
-  if (lane == 0) prefetch_panel(P, nf, nc);
-  T dinv[R];
-#pragma unroll
-  for (int q = 0; q < R; ++q) {
-    const int i = lane + 32 * q;
-    dinv[q] = i < nc ? T(1) / P[i + (size_t)i * nf] : T(1);
-  }
-  T* Vf = V + F.v_off[f] * nrhs;
-  const int rb = gridDim.y > 1 ? (int)blockIdx.y : 0, re = gridDim.y > 1 ? rb + 1 : nrhs;   // one RHS per CTA row
-  for (int r = rb; r < re; ++r) {
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      const int i = lane + 32 * q;
-      vs[i] = i < nc ? X[first + i + r * ldx] : T(0);
-    }
-    __syncwarp();
-    gather_children<T, R>(F, f, V, nrhs, r, vs, lane);
-    T v[R];
-#pragma unroll
-    for (int q = 0; q < R; ++q) v[q] = vs[lane + 32 * q];
-    __syncwarp();
-    // columns in groups of G with predicated (not early-exited) steps, so the
-    // group's loads issue together: one memory latency per group
-    constexpr int G = 8;
-    for (int k0 = 0; k0 < nc; k0 += 32) {
-      const int qb = k0 >> 5, kn = min(32, nc - k0);
-      const T dk = pick(dinv, qb);
-      for (int g = 0; g < kn; g += G) {
-        T l[G][R];
-#pragma unroll
-        for (int u = 0; u < G; ++u) {
-          const int k = k0 + g + u;
-          const T* Pk = P + (size_t)k * nf;
-#pragma unroll
-          for (int q = 0; q < R; ++q) {
-            const int i = lane + 32 * q;
-            l[u][q] = (g + u < kn && i > k && i < nf) ? Pk[i] : T(0);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < G; ++u) {
-          if (g + u < kn) {
-            const int kk = g + u, k = k0 + kk;
-            const T yk = __shfl_sync(0xffffffffu, pick(v, qb) * dk, kk);
-#pragma unroll
-            for (int q = 0; q < R; ++q)
-              if (lane + 32 * q > k) v[q] -= l[u][q] * yk;
-            if (lane == kk) put(v, qb, yk);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      const int i = lane + 32 * q;
-      if (i < nc) X[first + i + r * ldx] = v[q];
-      else if (i < nf) Vf[(int64_t)r * nf + i] = v[q];
-    }
-  }
-}
-
-template <typename T, int R>
-__global__ void __launch_bounds__(kSWarps * 32) k_fwd_small(DevFronts F, const int32_t* list, int count,
-                                                            const T* __restrict__ panel, T* X, int64_t ldx, T* V,
-                                                            int nrhs) {
-  __shared__ T vbuf[kSWarps][32 * R];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int slot = blockIdx.x * kSWarps + warp;
-  if (slot >= count) return;
-  fwd_small_front<T, R>(F, list[slot], panel, X, ldx, V, nrhs, vbuf[warp], lane);
-}
-
-template <typename T, int R>
-__device__ __forceinline__ void bwd_small_front(const DevFronts& F, int f, const T* __restrict__ panel, T* X,
-                                                int64_t ldx, int nrhs, T* xs, T* tile, int lane) {
-  const int nc = F.nc[f], nf = nc + F.nr[f], first = F.first[f];
-  const int32_t* lr = F.lrow + F.lrow_off[f];
-  const T* P = panel + F.panel_off[f];
-  if (lane == 0) prefetch_panel(P, nf, nc);
-  const int rb = gridDim.y > 1 ? (int)blockIdx.y : 0, re = gridDim.y > 1 ? rb + 1 : nrhs;   // one RHS per CTA row
-  for (int r = rb; r < re; ++r) {
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      const int i = lane + 32 * q;
-      xs[i] = i < nc ? X[first + i + r * ldx] : (i < nf ? X[lr[i - nc] + r * ldx] : T(0));
-    }
-    __syncwarp();
-    for (int b = (nc - 1) >> 5; b >= 0; --b) {
-      const int j0 = 32 * b, e = min(j0 + 32, nc), kn = e - j0;   // the block's columns [j0, e)
-      T s = T(0);
-      if constexpr (R == 1) {
-        // nf <= 32: the whole panel in one pass, lanes over rows (one memory
-        // latency): triangle rows raw and lower, rows below nc as products
-        // with x, summed per column in row order
-        const int i = lane;
-        const bool tri = i < nc, ok = i < nf;
-        const T xi = (!tri && ok) ? xs[i] : T(0);
-        T l[32];
-#pragma unroll
-        for (int kk = 0; kk < 32; ++kk) l[kk] = (ok && kk < nc && (!tri || kk <= i)) ? P[i + (size_t)kk * nf] : T(0);
-#pragma unroll
-        for (int kk = 0; kk < 32; ++kk) tile[lane * kTileLd + kk] = tri ? l[kk] : l[kk] * xi;
-        __syncwarp();
-#pragma unroll
-        for (int ii = 0; ii < 32; ++ii) {
-          const T v = tile[ii * kTileLd + lane];
-          if (ii >= nc && ii < nf) s += v;
-        }
-      } else {
-        // rows below the triangle [e, nf), lanes over rows, 8 columns at a time:
-        // tile(lane, kk) = sum over the lane's rows i of L(i, j0+kk) x_i
-        for (int g = 0; g < kn; g += 8) {
-          T acc[8];
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk) acc[kk] = T(0);
-          for (int i0 = e; i0 < nf; i0 += 32) {
-            const int i = i0 + lane;
-            const bool ok = i < nf;
-            const T xi = ok ? xs[i] : T(0);
-            const T* Pi = P + i + (size_t)(j0 + g) * nf;
-            T l[8];
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk) l[kk] = (ok && g + kk < kn) ? Pi[(size_t)kk * nf] : T(0);
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk) acc[kk] += l[kk] * xi;
-          }
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk) tile[lane * kTileLd + g + kk] = acc[kk];
-        }
-        __syncwarp();
-        // columns >= kn of the tile are not written: unused
-#pragma unroll
-        for (int j = 0; j < 32; ++j) s += tile[j * kTileLd + lane];
-        __syncwarp();
-        // the triangle, read lanes over rows (row j0 + lane, columns j0 .. row)
-        // into the tile; lane k then reads column k from it
-        {
-          const int i = j0 + lane;
-          const T* Pi = P + i + (size_t)j0 * nf;
-#pragma unroll
-          for (int h = 0; h < 32; h += 16) {
-            T l[16];
-#pragma unroll
-            for (int kk = 0; kk < 16; ++kk) l[kk] = (h + kk <= lane && lane < kn) ? Pi[(size_t)(h + kk) * nf] : T(0);
-#pragma unroll
-            for (int kk = 0; kk < 16; ++kk) tile[lane * kTileLd + h + kk] = l[kk];
-          }
-        }
-      }
-      __syncwarp();
-      const T dk = lane < kn ? T(1) / tile[lane * kTileLd + lane] : T(1);
-      T t = lane < kn ? xs[j0 + lane] - s : T(0);
-#pragma unroll 8
-      for (int ii = 31; ii >= 0; --ii) {
-        if (ii >= kn) continue;
-        const T lv = tile[ii * kTileLd + lane];    // L(j0 + ii, j0 + lane)
-        const T xi = __shfl_sync(0xffffffffu, t * dk, ii);
-        if (lane == ii) t = xi;
-        else if (lane < ii) t -= lv * xi;
-      }
-      __syncwarp();
-      if (lane < kn) xs[j0 + lane] = t;
-      __syncwarp();
-    }
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      const int i = lane + 32 * q;
-      if (i < nc) X[first + i + r * ldx] = xs[i];
-    }
-    __syncwarp();
-  }
-}
-
-template <typename T, int R>
-__global__ void __launch_bounds__(kSWarps * 32, 6) k_bwd_small(DevFronts F, const int32_t* list, int count,
-                                                            const T* __restrict__ panel, T* X, int64_t ldx, int nrhs) {
-  __shared__ T xbuf[kSWarps][32 * R];
-  __shared__ T tbuf[kSWarps][32 * kTileLd];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int slot = blockIdx.x * kSWarps + warp;
-  if (slot >= count) return;
-  bwd_small_front<T, R>(F, list[slot], panel, X, ldx, nrhs, xbuf[warp], tbuf[warp], lane);
-}
-
 // ---- large fronts: the solve vector of front f lives in V (nf per RHS) --------
 // Panel steps of kSolveB = 128 columns use the inverted diagonal blocks kept
 // from the factorization (Li = L_ss^{-1}), one launch per step:
@@ -1385,7 +714,6 @@ __global__ void __launch_bounds__(kSWarps * 32, 6) k_bwd_small(DevFronts F, cons
 //             x_s = Li^T t_s (k_bwd_large_step)
 // The diagonal solves write the front's own entries of X directly.
 constexpr int kRhsG = 8;      // right-hand sides per pass
-constexpr int kMrhsMin = 8;   // from this many right-hand sides on, GEMM-shaped large-front steps
 constexpr int kFwdRows = 32;  // rows per CTA of k_fwd_large_rest
 
 // y_s = Li v_s by one CTA of 256 threads: thread (row i, half h) sums k in
@@ -1781,6 +1109,77 @@ __global__ void __launch_bounds__(256) k_bwd_large_fused(DevFronts F, const int4
   }
 }
 
+// Gathers of a level with many fronts and several right-hand sides: eight
+// right-hand sides per CTA, a warp each (no CTA-wide barrier between children),
+// eight rows per lane in flight.  With one CTA per front and right-hand side
+// these levels paid each CTA's chain of loads for a few hundred rows: 218 us
+// against this form's figure in launch_fwd_large for 928 fronts x 64.
+constexpr int kGatherRhs = 8;
+template <typename T>
+__global__ void __launch_bounds__(32 * kGatherRhs) k_fwd_gather_warp(DevFronts F, const int32_t* list, const T* X,
+                                                                     int64_t ldx, T* V, int nrhs) {
+  constexpr int U = 8;
+  const int f = list[blockIdx.x], lane = threadIdx.x & 31, r = blockIdx.y * kGatherRhs + (threadIdx.x >> 5);
+  if (r >= nrhs) return;
+  const int nc = F.nc[f], nf = nc + F.nr[f], first = F.first[f];
+  T* Vf = V + F.v_off[f] * nrhs + (int64_t)r * nf;
+  const T* Xr = X + first + r * ldx;
+  for (int i0 = lane; i0 < nf; i0 += 32 * U) {
+    T v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = i0 + 32 * u < nc ? Xr[i0 + 32 * u] : T(0);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i0 + 32 * u < nf) Vf[i0 + 32 * u] = v[u];
+  }
+  for (int t = F.child_ptr[f]; t < F.child_ptr[f + 1]; ++t) {
+    __syncwarp();
+    const int c = F.child[t];
+    const int ncc = F.nc[c], nrc = F.nr[c];
+    const T* Vc = V + F.v_off[c] * nrhs + (int64_t)r * (ncc + nrc) + ncc;
+    const int32_t* loc = F.local + F.lrow_off[c];
+    for (int i0 = lane; i0 < nrc; i0 += 32 * U) {
+      int li[U];
+      T cv[U], ov[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + 32 * u;
+        li[u] = i < nrc ? loc[i] - 1 : -1;
+        cv[u] = i < nrc ? Vc[i] : T(0);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) ov[u] = li[u] >= 0 ? Vf[li[u]] : T(0);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (li[u] >= 0) Vf[li[u]] = ov[u] + cv[u];
+    }
+  }
+}
+template <typename T>
+__global__ void __launch_bounds__(32 * kGatherRhs) k_bwd_gather_warp(DevFronts F, const int32_t* list, const T* X,
+                                                                     int64_t ldx, T* V, int nrhs) {
+  constexpr int U = 8;
+  const int f = list[blockIdx.x], lane = threadIdx.x & 31, r = blockIdx.y * kGatherRhs + (threadIdx.x >> 5);
+  if (r >= nrhs) return;
+  const int nc = F.nc[f], nf = nc + F.nr[f], first = F.first[f];
+  const int32_t* lr = F.lrow + F.lrow_off[f];
+  T* Vf = V + F.v_off[f] * nrhs + (int64_t)r * nf;
+  for (int i0 = lane; i0 < nf; i0 += 32 * U) {
+    int gi[U];
+    T v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + 32 * u;
+      gi[u] = i < nc ? first + i : (i < nf ? lr[i - nc] : -1);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = gi[u] >= 0 ? X[gi[u] + r * ldx] : T(0);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (gi[u] >= 0) Vf[i0 + 32 * u] = v[u];
+  }
+}
+
 template <typename T>
 __global__ void k_bwd_large_gather(DevFronts F, const int32_t* list, const T* X, int64_t ldx, T* V, int nrhs) {
   const int f = list[blockIdx.x];
@@ -2064,11 +1463,6 @@ __global__ void k_fill_int(int32_t* p, int32_t v, int64_t n) {
 constexpr int kNumSms = 148;
 inline int grid_1d(int64_t n, int threads = 256) { return clamp_grid(ceil_div(n, threads), 148 * 16); }
 
-template <typename T>
-size_t small_front_smem(int nf_max) {   // packed front, kSfW pivot scales, a staged local_index
-  return ((size_t)nf_max * (nf_max + 1) / 2 + kSfW) * sizeof(T) + (size_t)nf_max * sizeof(int);
-}
-
 // Dynamic shared memory above 48 KB is opted into once per kernel at handle
 // creation (prepare_kernels), never inside a stream capture.
 constexpr int kMaxDynSmem = 227 * 1024;
@@ -2087,9 +1481,9 @@ void set_smem(KernelT, size_t) {}
 cudaError_t prepare_kernels() {
   cudaError_t e = cudaSuccess;
   auto chk = [&](cudaError_t r) { if (r != cudaSuccess && e == cudaSuccess) e = r; };
-  chk(opt_in(k_small_front<double, false>)); chk(opt_in(k_small_front<float, false>));
-  chk(opt_in(k_small_front<double, true>)); chk(opt_in(k_small_front<float, true>));
   chk(opt_in(k_update_dmma));
+  chk(prepare_small_fronts());
+  chk(prepare_small_solve());
   chk(prepare_panel());
   chk(prepare_update_tc());
   chk(prepare_update_tcq());
@@ -2108,6 +1502,11 @@ void launch_assembly_map(const DevFronts& F, const int32_t* col_front, const int
     k_assembly_map<<<ceil_div(n_total, 256), 256, 0, st>>>(F, col_front, acol_ptr, arow, ccs_src, sidx, a_src, a_pos,
                                                            n_total);
 }
+void launch_records(const DevFronts& F, const int32_t* lists, int list_len, FrontRec* rec, int num_child,
+                    ChildRec* crec, cudaStream_t st) {
+  if (list_len > 0) k_front_records<<<ceil_div(list_len, 256), 256, 0, st>>>(F, lists, list_len, rec);
+  if (num_child > 0) k_child_records<<<ceil_div(num_child, 256), 256, 0, st>>>(F, num_child, crec);
+}
 void launch_bli_count(const DevFronts& F, const int32_t* fronts, int count, int nb, int32_t* groups, cudaStream_t st) {
   if (count > 0) k_bli_count<<<ceil_div(count, 128), 128, 0, st>>>(F, fronts, count, nb, groups);
 }
@@ -2119,21 +1518,6 @@ void launch_bli_fill(const DevFronts& F, const int32_t* fronts, int count, int n
                                                      cnum, offset, rebuilt);
 }
 
-template <typename T>
-void launch_small_fronts(const DevFronts& F, const int32_t* list, int count, int nf_max, const double* a, T* panel,
-                         T* upool, int32_t* info, cudaStream_t st) {
-  if (count <= 0) return;
-  if (nf_max <= kWF) {
-    k_small_warp<T><<<ceil_div(count, kWFWarps), kWFWarps * 32, 0, st>>>(F, list, count, a, panel, upool, info);
-    return;
-  }
-  size_t sm = small_front_smem<T>(nf_max);
-  // 128 threads per front, so that shared memory and registers (not the
-  // thread count) bound the fronts in flight per SM (measured faster than 256
-  // on the 2,000-system batch, both variants)
-  if (nf_max > 64) k_small_front<T, true><<<count, 128, sm, st>>>(F, list, a, panel, upool, info);
-  else k_small_front<T, false><<<count, 128, sm, st>>>(F, list, a, panel, upool, info);
-}
 template <typename T>
 void launch_zero_large(const DevFronts& F, const int32_t* list, int count, int64_t max_cols, T* panel, T* upool,
                        cudaStream_t st) {
@@ -2202,31 +1586,6 @@ int launch_update(const DevFronts& F, const int32_t* list, int count, int step, 
   return 1;
 }
 
-// one launch per size bin (nf_max <= 32 R, R <= kSmallFrontMax / 32 = 4)
-template <typename T>
-void launch_fwd_small(const DevFronts& F, const int32_t* list, int count, int nf_max, const T* panel, T* X,
-                      int64_t ldx, T* V, int nrhs, cudaStream_t st) {
-  if (count <= 0) return;
-  const dim3 grid(ceil_div(count, kSWarps), nrhs >= kMrhsMin ? nrhs : 1), block(kSWarps * 32);
-  switch (ceil_div(nf_max, 32)) {
-    case 1: k_fwd_small<T, 1><<<grid, block, 0, st>>>(F, list, count, panel, X, ldx, V, nrhs); break;
-    case 2: k_fwd_small<T, 2><<<grid, block, 0, st>>>(F, list, count, panel, X, ldx, V, nrhs); break;
-    case 3: k_fwd_small<T, 3><<<grid, block, 0, st>>>(F, list, count, panel, X, ldx, V, nrhs); break;
-    default: k_fwd_small<T, 4><<<grid, block, 0, st>>>(F, list, count, panel, X, ldx, V, nrhs); break;
-  }
-}
-template <typename T>
-void launch_bwd_small(const DevFronts& F, const int32_t* list, int count, int nf_max, const T* panel, T* X,
-                      int64_t ldx, int nrhs, cudaStream_t st) {
-  if (count <= 0) return;
-  const dim3 grid(ceil_div(count, kSWarps), nrhs >= kMrhsMin ? nrhs : 1), block(kSWarps * 32);
-  switch (ceil_div(nf_max, 32)) {
-    case 1: k_bwd_small<T, 1><<<grid, block, 0, st>>>(F, list, count, panel, X, ldx, nrhs); break;
-    case 2: k_bwd_small<T, 2><<<grid, block, 0, st>>>(F, list, count, panel, X, ldx, nrhs); break;
-    case 3: k_bwd_small<T, 3><<<grid, block, 0, st>>>(F, list, count, panel, X, ldx, nrhs); break;
-    default: k_bwd_small<T, 4><<<grid, block, 0, st>>>(F, list, count, panel, X, ldx, nrhs); break;
-  }
-}
 // a warp per right-hand side once the level's CTAs of eight still fill the chip (below, the
 // long fronts of a small level want a CTA each)
 bool gather_by_warp(int count, int nrhs) { return nrhs > 1 && (int64_t)count * ceil_div(nrhs, kGatherRhs) >= 2 * kNumSms; }
@@ -2379,18 +1738,12 @@ void launch_remap_int(const int32_t* map, int32_t* a, int64_t n, cudaStream_t st
 }
 
 #define MFD_INSTANTIATE(T)                                                                                          \
-  template void launch_small_fronts<T>(const DevFronts&, const int32_t*, int, int, const double*, T*, T*, int32_t*, \
-                                       cudaStream_t);                                                              \
   template void launch_zero_large<T>(const DevFronts&, const int32_t*, int, int64_t, T*, T*, cudaStream_t);         \
   template void launch_assemble_large<T>(const DevFronts&, const int32_t*, int, int, const double*, T*,             \
                                          cudaStream_t);                                                            \
   template void launch_extend_add<T>(const DevFronts&, const int32_t*, int, int, T*, T*, cudaStream_t);             \
   template int launch_update<T>(const DevFronts&, const int32_t*, int, int, int, int, T*, T*, int, cudaStream_t,    \
                                  UpdBand, int, bool);                                                              \
-  template void launch_fwd_small<T>(const DevFronts&, const int32_t*, int, int, const T*, T*, int64_t, T*, int,    \
-                                    cudaStream_t);                                                                 \
-  template void launch_bwd_small<T>(const DevFronts&, const int32_t*, int, int, const T*, T*, int64_t, int,         \
-                                    cudaStream_t);                                                                 \
   template void launch_fwd_large<T>(const DevFronts&, const int32_t*, int, int, int, const T*, const T*, T*,       \
                                     int64_t, T*, int32_t*, int, cudaStream_t, int64_t*, bool, bool);               \
   template void launch_bwd_large<T>(const DevFronts&, const int32_t*, int, int, int, const T*, const T*, T*,       \

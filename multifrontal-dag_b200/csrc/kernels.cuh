@@ -114,14 +114,19 @@ void launch_local_index(const DevFronts& F, int32_t* local, int num_front, cudaS
 void launch_assembly_map(const DevFronts& F, const int32_t* col_front, const int32_t* acol_ptr, const int32_t* arow,
                          const int32_t* ccs_src, int32_t* sidx, int32_t* a_src, int32_t* a_pos, int n_total,
                          cudaStream_t st);
+void launch_records(const DevFronts& F, const int32_t* lists, int list_len, FrontRec* rec, int num_child,
+                    ChildRec* crec, cudaStream_t st);
 void launch_bli_count(const DevFronts& F, const int32_t* fronts, int count, int nb, int32_t* groups, cudaStream_t st);
 void launch_bli_fill(const DevFronts& F, const int32_t* fronts, int count, int nb, const int32_t* group_base,
                      const int32_t* index_base, int32_t* block_ptr, int32_t* pnum, int32_t* cnum, int32_t* offset,
                      int32_t* rebuilt, cudaStream_t st);
 
 // ---- factorization -----------------------------------------------------------
+// One size bin of a level's small fronts (nf <= nf_max <= kSmallFrontMax), small_front.cu; rec: the
+// bin's records.
+cudaError_t prepare_small_fronts();
 template <typename T>
-void launch_small_fronts(const DevFronts& F, const int32_t* list, int count, int nf_max, const double* a, T* panel,
+void launch_small_fronts(const DevFronts& F, const FrontRec* rec, int count, int nf_max, const double* a, T* panel,
                          T* upool, int32_t* info, cudaStream_t st);
 template <typename T>
 void launch_zero_large(const DevFronts& F, const int32_t* list, int count, int64_t max_cols, T* panel, T* upool,
@@ -199,15 +204,16 @@ int launch_update_tcq(const DevFronts& F, const int32_t* list, int count, int st
 int update_grid(int T, int tw, UpdBand band);
 
 // ---- solves --------------------------------------------------------------------
-// Small fronts (one size bin, nf <= nf_max <= kSmallFrontMax): one warp per front.
+// Small fronts (nf <= nf_max <= kSmallFrontMax), small_solve.cu; panel_elems: the most (nf | 1) nc of the list.
+cudaError_t prepare_small_solve();
 template <typename T>
-void launch_fwd_small(const DevFronts& F, const int32_t* list, int count, int nf_max, const T* panel, T* X,
-                      int64_t ldx, T* V, int nrhs, cudaStream_t st);
+void launch_fwd_small(const DevFronts& F, const FrontRec* rec, int count, int nf_max, int panel_elems, const T* panel,
+                      T* X, int64_t ldx, T* V, int nrhs, cudaStream_t st);
 template <typename T>
-void launch_bwd_small(const DevFronts& F, const int32_t* list, int count, int nf_max, const T* panel, T* X,
-                      int64_t ldx, int nrhs, cudaStream_t st);
+void launch_bwd_small(const DevFronts& F, const FrontRec* rec, int count, int nf_max, int panel_elems, const T* panel,
+                      T* X, int64_t ldx, int nrhs, cudaStream_t st);
 // Large fronts: dinv holds the inverted 128 x 128 diagonal blocks the factorization kept (DevFronts::d_off).
-// fused: only the gather runs here (single right-hand side; launch_large_fused does the steps)
+// fused: only the gather runs here (launch_large_fused or launch_large_multi does the steps)
 template <typename T>
 void launch_fwd_large(const DevFronts& F, const int32_t* list, int count, int max_nc, int max_nf, const T* panel,
                       const T* dinv, T* X, int64_t ldx, T* V, int32_t* cnt, int nrhs, cudaStream_t st,

@@ -16,6 +16,19 @@
 
 namespace mfd {
 
+// A front as the small-front kernels read it: one 64-byte record per entry of the launch lists.
+struct alignas(16) FrontRec {
+  int32_t nc, nr, first, lrow_off;
+  int32_t a_beg, a_end, child_beg, child_end;
+  int64_t panel_off, u_off;
+  int64_t v_off, pad;
+};
+// One record per entry of DevFronts::child.
+struct alignas(16) ChildRec {
+  int32_t nc, nr, lrow_off, pad;
+  int64_t u_off, v_off;
+};
+
 // Pointers into the device copies of the per-front tables (all 0-based).
 struct DevFronts {
   const int32_t* nc;          // supernode columns
@@ -24,6 +37,7 @@ struct DevFronts {
   const int32_t* parent;      // parent front, -1 for a root
   const int32_t* child_ptr;   // children of f: child[child_ptr[f] .. child_ptr[f+1])
   const int32_t* child;       // ascending (the reference's tree_child order)
+  const ChildRec* crec;       // the children's records, as child
   const int64_t* panel_off;   // element offset of the panel in the panel pool
   const int64_t* u_off;       // element offset of the update matrix in the update pool
   const int32_t* lrow_off;    // offset of f's L rows in lrow / local
@@ -52,12 +66,12 @@ struct LaunchList {          // a list of front ids in the device list pool
 };
 
 struct LevelPlan {
-  std::vector<LaunchList> small;     // fused one-CTA fronts, one list per size bin
+  std::vector<LaunchList> small;     // fused one-warp or one-CTA fronts, one list per size bin
+  std::vector<LaunchList> small_solve;   // the same for the solves: bins up to 32 rows in one list
   LaunchList large;                  // blocked fronts (sorted by nc descending)
   std::vector<LaunchList> ext_add;   // per child rank: children of large fronts
   std::vector<LaunchList> steps;     // per panel step: prefix of `large`; param = TRSM row blocks,
                                      // param2 = 128-tiles, param3 = 64-tiles of the trailing triangle
-  std::vector<LaunchList> solve_steps;
   // per panel step: how many fronts of the step's list (in order) need 4, 3, 2, 1
   // sub-blocks of 32 columns in the diagonal-block POTRF
   std::vector<std::array<int32_t, 4>> potrf_cls;
