@@ -193,6 +193,8 @@ struct mfd_handle {
   // backward tickets, then forward flags, backward flags and backward update-row counters,
   // one per front, panel step and RHS tile (zeroed before every solve)
   DBuf<int32_t> d_stasks, d_ssync;
+  DBuf<int32_t> d_inv;
+  DBuf<int64_t> d_inv_off;
   DBuf<FrontRec> d_rec;
   DBuf<ChildRec> d_crec;
   DBuf<int64_t> d_panel_off, d_u_off, d_v_off, d_s_off, d_d_off, d_q_off;
@@ -447,19 +449,16 @@ int build_plan(mfd_handle* h) {
     L.large.count = (int32_t)large.size();
     h->max_large_count = std::max(h->max_large_count, L.large.count);
     int max_entries = 0;
-    int64_t max_elems = 0;
     int max_nc = 0;
     for (int32_t g : large) {
       const HostFront& fr = h->fronts[g];
       int nf = fr.nc + fr.nr;
       max_entries = std::max(max_entries, h->h_a_beg[g + 1] - h->h_a_beg[g]);
-      max_elems = std::max<int64_t>(max_elems, nf);
       max_nc = std::max(max_nc, fr.nc);
       L.large_max_nf = std::max(L.large_max_nf, nf);
     }
     L.large.param = max_entries;
     L.large.param2 = max_nc;
-    L.large_zero_elems = max_elems;
     // packed operands of the FP32 tensor-core update: the level's large fronts side by side,
     // each with the 128-row blocks of its largest step (step 0); reused level after level
     {
@@ -471,24 +470,6 @@ int build_plan(mfd_handle* h) {
         q += (nrem + kFactB - 1) / kFactB * kPackedBlockElems;
       }
       h->q_elems = std::max(h->q_elems, q);
-    }
-    // extend-add by child rank
-    for (int rank = 0;; ++rank) {
-      std::vector<int32_t> kids;
-      int max_nr = 0;
-      for (int32_t g : large) {
-        int32_t t = h->h_child_ptr[g] + rank;
-        if (t < h->h_child_ptr[g + 1]) {
-          kids.push_back(h->h_child[t]);
-          max_nr = std::max(max_nr, h->fronts[h->h_child[t]].nr);
-        }
-      }
-      if (kids.empty()) break;
-      LaunchList ll;
-      ll.off = push_list(h, kids);
-      ll.count = (int32_t)kids.size();
-      ll.param = max_nr;
-      L.ext_add.push_back(ll);
     }
     // panel steps: prefix of the nc-sorted list
     int steps = (max_nc + kFactB - 1) / kFactB;
@@ -749,6 +730,29 @@ int upload_plan(mfd_handle* h) {
     }
   }
 
+  // the children of large fronts: the inverse of their local index
+  {
+    std::vector<int64_t> ioff(nfr, 0);
+    std::vector<int32_t> kids;
+    int64_t len = 0;
+    const int sfm = small_front_max(h);
+    for (int32_t g = 0; g < nfr; ++g) {
+      const int32_t p = h->fronts[g].parent;
+      if (p < 0 || h->fronts[p].nc + h->fronts[p].nr <= sfm) continue;
+      ioff[g] = len;
+      len += h->fronts[p].nc + h->fronts[p].nr;
+      kids.push_back(g);
+    }
+    CK(h->d_inv.alloc(len));
+    CK(h->d_inv_off.upload(ioff, st));
+    F.inv = h->d_inv.p;
+    F.inv_off = h->d_inv_off.p;
+    DBuf<int32_t> d_kids;
+    CK(d_kids.upload(kids, st));
+    launch_inverse_index(F, d_kids.p, (int)kids.size(), h->d_inv.p, st);
+    CK(cudaStreamSynchronize(st));       // d_kids and the host tables go out of scope
+  }
+
   h->setup_s[2] = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   t0 = std::chrono::steady_clock::now();
   // permuted full CSR (both triangles) for residuals
@@ -947,30 +951,24 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
       if (nside) side_join(h, st, nside);
       continue;
     }
-    double zb = 0, ab = 0;
+    double gf = 0, gb = 0, ab = 0;
     if (prof)
       for (int i = 0; i < L.large.count; ++i) {
-        const HostFront& f = h->fronts[hl[L.large.off + i]];
-        zb += w * ((double)(f.nc + f.nr) * f.nc - (double)f.nc * (f.nc - 1) / 2 + (double)f.nr * (f.nr + 1) / 2);
-        ab += 12.0 * (h->h_a_beg[hl[L.large.off + i] + 1] - h->h_a_beg[hl[L.large.off + i]]);
-      }
-    record(h, st, MFD_K_ZERO, 0, zb,
-           [&] { launch_zero_large<T>(F, lists + L.large.off, L.large.count, L.large_zero_elems, panel, upool, st); });
-    record(h, st, MFD_K_ASSEMBLE, 0, ab,
-           [&] { launch_assemble_large<T>(F, lists + L.large.off, L.large.count, L.large.param, a, panel, st); });
-    n += 2;
-    for (const LaunchList& e : L.ext_add) {
-      double fl = 0, by = 0;
-      if (prof)
-        for (int i = 0; i < e.count; ++i) {
-          double c = h->fronts[hl[e.off + i]].nr;
-          fl += c * (c + 1) / 2;
-          by += 3 * w * c * (c + 1) / 2 + 4.0 * c;
+        const int32_t g = hl[L.large.off + i];
+        const HostFront& f = h->fronts[g];
+        gb += w * ((double)(f.nc + f.nr) * f.nc - (double)f.nc * (f.nc - 1) / 2 + (double)f.nr * (f.nr + 1) / 2);
+        for (int32_t t = h->h_child_ptr[g]; t < h->h_child_ptr[g + 1]; ++t) {
+          const double c = h->fronts[h->h_child[t]].nr;
+          gf += c * (c + 1) / 2;
+          gb += w * c * (c + 1) / 2 + 4.0 * c;
         }
-      record(h, st, MFD_K_EXTEND_ADD, fl, by,
-             [&] { launch_extend_add<T>(F, lists + e.off, e.count, e.param, panel, upool, st); });
-      ++n;
-    }
+        ab += 12.0 * (h->h_a_beg[g + 1] - h->h_a_beg[g]);
+      }
+    record(h, st, MFD_K_EXTEND_ADD, gf, gb,
+           [&] { launch_build_large<T>(F, lists + L.large.off, L.large.count, L.large_max_nf, panel, upool, st); });
+    record(h, st, MFD_K_ASSEMBLE, 0, ab,
+           [&] { launch_assemble_large<T>(F, lists + L.large.off, L.large.count, L.large.param, a, panel, upool, st); });
+    n += 2;
     // Lookahead (on unless reserved[1] = 1; profiling runs the serial schedule so
     // that every kernel is timed alone) with deferred updates (groups of D =
     // h->defer panel steps, update_k_range): after the TRSM of step s the next

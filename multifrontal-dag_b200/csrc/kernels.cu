@@ -221,103 +221,104 @@ __global__ void k_bli_fill(DevFronts F, const int32_t* fronts, int count, int nb
 // factorization
 // ============================================================================
 
-// Zero the lower triangles of a large front's panel (nf x nc) and update
-// matrix (nr x nr): one warp per column, grid-stride over columns.
+// Inverse of a child's local index: for every position of the parent front the
+// child's row there, or -1 (children of large fronts, at F.inv_off).
+__global__ void k_inverse_index(DevFronts F, const int32_t* kids, int32_t* inv) {
+  const int c = kids[blockIdx.x], p = F.parent[c];
+  const int nfp = F.nc[p] + F.nr[p], nrc = F.nr[c];
+  int32_t* v = inv + F.inv_off[c];
+  for (int i = threadIdx.x; i < nfp; i += blockDim.x) v[i] = -1;
+  __syncthreads();
+  const int32_t* loc = F.local + F.lrow_off[c];
+  for (int i = threadIdx.x; i < nrc; i += blockDim.x) v[loc[i] - 1] = i;
+}
+
+// Extend-add of a level's large fronts, gathered: every lower entry of a
+// front's panel and update matrix is written once, as the sum of its children's
+// entries there in child order (zero where no child has one; more than two
+// children are taken two at a time).  A warp takes the column pair (j, nf-1-j),
+// nf + 1 entries whatever j, lanes over rows, four rows of two children in
+// flight; a child without column j costs nothing.
+// What bounds it is HBM: per entry two reads and one write, where zeroing and
+// one scatter launch per child rank moved seven (64^3 Laplacian, FP64: 6.5 ms
+// a factorization in 78 launches).
 template <typename T>
-__global__ void k_zero_large(DevFronts F, const int32_t* list, T* panel, T* upool) {
+__global__ void __launch_bounds__(256) k_gather_children(DevFronts F, const int32_t* list, T* panel, T* upool) {
+  constexpr int U = 4;
   const int f = list[blockIdx.y];
   const int nc = F.nc[f], nr = F.nr[f], nf = nc + nr;
   T* P = panel + F.panel_off[f];
-  T* U = upool + F.u_off[f];
-  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int j = blockIdx.x * nw + (threadIdx.x >> 5); j < nc + nr; j += gridDim.x * nw) {
-    if (j < nc) {
-      T* col = P + (size_t)j * nf;
-      for (int i = j + lane; i < nf; i += 32) col[i] = T(0);
-    } else {
-      const int jj = j - nc;
-      T* col = U + (size_t)jj * nr;
-      for (int i = jj + lane; i < nr; i += 32) col[i] = T(0);
-    }
-  }
-}
-
-template <typename T>
-__global__ void k_assemble_large(DevFronts F, const int32_t* list, const double* __restrict__ a, T* panel) {
-  const int f = list[blockIdx.y];
-  T* P = panel + F.panel_off[f];
-  for (int k = F.a_beg[f] + blockIdx.x * blockDim.x + threadIdx.x; k < F.a_beg[f + 1]; k += gridDim.x * blockDim.x)
-    P[F.a_pos[k]] = T(a[F.a_src[k]]);
-}
-
-// Extend-add of one child per parent (children of one rank, so no two CTAs of a
-// launch write the same parent entry): warp per child column, lanes over rows.
-template <typename T>
-__global__ void __launch_bounds__(256) k_extend_add(DevFronts F, const int32_t* list, T* panel, T* upool) {
-  const int c = list[blockIdx.y];
-  const int p = F.parent[c];
-  const int nrc = F.nr[c];
-  const int ncp = F.nc[p], nrp = F.nr[p], nfp = ncp + nrp;
-  const T* __restrict__ Uc = upool + F.u_off[c];
-  T* Pp = panel + F.panel_off[p];
-  T* Up = upool + F.u_off[p];
-  const int32_t* __restrict__ loc = F.local + F.lrow_off[c];
+  T* Uf = upool + F.u_off[f];
+  const int cb = F.child_ptr[f], ce = F.child_ptr[f + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int j = blockIdx.x * nw + warp; j < nrc; j += gridDim.x * nw) {
-    const int lj = loc[j] - 1;
-    const T* src = Uc + (size_t)j * nrc;
-    if (lj < ncp) {
-      T* dst = Pp + (size_t)lj * nfp;
-      for (int i = j + lane; i < nrc; i += 32) dst[loc[i] - 1] += src[i];
-    } else {
-      T* dst = Up + (size_t)(lj - ncp) * nrp - ncp;
-      for (int i = j + lane; i < nrc; i += 32) dst[loc[i] - 1] += src[i];
-    }
-  }
-}
-
-// FP32 form: warps take column pairs (j, nrc-1-j), nrc + 1 entries per pair,
-// lanes over rows with four rows per lane in flight (the source and
-// local-index reads, then the parent reads, then the stores).  Measured on the
-// 64^3 Laplacian: FP32 4.1 -> 2.9 ms per factorization; for FP64 (twice the
-// bytes per entry, already near the bandwidth the scatter reaches) the same
-// scheme was slower (5.0 -> 5.6 ms), so FP64 keeps the kernel above.
-template <typename T>
-__global__ void __launch_bounds__(256) k_extend_add_ilp(DevFronts F, const int32_t* list, T* panel, T* upool) {
-  const int c = list[blockIdx.y];
-  const int p = F.parent[c];
-  const int nrc = F.nr[c];
-  const int ncp = F.nc[p], nrp = F.nr[p], nfp = ncp + nrp;
-  const T* __restrict__ Uc = upool + F.u_off[c];
-  T* Pp = panel + F.panel_off[p];
-  T* Up = upool + F.u_off[p];
-  const int32_t* __restrict__ loc = F.local + F.lrow_off[c];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int ntask = (nrc + 1) / 2;
-  for (int q = blockIdx.x * nw + warp; q < ntask; q += gridDim.x * nw) {
+  const int pairs = (nf + 1) / 2;
+  for (int q = blockIdx.x * nw + warp; q < pairs; q += gridDim.x * nw) {
 #pragma unroll 1
     for (int hh = 0; hh < 2; ++hh) {
-      const int j = hh ? nrc - 1 - q : q;
+      const int j = hh ? nf - 1 - q : q;
       if (hh && j == q) break;
-      const int lj = __ldg(&loc[j]) - 1;
-      const T* src = Uc + (size_t)j * nrc;
-      T* dst = lj < ncp ? Pp + (size_t)lj * nfp : Up + (size_t)(lj - ncp) * nrp - ncp;
-      for (int i0 = j + lane; i0 < nrc; i0 += 128) {
-        int li[4];
-        T v[4], d[4];
+      T* dst = j < nc ? P + (size_t)j * nf : Uf + (size_t)(j - nc) * nr - nc;   // entry (i, j) at dst[i]
+#pragma unroll 1
+      for (int t0 = cb; t0 == cb || t0 < ce; t0 += 2) {
+        const int32_t* iv[2] = {nullptr, nullptr};
+        const T* col[2] = {nullptr, nullptr};
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int i = i0 + 32 * u;
-          v[u] = i < nrc ? src[i] : T(0);
-          li[u] = i < nrc ? __ldg(&loc[i]) - 1 : -1;
+        for (int s = 0; s < 2; ++s)
+          if (t0 + s < ce) {
+            const int c = F.child[t0 + s];
+            const int32_t* v = F.inv + F.inv_off[c];
+            const int cj = v[j];
+            if (cj >= 0) {
+              iv[s] = v;
+              col[s] = upool + F.u_off[c] + (size_t)cj * F.nr[c];
+            }
+          }
+        const bool first = t0 == cb;
+        if (!first && iv[0] == nullptr && iv[1] == nullptr) continue;
+        for (int i0 = j + lane; i0 < nf; i0 += 32 * U) {
+          int ci[2][U];
+          T x[2][U], d[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int i = i0 + 32 * u;
+#pragma unroll
+            for (int s = 0; s < 2; ++s) ci[s][u] = iv[s] != nullptr && i < nf ? __ldg(iv[s] + i) : -1;
+            d[u] = !first && i < nf ? dst[i] : T(0);
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int s = 0; s < 2; ++s) x[s][u] = ci[s][u] >= 0 ? col[s][ci[s][u]] : T(0);
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int i = i0 + 32 * u;
+            if (i < nf) dst[i] = (d[u] + x[0][u]) + x[1][u];
+          }
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) d[u] = li[u] >= 0 ? dst[li[u]] : T(0);
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (li[u] >= 0) dst[li[u]] = d[u] + v[u];
       }
     }
+  }
+}
+
+// A's entries of the large fronts, each with its children's contributions on
+// top (A first, then the children in order): written over what the gather put
+// there, so that an entry of A is set, not added.
+template <typename T>
+__global__ void k_assemble_large(DevFronts F, const int32_t* list, const double* __restrict__ a, T* panel,
+                                 const T* __restrict__ upool) {
+  const int f = list[blockIdx.y];
+  const int nf = F.nc[f] + F.nr[f], cb = F.child_ptr[f], ce = F.child_ptr[f + 1];
+  T* P = panel + F.panel_off[f];
+  for (int k = F.a_beg[f] + blockIdx.x * blockDim.x + threadIdx.x; k < F.a_beg[f + 1]; k += gridDim.x * blockDim.x) {
+    const int pos = F.a_pos[k], j = pos / nf, i = pos - j * nf;
+    T v = T(a[F.a_src[k]]);
+    for (int t = cb; t < ce; ++t) {
+      const int c = F.child[t];
+      const int32_t* iv = F.inv + F.inv_off[c];
+      const int cj = iv[j], ci = iv[i];
+      if (cj >= 0 && ci >= 0) v += upool[F.u_off[c] + ci + (size_t)cj * F.nr[c]];
+    }
+    P[pos] = v;
   }
 }
 
@@ -1518,31 +1519,23 @@ void launch_bli_fill(const DevFronts& F, const int32_t* fronts, int count, int n
                                                      cnum, offset, rebuilt);
 }
 
+void launch_inverse_index(const DevFronts& F, const int32_t* kids, int count, int32_t* inv, cudaStream_t st) {
+  if (count > 0) k_inverse_index<<<count, 128, 0, st>>>(F, kids, inv);
+}
 template <typename T>
-void launch_zero_large(const DevFronts& F, const int32_t* list, int count, int64_t max_cols, T* panel, T* upool,
-                       cudaStream_t st) {
+void launch_build_large(const DevFronts& F, const int32_t* list, int count, int max_nf, T* panel, T* upool,
+                        cudaStream_t st) {
   if (count <= 0) return;
-  dim3 grid(clamp_grid(ceil_div(max_cols, 8), 512), count);
-  k_zero_large<T><<<grid, 256, 0, st>>>(F, list, panel, upool);
+  // one warp per column pair of the largest front, at most 1,024 CTAs per front
+  const int gx = std::max(1, std::min(ceil_div((max_nf + 1) / 2, 8), 1024));
+  k_gather_children<T><<<dim3(gx, count), 256, 0, st>>>(F, list, panel, upool);
 }
 template <typename T>
 void launch_assemble_large(const DevFronts& F, const int32_t* list, int count, int max_entries, const double* a,
-                           T* panel, cudaStream_t st) {
+                           T* panel, const T* upool, cudaStream_t st) {
   if (count <= 0) return;
   dim3 grid(clamp_grid(ceil_div(max_entries, 256), 256), count);
-  k_assemble_large<T><<<grid, 256, 0, st>>>(F, list, a, panel);
-}
-template <typename T>
-void launch_extend_add(const DevFronts& F, const int32_t* list, int count, int max_nr, T* panel, T* upool,
-                       cudaStream_t st) {
-  if (count <= 0) return;
-  if constexpr (sizeof(T) == 4) {   // one warp per column pair of the largest child, at most 1,024 CTAs per child
-    const int gx = std::max(1, std::min(ceil_div((max_nr + 1) / 2, 8), 1024));
-    k_extend_add_ilp<T><<<dim3(gx, count), 256, 0, st>>>(F, list, panel, upool);
-    return;
-  }
-  dim3 grid(clamp_grid(ceil_div(max_nr, 8), 1024), count);
-  k_extend_add<T><<<grid, 256, 0, st>>>(F, list, panel, upool);
+  k_assemble_large<T><<<grid, 256, 0, st>>>(F, list, a, panel, upool);
 }
 int update_grid(int T, int tw, UpdBand band) {
   const int c1 = kFactB / tw, jlo = band.blo * c1;
@@ -1738,10 +1731,9 @@ void launch_remap_int(const int32_t* map, int32_t* a, int64_t n, cudaStream_t st
 }
 
 #define MFD_INSTANTIATE(T)                                                                                          \
-  template void launch_zero_large<T>(const DevFronts&, const int32_t*, int, int64_t, T*, T*, cudaStream_t);         \
-  template void launch_assemble_large<T>(const DevFronts&, const int32_t*, int, int, const double*, T*,             \
+  template void launch_build_large<T>(const DevFronts&, const int32_t*, int, int, T*, T*, cudaStream_t);            \
+  template void launch_assemble_large<T>(const DevFronts&, const int32_t*, int, int, const double*, T*, const T*,   \
                                          cudaStream_t);                                                            \
-  template void launch_extend_add<T>(const DevFronts&, const int32_t*, int, int, T*, T*, cudaStream_t);             \
   template int launch_update<T>(const DevFronts&, const int32_t*, int, int, int, int, T*, T*, int, cudaStream_t,    \
                                  UpdBand, int, bool);                                                              \
   template void launch_fwd_large<T>(const DevFronts&, const int32_t*, int, int, int, const T*, const T*, T*,       \

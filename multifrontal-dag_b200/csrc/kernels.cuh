@@ -128,15 +128,15 @@ cudaError_t prepare_small_fronts();
 template <typename T>
 void launch_small_fronts(const DevFronts& F, const FrontRec* rec, int count, int nf_max, const double* a, T* panel,
                          T* upool, int32_t* info, cudaStream_t st);
+// A level's large fronts before their panel steps: build writes every lower entry as the sum of
+// the children's (max_nf: the largest front), assemble then sets A's entries on top.
+void launch_inverse_index(const DevFronts& F, const int32_t* kids, int count, int32_t* inv, cudaStream_t st);
 template <typename T>
-void launch_zero_large(const DevFronts& F, const int32_t* list, int count, int64_t max_cols, T* panel, T* upool,
-                       cudaStream_t st);
+void launch_build_large(const DevFronts& F, const int32_t* list, int count, int max_nf, T* panel, T* upool,
+                        cudaStream_t st);
 template <typename T>
 void launch_assemble_large(const DevFronts& F, const int32_t* list, int count, int max_entries, const double* a,
-                           T* panel, cudaStream_t st);
-template <typename T>
-void launch_extend_add(const DevFronts& F, const int32_t* list, int count, int max_nr, T* panel, T* upool,
-                       cudaStream_t st);
+                           T* panel, const T* upool, cudaStream_t st);
 // Panel step s of the blocked large-front factorization (columns s*kFactB ..), panel.cu:
 //   potrf  : one CTA per front; L11 into the panel and, in packed 8 x 8 blocks with the diagonal
 //            ones inverted, into list slot i's kPackedPanelElems doubles of `packed`

@@ -43,6 +43,8 @@ struct DevFronts {
   const int32_t* lrow_off;    // offset of f's L rows in lrow / local
   const int32_t* lrow;        // L rows, global permuted 0-based
   const int32_t* local;       // reference local_index values (1-based positions in the parent front)
+  const int32_t* inv;         // children of large fronts: the child's row at every position of the parent, or -1
+  const int64_t* inv_off;     // offset of a child's part of inv
   const int32_t* a_beg;       // entries of A assembled into f: [a_beg[f], a_beg[f+1])
   const int32_t* a_src;       // per A entry: index into the caller's value array
   const int32_t* a_pos;       // per A entry: row + col*nf inside the front
@@ -69,7 +71,6 @@ struct LevelPlan {
   std::vector<LaunchList> small;     // fused one-warp or one-CTA fronts, one list per size bin
   std::vector<LaunchList> small_solve;   // the same for the solves: bins up to 32 rows in one list
   LaunchList large;                  // blocked fronts (sorted by nc descending)
-  std::vector<LaunchList> ext_add;   // per child rank: children of large fronts
   std::vector<LaunchList> steps;     // per panel step: prefix of `large`; param = TRSM row blocks,
                                      // param2 = 128-tiles, param3 = 64-tiles of the trailing triangle
   // per panel step: how many fronts of the step's list (in order) need 4, 3, 2, 1
@@ -79,7 +80,6 @@ struct LevelPlan {
   // in the solve task pool, forward and backward
   LaunchList fwd_tasks, bwd_tasks;
   int32_t large_max_nf = 0;
-  int64_t large_zero_elems = 0;
 };
 
 }  // namespace mfd
