@@ -180,6 +180,7 @@ struct mfd_handle {
   int32_t solve_flags = 0;                          // per front and panel step, one sweep's worth
   int64_t bw_part_elems = 0;                        // backward sweep partial sums, largest level
   void* d_bwpart = nullptr;                         // T, the backward sweep's partial sums
+  void* d_exch = nullptr;                           // single-RHS sweeps: n_total exchange entries of 2 sizeof(T)
   std::vector<int> small_bins;
   int64_t panel_elems = 0, upool_elems = 0, v_elems = 0, s_elems = 0, dinv_elems = 0;
   int64_t q_elems = 0;                              // packed FP32 update operands of one step parity
@@ -192,7 +193,7 @@ struct mfd_handle {
   // fused solve: the tasks, and [0] expiry flag, [1 + 2 l] / [2 + 2 l] level l's forward /
   // backward tickets, then forward flags, backward flags and backward update-row counters,
   // one per front, panel step and RHS tile (zeroed before every solve)
-  DBuf<int32_t> d_stasks, d_ssync;
+  DBuf<int32_t> d_stasks, d_ssync, d_epoch;
   DBuf<int32_t> d_inv;
   DBuf<int64_t> d_inv_off;
   DBuf<FrontRec> d_rec;
@@ -250,7 +251,7 @@ struct mfd_handle {
     for (auto& kv : g_solve) cudaGraphExecDestroy(kv.second);
     for (auto& kv : g_ir) cudaGraphExecDestroy(kv.second);
     if (bst) cudaStreamDestroy(bst);
-    for (void* p : {d_panel, d_upool, d_diag, d_X, d_V, d_S, static_cast<void*>(d_q), static_cast<void*>(d_packed), d_bwpart})
+    for (void* p : {d_panel, d_upool, d_diag, d_X, d_V, d_S, static_cast<void*>(d_q), static_cast<void*>(d_packed), d_bwpart, d_exch})
       if (p) cudaFree(p);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
@@ -605,10 +606,7 @@ int upload_plan(mfd_handle* h) {
   F.a_src = h->d_a_src.p; F.a_pos = h->d_a_pos.p; F.v_off = h->d_v_off.p; F.s_off = h->d_s_off.p;
   F.d_off = h->d_d_off.p;
   F.q_off = h->d_q_off.p;
-  CK(h->d_rec.alloc(h->h_lists.size()));
-  CK(h->d_crec.alloc(h->h_child.size()));
-  F.crec = h->d_crec.p;
-  launch_records(F, h->d_lists.p, (int)h->h_lists.size(), h->d_rec.p, (int)h->h_child.size(), h->d_crec.p, st);
+
 
   // permuted global A structure, value sources, front of every column
   std::vector<int32_t> acol(h->n_total + 1), arow(h->nnz_total), src(h->nnz_total), colf(h->n_total),
@@ -750,6 +748,10 @@ int upload_plan(mfd_handle* h) {
     DBuf<int32_t> d_kids;
     CK(d_kids.upload(kids, st));
     launch_inverse_index(F, d_kids.p, (int)kids.size(), h->d_inv.p, st);
+    CK(h->d_rec.alloc(h->h_lists.size()));
+    CK(h->d_crec.alloc(h->h_child.size()));
+    F.crec = h->d_crec.p;
+    launch_records(F, h->d_lists.p, (int)h->h_lists.size(), h->d_rec.p, (int)h->h_child.size(), h->d_crec.p, st);
     CK(cudaStreamSynchronize(st));       // d_kids and the host tables go out of scope
   }
 
@@ -820,6 +822,12 @@ int ensure_rhs(mfd_handle* h, int nrhs) {
   size_t esz = h->fp32 ? sizeof(float) : sizeof(double);
   for (void** p : {&h->d_X, &h->d_V, &h->d_S, &h->d_bwpart})
     if (*p) { cudaFree(*p); *p = nullptr; }
+  if (!h->d_exch && solve_fused(h, 1)) {
+    CK(cudaMalloc(&h->d_exch, (size_t)h->n_total * 2 * esz));
+    CK(cudaMemsetAsync(h->d_exch, 0, (size_t)h->n_total * 2 * esz, h->st));
+    CK(h->d_epoch.alloc(1));
+    CK(cudaMemsetAsync(h->d_epoch.p, 0, sizeof(int32_t), h->st));
+  }
   int widest = nrhs;                        // the most right-hand sides up to nrhs that take the fused sweeps
   while (widest > 1 && !solve_fused(h, widest)) --widest;
   CK(h->d_ssync.alloc(solve_sync_ints(h, solve_fused(h, widest) ? widest : 1)));
@@ -1147,7 +1155,7 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
   const int64_t nflags = h->solve_flags * multi_tiles(nrhs);
   int32_t* bwd_flags = fwd_flags + nflags;
   if (fused) {                              // a kernel, not a memset node: this also runs in the refinement loop's body
-    launch_fill_int(ssync, 0, solve_sync_ints(h, nrhs), st);
+    launch_solve_begin(ssync, solve_sync_ints(h, nrhs), h->d_epoch.p, st);
     ++n;
   }
   // a level's fused sweep
@@ -1157,8 +1165,8 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
     int32_t* flags = backward ? bwd_flags : fwd_flags;
     T* part = static_cast<T*>(h->d_bwpart);
     if (nrhs == 1)
-      launch_large_fused<T>(F, stasks + tl.off, tl.count, backward, ticket, flags, ssync, panel, dinv, X, V, st,
-                            h->d_info.p + 2, part, bwd_flags + nflags);
+      launch_large_fused<T>(F, stasks + tl.off, tl.count, backward, ticket, ssync, h->d_epoch.p, panel, dinv, X, V,
+                            h->d_exch, st, h->d_info.p + 2, part, bwd_flags + nflags);
     else
       launch_large_multi<T>(F, stasks + tl.off, tl.count, backward, ticket, flags, ssync, panel, dinv, X, ldx, V, nrhs, st,
                             h->d_info.p + 2, part, bwd_flags + nflags);
@@ -1197,9 +1205,10 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
       double fl = 0, by = 0;
       work(L.large, fl, by);
       record(h, st, MFD_K_SOLVE_LARGE, fl, by, [&] {
-        launch_fwd_large<T>(F, lists + L.large.off, L.large.count, L.large.param2, L.large_max_nf, panel, dinv, X,
-                            ldx, V, h->d_cnt.p, nrhs, st, &n, solve_pdl, fused);
         if (fused) sweep(L, false);
+        else
+          launch_fwd_large<T>(F, lists + L.large.off, L.large.count, L.large.param2, L.large_max_nf, panel, dinv, X, ldx,
+                              V, h->d_cnt.p, nrhs, st, &n, solve_pdl);
       });
     }
     if (nside) side_join(h, st, nside);
@@ -1221,9 +1230,10 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
       double fl = 0, by = 0;
       work(L.large, fl, by);
       record(h, st, MFD_K_SOLVE_LARGE, fl, by, [&] {
-        launch_bwd_large<T>(F, lists + L.large.off, L.large.count, L.large.param2, L.large_max_nf, panel, dinv, X,
-                            ldx, V, S, h->d_cnt.p, nrhs, st, &n, solve_pdl, fused);
         if (fused) sweep(L, true);
+        else
+          launch_bwd_large<T>(F, lists + L.large.off, L.large.count, L.large.param2, L.large_max_nf, panel, dinv, X, ldx,
+                              V, S, h->d_cnt.p, nrhs, st, &n, solve_pdl);
       });
     }
     if (nside) side_join(h, st, nside);

@@ -24,7 +24,6 @@
 
 #include "chol_smem.cuh"
 #include "kernels.cuh"
-#include "sweep_sync.cuh"
 
 namespace mfd {
 
@@ -161,7 +160,7 @@ __global__ void k_child_records(DevFronts F, int n, ChildRec* rec) {
   const int c = F.child[k];
   ChildRec r;
   r.nc = F.nc[c]; r.nr = F.nr[c]; r.lrow_off = F.lrow_off[c]; r.pad = 0;
-  r.u_off = F.u_off[c]; r.v_off = F.v_off[c];
+  r.u_off = F.u_off[c]; r.v_off = F.v_off[c]; r.inv_off = F.inv_off[c]; r.pad2 = 0;
   rec[k] = r;
 }
 
@@ -771,19 +770,17 @@ __device__ void fwd_diag_cta(const DevFronts& F, int f, int step, int slot, cons
 template <typename T>
 __global__ void __launch_bounds__(256) k_fwd_large_gather(DevFronts F, const int32_t* list,
                                                           const T* __restrict__ dinv, T* X, int64_t ldx, T* V,
-                                                          int nrhs, int diag0) {
+                                                          int nrhs) {
   __shared__ T vs[kSolveB * kRhsG];
   __shared__ T hs[kSolveB * kRhsG];
   const int f = list[blockIdx.x];
   const int nc = F.nc[f], nf = nc + F.nr[f], first = F.first[f];
   T* Vbase = V + F.v_off[f] * nrhs;
-  // one right-hand side per CTA when the grid has a y extent (many RHS)
-  const int rb = gridDim.y > 1 ? (int)blockIdx.y : 0, re = gridDim.y > 1 ? rb + 1 : nrhs;
   // loads batched kGU per thread (in flight together); each entry takes one
   // add per child, children in order
   constexpr int kGU = 4;
   const int nt = blockDim.x;
-  for (int r = rb; r < re; ++r) {
+  for (int r = 0; r < nrhs; ++r) {
     T* Vf = Vbase + (int64_t)r * nf;
     for (int i0 = threadIdx.x; i0 < nf; i0 += kGU * nt) {
       T xv[kGU];
@@ -820,7 +817,6 @@ __global__ void __launch_bounds__(256) k_fwd_large_gather(DevFronts F, const int
       __syncthreads();
     }
   }
-  if (!diag0) return;                                     // the fused sweep follows
   __threadfence_block();
   fwd_diag_cta(F, f, 0, blockIdx.x, dinv, X, ldx, Vbase, nf, nrhs, vs, hs);
 }
@@ -894,302 +890,14 @@ __global__ void __launch_bounds__(256) k_fwd_large_rest(DevFronts F, const int32
   if (threadIdx.x == 0) cnt[blockIdx.y] = 0;
 }
 
-// ---- single right-hand side: a level's large-front sweep in one launch ----------
-// The sweep is a list of tasks in dependency order: forward, for each panel step
-// s the diagonal-block task (f, s) of every front (y_s = Li (v_s - sum_{t<s}
-// L_st y_t)), then the rest-row tasks (128 rows below the front's columns each,
-// v_rest -= sum_t L_rest,t y_t); backward, for s from the last step down the
-// column-block task (f, s) of every front (x_s = Li^T (v_s - L_below,s^T
-// x_below)).  A CTA takes the next task from a ticket counter, so a task only
-// waits (on the per-front, per-step flags the producing tasks release) for
-// tasks that CTAs already running have taken: the sweep always progresses.
-// Every wait is bounded (~1 s); on expiry the CTA raises `expired` and stops
-// (the solve reports MFD_E_TIMEOUT).  Each task's sums have a fixed order, so
-// the sweep is deterministic.
-constexpr int kFuseRows = 128;                // rows of a forward rest task
-
-// forward: thread (row r0 + (t mod 128), half t / 128) sums its half of each
-// step's 128 columns; the step's 64 panel entries are loaded before the wait on
-// y_s (they do not depend on it)
-template <typename T>
-__global__ void __launch_bounds__(256) k_fwd_large_fused(DevFronts F, const int4* __restrict__ tasks, int ntask,
-                                                         int32_t* ticket, int32_t* flags, int32_t* expired,
-                                                         const T* __restrict__ panel, const T* __restrict__ dinv,
-                                                         T* X, T* V, const int32_t* test_req) {
-  __shared__ int sh_t, sh_ok;
-  __shared__ T ys[kSolveB];
-  __shared__ T part[kFuseRows];
-  if (threadIdx.x == 0) sh_t = atomicAdd(ticket, 1);
-  __syncthreads();
-  const int t = sh_t;
-  if (t >= ntask) return;
-  const int4 tk = tasks[t];
-  const int f = tk.x, code = tk.y;
-  int32_t* fl = flags + tk.z;
-  const bool probe = *test_req != 0;
-  const int nc = F.nc[f], nf = nc + F.nr[f];
-  const int r0 = code >= 0 ? code * kSolveB : nc + (-1 - code) * kFuseRows;
-  const int r1 = code >= 0 ? min(nc, r0 + kSolveB) : min(nf, r0 + kFuseRows);
-  const int nsteps = code >= 0 ? code : (nc + kSolveB - 1) / kSolveB;   // steps whose y this task consumes
-  const T* P = panel + F.panel_off[f];
-  T* Vf = V + F.v_off[f];
-  const int tid = threadIdx.x, ri = tid & (kFuseRows - 1), h = tid >> 7;
-  const int i = r0 + ri;
-  const bool valid = i < r1;
-  T acc = T(0);
-  for (int s = 0; s < nsteps; ++s) {
-    const int c0 = s * kSolveB, w = min(kSolveB, nc - c0);
-    T l[64];
-    const T* pc = P + (valid ? i : 0) + (size_t)(c0 + 64 * h) * nf;
-#pragma unroll
-    for (int k = 0; k < 64; ++k) l[k] = (valid && 64 * h + k < w) ? pc[(size_t)k * nf] : T(0);
-    if (!cta_wait_flag(fl + s, expired, &sh_ok, probe)) return;
-    if (tid < kSolveB) ys[tid] = tid < w ? __ldcg(&Vf[c0 + tid]) : T(0);
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 64; ++k) acc += l[k] * ys[64 * h + k];
-    __syncthreads();
-  }
-  if (h == 1) part[ri] = acc;
-  __syncthreads();
-  T v = T(0);
-  if (h == 0 && valid) v = Vf[i] - (acc + part[ri]);
-  if (code < 0) {
-    if (h == 0 && valid) Vf[i] = v;
-    return;
-  }
-  if (h == 0) ys[ri] = valid ? v : T(0);
-  __syncthreads();
-  const T* Li = inv_block(F, dinv, f, code);    // zero outside its w x w part
-  T y = T(0);
-#pragma unroll 16
-  for (int k = 0; k < 64; ++k) y += Li[ri + (size_t)(64 * h + k) * kSolveB] * ys[64 * h + k];
-  if (h == 1) part[ri] = y;
-  __syncthreads();
-  if (h == 0 && valid) {
-    const T yy = y + part[ri];
-    Vf[i] = yy;
-    X[F.first[f] + i] = yy;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    st_release_i32(fl + code, 1);
-  }
-}
-
-// backward: warp w takes columns 16 w .. 16 w + 15 of the block, lanes rows;
-// the rows below the block in the update part (their x known from the gather)
-// first, then the later diagonal blocks of the front from the last one down,
-// each after its flag (its panel entries loaded before the wait); a butterfly
-// transpose-reduce leaves column 16 w + (l mod 16)'s sum in lane l.
-template <typename T>
-__device__ __forceinline__ void bwd_rows_acc(const T* P, int nf, int c0, int w, int ra, int rb, const T* Vf, bool cg,
-                                             int wc, int lane, T (&acc)[16]) {
-  for (int rr = ra; rr < rb; rr += 32) {
-    const int r = rr + lane;
-    const bool ok = r < rb;
-    const T xv = ok ? (cg ? __ldcg(&Vf[r]) : Vf[r]) : T(0);
-    const T* pr = P + (ok ? r : ra) + (size_t)(c0 + wc) * nf;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) acc[j] += (ok && wc + j < w ? pr[(size_t)j * nf] : T(0)) * xv;
-  }
-}
-
-// butterfly transpose-reduce of 16 per-lane column sums: lane l ends with column (l mod 16)'s sum
-template <typename T>
-__device__ __forceinline__ T transpose_reduce16(T (&acc)[16], int lane) {
-#pragma unroll
-  for (int sft = 8; sft >= 1; sft >>= 1) {
-    const bool up = (lane & sft) != 0;
-#pragma unroll
-    for (int j = 0; j < sft; ++j) {
-      const T send = up ? acc[j] : acc[j + sft];
-      const T keep = up ? acc[j + sft] : acc[j];
-      acc[j] = keep + __shfl_xor_sync(0xffffffffu, send, sft);
-    }
-  }
-  return acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 16);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_bwd_large_fused(DevFronts F, const int4* __restrict__ tasks, int ntask,
-                                                         int32_t* ticket, int32_t* flags, int32_t* expired,
-                                                         const T* __restrict__ panel, const T* __restrict__ dinv,
-                                                         T* X, T* V, T* part, int32_t* counters,
-                                                         const int32_t* test_req) {
-  __shared__ int sh_t, sh_ok;
-  __shared__ T ts[kSolveB];
-  if (threadIdx.x == 0) sh_t = atomicAdd(ticket, 1);
-  __syncthreads();
-  const int t = sh_t;
-  if (t >= ntask) return;
-  const int4 tk = tasks[t];
-  const int f = tk.x;
-  int32_t* fl = flags + tk.z;
-  const bool probe = *test_req != 0;
-  const int nc = F.nc[f], nr = F.nr[f], nf = nc + nr;
-  const int nsteps = (nc + kSolveB - 1) / kSolveB;
-  const int nch = (nr + kBwdRestRows - 1) / kBwdRestRows;
-  const T* P = panel + F.panel_off[f];
-  T* Vf = V + F.v_off[f];
-  T* Pt = part + tk.w;                        // the front's partial sums: [step][chunk][128]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wc = 16 * warp;
-  T acc[16];
-#pragma unroll
-  for (int j = 0; j < 16; ++j) acc[j] = T(0);
-  if (tk.y < 0) {                             // update-row chunk j against column block s (x gathered)
-    const int code = -1 - tk.y, s = code >> 16, j = code & 0xffff;
-    const int c0 = s * kSolveB, w = min(kSolveB, nc - c0);
-    const int ra = nc + j * kBwdRestRows;
-    bwd_rows_acc(P, nf, c0, w, ra, min(nf, ra + kBwdRestRows), Vf, false, wc, lane, acc);
-    const T sum = transpose_reduce16(acc, lane);
-    if (lane < 16) Pt[((size_t)s * nch + j) * kSolveB + wc + lane] = sum;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      atomicAdd(&counters[tk.z + s], 1);
-    }
-    return;
-  }
-  const int s = tk.y;
-  const int c0 = s * kSolveB, w = min(kSolveB, nc - c0);
-  for (int b = nsteps - 1; b > s; --b) {                                   // later diagonal blocks
-    const int ra = b * kSolveB, rb = min(nc, ra + kSolveB);
-    T l[4][16];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int r = ra + lane + 32 * q;
-      const T* pr = P + (r < rb ? r : ra) + (size_t)(c0 + wc) * nf;
-#pragma unroll
-      for (int j = 0; j < 16; ++j) l[q][j] = (r < rb && wc + j < w) ? pr[(size_t)j * nf] : T(0);
-    }
-    if (!cta_wait_flag(fl + b, expired, &sh_ok, probe)) return;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int r = ra + lane + 32 * q;
-      const T xv = r < rb ? __ldcg(&Vf[r]) : T(0);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) acc[j] += l[q][j] * xv;
-    }
-  }
-  const T dsum = transpose_reduce16(acc, lane);           // lane l: column wc + (l mod 16), diagonal blocks
-  // the update rows' partial sums, chunk by chunk in order, once every chunk task has counted in
-  if (nch > 0 && !cta_wait_flag(counters + tk.z + s, expired, &sh_ok, probe, nch)) return;
-  if (lane < 16) {
-    const int c = wc + lane;
-    T rsum = T(0);
-    for (int j = 0; j < nch; ++j) rsum += __ldcg(&Pt[((size_t)s * nch + j) * kSolveB + c]);
-    ts[c] = c < w ? Vf[c0 + c] - (rsum + dsum) : T(0);
-  }
-  __syncthreads();
-  // x = Li^T t: column i of Li against t, lanes over k (coalesced), 16 columns per warp
-  const T* Li = inv_block(F, dinv, f, s);
-  T tv[kSolveB / 32];
-#pragma unroll
-  for (int q = 0; q < kSolveB / 32; ++q) tv[q] = ts[lane + 32 * q];
-  const int first = F.first[f];
-#pragma unroll 4
-  for (int cc = 0; cc < 16; ++cc) {
-    const int i = wc + cc;
-    const T* lcol = Li + (size_t)i * kSolveB + lane;
-    T sum = T(0);
-#pragma unroll
-    for (int q = 0; q < kSolveB / 32; ++q) sum += lcol[32 * q] * tv[q];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (lane == 0 && i < w) {
-      Vf[c0 + i] = sum;
-      X[first + c0 + i] = sum;
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    st_release_i32(fl + s, 1);
-  }
-}
-
-// Gathers of a level with many fronts and several right-hand sides: eight
-// right-hand sides per CTA, a warp each (no CTA-wide barrier between children),
-// eight rows per lane in flight.  With one CTA per front and right-hand side
-// these levels paid each CTA's chain of loads for a few hundred rows: 218 us
-// against this form's figure in launch_fwd_large for 928 fronts x 64.
-constexpr int kGatherRhs = 8;
-template <typename T>
-__global__ void __launch_bounds__(32 * kGatherRhs) k_fwd_gather_warp(DevFronts F, const int32_t* list, const T* X,
-                                                                     int64_t ldx, T* V, int nrhs) {
-  constexpr int U = 8;
-  const int f = list[blockIdx.x], lane = threadIdx.x & 31, r = blockIdx.y * kGatherRhs + (threadIdx.x >> 5);
-  if (r >= nrhs) return;
-  const int nc = F.nc[f], nf = nc + F.nr[f], first = F.first[f];
-  T* Vf = V + F.v_off[f] * nrhs + (int64_t)r * nf;
-  const T* Xr = X + first + r * ldx;
-  for (int i0 = lane; i0 < nf; i0 += 32 * U) {
-    T v[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) v[u] = i0 + 32 * u < nc ? Xr[i0 + 32 * u] : T(0);
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (i0 + 32 * u < nf) Vf[i0 + 32 * u] = v[u];
-  }
-  for (int t = F.child_ptr[f]; t < F.child_ptr[f + 1]; ++t) {
-    __syncwarp();
-    const int c = F.child[t];
-    const int ncc = F.nc[c], nrc = F.nr[c];
-    const T* Vc = V + F.v_off[c] * nrhs + (int64_t)r * (ncc + nrc) + ncc;
-    const int32_t* loc = F.local + F.lrow_off[c];
-    for (int i0 = lane; i0 < nrc; i0 += 32 * U) {
-      int li[U];
-      T cv[U], ov[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int i = i0 + 32 * u;
-        li[u] = i < nrc ? loc[i] - 1 : -1;
-        cv[u] = i < nrc ? Vc[i] : T(0);
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) ov[u] = li[u] >= 0 ? Vf[li[u]] : T(0);
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (li[u] >= 0) Vf[li[u]] = ov[u] + cv[u];
-    }
-  }
-}
-template <typename T>
-__global__ void __launch_bounds__(32 * kGatherRhs) k_bwd_gather_warp(DevFronts F, const int32_t* list, const T* X,
-                                                                     int64_t ldx, T* V, int nrhs) {
-  constexpr int U = 8;
-  const int f = list[blockIdx.x], lane = threadIdx.x & 31, r = blockIdx.y * kGatherRhs + (threadIdx.x >> 5);
-  if (r >= nrhs) return;
-  const int nc = F.nc[f], nf = nc + F.nr[f], first = F.first[f];
-  const int32_t* lr = F.lrow + F.lrow_off[f];
-  T* Vf = V + F.v_off[f] * nrhs + (int64_t)r * nf;
-  for (int i0 = lane; i0 < nf; i0 += 32 * U) {
-    int gi[U];
-    T v[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int i = i0 + 32 * u;
-      gi[u] = i < nc ? first + i : (i < nf ? lr[i - nc] : -1);
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) v[u] = gi[u] >= 0 ? X[gi[u] + r * ldx] : T(0);
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (gi[u] >= 0) Vf[i0 + 32 * u] = v[u];
-  }
-}
-
 template <typename T>
 __global__ void k_bwd_large_gather(DevFronts F, const int32_t* list, const T* X, int64_t ldx, T* V, int nrhs) {
   const int f = list[blockIdx.x];
   const int nc = F.nc[f], nf = nc + F.nr[f], first = F.first[f];
   const int32_t* lr = F.lrow + F.lrow_off[f];
-  const int rb = gridDim.y > 1 ? (int)blockIdx.y : 0, re = gridDim.y > 1 ? rb + 1 : nrhs;
   constexpr int kGU = 4;                     // loads in flight per thread
   const int nt = blockDim.x;
-  for (int r = rb; r < re; ++r) {
+  for (int r = 0; r < nrhs; ++r) {
     T* Vf = V + F.v_off[f] * nrhs + (int64_t)r * nf;
     for (int i0 = threadIdx.x; i0 < nf; i0 += kGU * nt) {
       int gi[kGU];
@@ -1485,6 +1193,7 @@ cudaError_t prepare_kernels() {
   chk(opt_in(k_update_dmma));
   chk(prepare_small_fronts());
   chk(prepare_small_solve());
+  chk(prepare_solve_single());
   chk(prepare_panel());
   chk(prepare_update_tc());
   chk(prepare_update_tcq());
@@ -1579,22 +1288,12 @@ int launch_update(const DevFronts& F, const int32_t* list, int count, int step, 
   return 1;
 }
 
-// a warp per right-hand side once the level's CTAs of eight still fill the chip (below, the
-// long fronts of a small level want a CTA each)
-bool gather_by_warp(int count, int nrhs) { return nrhs > 1 && (int64_t)count * ceil_div(nrhs, kGatherRhs) >= 2 * kNumSms; }
 template <typename T>
 void launch_fwd_large(const DevFronts& F, const int32_t* list, int count, int max_nc, int max_nf, const T* panel,
                       const T* dinv, T* X, int64_t ldx, T* V, int32_t* cnt, int nrhs, cudaStream_t st,
-                      int64_t* launches, bool pdl, bool fused) {
+                      int64_t* launches, bool pdl) {
   if (count <= 0) return;
-  // fused: one right-hand side per CTA row, the steps follow as one launch
-  if (fused && gather_by_warp(count, nrhs))
-    k_fwd_gather_warp<T><<<dim3(count, ceil_div(nrhs, kGatherRhs)), 32 * kGatherRhs, 0, st>>>(F, list, X, ldx, V, nrhs);
-  else k_fwd_large_gather<T><<<dim3(count, fused ? nrhs : 1), 256, 0, st>>>(F, list, dinv, X, ldx, V, nrhs, fused ? 0 : 1);
-  if (fused) {
-    if (launches) *launches += 1;
-    return;
-  }
+  k_fwd_large_gather<T><<<count, 256, 0, st>>>(F, list, dinv, X, ldx, V, nrhs);
   const int steps = ceil_div(max_nc, kSolveB);
   const int chunks = std::max(1, ceil_div(max_nf, kFwdRows));
   for (int s = 0; s < steps; ++s)
@@ -1605,15 +1304,9 @@ void launch_fwd_large(const DevFronts& F, const int32_t* list, int count, int ma
 template <typename T>
 void launch_bwd_large(const DevFronts& F, const int32_t* list, int count, int max_nc, int max_nf, const T* panel,
                       const T* dinv, T* X, int64_t ldx, T* V, T* scratch, int32_t* cnt, int nrhs, cudaStream_t st,
-                      int64_t* launches, bool pdl, bool fused) {
+                      int64_t* launches, bool pdl) {
   if (count <= 0) return;
-  if (fused && gather_by_warp(count, nrhs))
-    k_bwd_gather_warp<T><<<dim3(count, ceil_div(nrhs, kGatherRhs)), 32 * kGatherRhs, 0, st>>>(F, list, X, ldx, V, nrhs);
-  else k_bwd_large_gather<T><<<dim3(count, fused ? nrhs : 1), 256, 0, st>>>(F, list, X, ldx, V, nrhs);
-  if (fused) {
-    if (launches) *launches += 1;
-    return;
-  }
+  k_bwd_large_gather<T><<<count, 256, 0, st>>>(F, list, X, ldx, V, nrhs);
   const int steps = ceil_div(max_nc, kSolveB);
   const int chunks = std::max(1, ceil_div(max_nf, kSolveRows));
   for (int s = steps - 1; s >= 0; --s)
@@ -1621,19 +1314,6 @@ void launch_bwd_large(const DevFronts& F, const int32_t* list, int count, int ma
              scratch, cnt, nrhs);
   if (launches) *launches += 1 + steps;
 }
-template <typename T>
-void launch_large_fused(const DevFronts& F, const int4* tasks, int ntask, bool backward, int32_t* ticket,
-                        int32_t* flags, int32_t* expired, const T* panel, const T* dinv, T* X, T* V, cudaStream_t st,
-                        const int32_t* test_req, T* part, int32_t* counters) {
-  if (ntask <= 0) return;
-  if (backward)
-    k_bwd_large_fused<T><<<ntask, 256, 0, st>>>(F, tasks, ntask, ticket, flags, expired, panel, dinv, X, V, part,
-                                                counters, test_req);
-  else
-    k_fwd_large_fused<T><<<ntask, 256, 0, st>>>(F, tasks, ntask, ticket, flags, expired, panel, dinv, X, V,
-                                                test_req);
-}
-
 template <typename T>
 void launch_permute_in(const double* b, int64_t ldb, const int32_t* perm, T* X, int64_t ldx, int64_t n, int nrhs,
                        cudaStream_t st) {
@@ -1737,11 +1417,9 @@ void launch_remap_int(const int32_t* map, int32_t* a, int64_t n, cudaStream_t st
   template int launch_update<T>(const DevFronts&, const int32_t*, int, int, int, int, T*, T*, int, cudaStream_t,    \
                                  UpdBand, int, bool);                                                              \
   template void launch_fwd_large<T>(const DevFronts&, const int32_t*, int, int, int, const T*, const T*, T*,       \
-                                    int64_t, T*, int32_t*, int, cudaStream_t, int64_t*, bool, bool);               \
+                                    int64_t, T*, int32_t*, int, cudaStream_t, int64_t*, bool);                     \
   template void launch_bwd_large<T>(const DevFronts&, const int32_t*, int, int, int, const T*, const T*, T*,       \
-                                    int64_t, T*, T*, int32_t*, int, cudaStream_t, int64_t*, bool, bool);           \
-  template void launch_large_fused<T>(const DevFronts&, const int4*, int, bool, int32_t*, int32_t*, int32_t*,      \
-                                      const T*, const T*, T*, T*, cudaStream_t, const int32_t*, T*, int32_t*);     \
+                                    int64_t, T*, T*, int32_t*, int, cudaStream_t, int64_t*, bool);                 \
   template void launch_permute_in<T>(const double*, int64_t, const int32_t*, T*, int64_t, int64_t, int,            \
                                      cudaStream_t);                                                                \
   template void launch_permute_out<T>(const T*, int64_t, const int32_t*, double*, int64_t, int64_t, int,           \

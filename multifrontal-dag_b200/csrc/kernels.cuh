@@ -213,31 +213,32 @@ template <typename T>
 void launch_bwd_small(const DevFronts& F, const FrontRec* rec, int count, int nf_max, int panel_elems, const T* panel,
                       T* X, int64_t ldx, int nrhs, cudaStream_t st);
 // Large fronts: dinv holds the inverted 128 x 128 diagonal blocks the factorization kept (DevFronts::d_off).
-// fused: only the gather runs here (launch_large_fused or launch_large_multi does the steps)
+// One launch per panel step (the fallback of launch_large_fused / launch_large_multi).
 template <typename T>
 void launch_fwd_large(const DevFronts& F, const int32_t* list, int count, int max_nc, int max_nf, const T* panel,
                       const T* dinv, T* X, int64_t ldx, T* V, int32_t* cnt, int nrhs, cudaStream_t st,
-                      int64_t* launches, bool pdl, bool fused = false);
+                      int64_t* launches, bool pdl);
 // cnt: one zero-initialised ticket per list slot (left zero again on exit)
 template <typename T>
 void launch_bwd_large(const DevFronts& F, const int32_t* list, int count, int max_nc, int max_nf, const T* panel,
                       const T* dinv, T* X, int64_t ldx, T* V, T* scratch, int32_t* cnt, int nrhs, cudaStream_t st,
-                      int64_t* launches, bool pdl, bool fused = false);
+                      int64_t* launches, bool pdl);
 // A level's single-RHS large-front sweep as one launch over its task list (4 ints per task:
-// front, code, flag base, 0; forward code >= 0: diagonal block, < 0: rest rows chunk -1 - code;
-// backward code: column block).  ticket: zero before the launch; flags: zero before the sweep
-// (one per front and panel step); expired: raised when a bounded wait gives up.
-// test_req (read once per CTA): nonzero makes every wait run out after ~1 ms (a test of the
-// expiry path).
-// Backward: tasks with code < 0 are partial sums of update-row chunk j (kBwdRestRows rows)
-// against column block s (code = -1 - (s << 16 | j)), written to part (front base in the
-// task's fourth int) and counted in counters (one per front and step); code >= 0 is the
-// column block, which sums its chunks' partials in chunk order.
+// front, code, flag base, partial-sum base; solve_single.cu).  Forward code >= 0: diagonal block,
+// < 0: rest rows chunk -1 - code.  Backward code < 0: partial sums of update-row chunk j
+// (kBwdRestRows rows) against column block s (code = -1 - (s << 16 | j)), written to part and
+// counted in counters (one per front and step); code >= 0: column block, which adds its chunks'
+// partials in chunk order.  ticket and counters: zero before the launch; expired: raised when a
+// bounded wait gives up; epoch: the sweep's number (launch_solve_begin); exch: n_total exchange
+// entries of 2 sizeof(T), zero at allocation.  test_req (read once per CTA): nonzero makes every
+// wait run out after ~1 ms (a test of the expiry path).
 constexpr int kBwdRestRows = 256;
+cudaError_t prepare_solve_single();
+void launch_solve_begin(int32_t* sync, int64_t n, int32_t* epoch, cudaStream_t st);
 template <typename T>
 void launch_large_fused(const DevFronts& F, const int4* tasks, int ntask, bool backward, int32_t* ticket,
-                        int32_t* flags, int32_t* expired, const T* panel, const T* dinv, T* X, T* V, cudaStream_t st,
-                        const int32_t* test_req, T* part = nullptr, int32_t* counters = nullptr);
+                        int32_t* expired, const int32_t* epoch, const T* panel, const T* dinv, T* X, T* V, void* exch,
+                        cudaStream_t st, const int32_t* test_req, T* part = nullptr, int32_t* counters = nullptr);
 // The same sweep for several right-hand sides (solve_multi.cu), each task split into
 // multi_tiles(nrhs) tiles: flags and counters hold as many entries per front and panel
 // step, part multi_part(nrhs) times the single-RHS size.

@@ -27,6 +27,7 @@ struct alignas(16) FrontRec {
 struct alignas(16) ChildRec {
   int32_t nc, nr, lrow_off, pad;
   int64_t u_off, v_off;
+  int64_t inv_off, pad2;
 };
 
 // Pointers into the device copies of the per-front tables (all 0-based).

@@ -33,12 +33,15 @@ constexpr int kHalf = 8;          // blocks of eight columns per register half
 // The 128 x (8 NB) block of the vectors (column stride ld, `rows` rows, `cols`
 // columns valid) as B fragments: element (k, n) at Y[(n / 8) 1024 + (k / 8) 64 +
 // 8 (n % 8) + k % 8], zero outside.  Read past L1: other CTAs wrote it.
+// idx (may be null): row k is row idx[k] of v.
 template <int NB, typename T>
-__device__ __forceinline__ void stage_vectors(double* Y, const T* v, int64_t ld, int rows, int cols) {
+__device__ __forceinline__ void stage_vectors(double* Y, const T* v, int64_t ld, int rows, int cols,
+                                              const int32_t* idx = nullptr) {
+  const int k = threadIdx.x & 127, kr = k < rows ? (idx ? idx[k] : k) : 0;
 #pragma unroll
   for (int u = 0; u < 4 * NB; ++u) {
-    const int e = threadIdx.x + 256 * u, k = e & 127, n = e >> 7;
-    Y[(n >> 3) * 1024 + (k >> 3) * 64 + (n & 7) * 8 + (k & 7)] = k < rows && n < cols ? (double)__ldcg(v + n * ld + k) : 0.0;
+    const int n = (threadIdx.x >> 7) + 2 * u;
+    Y[(n >> 3) * 1024 + (k >> 3) * 64 + (n & 7) * 8 + (k & 7)] = k < rows && n < cols ? (double)__ldcg(v + n * ld + kr) : 0.0;
   }
 }
 
@@ -106,6 +109,31 @@ __device__ __forceinline__ void zero(double2 (&v)[2][NB]) {
     for (int n = 0; n < NB; ++n) v[m][n] = make_double2(0.0, 0.0);
 }
 
+// gather_row (sweep_sync.cuh) for right-hand sides rc + 8 n and rc + 8 n + 1, n < NB, below re; row i < 0: zeros
+template <int NB, typename T>
+__device__ __forceinline__ void gather_rows(double2 (&v)[NB], const DevFronts& F, int f, int i, int nc, const T* Xf,
+                                            int64_t ldx, const T* V, int nrhs, int rc, int re) {
+#pragma unroll
+  for (int n = 0; n < NB; ++n) {
+    const int r = rc + 8 * n;
+    v[n].x = i >= 0 && i < nc && r < re ? (double)Xf[i + (int64_t)r * ldx] : 0.0;
+    v[n].y = i >= 0 && i < nc && r + 1 < re ? (double)Xf[i + (int64_t)(r + 1) * ldx] : 0.0;
+  }
+  if (i < 0) return;
+  for (int t = F.child_ptr[f], ce = F.child_ptr[f + 1]; t < ce; ++t) {
+    const ChildRec c = F.crec[t];
+    const int ci = F.inv[c.inv_off + i];
+    if (ci < 0) continue;
+    const int ld = c.nc + c.nr;
+    const T* p = V + c.v_off * nrhs + (int64_t)rc * ld + c.nc + ci;
+#pragma unroll
+    for (int n = 0; n < NB; ++n) {
+      if (rc + 8 * n < re) v[n].x += (double)p[(int64_t)(8 * n) * ld];
+      if (rc + 8 * n + 1 < re) v[n].y += (double)p[(int64_t)(8 * n + 1) * ld];
+    }
+  }
+}
+
 // Forward: task (f, s, tile): y_s = Li (v_s - sum_{t<s} L_st y_t); rest tasks
 // (128 rows below the columns): v -= sum_t L_rest,t y_t.  Warp w has rows
 // 16 w .. 16 w + 15 of the task.
@@ -135,17 +163,14 @@ __global__ void __launch_bounds__(256, 2)
   const int ri = 16 * warp + g;                            // rows r0 + ri and r0 + ri + 8
   double2 acc[2][NB];
   zero(acc);
-  // the task's own rows of the vectors (written by the gather), off the chain of steps
+  // the task's own rows of the vectors, gathered here (each row once), off the chain of steps
   double2 v[2][NB];
+  const int first = F.first[f];
 #pragma unroll
-  for (int m = 0; m < 2; ++m)
-#pragma unroll
-    for (int n = 0; n < NB; ++n) {
-      const int r = r0 + ri + 8 * m, c = 8 * n + q2;
-      const T* p = Vf + (int64_t)c * nf + r;
-      v[m][n].x = r < r1 && c < cols ? (double)p[0] : 0.0;
-      v[m][n].y = r < r1 && c + 1 < cols ? (double)p[nf] : 0.0;
-    }
+  for (int m = 0; m < 2; ++m) {
+    const int r = r0 + ri + 8 * m;
+    gather_rows<NB>(v[m], F, f, r < r1 ? r : -1, nc, X + first, ldx, V, nrhs, c0r + q2, c0r + cols);
+  }
   T a[2][kHalf][2];
   for (int s = 0; s < nsteps; ++s) {
     const int c0 = s * kSolveB, w = min(kSolveB, nc - c0), kb = (w + 7) >> 3;
@@ -181,7 +206,6 @@ __global__ void __launch_bounds__(256, 2)
       mul_half(v, a, Y, kHalf, kb, lane);
     }
   }
-  const int first = F.first[f];
 #pragma unroll
   for (int m = 0; m < 2; ++m) {
     const int r = r0 + ri + 8 * m;
@@ -206,13 +230,13 @@ __global__ void __launch_bounds__(256, 2)
 }
 
 // Backward: first the partial sums over the update rows (chunks of
-// kBwdRestRows, x gathered), then the column blocks from the last down: x_s =
+// kBwdRestRows, their x known from the ancestors), then the column blocks from the last down: x_s =
 // Li^T (v_s - L_below,s^T x_below), the chunks' partials added in chunk order.
 // part: [front's step and chunk][tile][128 columns][8 NB].
 template <typename T, int NB>
 __global__ void __launch_bounds__(256, 2)
     k_bwd_multi(DevFronts F, const int4* __restrict__ tasks, int ntask, int tiles, int stride, int32_t* ticket, int32_t* flags,
-                int32_t* expired, const T* __restrict__ panel, const T* __restrict__ dinv, T* X, int64_t ldx, T* V,
+                int32_t* expired, const T* __restrict__ panel, const T* __restrict__ dinv, T* X, int64_t ldx,
                 int nrhs, T* part, int32_t* counters, const int32_t* test_req) {
   __shared__ int sh_t, sh_ok;
   __shared__ __align__(16) double Y[NB * 1024];
@@ -229,7 +253,9 @@ __global__ void __launch_bounds__(256, 2)
   const int nsteps = (nc + kSolveB - 1) / kSolveB, nch = (nr + kBwdRestRows - 1) / kBwdRestRows;
   const int c0r = tile * 8 * NB, cols = min(8 * NB, nrhs - c0r);
   const T* P = panel + F.panel_off[f];
-  T* Vf = V + F.v_off[f] * nrhs + (int64_t)c0r * nf;
+  const int first = F.first[f];
+  T* Xt = X + (int64_t)c0r * ldx;                          // the tile's right-hand sides
+  const int32_t* lr = F.lrow + F.lrow_off[f] - nc;         // row r >= nc of the front is row lr[r] of X
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q2 = 2 * (lane & 3);
   const int ci = 16 * warp + g;                            // columns c0 + ci and c0 + ci + 8
   // this lane's first entry of partial (s, j)
@@ -242,7 +268,8 @@ __global__ void __launch_bounds__(256, 2)
   // acc += (rows [ra, rb) of column block Pc)^T x, the first half of the rows loaded
   auto finish_rows = [&](const T* Pc, int w, int ra, int rb) {
     const int kb = (rb - ra + 7) >> 3;
-    stage_vectors<NB>(Y, Vf + ra, nf, rb - ra, cols);
+    if (ra < nc) stage_vectors<NB>(Y, Xt + first + ra, ldx, rb - ra, cols);
+    else stage_vectors<NB>(Y, Xt, ldx, rb - ra, cols, lr + ra);
     __syncthreads();
     mul_half(acc, a, Y, 0, kb, lane);
     if (kb > kHalf) {
@@ -284,9 +311,9 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
     for (int n = 0; n < NB; ++n) {
       const int i = ci + 8 * m, c = 8 * n + q2;
-      const T* p = Vf + (int64_t)c * nf + c0 + i;
+      const T* p = Xt + (int64_t)c * ldx + first + c0 + i;
       v[m][n].x = i < w && c < cols ? (double)p[0] : 0.0;
-      v[m][n].y = i < w && c + 1 < cols ? (double)p[nf] : 0.0;
+      v[m][n].y = i < w && c + 1 < cols ? (double)p[ldx] : 0.0;
     }
   for (int b = nsteps - 1; b > s; --b) {                   // later diagonal blocks
     const int ra = b * kSolveB, rb = min(nc, ra + kSolveB);
@@ -330,7 +357,6 @@ __global__ void __launch_bounds__(256, 2)
     load_cols(a, Li, kSolveB, ci, kSolveB, w, 1, q2);
     mul_half(acc, a, Y, kHalf, kb, lane);
   }
-  const int first = F.first[f];
 #pragma unroll
   for (int m = 0; m < 2; ++m) {
     const int i = ci + 8 * m;
@@ -341,9 +367,7 @@ __global__ void __launch_bounds__(256, 2)
       for (int e = 0; e < 2; ++e) {
         const int c = 8 * n + q2 + e;
         if (c >= cols) continue;
-        const T x = (T)(e ? acc[m][n].y : acc[m][n].x);
-        Vf[(int64_t)c * nf + c0 + i] = x;
-        X[first + c0 + i + (int64_t)(c0r + c) * ldx] = x;
+        Xt[first + c0 + i + (int64_t)c * ldx] = (T)(e ? acc[m][n].y : acc[m][n].x);
       }
   }
   __syncthreads();
@@ -364,7 +388,7 @@ void launch_large_multi(const DevFronts& F, const int4* tasks, int ntask, bool b
   auto go = [&](auto fwd, auto bwd, int width) {
     const int tiles = (nrhs + width - 1) / width;
     if (backward)
-      bwd<<<ntask * tiles, 256, 0, st>>>(F, tasks, ntask, tiles, stride, ticket, flags, expired, panel, dinv, X, ldx, V,
+      bwd<<<ntask * tiles, 256, 0, st>>>(F, tasks, ntask, tiles, stride, ticket, flags, expired, panel, dinv, X, ldx,
                                          nrhs, part, counters, test_req);
     else
       fwd<<<ntask * tiles, 256, 0, st>>>(F, tasks, ntask, tiles, stride, ticket, flags, expired, panel, dinv, X, ldx, V,

@@ -1,9 +1,12 @@
-// Device-side flags of the fused solve sweeps: bounded waits, acquire / release.
+// Shared by the fused solve sweeps: device-side flags (bounded waits, acquire /
+// release) and the forward gather.
 #pragma once
 #include <cuda_runtime.h>
 
 #include <climits>
 #include <cstdint>
+
+#include "plan.hpp"
 
 namespace mfd {
 
@@ -42,6 +45,31 @@ __device__ __forceinline__ bool cta_wait_flag(const int32_t* flag, int32_t* expi
   }
   __syncthreads();
   return *sh_ok != 0;
+}
+
+// Entry i of front f's vector before its panel steps: its own right-hand side
+// (Xf: the front's first column) plus the children's update vectors in child
+// order (V: nrhs columns per front, column r), two children's loads in flight.
+template <typename T>
+__device__ __forceinline__ T gather_row(const DevFronts& F, int f, int i, int nc, const T* Xf, const T* V, int nrhs,
+                                        int r) {
+  T v = i < nc ? Xf[i] : T(0);
+  const int ce = F.child_ptr[f + 1];
+  for (int t = F.child_ptr[f]; t < ce; t += 2) {
+    T x[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      x[s] = T(0);
+      if (t + s < ce) {
+        const ChildRec c = F.crec[t + s];
+        const int ci = F.inv[c.inv_off + i];
+        if (ci >= 0) x[s] = V[c.v_off * nrhs + (int64_t)r * (c.nc + c.nr) + c.nc + ci];
+      }
+    }
+    v += x[0];
+    v += x[1];
+  }
+  return v;
 }
 
 }  // namespace mfd
