@@ -42,9 +42,13 @@ int fail(int code, const std::string& msg) {
 constexpr int64_t kAlign = 32;  // elements; keeps every front 256-byte aligned in FP64
 constexpr int kResMulti = 4;     // from this many right-hand sides on, one multi-column residual per IR sweep
 constexpr int kPotrfSplitMin = 148;   // fronts in a panel step above which POTRF launches per width class
-// panel steps per deferred trailing update: FP64 2 (64^3 Laplacian 38.1 -> 37.7 ms: K = 256 per pass
-// halves the C traffic of the DMMA update); FP32 1 (the packed-operand tensor-core update needs it)
-constexpr int kDeferDefaultFp64 = 2, kDeferDefaultFp32 = 1;
+// panel steps per deferred trailing update: K = 256 per pass halves the update's C traffic, which
+// counts on levels whose trailing matrices pass through HBM, their lower triangles above half of the
+// 126 MB L2 (80^3 diffusion, mixed: 45.7 -> 40.7 ms).  Below, a deferred update only lengthens the
+// panel chain (elasticity 21^3, mixed, with it on every level: 6.00 -> 6.16 ms).
+constexpr int kDeferDefault = 2;
+constexpr double kDeferBytes = 64e6;
+constexpr int kPackedDefer = 2;       // the most the packed-operand FP32 update takes
 int64_t align_up(int64_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
 template <typename T>
@@ -212,7 +216,7 @@ struct mfd_handle {
   void* d_upool = nullptr;
   void* d_diag = nullptr;
   double* d_packed = nullptr;                       // the current panel step's packed diagonal blocks, one per list slot
-  float* d_q = nullptr;                             // FP32: packed update operands, two step parities
+  float* d_q = nullptr;                             // FP32: packed update operands, 2 defer step buffers
   DBuf<double> d_a, d_b, d_xp, d_bp, d_r, d_norms, d_cnorms, d_xt;
   void* d_X = nullptr;   // T, n_total x nrhs
   void* d_V = nullptr;   // T
@@ -460,6 +464,15 @@ int build_plan(mfd_handle* h) {
     }
     L.large.param = max_entries;
     L.large.param2 = max_nc;
+    // deferral depth: the caller's (reserved[5]) on every level, the default where it pays
+    {
+      double bytes = 0;
+      for (int32_t g : large) {
+        const double nf = h->fronts[g].nc + h->fronts[g].nr;
+        bytes += (h->fp32 ? 4.0 : 8.0) * nf * nf / 2;
+      }
+      L.defer = h->opt.reserved[5] > 0 || bytes > kDeferBytes ? h->defer : 1;
+    }
     // packed operands of the FP32 tensor-core update: the level's large fronts side by side,
     // each with the 128-row blocks of its largest step (step 0); reused level after level
     {
@@ -789,10 +802,10 @@ int upload_plan(mfd_handle* h) {
   CK(cudaMalloc(&h->d_upool, std::max<int64_t>(h->upool_elems, 1) * esz));
   CK(cudaMalloc(&h->d_diag, (size_t)std::max<int64_t>(h->dinv_elems, 1) * esz));
   CK(cudaMalloc(&h->d_packed, (size_t)std::max(1, h->max_large_count) * kPackedPanelElems * sizeof(double)));
-  if (h->fp32 && h->q_elems > 0) {
-    CK(cudaMalloc(&h->d_q, (size_t)(2 * h->q_elems) * sizeof(float)));
+  if (h->fp32 && h->q_elems > 0 && h->defer <= kPackedDefer) {
+    CK(cudaMalloc(&h->d_q, (size_t)(2 * h->defer * h->q_elems) * sizeof(float)));
     // rows past a front's last row are never written and only reach discarded outputs; zero keeps them finite
-    CK(cudaMemsetAsync(h->d_q, 0, (size_t)(2 * h->q_elems) * sizeof(float), h->st));
+    CK(cudaMemsetAsync(h->d_q, 0, (size_t)(2 * h->defer * h->q_elems) * sizeof(float), h->st));
   }
   // the inverted diagonal blocks are written on their lower w x w part only: the rest stays zero
   CK(cudaMemsetAsync(h->d_diag, 0, (size_t)std::max<int64_t>(h->dinv_elems, 1) * esz, h->st));
@@ -992,11 +1005,12 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
     // Measured on the 64^3 Laplacian it costs 1-2 ms (early-launched CTAs wait on
     // SMs the side-stream update could use), so the default leaves it off.
     const bool pdl = h->opt.reserved[2] == 1 && !h->profiling;
-    const int D = h->defer;
-    // FP32 tensor-core update without deferral: the TRSM also writes the step's rows as
-    // packed TF32 hi / lo operands (two buffers by step parity: with D = 1 the bulk update
-    // of step s is complete before the TRSM of step s + 2 starts) for k_update_tcq
-    const bool tcq = sizeof(T) == 4 && (kind == 0 || kind == 2) && D == 1 && h->d_q != nullptr;
+    const int D = L.defer;
+    // FP32 tensor-core update: the TRSM also writes the step's rows as packed TF32 hi / lo
+    // operands for k_update_tcq, in 2 D buffers taken in turn: the bulk update of a group reads
+    // its own D, and is complete before the TRSM of the group after the next one starts
+    const bool tcq = sizeof(T) == 4 && (kind == 0 || kind == 2) && h->d_q != nullptr;
+    auto packed_rows = [&](size_t step) { return h->d_q + (step % (2 * D)) * h->q_elems; };
     int pend = -1;                            // step of the latest bulk on st2 not yet fully waited for
     for (size_t s = 0; s < L.steps.size(); ++s) {
       const LaunchList& p = L.steps[s];
@@ -1042,7 +1056,7 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
              });
       record(h, st, MFD_K_TRSM, tf, tb, [&] {
         launch_trsm<T>(F, lists + p.off, p.count, (int)s, p.param, std::min(kFactB, L.large.param2 - (int)s * kFactB),
-                       panel, h->d_packed, st, pdl, tcq ? h->d_q + (s & 1) * h->q_elems : nullptr);
+                       panel, h->d_packed, st, pdl, tcq ? packed_rows(s) : nullptr);
       });
       n += 2;
       auto update = [&](cudaStream_t us, UpdBand band) {
@@ -1052,9 +1066,10 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
         record(h, us, MFD_K_UPDATE, fl, by, [&] {
           if constexpr (sizeof(T) == 4) {
             if (tcq) {
-              n += launch_update_tcq(F, lists + p.off, p.count, (int)s, p.param2, h->d_q + (s & 1) * h->q_elems,
-                                     reinterpret_cast<float*>(panel), reinterpret_cast<float*>(upool),
-                                     kind == 0 ? 1 : 0, h->d_info.p + 1, us, band, upd_pdl);
+              n += launch_update_tcq(F, lists + p.off, p.count, (int)s, p.param2, packed_rows(s),
+                                     s > 0 ? packed_rows(s - 1) : nullptr, reinterpret_cast<float*>(panel),
+                                     reinterpret_cast<float*>(upool), kind == 0 ? 1 : 0, h->d_info.p + 1, us, band, D,
+                                     upd_pdl);
               return;
             }
             if (kind == 0 || kind == 2) {
@@ -1565,7 +1580,7 @@ int create_common(mfd_handle** out, std::vector<Symbolic>&& syms, const mfd_opti
   for (int k = 0; k < mfd_handle::kMaxDefer; ++k) CK(cudaEventCreateWithFlags(&h->ev_part[k], cudaEventDisableTiming));
   // deferred updates: reserved[5] = group size (1 = none); 0 = default
   h->defer = h->opt.reserved[5] > 0 ? std::min(h->opt.reserved[5], mfd_handle::kMaxDefer)
-                                     : (h->opt.precision == MFD_PREC_FP32_IR ? kDeferDefaultFp32 : kDeferDefaultFp64);
+                                     : kDeferDefault;
   CK(cudaEventCreateWithFlags(&h->ev_lvl, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&h->ev_inv, cudaEventDisableTiming));
   CK(cudaStreamCreateWithPriority(&h->sinv, cudaStreamNonBlocking, prio_lo));
@@ -1817,7 +1832,7 @@ int mfd_autotune(mfd_handle* h, const double* a, int32_t repeats, mfd_options* b
       mfd_options o = base;
       o.reserved[0] = kinds[ki];
       o.reserved[5] = d;
-      const int base_d = base.reserved[5] > 0 ? base.reserved[5] : (fp32 ? kDeferDefaultFp32 : kDeferDefaultFp64);
+      const int base_d = base.reserved[5] > 0 ? base.reserved[5] : kDeferDefault;
       if (kinds[ki] == base.reserved[0] && d == base_d) continue;   // timed in stage 1
       int rc = consider(o);
       if (rc) return rc;

@@ -184,7 +184,7 @@ int launch_update_tc(const DevFronts& F, const int32_t* list, int count, int ste
 // base = first row below the block), each as 16 K chunks of 8 columns, each chunk a TF32 hi
 // block then a lo block (x - hi), 1024 floats each in the canonical K-major no-swizzle UMMA
 // layout (8-row x 16-byte core matrices; 16 bytes between the two k-cores, 256 between
-// 8-row groups).  Columns past the block width are zero.  Two buffers, by step parity.
+// 8-row groups).  Columns past the block width are zero.
 constexpr int64_t kPackedBlockElems = 16 * 2 * 1024;   // one 128-row block: 16 chunks x (hi, lo)
 #ifdef __CUDACC__
 __host__ __device__ constexpr int64_t packed_block_elems() { return kPackedBlockElems; }
@@ -194,12 +194,12 @@ __device__ __forceinline__ int64_t packed_offset(int row, int k, int hl) {   // 
          (kk >> 2) * 32 + (kk & 3);
 }
 #endif
-// Trailing update of an FP32 step with deferral depth 1 from the packed operands q (this
-// step's parity buffer): warp-specialised tcgen05 pipeline (update_tc.cu).
+// Trailing update of an FP32 step (deferral depth 1 or 2) from the packed operands, q the step's
+// and qprev the previous step's: warp-specialised tcgen05 pipeline (update_tc.cu).
 cudaError_t prepare_update_tcq();
 int launch_update_tcq(const DevFronts& F, const int32_t* list, int count, int step, int T128, const float* q,
-                      float* panel, float* upool, int split, int32_t* err, cudaStream_t st, UpdBand band = {},
-                      bool pdl = false);
+                      const float* qprev, float* panel, float* upool, int split, int32_t* err, cudaStream_t st,
+                      UpdBand band = {}, int defer = 1, bool pdl = false);
 // grid size of an update launch over a band of the T x T lower tiles of width tw
 int update_grid(int T, int tw, UpdBand band);
 

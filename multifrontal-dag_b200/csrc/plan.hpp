@@ -81,6 +81,7 @@ struct LevelPlan {
   // in the solve task pool, forward and backward
   LaunchList fwd_tasks, bwd_tasks;
   int32_t large_max_nf = 0;
+  int32_t defer = 1;                 // panel steps per deferred trailing update
 };
 
 }  // namespace mfd

@@ -335,9 +335,10 @@ __device__ __forceinline__ bool mbar_wait_ab(uint32_t mbar, uint32_t parity, vol
 }
 
 __global__ void __launch_bounds__(kTcThreads, 2) k_update_tcq(DevFronts F, const int32_t* list, int step,
-                                                              const float* __restrict__ q, float* panel,
+                                                              const float* __restrict__ q,
+                                                              const float* __restrict__ qprev, float* panel,
                                                               float* upool, int split, int32_t* err, int blo,
-                                                              int bhi) {
+                                                              int bhi, int defer) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const int f = list[blockIdx.y];
   const int nc = F.nc[f], nr = F.nr[f], nf = nc + nr;
@@ -350,15 +351,25 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_update_tcq(DevFronts F, const
   const int T = (nrem + kTcTile - 1) / kTcTile;
   int ti, tj, kbeg, kend;
   if (!select_tile(T, kTcTile, blo, bhi, blockIdx.x, ti, tj)) return;
-  if (!update_k_range(nc, step, 1, tj, kTcTile, kbeg, kend)) return;
+  if (!update_k_range(nc, step, defer, tj, kTcTile, kbeg, kend)) return;
   const int nchunk = (kend - kbeg + 7) / 8;         // K = 8 chunks of the packed operands
+  // a group of two steps: the first kPrevChunks come from the previous step's rows, one 128-row
+  // block further down there (the step's own width is 128: a narrower one is a group of its own)
+  constexpr int kPrevChunks = kFactB / 8;
+  const bool two = kbeg < c0;
   const int nst = (nchunk + kQStageChunks - 1) / kQStageChunks;
   const int i0 = base + ti * kTcTile, j0 = base + tj * kTcTile;
   const bool diag = ti == tj;
   float* P = panel + F.panel_off[f];
   float* U = upool + F.u_off[f];
-  const float* QA = q + F.q_off[f] + (int64_t)ti * packed_block_elems();
-  const float* QB = q + F.q_off[f] + (int64_t)tj * packed_block_elems();
+  const int64_t qo = F.q_off[f];
+  const int test_req = err[1];
+  // chunk c of the rows of tile index t
+  auto operand = [&](int t, int c) {
+    const float* b = two && c < kPrevChunks ? qprev + (int64_t)(t + 1) * packed_block_elems()
+                                            : q + (int64_t)t * packed_block_elems() - (two ? kPrevChunks * 2048 : 0);
+    return b + qo + (int64_t)c * 2048;
+  };
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw);
@@ -417,7 +428,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_update_tcq(DevFronts F, const
   };
   if (!full) load_c(0);
 
-  if (err[1]) {                     // test request: every CTA waits on a barrier nothing arrives at
+  if (test_req) {                   // test request: every CTA waits on a barrier nothing arrives at
     if (tid == 0) mbar_wait_ab(bar_probe, 0, abort_flag, kProbeLimit);
   }
   __syncthreads();
@@ -433,12 +444,12 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_update_tcq(DevFronts F, const
                    : "memory");
       const uint32_t dA = sb + s * kQStageBytes;
       asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dA),
-                   "l"(QA + (int64_t)c * kQStageChunks * 2048), "r"(opb), "r"(fb)
+                   "l"(operand(ti, c * kQStageChunks)), "r"(opb), "r"(fb)
                    : "memory");
       if (!diag)
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                          dA + kQOpStage),
-                     "l"(QB + (int64_t)c * kQStageChunks * 2048), "r"(opb), "r"(fb)
+                     "l"(operand(tj, c * kQStageChunks)), "r"(opb), "r"(fb)
                      : "memory");
       produced = c + 1;
     }
@@ -515,11 +526,12 @@ cudaError_t prepare_update_tcq() {
 }
 
 int launch_update_tcq(const DevFronts& F, const int32_t* list, int count, int step, int T128, const float* q,
-                      float* panel, float* upool, int split, int32_t* err, cudaStream_t st, UpdBand band, bool pdl) {
+                      const float* qprev, float* panel, float* upool, int split, int32_t* err, cudaStream_t st,
+                      UpdBand band, int defer, bool pdl) {
   const int g = update_grid(T128, kTcTile, band);
   if (count <= 0 || g <= 0) return 0;
-  launch_k(k_update_tcq, dim3(g, count), dim3(kTcThreads), kQSmem, st, pdl, F, list, step, q, panel, upool, split,
-           err, band.blo, band.bhi);
+  launch_k(k_update_tcq, dim3(g, count), dim3(kTcThreads), kQSmem, st, pdl, F, list, step, q, qprev, panel, upool,
+           split, err, band.blo, band.bhi, defer);
   return 1;
 }
 
