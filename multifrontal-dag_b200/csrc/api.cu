@@ -11,6 +11,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <set>
 #include <string>
 #include <thread>
@@ -135,9 +136,63 @@ struct BestFit {
   }
 };
 
-struct SmallBin {
-  int nf_max;
+// What a factorization or solve tells the host, written by its last kernel: page-locked, so that
+// one stream synchronisation is all the host waits for.
+struct HostStatus {
+  int32_t info[4];                          // as mfd_handle::d_info
+  double anorm;
+  double norms[5];                          // of the residual (launch_norms)
+  double ir_d[2];                           // refinement state (launch_ir_check)
+  int32_t ir_i[2];
+  int32_t expired;
 };
+// One page-locked block for the process, cut into slots (a handle takes one and gives it back);
+// page-locking memory per handle would cost more than a small handle's set-up.
+class StatusPool {
+ public:
+  HostStatus* take() {
+    std::lock_guard<std::mutex> lk(mu_);
+    if (!base_) {
+      void* p = nullptr;
+      if (cudaHostAlloc(&p, kSlots * kSlotBytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+      }
+      base_ = static_cast<char*>(p);
+      for (int i = kSlots; i-- > 0;) free_.push_back(i);
+    }
+    if (!free_.empty()) {
+      const int i = free_.back();
+      free_.pop_back();
+      return reinterpret_cast<HostStatus*>(base_ + i * kSlotBytes);
+    }
+    void* p = nullptr;                      // every slot in use: an allocation of its own
+    if (cudaHostAlloc(&p, kSlotBytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    return static_cast<HostStatus*>(p);
+  }
+  void give(HostStatus* s) {
+    if (!s) return;
+    std::lock_guard<std::mutex> lk(mu_);
+    char* p = reinterpret_cast<char*>(s);
+    if (base_ && p >= base_ && p < base_ + kSlots * kSlotBytes) free_.push_back((int)((p - base_) / kSlotBytes));
+    else cudaFreeHost(p);
+  }
+
+ private:
+  static constexpr int kSlots = 256;
+  static constexpr size_t kSlotBytes = 256;
+  static_assert(sizeof(HostStatus) <= kSlotBytes, "slot size");
+  std::mutex mu_;
+  char* base_ = nullptr;
+  std::vector<int> free_;
+};
+StatusPool& status_pool() {
+  static StatusPool* p = new StatusPool();  // never destroyed: handles may outlive static destruction
+  return *p;
+}
 
 }  // namespace
 }  // namespace mfd
@@ -229,6 +284,8 @@ struct mfd_handle {
 
   bool factored = false;
   bool expire_waits = false;                        // test request (mfd_test_expire_waits)
+  bool expire_on_device = false;                    // its value in d_info[2]
+  HostStatus* status = nullptr;
   int64_t pivot_fallbacks = 0;                      // FP32 diagonal sub-blocks redone in FP64, last factorize
   int64_t launches_factor = 0, launches_solve = 0;
   double factor_ms = 0, solve_ms = 0, anorm = 0;
@@ -250,6 +307,7 @@ struct mfd_handle {
 
   ~mfd_handle() {
     if (st) cudaStreamSynchronize(st);
+    status_pool().give(status);
     for (cudaEvent_t e : event_pool) cudaEventDestroy(e);
     if (g_factor) cudaGraphExecDestroy(g_factor);
     for (auto& kv : g_solve) cudaGraphExecDestroy(kv.second);
@@ -944,15 +1002,23 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
   const double w = sizeof(T);
   const bool prof = h->profiling;
   const int32_t* hl = h->h_lists.data();
-  launch_fill_int(h->d_info.p, INT_MAX, 1, st);
-  launch_fill_int(h->d_info.p + 1, 0, 1, st);
-  launch_fill_int(h->d_info.p + 3, 0, 1, st);
-  n += 3;
+  launch_factor_begin(h->d_info.p, st);
+  ++n;
   // trailing update: 0 tensor cores (FP64: DMMA in 128 x 64 halves, two CTAs per SM; FP32: tcgen05 3xTF32),
   // 1 FFMA tiles, 2 tcgen05 1xTF32 (FP32), 3 FP64 DMMA in whole 128 x 128 tiles, one CTA per SM
   const int kind = h->opt.reserved[0];
   const bool side = side_streams(h);
-  bool inverting = false;                   // launches on h->sinv to wait for
+  // values of the permuted full matrix for residuals, next to the factorization
+  cudaStream_t si = side ? h->sinv : st;
+  if (side) {
+    cudaEventRecord(h->ev_inv, st);
+    cudaStreamWaitEvent(si, h->ev_inv, 0);
+  }
+  record(h, si, MFD_K_OTHER, 0, 0, [&] {
+    launch_gather_values(a, h->d_csr_src.p, h->d_csr_val.p, (int64_t)h->d_csr_val.n, si);
+    launch_row_abs_max(h->d_csr_ptr.p, h->d_csr_val.p, h->n_total, h->d_norms.p + 7, si);
+  });
+  n += 2;
   for (const LevelPlan& L : h->levels) {
     // the level's small-front bins and its large fronts are independent (their
     // children are on lower levels; their update matrices are distinct blocks)
@@ -1112,11 +1178,9 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
       }
     }
     // the inverted diagonal blocks serve the solves only: next to the rest of the factorization
-    cudaStream_t si = side ? h->sinv : st;
     if (side) {
       cudaEventRecord(h->ev_inv, st);
       cudaStreamWaitEvent(si, h->ev_inv, 0);
-      inverting = true;
     }
     double vf = 0, vb = 0;
     if (prof)
@@ -1133,16 +1197,12 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
     ++n;
     if (nside) side_join(h, st, nside);
   }
-  if (inverting) {
-    cudaEventRecord(h->ev_inv, h->sinv);
+  if (side) {
+    cudaEventRecord(h->ev_inv, si);
     cudaStreamWaitEvent(st, h->ev_inv, 0);
   }
-  // values of the permuted full matrix for residuals
-  record(h, st, MFD_K_OTHER, 0, 0, [&] {
-    launch_gather_values(a, h->d_csr_src.p, h->d_csr_val.p, (int64_t)h->d_csr_val.n, st);
-    launch_row_abs_max(h->d_csr_ptr.p, h->d_csr_val.p, h->n_total, h->d_norms.p + 7, st);
-  });
-  n += 2;
+  launch_factor_report(h->d_info.p, h->d_norms.p + 7, h->status->info, &h->status->anorm, st);
+  ++n;
   return n;
 }
 
@@ -1288,27 +1348,31 @@ bool is_device_ptr(const void* p) {
   return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
 }
 
+// the test request (mfd_test_expire_waits) into d_info[2], when it changed
+void set_test_request(mfd_handle* h) {
+  if (h->expire_waits == h->expire_on_device) return;
+  launch_fill_int(h->d_info.p + 2, h->expire_waits ? 1 : 0, 1, h->st);
+  h->expire_on_device = h->expire_waits;
+}
+
 int do_factorize(mfd_handle* h, const double* a) {
   if (!a) return fail(MFD_E_ARG, "null values");
   CK(cudaSetDevice(h->device));
   cudaMemcpyKind kind = is_device_ptr(a) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   CK(cudaMemcpyAsync(h->d_a.p, a, sizeof(double) * h->a_len, kind, h->st));
-  launch_fill_int(h->d_info.p + 2, h->expire_waits ? 1 : 0, 1, h->st);
+  set_test_request(h);
   CK(cudaEventRecord(h->ev0, h->st));
   int rc = h->fp32 ? run_graph(h, &h->g_factor, [&](cudaStream_t s) { h->launches_factor = enqueue_factor<float>(h, s); })
                    : run_graph(h, &h->g_factor, [&](cudaStream_t s) { h->launches_factor = enqueue_factor<double>(h, s); });
   if (rc) return rc;
   CK(cudaEventRecord(h->ev1, h->st));
-  int32_t infos[4] = {0, 0, 0, 0};
-  double anorm = 0;
-  CK(cudaMemcpyAsync(infos, h->d_info.p, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, h->st));
-  CK(cudaMemcpyAsync(&anorm, h->d_norms.p + 7, sizeof(double), cudaMemcpyDeviceToHost, h->st));
   CK(cudaStreamSynchronize(h->st));
+  const int32_t* infos = h->status->info;
   float ms = 0;
   cudaEventElapsedTime(&ms, h->ev0, h->ev1);
   collect_profile(h);
   h->factor_ms = ms;
-  h->anorm = anorm;
+  h->anorm = h->status->anorm;
   h->pivot_fallbacks = infos[3];
   h->time_info[6] = ms * 1e-3;
   h->factored = true;
@@ -1328,43 +1392,46 @@ int do_factorize(mfd_handle* h, const double* a) {
   return MFD_OK;
 }
 
-template <typename T>
-int solve_core(mfd_handle* h, int nrhs) {
-  auto it = h->g_solve.find(nrhs);
+// One FP64 solve of d_b in place: permutation, both sweeps, the timing event, with `report` the
+// residual of the first right-hand side and its norms, the inverse permutation, the status.
+int fp64_solve(mfd_handle* h, int nrhs, bool report) {
+  const int64_t n = h->n_total;
+  double* X = static_cast<double*>(h->d_X);
+  const int key = 2 * nrhs + (report ? 1 : 0);
+  auto it = h->g_solve.find(key);
   cudaGraphExec_t exec = it == h->g_solve.end() ? nullptr : it->second;
-  int rc = run_graph(h, &exec, [&](cudaStream_t s) { h->launches_solve = enqueue_solve_core<T>(h, nrhs, s); });
-  if (exec) h->g_solve[nrhs] = exec;
+  const bool graph = h->opt.use_graph && !h->profiling, side = report && side_streams(h);
+  int rc = run_graph(h, &exec, [&](cudaStream_t s) {
+    if (report) {                                    // next to the sweeps: d_b stands until the end
+      if (side) {
+        cudaEventRecord(h->ev_inv, s);
+        cudaStreamWaitEvent(h->sinv, h->ev_inv, 0);
+      }
+      launch_permute_in<double>(h->d_b.p, n, h->d_perm.p, h->d_bp.p, n, n, 1, side ? h->sinv : s);
+      if (side) cudaEventRecord(h->ev_inv, h->sinv);
+    }
+    launch_permute_in<double>(h->d_b.p, n, h->d_perm.p, X, n, n, nrhs, s);
+    h->launches_solve = enqueue_solve_core<double>(h, nrhs, s);
+    cudaEventRecordWithFlags(h->ev1, s, graph ? cudaEventRecordExternal : cudaEventRecordDefault);
+    if (report) {
+      if (side) cudaStreamWaitEvent(s, h->ev_inv, 0);
+      launch_residual(h->d_csr_ptr.p, h->d_csr_col.p, h->d_csr_val.p, X, h->d_bp.p, h->d_r.p, n, s);
+      launch_norms(h->d_r.p, X, h->d_bp.p, n, h->d_norms.p, s);
+    }
+    launch_permute_out<double>(X, n, h->d_perm.p, h->d_b.p, n, n, nrhs, s);
+    launch_solve_report(report ? h->d_norms.p : nullptr, nullptr, nullptr, solve_fused(h, nrhs) ? h->d_ssync.p : nullptr,
+                        h->status->norms, nullptr, nullptr, &h->status->expired, s);
+  });
+  if (exec) h->g_solve[key] = exec;
   return rc;
-}
-
-int residual_report(mfd_handle* h, const double* xp, const double* bp, mfd_report* rep, double* bwd) {
-  launch_residual(h->d_csr_ptr.p, h->d_csr_col.p, h->d_csr_val.p, xp, bp, h->d_r.p, h->n_total, h->st);
-  launch_norms(h->d_r.p, xp, bp, h->n_total, h->d_norms.p, h->st);
-  double nv[5];
-  CK(cudaMemcpyAsync(nv, h->d_norms.p, 5 * sizeof(double), cudaMemcpyDeviceToHost, h->st));
-  CK(cudaStreamSynchronize(h->st));
-  double denom = h->anorm * nv[1] + nv[2];
-  *bwd = denom > 0 ? nv[0] / denom : nv[0];
-  if (rep) {
-    rep->backward_error = *bwd;
-    rep->residual_ref = nv[4] > 0 ? std::sqrt(nv[3]) / std::sqrt(nv[4]) : std::sqrt(nv[3]);
-  }
-  return MFD_OK;
 }
 
 // One refinement sweep on `st`: x_32 = r in FP32, the FP32 solve, x += x_32
 // in FP64, r = b - A x and the per-column norms (launch_norms layout) in FP64.
-// graph_solve: the FP32 solve as its cached graph (host-driven loop), else its
-// launches directly (inside the refinement graph's body).
-int ir_sweep(mfd_handle* h, int nrhs, cudaStream_t st, bool graph_solve) {
+int ir_sweep(mfd_handle* h, int nrhs, cudaStream_t st) {
   const int64_t n = h->n_total;
   launch_to_t<float>(h->d_r.p, static_cast<float*>(h->d_X), n * nrhs, st);
-  if (graph_solve) {
-    int rc = solve_core<float>(h, nrhs);
-    if (rc) return rc;
-  } else {
-    h->launches_solve = enqueue_solve_core<float>(h, nrhs, st);
-  }
+  h->launches_solve = enqueue_solve_core<float>(h, nrhs, st);
   launch_axpy_from_t<float>(static_cast<float*>(h->d_X), h->d_xp.p, n * nrhs, st);
   if (nrhs >= kResMulti) {               // A read once for all columns
     launch_residual_multi(h->d_csr_ptr.p, h->d_csr_col.p, h->d_csr_val.p, h->d_xp.p, h->d_xt.p, h->d_bp.p,
@@ -1415,7 +1482,7 @@ int ir_graph(mfd_handle* h, int nrhs) {
       cudaGraph_t body = cp.conditional.phGraph_out[0];
       e = cudaStreamBeginCaptureToGraph(h->bst, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
       if (e == cudaSuccess) {
-        int rc = ir_sweep(h, nrhs, h->bst, /*graph_solve=*/false);
+        int rc = ir_sweep(h, nrhs, h->bst);
         launch_ir_check(h->d_cnorms.p, h->d_norms.p + 7, nrhs, h->opt.ir_tol, maxit, h->d_ir_prev.p, h->d_ir_i.p,
                         h->d_ir_d.p, cond, h->bst);
         cudaGraph_t got = nullptr;
@@ -1425,6 +1492,8 @@ int ir_graph(mfd_handle* h, int nrhs) {
       }
     }
     launch_permute_out<double>(h->d_xp.p, n, h->d_perm.p, h->d_b.p, n, n, nrhs, st);
+    launch_solve_report(nullptr, h->d_ir_i.p, h->d_ir_d.p, solve_fused(h, nrhs) ? h->d_ssync.p : nullptr, nullptr,
+                        h->status->ir_i, h->status->ir_d, &h->status->expired, st);
     cudaGraph_t outer = nullptr;
     cudaError_t e3 = cudaStreamEndCapture(st, &outer);
     if (e == cudaSuccess) e = e3;
@@ -1455,41 +1524,22 @@ int do_solve(mfd_handle* h, double* b, int nrhs, int64_t ldb, mfd_report* rep) {
     CK(cudaMemcpy2DAsync(h->d_b.p, sizeof(double) * n, b, sizeof(double) * ldb, sizeof(double) * n, nrhs,
                          dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
   }
-  launch_fill_int(h->d_info.p + 2, h->expire_waits ? 1 : 0, 1, st);   // test request (mfd_test_expire_waits)
+  set_test_request(h);
   CK(cudaEventRecord(h->ev0, st));
   int iters = 0;
   double bwd = 0;
-  bool want_report = rep != nullptr || h->fp32;
+  const bool ir_graphed = h->fp32 && h->opt.use_graph && !h->profiling;
+  h->status->expired = 0;
   if (!h->fp32) {
-    launch_permute_in<double>(h->d_b.p, n, h->d_perm.p, static_cast<double*>(h->d_X), n, n, nrhs, st);
-    rc = solve_core<double>(h, nrhs);
+    rc = fp64_solve(h, nrhs, rep != nullptr);
     if (rc) return rc;
-    CK(cudaEventRecord(h->ev1, st));
-    if (want_report) {
-      launch_permute_in<double>(h->d_b.p, n, h->d_perm.p, h->d_bp.p, n, n, 1, st);
-      rc = residual_report(h, static_cast<double*>(h->d_X), h->d_bp.p, rep, &bwd);
-      if (rc) return rc;
-    }
-    launch_permute_out<double>(static_cast<double*>(h->d_X), n, h->d_perm.p, h->d_b.p, n, n, nrhs, st);
-  } else if (h->opt.use_graph && !h->profiling) {
+  } else if (ir_graphed) {
     // FP32 factor + FP64 iterative refinement as one graph per right-hand-side
     // count: the sweeps run in a WHILE node whose last kernel applies the
     // convergence test on the device, so the host waits once per solve
     rc = ir_graph(h, nrhs);
     if (rc) return rc;
-    int32_t si[2];
-    double sd[2];
-    CK(cudaMemcpyAsync(si, h->d_ir_i.p, sizeof(si), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(sd, h->d_ir_d.p, sizeof(sd), cudaMemcpyDeviceToHost, st));
     CK(cudaEventRecord(h->ev1, st));
-    CK(cudaStreamSynchronize(st));
-    iters = si[0];
-    bwd = sd[0];
-    if (rep) {
-      rep->backward_error = bwd;
-      rep->residual_ref = sd[1];
-    }
-    if (!(bwd <= h->opt.ir_tol)) rc = MFD_E_NOCONV;
   } else {
     // FP32 factor + FP64 iterative refinement, all right-hand sides together,
     // the convergence test on the host after every sweep (schedule without
@@ -1502,7 +1552,7 @@ int do_solve(mfd_handle* h, double* b, int nrhs, int64_t ldb, mfd_report* rep) {
     double worst_ref = 0;
     int it = 0;
     for (; it < maxit; ++it) {
-      rc = ir_sweep(h, nrhs, st, /*graph_solve=*/true);
+      rc = ir_sweep(h, nrhs, st);
       if (rc) return rc;
       CK(cudaMemcpyAsync(nv.data(), h->d_cnorms.p, sizeof(double) * 8 * nrhs, cudaMemcpyDeviceToHost, st));
       CK(cudaStreamSynchronize(st));
@@ -1540,10 +1590,27 @@ int do_solve(mfd_handle* h, double* b, int nrhs, int64_t ldb, mfd_report* rep) {
     CK(cudaMemcpy2DAsync(b, sizeof(double) * ldb, h->d_b.p, sizeof(double) * n, sizeof(double) * n, nrhs,
                          dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
   }
-  int32_t expired = 0;                      // a bounded wait of the fused large-front sweeps gave up
-  if (solve_fused(h, nrhs)) CK(cudaMemcpyAsync(&expired, h->d_ssync.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+  if (h->fp32 && !ir_graphed)
+    launch_solve_report(nullptr, nullptr, nullptr, solve_fused(h, nrhs) ? h->d_ssync.p : nullptr, nullptr, nullptr, nullptr,
+                        &h->status->expired, st);
   CK(cudaStreamSynchronize(st));
-  if (expired) return fail(MFD_E_TIMEOUT, "a device wait of the solve timed out");
+  const HostStatus& hs = *h->status;
+  if (hs.expired) return fail(MFD_E_TIMEOUT, "a device wait of the solve timed out");   // of the large-front sweeps
+  if (!h->fp32 && rep) {
+    const double* nv = hs.norms;
+    const double denom = h->anorm * nv[1] + nv[2];
+    bwd = denom > 0 ? nv[0] / denom : nv[0];
+    rep->backward_error = bwd;
+    rep->residual_ref = nv[4] > 0 ? std::sqrt(nv[3]) / std::sqrt(nv[4]) : std::sqrt(nv[3]);
+  } else if (ir_graphed) {
+    iters = hs.ir_i[0];
+    bwd = hs.ir_d[0];
+    if (rep) {
+      rep->backward_error = bwd;
+      rep->residual_ref = hs.ir_d[1];
+    }
+    if (!(bwd <= h->opt.ir_tol)) rc = MFD_E_NOCONV;
+  }
   float ms = 0;
   cudaEventElapsedTime(&ms, h->ev0, h->ev1);
   collect_profile(h);
@@ -1570,6 +1637,8 @@ int create_common(mfd_handle** out, std::vector<Symbolic>&& syms, const mfd_opti
   h->sys = std::move(syms);
   CK(cudaSetDevice(h->device));
   CK(prepare_kernels());
+  h->status = status_pool().take();
+  if (!h->status) return fail(MFD_E_NOMEM, "no page-locked memory for a handle's status");
   int prio_lo = 0, prio_hi = 0;
   CK(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi));
   CK(cudaStreamCreateWithPriority(&h->st, cudaStreamNonBlocking, prio_hi));

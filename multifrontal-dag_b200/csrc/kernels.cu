@@ -1402,6 +1402,34 @@ void launch_ir_check(const double* norms, const double* anorm, int nrhs, double 
   k_ir_check<<<1, 32, 0, st>>>(norms, anorm, nrhs, tol, maxit, prev, st_i, st_d, cond);
 }
 
+__global__ void k_factor_begin(int32_t* info) {
+  info[0] = INT_MAX;
+  info[1] = 0;
+  info[3] = 0;
+}
+void launch_factor_begin(int32_t* info, cudaStream_t st) { k_factor_begin<<<1, 1, 0, st>>>(info); }
+__global__ void k_factor_report(const int32_t* info, const double* anorm, int32_t* h_info, double* h_anorm) {
+  if (threadIdx.x < 4) h_info[threadIdx.x] = info[threadIdx.x];
+  if (threadIdx.x == 4) *h_anorm = *anorm;
+}
+void launch_factor_report(const int32_t* info, const double* anorm, int32_t* h_info, double* h_anorm, cudaStream_t st) {
+  k_factor_report<<<1, 32, 0, st>>>(info, anorm, h_info, h_anorm);
+}
+__global__ void k_solve_report(const double* norms, const int32_t* ir_i, const double* ir_d, const int32_t* expired,
+                               double* h_norms, int32_t* h_ir_i, double* h_ir_d, int32_t* h_expired) {
+  const int t = threadIdx.x;
+  if (norms && t < 5) h_norms[t] = norms[t];
+  if (ir_i && t < 2) {
+    h_ir_i[t] = ir_i[t];
+    h_ir_d[t] = ir_d[t];
+  }
+  if (expired && t == 5) *h_expired = *expired;
+}
+void launch_solve_report(const double* norms, const int32_t* ir_i, const double* ir_d, const int32_t* expired,
+                         double* h_norms, int32_t* h_ir_i, double* h_ir_d, int32_t* h_expired, cudaStream_t st) {
+  k_solve_report<<<1, 32, 0, st>>>(norms, ir_i, ir_d, expired, h_norms, h_ir_i, h_ir_d, h_expired);
+}
+
 __global__ void k_remap_int(const int32_t* map, int32_t* a, int64_t n) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     a[i] = map[a[i]];

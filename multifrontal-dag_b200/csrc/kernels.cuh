@@ -272,6 +272,12 @@ void launch_to_t(const double* in, T* out, int64_t n, cudaStream_t st);
 template <typename T>
 void launch_axpy_from_t(const T* d, double* x, int64_t n, cudaStream_t st);
 void launch_fill_int(int32_t* p, int32_t v, int64_t n, cudaStream_t st);
+// First and last kernel of a factorization, last kernel of a solve: reset of info (first bad pivot,
+// expiry flag, fallback count); what the host reads, into its page-locked status (null: not written).
+void launch_factor_begin(int32_t* info, cudaStream_t st);
+void launch_factor_report(const int32_t* info, const double* anorm, int32_t* h_info, double* h_anorm, cudaStream_t st);
+void launch_solve_report(const double* norms, const int32_t* ir_i, const double* ir_d, const int32_t* expired,
+                         double* h_norms, int32_t* h_ir_i, double* h_ir_d, int32_t* h_expired, cudaStream_t st);
 // a[i] = map[a[i]] for i < n
 void launch_remap_int(const int32_t* map, int32_t* a, int64_t n, cudaStream_t st);
 
