@@ -43,6 +43,7 @@ int fail(int code, const std::string& msg) {
 constexpr int64_t kAlign = 32;  // elements; keeps every front 256-byte aligned in FP64
 constexpr int kResMulti = 4;     // from this many right-hand sides on, one multi-column residual per IR sweep
 constexpr int kPotrfSplitMin = 148;   // fronts in a panel step above which POTRF launches per width class
+constexpr int kWarpFrontsAtOnce = 148 * 24;   // one-warp fronts the chip holds at once
 // panel steps per deferred trailing update: K = 256 per pass halves the update's C traffic, which
 // counts on levels whose trailing matrices pass through HBM, their lower triangles above half of the
 // 126 MB L2 (80^3 diffusion, mixed: 45.7 -> 40.7 ms).  Below, a deferred update only lengthens the
@@ -216,11 +217,10 @@ struct mfd_handle {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // a level's independent launches (small-front size bins) on side streams,
   // forked from st at the level's start and joined back at its end
-  static constexpr int kSide = 6;
+  static constexpr int kSide = 4;
   cudaStream_t sst[kSide] = {};
   cudaEvent_t ev_lvl = nullptr, ev_side[kSide] = {};
-  cudaStream_t sinv = nullptr;                      // inverted diagonal blocks, off the panel chain
-  cudaEvent_t ev_inv = nullptr;
+  cudaEvent_t ev_inv = nullptr;                     // on bst: work next to the main chain
 
   // systems
   std::vector<Symbolic> sys;
@@ -294,7 +294,9 @@ struct mfd_handle {
   cudaGraphExec_t g_factor = nullptr;
   std::map<int, cudaGraphExec_t> g_solve;
   std::map<int, cudaGraphExec_t> g_ir;              // FP32 + FP64 refinement, whole loop per RHS count
-  cudaStream_t bst = nullptr;                       // captures the refinement loop's body
+  // captures the refinement loop's body; in other graphs what runs next to the main chain for a
+  // whole factorization or solve (inverted diagonal blocks, the residual's matrix and right-hand side)
+  cudaStream_t bst = nullptr;
   DBuf<int32_t> d_ir_i;                             // refinement state (launch_ir_init / launch_ir_check)
   DBuf<double> d_ir_d, d_ir_prev;
 
@@ -323,7 +325,6 @@ struct mfd_handle {
       if (e) cudaEventDestroy(e);
     if (ev_lvl) cudaEventDestroy(ev_lvl);
     if (ev_inv) cudaEventDestroy(ev_inv);
-    if (sinv) cudaStreamDestroy(sinv);
     for (int b = 0; b < kSide; ++b) {
       if (ev_side[b]) cudaEventDestroy(ev_side[b]);
       if (sst[b]) cudaStreamDestroy(sst[b]);
@@ -336,8 +337,6 @@ struct mfd_handle {
 namespace {
 
 int small_front_max(const mfd_handle* h) {
-  // fronts above 128 go to the blocked path: measured on the 64^3 Laplacian,
-  // 128 is as fast as 160 (FP64) and 1.3 ms faster than 224 (FP32)
   int lim = kSmallFrontMax;
   if (h->opt.small_front_max > 0) lim = std::min(lim, h->opt.small_front_max);
   return lim;
@@ -462,7 +461,7 @@ int build_plan(mfd_handle* h) {
     h->upool_elems = std::max<int64_t>(ff.top, kAlign);
   }
   // level launch lists
-  h->small_bins = std::vector<int>{16, 24, 32, 64, 96, 128};
+  h->small_bins = std::vector<int>{16, 24, 32, 64, 96, 128, 160};
   while (!h->small_bins.empty() && h->small_bins.back() > sfm) h->small_bins.pop_back();
   if (h->small_bins.empty() || h->small_bins.back() < sfm) h->small_bins.push_back(sfm);
   h->levels.assign(nlev, LevelPlan{});
@@ -477,11 +476,22 @@ int build_plan(mfd_handle* h) {
     LevelPlan& L = h->levels[l];
     std::vector<std::vector<int32_t>> bins(h->small_bins.size());
     std::vector<int32_t> large;
+    // the one-warp fronts in one launch sized for the largest unless they fill the chip more than
+    // once: below that the launches' number counts, not their warps' registers and shared memory
+    int warp_fronts = 0, warp_max = 0;
+    for (int32_t g : lev_fronts[l]) {
+      const int nf = h->fronts[g].nc + h->fronts[g].nr;
+      if (nf > 32) continue;
+      ++warp_fronts;
+      warp_max = std::max(warp_max, nf);
+    }
+    const bool split_warp_bins = warp_fronts > kWarpFrontsAtOnce;
     for (int32_t g : lev_fronts[l]) {
       int nf = h->fronts[g].nc + h->fronts[g].nr;
       if (nf <= sfm) {
+        const int fit = nf <= 32 && !split_warp_bins ? warp_max : nf;
         size_t b = 0;
-        while (h->small_bins[b] < nf) ++b;
+        while (h->small_bins[b] < fit) ++b;
         bins[b].push_back(g);
       } else {
         large.push_back(g);
@@ -799,8 +809,8 @@ int upload_plan(mfd_handle* h) {
     }
   }
 
-  // the children of large fronts: the inverse of their local index
-  {
+  // the children of large fronts: the inverse of their local index; the fronts' and children's records
+  if (h->max_large_count > 0) {
     std::vector<int64_t> ioff(nfr, 0);
     std::vector<int32_t> kids;
     int64_t len = 0;
@@ -819,12 +829,12 @@ int upload_plan(mfd_handle* h) {
     DBuf<int32_t> d_kids;
     CK(d_kids.upload(kids, st));
     launch_inverse_index(F, d_kids.p, (int)kids.size(), h->d_inv.p, st);
-    CK(h->d_rec.alloc(h->h_lists.size()));
-    CK(h->d_crec.alloc(h->h_child.size()));
-    F.crec = h->d_crec.p;
-    launch_records(F, h->d_lists.p, (int)h->h_lists.size(), h->d_rec.p, (int)h->h_child.size(), h->d_crec.p, st);
     CK(cudaStreamSynchronize(st));       // d_kids and the host tables go out of scope
   }
+  CK(h->d_rec.alloc(h->h_lists.size()));
+  CK(h->d_crec.alloc(h->h_child.size()));
+  F.crec = h->d_crec.p;
+  launch_records(F, h->d_lists.p, (int)h->h_lists.size(), h->d_rec.p, (int)h->h_child.size(), h->d_crec.p, st);
 
   h->setup_s[2] = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   t0 = std::chrono::steady_clock::now();
@@ -859,7 +869,8 @@ int upload_plan(mfd_handle* h) {
   CK(cudaMalloc(&h->d_panel, (std::max<int64_t>(h->panel_elems, 1) + 32) * esz));
   CK(cudaMalloc(&h->d_upool, std::max<int64_t>(h->upool_elems, 1) * esz));
   CK(cudaMalloc(&h->d_diag, (size_t)std::max<int64_t>(h->dinv_elems, 1) * esz));
-  CK(cudaMalloc(&h->d_packed, (size_t)std::max(1, h->max_large_count) * kPackedPanelElems * sizeof(double)));
+  if (h->max_large_count > 0)
+    CK(cudaMalloc(&h->d_packed, (size_t)h->max_large_count * kPackedPanelElems * sizeof(double)));
   if (h->fp32 && h->q_elems > 0 && h->defer <= kPackedDefer) {
     CK(cudaMalloc(&h->d_q, (size_t)(2 * h->defer * h->q_elems) * sizeof(float)));
     // rows past a front's last row are never written and only reach discarded outputs; zero keeps them finite
@@ -1009,7 +1020,7 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
   const int kind = h->opt.reserved[0];
   const bool side = side_streams(h);
   // values of the permuted full matrix for residuals, next to the factorization
-  cudaStream_t si = side ? h->sinv : st;
+  cudaStream_t si = side ? h->bst : st;
   if (side) {
     cudaEventRecord(h->ev_inv, st);
     cudaStreamWaitEvent(si, h->ev_inv, 0);
@@ -1405,10 +1416,10 @@ int fp64_solve(mfd_handle* h, int nrhs, bool report) {
     if (report) {                                    // next to the sweeps: d_b stands until the end
       if (side) {
         cudaEventRecord(h->ev_inv, s);
-        cudaStreamWaitEvent(h->sinv, h->ev_inv, 0);
+        cudaStreamWaitEvent(h->bst, h->ev_inv, 0);
       }
-      launch_permute_in<double>(h->d_b.p, n, h->d_perm.p, h->d_bp.p, n, n, 1, side ? h->sinv : s);
-      if (side) cudaEventRecord(h->ev_inv, h->sinv);
+      launch_permute_in<double>(h->d_b.p, n, h->d_perm.p, h->d_bp.p, n, n, 1, side ? h->bst : s);
+      if (side) cudaEventRecord(h->ev_inv, h->bst);
     }
     launch_permute_in<double>(h->d_b.p, n, h->d_perm.p, X, n, n, nrhs, s);
     h->launches_solve = enqueue_solve_core<double>(h, nrhs, s);
@@ -1643,7 +1654,7 @@ int create_common(mfd_handle** out, std::vector<Symbolic>&& syms, const mfd_opti
   CK(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi));
   CK(cudaStreamCreateWithPriority(&h->st, cudaStreamNonBlocking, prio_hi));
   CK(cudaStreamCreateWithPriority(&h->st2, cudaStreamNonBlocking, prio_lo));
-  CK(cudaStreamCreateWithPriority(&h->bst, cudaStreamNonBlocking, prio_hi));
+  CK(cudaStreamCreateWithPriority(&h->bst, cudaStreamNonBlocking, prio_lo));
   CK(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
   for (int k = 0; k < mfd_handle::kMaxDefer; ++k) CK(cudaEventCreateWithFlags(&h->ev_part[k], cudaEventDisableTiming));
@@ -1652,7 +1663,6 @@ int create_common(mfd_handle** out, std::vector<Symbolic>&& syms, const mfd_opti
                                      : kDeferDefault;
   CK(cudaEventCreateWithFlags(&h->ev_lvl, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&h->ev_inv, cudaEventDisableTiming));
-  CK(cudaStreamCreateWithPriority(&h->sinv, cudaStreamNonBlocking, prio_lo));
   for (int b = 0; b < mfd_handle::kSide; ++b) {
     CK(cudaStreamCreateWithPriority(&h->sst[b], cudaStreamNonBlocking, prio_lo));
     CK(cudaEventCreateWithFlags(&h->ev_side[b], cudaEventDisableTiming));

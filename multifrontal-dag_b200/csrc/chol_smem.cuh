@@ -61,196 +61,229 @@ __device__ __forceinline__ void named_barrier(int threads) {
   asm volatile("bar.sync %0, %1;" ::"n"(ID), "r"(threads) : "memory");
 }
 
-// One warp's share (warp u of nu) of the rank-8 update of block columns js ..
-// nbt - 1 by panel p: block rows in a there-and-back order, so that two rows of
-// a warp have as many blocks as any other two.  row_done(i) follows block row i.
-template <typename RowDone>
-__device__ __forceinline__ void panel_update(double* S, int p, int js, int nbt, int u, int nu, int lane,
-                                             RowDone&& row_done) {
-  const int fo = blk_frag(lane);
-  const double* Lp = S + blk_index(p, p, nbt) * kBlkElems + fo;       // block (i, p) at Lp + 64 (i - p)
-  for (int m = 0; js + m < nbt; m += 2 * nu) {
+// Row and column of the t-th tile of a lower triangle, row by row (the same for every size).
+__device__ __forceinline__ void tile_table(uint16_t* tab, int rows) {
+  for (int i = threadIdx.x >> 5; i < rows; i += blockDim.x >> 5)
+    for (int j = threadIdx.x & 31; j <= i; j += 32) tab[i * (i + 1) / 2 + j] = (uint16_t)(i << 8 | j);
+}
+
+// Block columns js .. nbt - 1 -= the K panels p .. p + K - 1, warp u of nu, in 2 x 2
+// blocks.  Shared memory bounds it (a block moves in 4 cycles): single blocks a
+// panel at a time take 16 cycles per block and panel, 2 x 2 of two panels 8.
+template <int K>
+__device__ __forceinline__ void panel_update(double* S, const uint16_t* tab, int p, int js, int nbt, int u, int nu,
+                                             int lane) {
+  const int fo = blk_frag(lane), T = (nbt - js + 1) / 2;
+  for (int t = u; t < T * (T + 1) / 2; t += nu) {
+    const int ij = tab[t], i0 = js + 2 * (ij >> 8), j0 = js + 2 * (ij & 255);
+    double2 a[K][2], b[K][2], c[2][2];
 #pragma unroll
-    for (int hh = 0; hh < 2; ++hh) {
-      const int i = js + m + (hh ? 2 * nu - 1 - u : u);
-      if (i >= nbt) continue;
-      double2 a = *reinterpret_cast<const double2*>(Lp + (i - p) * kBlkElems);
-      a.x = -a.x;
-      a.y = -a.y;
-      for (int j0 = js; j0 <= i; j0 += 4) {
-        double2 b[4], c[4];
+    for (int k = 0; k < K; ++k) {
+      const double* L = S + (blk_index(p + k, p + k, nbt) - (p + k)) * kBlkElems + fo;   // block (i, p + k) at L + 64 i
 #pragma unroll
-        for (int v = 0; v < 4; ++v)
-          if (j0 + v <= i) {
-            b[v] = *reinterpret_cast<const double2*>(Lp + (j0 + v - p) * kBlkElems);
-            c[v] = *reinterpret_cast<const double2*>(S + blk_index(i, j0 + v, nbt) * kBlkElems + fo);
-          }
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-          if (j0 + v <= i) dmma8(c[v], a, b[v]);
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-          if (j0 + v <= i) *reinterpret_cast<double2*>(S + blk_index(i, j0 + v, nbt) * kBlkElems + fo) = c[v];
+      for (int v = 0; v < 2; ++v) {
+        a[k][v] = *reinterpret_cast<const double2*>(L + min(i0 + v, nbt - 1) * kBlkElems);
+        b[k][v] = *reinterpret_cast<const double2*>(L + min(j0 + v, nbt - 1) * kBlkElems);
+        a[k][v] = make_double2(-a[k][v].x, -a[k][v].y);
       }
-      row_done(i);
     }
+    // block (i0 + v, j0 + w); above the diagonal or past the last block: not there
+    auto there = [&](int v, int w) { return i0 + v < nbt && j0 + w < nbt && i0 + v >= j0 + w; };
+    auto at = [&](int v, int w) { return reinterpret_cast<double2*>(S + blk_index(i0 + v, j0 + w, nbt) * kBlkElems + fo); };
+#pragma unroll
+    for (int v = 0; v < 2; ++v)
+#pragma unroll
+      for (int w = 0; w < 2; ++w)
+        if (there(v, w)) c[v][w] = *at(v, w);
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+      for (int v = 0; v < 2; ++v)
+#pragma unroll
+        for (int w = 0; w < 2; ++w)
+          if (there(v, w)) dmma8(c[v][w], a[k][v], b[k][w]);
+#pragma unroll
+    for (int v = 0; v < 2; ++v)
+#pragma unroll
+      for (int w = 0; w < 2; ++w)
+        if (there(v, w)) *at(v, w) = c[v][w];
+  }
+}
+// Block column p + 1 alone, one block per warp at a time.
+__device__ __forceinline__ void next_column_update(double* S, int p, int nbt, int u, int nu, int lane) {
+  const int fo = blk_frag(lane);
+  const double* L = S + (blk_index(p, p, nbt) - p) * kBlkElems + fo;
+  for (int i = p + 1 + u; i < nbt; i += nu) {
+    double2* C = reinterpret_cast<double2*>(S + blk_index(i, p + 1, nbt) * kBlkElems + fo);
+    double2 a = *reinterpret_cast<const double2*>(L + i * kBlkElems), c = *C;
+    dmma8(c, make_double2(-a.x, -a.y), *reinterpret_cast<const double2*>(L + (p + 1) * kBlkElems));
+    *C = c;
   }
 }
 
-// Scratch of chol_panels in shared memory, in doubles: two staged diagonal
-// blocks and the pivots' reciprocal roots; with small-pivot tracking the
-// diagonal entries its test compares with.
+// Scratch of chol_panels in shared memory, in doubles: two 4 x 4 exchange blocks,
+// the pivots' reciprocal roots, with small-pivot tracking the diagonal its test
+// compares with, and the tile table.
 __host__ __device__ constexpr int chol_scratch_elems(int max_rows, bool track) {
-  return 2 * kBlkElems + max_rows * (track ? 2 : 1);
+  return 32 + max_rows * (track ? 2 : 1) + (blk_count((max_rows / 8 + 1) / 2) + 3) / 4;
+}
+
+// Cholesky of the N x N lower block a (redundantly by every thread that calls
+// it), the thread's own row x carried along: x <- x L^{-T}.  a[k][k] ends as the
+// pivots (a non-positive one counts as 1), y as their 1 / sqrt; nothing but the
+// arithmetic is on the chain, the caller looks at the pivots afterwards.
+template <int N>
+__device__ __forceinline__ void chol_row(double (&a)[N][N], double* x, double (&y)[N]) {
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const double r = rsqrt(a[k][k]);
+    y[k] = a[k][k] > 0.0 ? r : 1.0;
+    x[k] *= y[k];
+    double l[N];
+#pragma unroll
+    for (int i = k + 1; i < N; ++i) l[i] = a[i][k] * y[k];
+#pragma unroll
+    for (int j = k + 1; j < N; ++j) {
+#pragma unroll
+      for (int i = j; i < N; ++i) a[i][j] = fma(-l[i], l[j], a[i][j]);
+      x[j] = fma(-x[k], l[j], x[j]);
+    }
+  }
 }
 
 // Right-looking partial Cholesky of the first nbp of nbt block columns of S,
 // in place: L in the first nbp block columns, the Schur complement of the rest.
-// Run by (PW + UW) warps, nbt <= 4 PW.  Two roles:
-//   panel warps (the first PW, thread t owns row t): every thread factors the
-//     current 8 x 8 diagonal block redundantly in registers, its own row
-//     carried along as a ninth one, so that a pivot costs one 1/sqrt, one
-//     product and one multiply-add of latency and no exchange between lanes;
-//     then, with the finished panel visible, its row of the next block column;
-//   update warps: the panel's rank-8 update of the block columns after the
-//     next, on m8n8k4 DMMA, while the panel warps factor the next panel.
-// The last panel's update is shared by all warps.
-// Dinv (optional, nbp blocks): the inverses of the diagonal blocks.
-// track: dgs holds, per 32-column group, the diagonal as it stood when the
-// group was reached, and on_small() is called once per group with a pivot not
-// above 2^-12 of it; on_bad(j) with the first non-positive pivot (0-based).
-// The caller synchronises before (S complete) and after.
+// Run by NW warps with 8 nbt <= 32 NW; thread t owns row t.  Per block column:
+//   factor, by the warps with rows at or below the diagonal block: every thread
+//     factors it redundantly in registers, its own row carried along, so that a
+//     pivot needs no exchange between lanes; in two 4 x 4 blocks, rows 4..7 of L
+//     and the second block exchanged through shared memory;
+//   update: all warps, on m8n8k4 DMMA, two panels at a time.
+// rq (in scratch): 1 / L_kk.  track: on_small() once per 32-column group with a
+// pivot not above 2^-12 of the diagonal entry it had when the group was reached;
+// on_bad(j): a non-positive pivot (0-based; the first one counts).  The caller
+// synchronises before (S complete) and after.
 //
-// What bounds it: the pivot chain, 73 cycles per column (rsqrt 55, DMUL 9,
-// DFMA 9) plus about 400 per 8 columns for the exchange of the next diagonal
-// block and two barriers.
-template <int PW, int UW, bool kInv, bool kTrack, typename OnBad, typename OnSmall>
-__device__ __forceinline__ void chol_panels(double* S, double* scratch, double* Dinv, int nbp, int nbt, OnBad&& on_bad,
+// What bounds it: the chain of pivots, 105 cycles each (rsqrt 55, DMUL 9, DFMA 9,
+// the issue of one warp's FP64 at 4.5 cycles per instruction), 1,330 cycles per
+// eight columns with the exchanges; then the update's shared-memory traffic.
+// Measured alternatives, 128 x 128: factor and update side by side in different
+// warps 2,450 cycles per panel (both slow each other down), 8 x 8 blocks without
+// the exchanges 1,500 per factor and 175 registers for 110.
+constexpr int kCholRq = 32;       // offset of rq in the scratch
+template <int NW, bool kTrack, typename OnBad, typename OnSmall>
+__device__ __forceinline__ void chol_panels(double* S, double* scratch, int nbp, int nbt, OnBad&& on_bad,
                                             OnSmall&& on_small) {
-  double* Dst = scratch;                       // 2 x 64: the diagonal block being factored, by panel parity
-  double* rq = scratch + 2 * kBlkElems;         // 8 per panel: 1 / L_kk
-  double* dgs = rq + 32 * PW;                   // kTrack: reference diagonal
+  constexpr int N = 4;
+  double* low = scratch;                                 // rows 4..7 of the diagonal block: L's first four columns
+  double* next = scratch + 16;                            // and their last four, before the second 4 x 4 block
+  double* rq = scratch + kCholRq;
+  double* dgs = rq + 8 * nbp;                            // kTrack
+  uint16_t* tab = reinterpret_cast<uint16_t*>(dgs + (kTrack ? 8 * nbp : 0));
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  if (warp < PW) {
-    const int R = t >> 3, rr = t & 7;
-    double x[8];
+  const int R = t >> 3, rr = t & 7;
+  tile_table(tab, (nbt + 1) / 2);
+  bool small = false;
+  for (int p = 0; p < nbp; ++p) {
+    if (4 * warp + 3 >= p && 4 * warp < nbt) {           // the warp has rows at or below the diagonal block
+      const int bar = 32 * ((nbt + 3) / 4 - p / 4);      // threads of such warps
+      const double* D = S + blk_index(p, p, nbt) * kBlkElems;
+      const bool mine = R >= p && R < nbt;
+      double a[N][N], x[8], dg[N];
+      auto load = [&](auto at) {                         // at(i, c): columns 2 c, 2 c + 1 of row i
 #pragma unroll
-    for (int k = 0; k < 8; ++k) x[k] = 0.0;
-    if (R < nbt) blk_load_row(S + blk_index(R, 0, nbt) * kBlkElems, rr, x);
-    if (R == 0) blk_store_row(Dst, rr, x);
-    if (kTrack && R < 4 && R < nbp) dgs[t] = S[blk_index(R, R, nbt) * kBlkElems + blk_elem(rr, rr)];
-    named_barrier<1>(32 * PW);
-    bool reported = false, small = false;
-    for (int p = 0; p < nbp; ++p) {
-      if (4 * warp + 3 >= p && 4 * warp < nbt) {         // the warp still has rows at or below the diagonal block
-        double a[8][8];
-        const double* D = Dst + (p & 1) * kBlkElems;
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < N; ++i)
 #pragma unroll
           for (int c = 0; c <= i / 2; ++c) {
-            const double2 v = *reinterpret_cast<const double2*>(D + blk_elem(i, 2 * c));
+            const double2 v = at(i, c);
             a[i][2 * c] = v.x;
-            if (2 * c + 1 <= i) a[i][2 * c + 1] = v.y;
+            a[i][2 * c + 1] = v.y;
           }
+      };
+      load([&](int i, int c) { return *reinterpret_cast<const double2*>(D + blk_elem(i, 2 * c)); });
+      blk_load_row(S + blk_index(mine ? R : p, p, nbt) * kBlkElems, rr, x);
+      if constexpr (kTrack) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          double d = a[k][k];
-          if constexpr (kTrack) small |= !(d > dgs[8 * p + k] * (1.0 / 4096.0));
-          if (!(d > 0.0)) {                              // uniform: every thread holds the same block
-            if (!reported) {
-              if (t == 8 * p) on_bad(8 * p + k);
-              reported = true;
-            }
-            d = 1.0;
-          }
-          const double y = rsqrt(d);
-          if (t == 8 * p) rq[8 * p + k] = y;
-          x[k] *= y;
-          double l[8];
+        for (int k = 0; k < N; ++k) dg[k] = (p & 3) == 0 ? a[k][k] : dgs[8 * p + k];
+        if ((p & 3) == 0 && mine && R < min(p + 4, nbp)) dgs[t] = S[blk_index(R, R, nbt) * kBlkElems + blk_elem(rr, rr)];
+      }
+      auto factor = [&](int o) {                         // columns o .. o + N - 1 of the panel
+        double y[N];
+        chol_row<N>(a, x + o, y);
+        bool good = true;
 #pragma unroll
-          for (int i = k + 1; i < 8; ++i) l[i] = a[i][k] * y;
-#pragma unroll
-          for (int j = k + 1; j < 8; ++j) {
-#pragma unroll
-            for (int i = j; i < 8; ++i) a[i][j] = fma(-l[i], l[j], a[i][j]);
-            x[j] = fma(-x[k], l[j], x[j]);
-          }
+        for (int k = 0; k < N; ++k) {
+          good &= a[k][k] > 0.0;
+          if constexpr (kTrack) small |= !(a[k][k] > dg[k] * (1.0 / 4096.0));
         }
-        if (R >= p && R < nbt) blk_store_row(S + blk_index(R, p, nbt) * kBlkElems, rr, x);
-        if constexpr (kTrack)
-          if ((p & 3) == 3 || p + 1 == nbp) {
-            if (small && t == 8 * p) on_small();
-            small = false;
-          }
+        if (t == 8 * p) {
+#pragma unroll
+          for (int k = 0; k < N; k += 2) *reinterpret_cast<double2*>(rq + 8 * p + o + k) = make_double2(y[k], y[k + 1]);
+          if (!good)
+#pragma unroll
+            for (int k = N - 1; k >= 0; --k)             // the first one last: the caller keeps the smallest
+              if (!(a[k][k] > 0.0)) on_bad(8 * p + o + k);
+        }
+      };
+      factor(0);
+      if (R == p && rr >= 4) {
+        *reinterpret_cast<double2*>(low + 4 * (rr - 4)) = make_double2(x[0], x[1]);
+        *reinterpret_cast<double2*>(low + 4 * (rr - 4) + 2) = make_double2(x[2], x[3]);
       }
       __syncwarp();
-      named_barrier<0>(32 * (PW + UW));                  // panel p complete; every update up to panel p - 1 applied
-      if (p + 1 < nbp) {
-        if (4 * warp + 3 > p && 4 * warp < nbt) {
-          double c[8];
-          const int Rc = R > p && R < nbt ? R : p + 1;
-          blk_load_row(S + blk_index(Rc, p + 1, nbt) * kBlkElems, rr, c);
-          const double* Lj = S + blk_index(p + 1, p, nbt) * kBlkElems;
+      named_barrier<1>(bar);                           // also: every thread has read the diagonal block
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            double l[8];
-            blk_load_row(Lj, j, l);
+      for (int j = 0; j < 4; ++j) {
+        const double2 l0 = *reinterpret_cast<const double2*>(low + 4 * j), l1 = *reinterpret_cast<const double2*>(low + 4 * j + 2);
+        x[4 + j] = fma(-x[0], l0.x, x[4 + j]);
+        x[4 + j] = fma(-x[1], l0.y, x[4 + j]);
+        x[4 + j] = fma(-x[2], l1.x, x[4 + j]);
+        x[4 + j] = fma(-x[3], l1.y, x[4 + j]);
+      }
+      if (R == p && rr >= 4) {
+        *reinterpret_cast<double2*>(next + 4 * (rr - 4)) = make_double2(x[4], x[5]);
+        *reinterpret_cast<double2*>(next + 4 * (rr - 4) + 2) = make_double2(x[6], x[7]);
+      }
+      __syncwarp();
+      named_barrier<1>(bar);
+      load([&](int i, int c) { return *reinterpret_cast<const double2*>(next + 4 * i + 2 * c); });
+      if constexpr (kTrack) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) c[j] = fma(-x[k], l[k], c[j]);
-          }
-          if (R == p + 1) {
-            blk_store_row(Dst + ((p + 1) & 1) * kBlkElems, rr, c);
-            if constexpr (kTrack)
-              if ((p & 3) == 3) {
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
-                  if (k == rr) dgs[t] = c[k];
-              }
-          }
-#pragma unroll
-          for (int k = 0; k < 8; ++k) x[k] = c[k];
+        for (int k = 0; k < 4; ++k) dg[k] = dgs[8 * p + 4 + k];
+      }
+      factor(4);
+      if (mine) blk_store_row(S + blk_index(R, p, nbt) * kBlkElems, rr, x);
+      if constexpr (kTrack)
+        if ((p & 3) == 3 || p + 1 == nbp) {
+          if (small && t == 8 * p) on_small();
+          small = false;
         }
-        __syncwarp();
-        named_barrier<1>(32 * PW);
-      } else {
-        panel_update(S, p, p + 1, nbt, warp, PW + UW, lane, [](int) {});
-      }
     }
-  } else {
-    const int u = warp - PW;
-    for (int p = 0; p < nbp; ++p) {
-      named_barrier<0>(32 * (PW + UW));
-      if (p + 1 < nbp) {                                 // the panel warps take block column p + 1
-        panel_update(S, p, p + 2, nbt, u, UW, lane, [&](int i) {
-          if constexpr (kTrack)                          // the next group's reference diagonal (its first block: above)
-            if ((p & 3) == 3 && i <= p + 4 && i < nbp) {
-              __syncwarp();
-              if (lane < 8) dgs[8 * i + lane] = S[blk_index(i, i, nbt) * kBlkElems + blk_elem(lane, lane)];
-            }
-        });
-      } else {
-        panel_update(S, p, p + 1, nbt, warp, PW + UW, lane, [](int) {});
-      }
-      if constexpr (kInv) {
-        if (u == p % UW && lane < 8) {                   // column `lane` of the inverse of the diagonal block
-          const double* L = S + blk_index(p, p, nbt) * kBlkElems;
-          double z[8];
-#pragma unroll
-          for (int k = 0; k < 8; ++k) z[k] = k == lane ? 1.0 : 0.0;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            z[k] *= rq[8 * p + k];
-#pragma unroll
-            for (int i = k + 1; i < 8; ++i) z[i] = fma(-L[blk_elem(i, k)], z[k], z[i]);
-          }
-#pragma unroll
-          for (int k = 0; k < 8; ++k) Dinv[p * kBlkElems + blk_elem(k, lane)] = z[k];
-        }
-        __syncwarp();
-      }
-    }
+    __syncthreads();
+    // two panels at a time: after the first of a pair only the second's block column
+    if ((p & 1) == 0 && p + 1 < nbp) next_column_update(S, p, nbt, warp, NW, lane);
+    else if ((p & 1) == 0) panel_update<1>(S, tab, p, p + 1, nbt, warp, NW, lane);
+    else panel_update<2>(S, tab, p - 1, p + 1, nbt, warp, NW, lane);
+    __syncthreads();
   }
+}
+
+// Dinv (nbp blocks): the inverses of the diagonal blocks of L, one column per thread.
+__device__ __forceinline__ void invert_diagonal_blocks(const double* S, const double* rq, double* Dinv, int nbp, int nbt) {
+  const int t = threadIdx.x, p = t >> 3, c = t & 7;
+  if (p >= nbp) return;
+  const double* L = S + blk_index(p, p, nbt) * kBlkElems;
+  double z[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) z[k] = k == c ? 1.0 : 0.0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    z[k] *= rq[8 * p + k];
+#pragma unroll
+    for (int i = k + 1; i < 8; ++i) z[i] = fma(-L[blk_elem(i, k)], z[k], z[i]);
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) Dinv[p * kBlkElems + blk_elem(k, c)] = z[k];
 }
 
 // One warp, eight rows: acc (8 x 8 nb, fragments) <- acc L^{-T}, L packed with

@@ -160,7 +160,7 @@ __global__ void k_child_records(DevFronts F, int n, ChildRec* rec) {
   const int c = F.child[k];
   ChildRec r;
   r.nc = F.nc[c]; r.nr = F.nr[c]; r.lrow_off = F.lrow_off[c]; r.pad = 0;
-  r.u_off = F.u_off[c]; r.v_off = F.v_off[c]; r.inv_off = F.inv_off[c]; r.pad2 = 0;
+  r.u_off = F.u_off[c]; r.v_off = F.v_off[c]; r.inv_off = F.inv_off ? F.inv_off[c] : 0; r.pad2 = 0;
   rec[k] = r;
 }
 

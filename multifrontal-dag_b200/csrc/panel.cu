@@ -19,15 +19,15 @@ namespace mfd {
 
 namespace {
 
-// Widest block of a k_potrf class: 32 NSB columns; panel warps = NSB (one row
-// per thread), update warps to match the trailing blocks.
+// Widest block of a k_potrf class: 32 NSB columns, one row per thread of the
+// first NSB warps, more warps for the trailing updates of the wider ones.
 template <int NSB>
-__host__ __device__ constexpr int potrf_uwarps() {
-  return NSB == 1 ? 1 : NSB == 2 ? 2 : NSB == 3 ? 5 : 8;
+__host__ __device__ constexpr int potrf_warps() {
+  return NSB == 1 ? 1 : NSB == 2 ? 4 : NSB == 3 ? 8 : 12;
 }
 template <int NSB>
 __host__ __device__ constexpr int potrf_threads() {
-  return 32 * (NSB + potrf_uwarps<NSB>());
+  return 32 * potrf_warps<NSB>();
 }
 template <int NSB>
 __host__ __device__ constexpr size_t potrf_smem() {
@@ -67,7 +67,7 @@ template <typename T, int NSB>
 __global__ void __launch_bounds__(potrf_threads<NSB>(), 1) k_potrf(DevFronts F, const int32_t* list, int slot0,
                                                                    int step, T* panel, double* packed, int32_t* info,
                                                                    int info_stride, int32_t* fallbacks) {
-  constexpr int UW = potrf_uwarps<NSB>(), NW = NSB + UW, NT = 32 * NW;
+  constexpr int NW = potrf_warps<NSB>(), NT = 32 * NW;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* S = reinterpret_cast<double*>(smem_raw);
   double* Dinv = S + (size_t)blk_count(4 * NSB) * kBlkElems;
@@ -83,15 +83,15 @@ __global__ void __launch_bounds__(potrf_threads<NSB>(), 1) k_potrf(DevFronts F, 
   load_block(P, nf, w, nb, S, NW);
   __syncthreads();
   int32_t* my_info = info + (size_t)info_stride * slot;
-  chol_panels<NSB, UW, true, sizeof(T) == 4>(
-      S, scratch, Dinv, nb, nb,
+  chol_panels<NW, sizeof(T) == 4>(
+      S, scratch, nb, nb,
       [&](int j) {
         if (j < w) atomicMin(my_info, F.first[f] + c0 + j + 1);
       },
       [&] {
         if (fallbacks) atomicAdd(fallbacks, 1);
       });
-  __syncthreads();
+  invert_diagonal_blocks(S, scratch + kCholRq, Dinv, nb, nb);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double2* Q = reinterpret_cast<double2*>(packed + (size_t)slot * kPackedPanelElems);
   for (int e = tid; e < blk_count(nb) * 32; e += NT) Q[e] = reinterpret_cast<const double2*>(S)[e];

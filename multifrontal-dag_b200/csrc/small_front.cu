@@ -1,9 +1,9 @@
-// Fused small fronts (nf <= 128): zero, assemble A, extend-add the children in
+// Fused small fronts (nf <= 160): zero, assemble A, extend-add the children in
 // order, partial Cholesky of the nc supernode columns and the Schur complement,
 // all on chip; the factor panel and the update matrix are written once.
 //
 //   k_small_warp  : nf <= 32, one warp per front, one row per lane in registers
-//   k_small_block : nf <= 128, one CTA per front on 8 x 8 blocks (chol_smem.cuh)
+//   k_small_block : nf <= 160, one CTA per front on 8 x 8 blocks (chol_smem.cuh)
 //
 // Both start from the front's record and its children's (FrontRec, ChildRec).
 // What bound them was latency: a chain of six dependent loads before the first
@@ -40,10 +40,10 @@ __device__ __forceinline__ float rsqrt_of<float>(float x) { return rsqrtf(x); }
 constexpr int kWarps = 4;
 
 template <typename T, int NF>
-__global__ void __launch_bounds__(kWarps * 32) k_small_warp(DevFronts F, const FrontRec* __restrict__ recs, int count,
+__global__ void __launch_bounds__(kWarps * 32, NF <= 24 ? 8 : 6) k_small_warp(DevFronts F, const FrontRec* __restrict__ recs, int count,
                                                             const double* __restrict__ a, T* __restrict__ panel,
                                                             T* __restrict__ upool, int32_t* info) {
-  constexpr int LD = NF + 1, CU = 8;
+  constexpr int LD = NF + 1, CU = 4;
   __shared__ T sbuf[kWarps][NF * LD];
   __shared__ T cbuf[kWarps][2][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -162,25 +162,23 @@ __global__ void __launch_bounds__(kWarps * 32) k_small_warp(DevFronts F, const F
   }
 }
 
-// ---- nf <= 128: one CTA per front ------------------------------------------------
+// ---- nf <= 160: one CTA per front ------------------------------------------------
 // The nc pivot columns are padded to a multiple of eight with an identity, so
 // that the pivot and the update part split at a block boundary (dummy columns
 // couple to nothing).  Shared memory in FP64 for either storage type.
 constexpr int kChildBatch = 4;    // children whose local indices are staged together
-constexpr int kStageRows = 128;
+constexpr int kStageRows = kSmallFrontMax;
 
 template <int NF>
 __host__ __device__ constexpr int block_rows() { return (NF + 7 + 7) / 8; }      // block rows with the padding
 template <int NF>
-__host__ __device__ constexpr int block_pwarps() { return (block_rows<NF>() + 3) / 4; }
+__host__ __device__ constexpr int block_warps() { return NF <= 64 ? 4 : NF <= 96 ? 6 : 8; }
 template <int NF>
-__host__ __device__ constexpr int block_uwarps() { return NF <= 64 ? 1 : NF <= 96 ? 2 : 3; }
-template <int NF>
-__host__ __device__ constexpr int block_threads() { return 32 * (block_pwarps<NF>() + block_uwarps<NF>()); }
+__host__ __device__ constexpr int block_threads() { return 32 * block_warps<NF>(); }
 // shared memory for fronts of at most nf rows
 template <int NF>
 size_t block_smem(int nf) {
-  return sizeof(double) * ((size_t)blk_count((nf + 14) / 8) * kBlkElems + chol_scratch_elems(32 * block_pwarps<NF>(), false)) +
+  return sizeof(double) * ((size_t)blk_count((nf + 14) / 8) * kBlkElems + chol_scratch_elems(8 * block_rows<NF>(), false)) +
          sizeof(uint8_t) * kChildBatch * kStageRows;
 }
 
@@ -216,17 +214,17 @@ __device__ __forceinline__ void extend_add(double* S, int nbt, const T* __restri
 }
 
 template <typename T, int NF>
-__global__ void __launch_bounds__(block_threads<NF>(), NF <= 64 ? 4 : NF <= 96 ? 2 : 2)
+__global__ void __launch_bounds__(block_threads<NF>(), NF <= 64 ? 6 : NF <= 96 ? 3 : NF <= 128 ? 2 : 1)
     k_small_block(DevFronts F, const FrontRec* __restrict__ recs, const double* __restrict__ a, T* __restrict__ panel,
                   T* __restrict__ upool, int32_t* info) {
-  constexpr int PW = block_pwarps<NF>(), UW = block_uwarps<NF>(), NT = block_threads<NF>(), NW = NT / 32;
+  constexpr int NW = block_warps<NF>(), NT = 32 * NW;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const FrontRec rec = recs[blockIdx.x];
   const int nc = rec.nc, nr = rec.nr, nf = nc + nr;
   const int nbp = (nc + 7) >> 3, pad = 8 * nbp - nc, nbt = (nf + pad + 7) >> 3;
   double* S = reinterpret_cast<double*>(smem_raw);
   double* scratch = S + blk_count(nbt) * kBlkElems;
-  uint8_t* sloc = reinterpret_cast<uint8_t*>(scratch + chol_scratch_elems(32 * PW, false));   // kChildBatch x kStageRows
+  uint8_t* sloc = reinterpret_cast<uint8_t*>(scratch + chol_scratch_elems(8 * block_rows<NF>(), false));   // kChildBatch x kStageRows
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nch = rec.child_end - rec.child_beg;
   // A's first entries and the first children's local indices are in flight while the front is zeroed
@@ -270,14 +268,14 @@ __global__ void __launch_bounds__(block_threads<NF>(), NF <= 64 ? 4 : NF <= 96 ?
         case 1: extend_add<1, 8>(S, nbt, U, loc, c.nr, lane, warp, NW); break;
         case 2: extend_add<2, 8>(S, nbt, U, loc, c.nr, lane, warp, NW); break;
         case 3: extend_add<3, 5>(S, nbt, U, loc, c.nr, lane, warp, NW); break;
-        default: extend_add<4, 4>(S, nbt, U, loc, c.nr, lane, warp, NW); break;
+        case 4: extend_add<4, 4>(S, nbt, U, loc, c.nr, lane, warp, NW); break;
+        default: extend_add<5, 3>(S, nbt, U, loc, c.nr, lane, warp, NW); break;
       }
       __syncthreads();
     }
   }
-  chol_panels<PW, UW, false, false>(
-      S, scratch, nullptr, nbp, nbt, [&](int j) { if (j < nc) atomicMin(info, rec.first + j + 1); }, [] {});
-  __syncthreads();
+  chol_panels<NW, false>(
+      S, scratch, nbp, nbt, [&](int j) { if (j < nc) atomicMin(info, rec.first + j + 1); }, [] {});
   T* P = panel + rec.panel_off;
   for (int j = warp; j < nc; j += NW)
     for (int i = j + lane; i < nf; i += 32) P[i + (size_t)j * nf] = (T)S[blk_addr(i < nc ? i : i + pad, j, nbt)];
@@ -298,6 +296,7 @@ cudaError_t prepare_small_fronts() {
   chk(k_small_block<double, 64>, block_smem<64>(64)); chk(k_small_block<float, 64>, block_smem<64>(64));
   chk(k_small_block<double, 96>, block_smem<96>(96)); chk(k_small_block<float, 96>, block_smem<96>(96));
   chk(k_small_block<double, 128>, block_smem<128>(128)); chk(k_small_block<float, 128>, block_smem<128>(128));
+  chk(k_small_block<double, 160>, block_smem<160>(160)); chk(k_small_block<float, 160>, block_smem<160>(160));
   return e;
 }
 
@@ -313,8 +312,10 @@ void launch_small_fronts(const DevFronts& F, const FrontRec* rec, int count, int
     k_small_block<T, 64><<<count, block_threads<64>(), block_smem<64>(nf_max), st>>>(F, rec, a, panel, upool, info);
   else if (nf_max <= 96)
     k_small_block<T, 96><<<count, block_threads<96>(), block_smem<96>(nf_max), st>>>(F, rec, a, panel, upool, info);
-  else
+  else if (nf_max <= 128)
     k_small_block<T, 128><<<count, block_threads<128>(), block_smem<128>(nf_max), st>>>(F, rec, a, panel, upool, info);
+  else
+    k_small_block<T, 160><<<count, block_threads<160>(), block_smem<160>(nf_max), st>>>(F, rec, a, panel, upool, info);
 }
 
 #define MFD_INSTANTIATE_SMALL(T)                                                                                \

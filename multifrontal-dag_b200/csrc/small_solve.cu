@@ -1,5 +1,5 @@
-// Triangular solves of small fronts (nf <= 128): nf <= 32 one warp per front,
-// four per CTA; above, one CTA of two or four warps per front.
+// Triangular solves of small fronts (nf <= 160): nf <= 32 one warp per front,
+// four per CTA; above, one CTA of two to five warps per front.
 //
 // The panel goes to shared memory with cp.async, every copy in flight at once
 // and next to the front's vectors and its children's, with an odd leading
@@ -26,7 +26,7 @@ namespace mfd {
 namespace {
 
 template <int R>
-__host__ __device__ constexpr int warps_per_front() { return R == 1 ? 1 : R == 2 ? 2 : 4; }
+__host__ __device__ constexpr int warps_per_front() { return R == 1 ? 1 : R == 2 ? 2 : R <= 4 ? 4 : 5; }
 template <int R>
 __host__ __device__ constexpr int fronts_per_cta() { return R == 1 ? 4 : 1; }
 template <int R>
@@ -240,7 +240,8 @@ size_t small_solve_smem(int nf_max, int panel_elems) {
     case 1: return sizeof(T) * fronts_per_cta<1>() * (size_t)front_elems<1>(panel_elems);
     case 2: return sizeof(T) * (size_t)front_elems<2>(panel_elems);
     case 3: return sizeof(T) * (size_t)front_elems<3>(panel_elems);
-    default: return sizeof(T) * (size_t)front_elems<4>(panel_elems);
+    case 4: return sizeof(T) * (size_t)front_elems<4>(panel_elems);
+    default: return sizeof(T) * (size_t)front_elems<5>(panel_elems);
   }
 }
 
@@ -257,7 +258,8 @@ cudaError_t prepare_small_solve() {
       case 1: chk(k_fwd_small<T, 1>, bytes); chk(k_bwd_small<T, 1>, bytes); break;
       case 2: chk(k_fwd_small<T, 2>, bytes); chk(k_bwd_small<T, 2>, bytes); break;
       case 3: chk(k_fwd_small<T, 3>, bytes); chk(k_bwd_small<T, 3>, bytes); break;
-      default: chk(k_fwd_small<T, 4>, bytes); chk(k_bwd_small<T, 4>, bytes); break;
+      case 4: chk(k_fwd_small<T, 4>, bytes); chk(k_bwd_small<T, 4>, bytes); break;
+      default: chk(k_fwd_small<T, 5>, bytes); chk(k_bwd_small<T, 5>, bytes); break;
     }
   };
   for (int nf = 32; nf <= kSmallFrontMax; nf += 32) {
@@ -279,7 +281,8 @@ void launch_fwd_small(const DevFronts& F, const FrontRec* rec, int count, int nf
     case 1: go(k_fwd_small<T, 1>, fronts_per_cta<1>(), solve_threads<1>()); break;
     case 2: go(k_fwd_small<T, 2>, 1, solve_threads<2>()); break;
     case 3: go(k_fwd_small<T, 3>, 1, solve_threads<3>()); break;
-    default: go(k_fwd_small<T, 4>, 1, solve_threads<4>()); break;
+    case 4: go(k_fwd_small<T, 4>, 1, solve_threads<4>()); break;
+    default: go(k_fwd_small<T, 5>, 1, solve_threads<5>()); break;
   }
 }
 template <typename T>
@@ -294,7 +297,8 @@ void launch_bwd_small(const DevFronts& F, const FrontRec* rec, int count, int nf
     case 1: go(k_bwd_small<T, 1>, fronts_per_cta<1>(), solve_threads<1>()); break;
     case 2: go(k_bwd_small<T, 2>, 1, solve_threads<2>()); break;
     case 3: go(k_bwd_small<T, 3>, 1, solve_threads<3>()); break;
-    default: go(k_bwd_small<T, 4>, 1, solve_threads<4>()); break;
+    case 4: go(k_bwd_small<T, 4>, 1, solve_threads<4>()); break;
+    default: go(k_bwd_small<T, 5>, 1, solve_threads<5>()); break;
   }
 }
 

@@ -100,8 +100,12 @@ __device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_grou
 // Task (f, s): y_s = Li (v_s - sum_{t<s} L_st y_t); rest tasks (128 rows below
 // the columns): v -= sum_t L_rest,t y_t.  Thread (row r0 + (t mod 128), half
 // t / 128) takes its half of each step's 128 columns.
-template <typename T>
-__global__ void __launch_bounds__(256) k_fwd_single(DevFronts F, const int4* __restrict__ tasks, int ntask,
+//
+// N: columns per half step in flight: 64, all of them, before the wait; in FP64 32
+// where the level has more tasks than SMs, so that two CTAs share an SM (in FP32
+// two do with 64).
+template <typename T, int N>
+__global__ void __launch_bounds__(256, N == 64 && sizeof(T) == 8 ? 1 : 2) k_fwd_single(DevFronts F, const int4* __restrict__ tasks, int ntask,
                                                     int32_t* ticket, int32_t* expired, const int32_t* epoch,
                                                     const T* __restrict__ panel, const T* __restrict__ dinv, T* X, T* V,
                                                     typename Exchange<T>::Word* E, const int32_t* test_req) {
@@ -131,10 +135,13 @@ __global__ void __launch_bounds__(256) k_fwd_single(DevFronts F, const int4* __r
   T acc[4] = {T(0), T(0), T(0), T(0)};
   for (int s = 0; s < nsteps; ++s) {
     const int c0 = s * kSolveB, w = min(kSolveB, nc - c0);
-    T l[64];
+    T l[N];
     const T* pc = P + (valid ? i : 0) + (size_t)(c0 + 64 * h) * nf;
+    auto load = [&](int o) {
 #pragma unroll
-    for (int k = 0; k < 64; ++k) l[k] = (valid && 64 * h + k < w) ? pc[(size_t)k * nf] : T(0);
+      for (int k = 0; k < N; ++k) l[k] = (valid && 64 * h + o + k < w) ? pc[(size_t)(o + k) * nf] : T(0);
+    };
+    load(0);
     bool ok = true;
     if (tid < kSolveB) {
       T y = T(0);
@@ -147,7 +154,11 @@ __global__ void __launch_bounds__(256) k_fwd_single(DevFronts F, const int4* __r
     }
     const T* y = ys[s & 1] + 64 * h;
 #pragma unroll
-    for (int k = 0; k < 64; ++k) acc[k & 3] += l[k] * y[k];
+    for (int o = 0; o < 64; o += N) {
+      if (o > 0) load(o);
+#pragma unroll
+      for (int k = 0; k < N; ++k) acc[k & 3] += l[k] * y[o + k];
+    }
   }
   const T a = (acc[0] + acc[1]) + (acc[2] + acc[3]);
   if (h == 1) part[0][ri] = a;
@@ -200,8 +211,11 @@ __device__ __forceinline__ T transpose_reduce16(T (&acc)[16], int lane) {
 // the last down: x_s = Li^T (v_s - L_below,s^T x_below), the chunks' partials
 // added in chunk order, before the wait on the later blocks.  Warp w takes
 // columns 16 w .. 16 w + 15 of the block, lanes rows.
-template <typename T>
-__global__ void __launch_bounds__(256) k_bwd_single(DevFronts F, const int4* __restrict__ tasks, int ntask,
+//
+// Q: 32-row pieces of a later block in flight: 4, the block, before the wait, or 2
+// (as N above).
+template <typename T, int Q>
+__global__ void __launch_bounds__(256, Q == 4 && sizeof(T) == 8 ? 1 : 2) k_bwd_single(DevFronts F, const int4* __restrict__ tasks, int ntask,
                                                     int32_t* ticket, int32_t* expired, const int32_t* epoch,
                                                     const T* __restrict__ panel, const T* __restrict__ dinv, T* X,
                                                     typename Exchange<T>::Word* E, T* part, int32_t* counters,
@@ -265,25 +279,28 @@ __global__ void __launch_bounds__(256) k_bwd_single(DevFronts F, const int4* __r
   bool good = true;
   for (int b = nsteps - 1; b > s && good; --b) {                           // later diagonal blocks
     const int ra = b * kSolveB, rb = min(nc, ra + kSolveB);
-    T l[4][16];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int r = ra + lane + 32 * q;
-      const T* pr = P + (r < rb ? r : ra) + (size_t)(c0 + wc) * nf;
+    for (int o = 0; o < 4; o += Q) {
+      T l[Q][16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) l[q][j] = (r < rb && wc + j < w) ? pr[(size_t)j * nf] : T(0);
+      for (int q = 0; q < Q; ++q) {
+        const int r = ra + lane + 32 * (o + q);
+        const T* pr = P + (r < rb ? r : ra) + (size_t)(c0 + wc) * nf;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) l[q][j] = (r < rb && wc + j < w) ? pr[(size_t)j * nf] : T(0);
+      }
+      T xv[Q];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int r = ra + lane + 32 * (o + q);
+        xv[q] = T(0);
+        if (r < rb && good) good = wait_value<T>(E + first + r, tag, xv[q], expired, probe);
+      }
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+#pragma unroll
+        for (int j = 0; j < 16; ++j) acc[j] += l[q][j] * xv[q];
     }
-    T xv[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int r = ra + lane + 32 * q;
-      xv[q] = T(0);
-      if (r < rb) good &= wait_value<T>(E + first + r, tag, xv[q], expired, probe);
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-      for (int j = 0; j < 16; ++j) acc[j] += l[q][j] * xv[q];
     good = __all_sync(0xffffffffu, good);
   }
   const T dsum = transpose_reduce16(acc, lane);           // lane l: column wc + (l mod 16), diagonal blocks
@@ -328,8 +345,9 @@ cudaError_t prepare_solve_single() {
     cudaError_t r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (r != cudaSuccess && e == cudaSuccess) e = r;
   };
-  chk(k_fwd_single<double>, kFoldElems * sizeof(double)); chk(k_bwd_single<double>, kFoldElems * sizeof(double));
-  chk(k_fwd_single<float>, kFoldElems * sizeof(float)); chk(k_bwd_single<float>, kFoldElems * sizeof(float));
+  chk(k_fwd_single<double, 64>, kFoldElems * sizeof(double)); chk(k_bwd_single<double, 4>, kFoldElems * sizeof(double));
+  chk(k_fwd_single<double, 32>, kFoldElems * sizeof(double)); chk(k_bwd_single<double, 2>, kFoldElems * sizeof(double));
+  chk(k_fwd_single<float, 64>, kFoldElems * sizeof(float)); chk(k_bwd_single<float, 4>, kFoldElems * sizeof(float));
   return e;
 }
 
@@ -344,11 +362,21 @@ void launch_large_fused(const DevFronts& F, const int4* tasks, int ntask, bool b
   if (ntask <= 0) return;
   auto* E = static_cast<typename Exchange<T>::Word*>(exch);
   const size_t sm = kFoldElems * sizeof(T);
-  if (backward)
-    k_bwd_single<T><<<ntask, 256, sm, st>>>(F, tasks, ntask, ticket, expired, epoch, panel, dinv, X, E, part, counters,
-                                            test_req);
-  else
-    k_fwd_single<T><<<ntask, 256, sm, st>>>(F, tasks, ntask, ticket, expired, epoch, panel, dinv, X, V, E, test_req);
+  auto bwd = [&](auto k) {
+    k<<<ntask, 256, sm, st>>>(F, tasks, ntask, ticket, expired, epoch, panel, dinv, X, E, part, counters, test_req);
+  };
+  auto fwd = [&](auto k) {
+    k<<<ntask, 256, sm, st>>>(F, tasks, ntask, ticket, expired, epoch, panel, dinv, X, V, E, test_req);
+  };
+  if constexpr (sizeof(T) == 8) {
+    if (ntask > 148) {
+      if (backward) bwd(k_bwd_single<T, 2>);
+      else fwd(k_fwd_single<T, 32>);
+      return;
+    }
+  }
+  if (backward) bwd(k_bwd_single<T, 4>);
+  else fwd(k_fwd_single<T, 64>);
 }
 
 #define MFD_INSTANTIATE_SINGLE(T)                                                                                  \

@@ -98,3 +98,29 @@ def test_several_rhs_expired_wait(precision):
     rep, rc = s.solve(X)
     assert rc == 0
     assert P.backward_error(p.n, p.col, p.row, p.val, X[:, 9], B[:, 9]) <= 1e-12
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("n", [1, 5, 15, 16, 17, 24, 25, 32, 33, 57, 64, 65, 89, 96, 97, 128, 129, 153, 160, 161])
+def test_small_front_sizes(n, precision):
+    """One dense front of n rows and columns: the edges of the one-warp sizes
+    (16, 24, 32), of the one-CTA sizes (64, 96, 128, 160), of their 8-column
+    blocks, and the first size of the blocked path.  Backward error against the
+    dense product: FP64 n eps, FP32 + refinement 1e-12."""
+    a = _spd(n, n)
+    col, rows, vals = [1], [], []
+    for j in range(n):
+        rows.extend(range(j + 1, n + 1))
+        vals.extend(a[j:, j])
+        col.append(len(rows) + 1)
+    s = H.Solver.analyze(n, np.array(col), np.array(rows), None, max_zero=0, precision=precision)
+    assert s.stats().num_front == 1
+    assert s.factorize(np.array(vals)) == 0
+    B = np.asfortranarray(np.random.default_rng(n).uniform(-1, 1, (n, 3)))
+    for X in (B[:, 0].copy(), B.copy(order="F")):
+        b = X.copy(order="F")
+        rep, rc = s.solve(X)
+        assert rc == 0
+        r = np.abs(b - a @ X).max()
+        den = np.abs(a).sum(axis=1).max() * np.abs(X).max() + np.abs(b).max()
+        assert r / den <= (1e-14 if precision == 0 else 1e-12)
