@@ -19,7 +19,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "mfdag", "libmfdag.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-SOURCES = ["analysis.cpp", "ordering.cpp", "partition.cpp", "kernels.cu", "small_front.cu", "small_solve.cu", "panel.cu", "solve_single.cu", "solve_multi.cu", "update_tc.cu", "api.cu", "noalloc.cu",
+SOURCES = ["analysis.cpp", "ordering.cpp", "partition.cpp", "kernels.cu", "small_front.cu", "small_solve.cu", "panel.cu", "solve_single.cu", "solve_multi.cu", "update_tc.cu", "update_dp.cu", "api.cu", "noalloc.cu",
            "input.cu"]
 
 

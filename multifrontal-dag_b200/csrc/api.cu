@@ -50,7 +50,9 @@ constexpr int kWarpFrontsAtOnce = 148 * 24;   // one-warp fronts the chip holds 
 // panel chain (elasticity 21^3, mixed, with it on every level: 6.00 -> 6.16 ms).
 constexpr int kDeferDefault = 2;
 constexpr double kDeferBytes = 64e6;
-constexpr int kPackedDefer = 2;       // the most the packed-operand FP32 update takes
+// FP64: levels whose largest front has this many rows pack the update's operands (below, the updates
+// are a few partly filled tiles and the panel itself is read)
+constexpr int kPackedDpRows = 768;
 int64_t align_up(int64_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
 template <typename T>
@@ -242,7 +244,7 @@ struct mfd_handle {
   void* d_exch = nullptr;                           // single-RHS sweeps: n_total exchange entries of 2 sizeof(T)
   std::vector<int> small_bins;
   int64_t panel_elems = 0, upool_elems = 0, v_elems = 0, s_elems = 0, dinv_elems = 0;
-  int64_t q_elems = 0;                              // packed FP32 update operands of one step parity
+  int64_t q_elems = 0;                              // packed update operands of one step
   int32_t max_large_count = 0, max_nf = 0;
   int64_t cost = 0, nonzero = 0;
 
@@ -271,7 +273,7 @@ struct mfd_handle {
   void* d_upool = nullptr;
   void* d_diag = nullptr;
   double* d_packed = nullptr;                       // the current panel step's packed diagonal blocks, one per list slot
-  float* d_q = nullptr;                             // FP32: packed update operands, 2 defer step buffers
+  void* d_q = nullptr;                              // T, packed update operands, 2 defer step buffers
   DBuf<double> d_a, d_b, d_xp, d_bp, d_r, d_norms, d_cnorms, d_xt;
   void* d_X = nullptr;   // T, n_total x nrhs
   void* d_V = nullptr;   // T
@@ -315,7 +317,7 @@ struct mfd_handle {
     for (auto& kv : g_solve) cudaGraphExecDestroy(kv.second);
     for (auto& kv : g_ir) cudaGraphExecDestroy(kv.second);
     if (bst) cudaStreamDestroy(bst);
-    for (void* p : {d_panel, d_upool, d_diag, d_X, d_V, d_S, static_cast<void*>(d_q), static_cast<void*>(d_packed), d_bwpart, d_exch})
+    for (void* p : {d_panel, d_upool, d_diag, d_X, d_V, d_S, d_q, static_cast<void*>(d_packed), d_bwpart, d_exch})
       if (p) cudaFree(p);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
@@ -541,15 +543,16 @@ int build_plan(mfd_handle* h) {
       }
       L.defer = h->opt.reserved[5] > 0 || bytes > kDeferBytes ? h->defer : 1;
     }
-    // packed operands of the FP32 tensor-core update: the level's large fronts side by side,
-    // each with the 128-row blocks of its largest step (step 0); reused level after level
-    {
+    // packed operands of the trailing update: the level's large fronts side by side, each with the
+    // 128-row blocks of its largest step (step 0); reused level after level
+    L.packed = h->defer <= kPackedDefer && (h->fp32 || L.large_max_nf >= kPackedDpRows);
+    if (L.packed) {
       int64_t q = 0;
       for (int32_t g : large) {
         HostFront& fr = h->fronts[g];
         const int64_t nrem = (int64_t)fr.nc + fr.nr - std::min(kFactB, fr.nc);
         fr.q_off = q;
-        q += (nrem + kFactB - 1) / kFactB * kPackedBlockElems;
+        q += (nrem + kFactB - 1) / kFactB * (h->fp32 ? kPackedBlockElems : (int64_t)kFactB * kFactB);
       }
       h->q_elems = std::max(h->q_elems, q);
     }
@@ -871,10 +874,11 @@ int upload_plan(mfd_handle* h) {
   CK(cudaMalloc(&h->d_diag, (size_t)std::max<int64_t>(h->dinv_elems, 1) * esz));
   if (h->max_large_count > 0)
     CK(cudaMalloc(&h->d_packed, (size_t)h->max_large_count * kPackedPanelElems * sizeof(double)));
-  if (h->fp32 && h->q_elems > 0 && h->defer <= kPackedDefer) {
-    CK(cudaMalloc(&h->d_q, (size_t)(2 * h->defer * h->q_elems) * sizeof(float)));
+  if (h->q_elems > 0) {
+    const size_t bytes = (size_t)(2 * h->defer * h->q_elems) * esz;
+    CK(cudaMalloc(&h->d_q, bytes));
     // rows past a front's last row are never written and only reach discarded outputs; zero keeps them finite
-    CK(cudaMemsetAsync(h->d_q, 0, (size_t)(2 * h->defer * h->q_elems) * sizeof(float), h->st));
+    CK(cudaMemsetAsync(h->d_q, 0, bytes, h->st));
   }
   // the inverted diagonal blocks are written on their lower w x w part only: the rest stays zero
   CK(cudaMemsetAsync(h->d_diag, 0, (size_t)std::max<int64_t>(h->dinv_elems, 1) * esz, h->st));
@@ -1083,11 +1087,11 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
     // SMs the side-stream update could use), so the default leaves it off.
     const bool pdl = h->opt.reserved[2] == 1 && !h->profiling;
     const int D = L.defer;
-    // FP32 tensor-core update: the TRSM also writes the step's rows as packed TF32 hi / lo
-    // operands for k_update_tcq, in 2 D buffers taken in turn: the bulk update of a group reads
-    // its own D, and is complete before the TRSM of the group after the next one starts
-    const bool tcq = sizeof(T) == 4 && (kind == 0 || kind == 2) && h->d_q != nullptr;
-    auto packed_rows = [&](size_t step) { return h->d_q + (step % (2 * D)) * h->q_elems; };
+    // packed operands: the TRSM also writes the step's rows for k_update_tcq / k_update_dp, in 2 D
+    // buffers taken in turn: the bulk update of a group reads its own D, and is complete before
+    // the TRSM of the group after the next one starts
+    const bool packed = L.packed && (kind == 0 || (sizeof(T) == 4 && kind == 2));
+    auto packed_rows = [&](size_t step) { return static_cast<T*>(h->d_q) + (step % (2 * D)) * h->q_elems; };
     int pend = -1;                            // step of the latest bulk on st2 not yet fully waited for
     for (size_t s = 0; s < L.steps.size(); ++s) {
       const LaunchList& p = L.steps[s];
@@ -1133,7 +1137,7 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
              });
       record(h, st, MFD_K_TRSM, tf, tb, [&] {
         launch_trsm<T>(F, lists + p.off, p.count, (int)s, p.param, std::min(kFactB, L.large.param2 - (int)s * kFactB),
-                       panel, h->d_packed, st, pdl, tcq ? packed_rows(s) : nullptr);
+                       panel, h->d_packed, st, pdl, packed ? packed_rows(s) : nullptr);
       });
       n += 2;
       auto update = [&](cudaStream_t us, UpdBand band) {
@@ -1142,7 +1146,7 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
         const bool upd_pdl = pdl && us == st;        // right behind the TRSM on the main stream
         record(h, us, MFD_K_UPDATE, fl, by, [&] {
           if constexpr (sizeof(T) == 4) {
-            if (tcq) {
+            if (packed) {
               n += launch_update_tcq(F, lists + p.off, p.count, (int)s, p.param2, packed_rows(s),
                                      s > 0 ? packed_rows(s - 1) : nullptr, reinterpret_cast<float*>(panel),
                                      reinterpret_cast<float*>(upool), kind == 0 ? 1 : 0, h->d_info.p + 1, us, band, D,
@@ -1153,6 +1157,15 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
               n += launch_update_tc(F, lists + p.off, p.count, (int)s, p.param2, reinterpret_cast<float*>(panel),
                                     reinterpret_cast<float*>(upool), kind == 0 ? 1 : 0, h->d_info.p + 1, us, band,
                                     D, upd_pdl);
+              return;
+            }
+          }
+          if constexpr (sizeof(T) == 8) {
+            // where 128 x 64 pieces fill the chip; launch_update's smaller ones read the panel
+            if (packed && (int64_t)2 * update_grid(p.param2, kUpdTile, band) * p.count > kNumSms) {
+              n += launch_update_dp(F, lists + p.off, p.count, (int)s, p.param2, static_cast<const double*>(h->d_q),
+                                    h->q_elems, 2 * D, reinterpret_cast<double*>(panel), reinterpret_cast<double*>(upool),
+                                    h->d_info.p + 1, us, band, D, upd_pdl);
               return;
             }
           }

@@ -1169,7 +1169,6 @@ __global__ void k_fill_int(int32_t* p, int32_t v, int64_t n) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) p[i] = v;
 }
 
-constexpr int kNumSms = 148;
 inline int grid_1d(int64_t n, int threads = 256) { return clamp_grid(ceil_div(n, threads), 148 * 16); }
 
 // Dynamic shared memory above 48 KB is opted into once per kernel at handle
@@ -1197,6 +1196,7 @@ cudaError_t prepare_kernels() {
   chk(prepare_panel());
   chk(prepare_update_tc());
   chk(prepare_update_tcq());
+  chk(prepare_update_dp());
   chk(opt_in(k_update_simt<double>)); chk(opt_in(k_update_simt<float>));
   chk(opt_in(k_update_dmma2<4, 2>)); chk(opt_in(k_update_dmma2<2, 1>));
   return e;

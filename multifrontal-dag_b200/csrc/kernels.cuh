@@ -11,6 +11,7 @@
 
 namespace mfd {
 
+constexpr int kNumSms = 148;
 constexpr int kSmallFrontMax = 160;   // widest front of the one-CTA / one-warp small-front kernels
 constexpr int kFactB = 128;          // column panel of the blocked large-front factorization
 constexpr int kTrRowsH = 64;         // rows per CTA of the panel TRSM
@@ -154,11 +155,11 @@ template <typename T>
 void launch_potrf(const DevFronts& F, const int32_t* list, int count, int step, T* panel, double* packed, int32_t* info,
                   cudaStream_t st, bool pdl = false, int info_stride = 0, int32_t* fallbacks = nullptr,
                   const int32_t* cls = nullptr);
-// max_w: the widest diagonal block of the step.  q (FP32 only, may be null): also write the solved
-// rows as packed TF32 operands of the tensor-core update (packed_offset below), at q + F.q_off[f].
+// max_w: the widest diagonal block of the step.  q (may be null): also write the solved rows as packed
+// operands of the update (FP32: TF32 hi / lo, packed_offset; FP64: packed_dp_offset), at q + F.q_off[f].
 template <typename T>
 void launch_trsm(const DevFronts& F, const int32_t* list, int count, int step, int row_blocks, int max_w, T* panel,
-                 const double* packed, cudaStream_t st, bool pdl = false, float* q = nullptr);
+                 const double* packed, cudaStream_t st, bool pdl = false, T* q = nullptr);
 template <typename T>
 void launch_invert(const DevFronts& F, const int32_t* list, int count, int steps, int max_w, const T* panel, T* linv,
                    cudaStream_t st);
@@ -200,6 +201,21 @@ cudaError_t prepare_update_tcq();
 int launch_update_tcq(const DevFronts& F, const int32_t* list, int count, int step, int T128, const float* q,
                       const float* qprev, float* panel, float* upool, int split, int32_t* err, cudaStream_t st,
                       UpdBand band = {}, int defer = 1, bool pdl = false);
+// The same for FP64 (update_dp.cu): 128-row blocks of 128 columns, kFactB * kFactB doubles each, in
+// chunks of 16 columns, [row][16] with column k at position 4 (k % 4) + (k % 16) / 4 and the
+// row's 16-byte pairs XORed by (row & 1).  Step t's rows at q + (t % nbuf) * buf; err[0] is raised
+// if a bounded wait expires.
+constexpr int kPackedDefer = 2;       // the deepest deferral the packed-operand updates take
+#ifdef __CUDACC__
+__device__ __forceinline__ int64_t packed_dp_offset(int row, int k) {   // row, k: 0-based within the step
+  const int r = row & 127, pos = 4 * (k & 3) + ((k & 15) >> 2);
+  return (int64_t)(row >> 7) * (kFactB * kFactB) + (k >> 4) * (kFactB * 16) + r * 16 + (pos ^ ((r & 1) << 1));
+}
+#endif
+cudaError_t prepare_update_dp();
+int launch_update_dp(const DevFronts& F, const int32_t* list, int count, int step, int T128, const double* q, int64_t buf,
+                     int nbuf, double* panel, double* upool, int32_t* err, cudaStream_t st, UpdBand band, int defer,
+                     bool pdl);
 // grid size of an update launch over a band of the T x T lower tiles of width tw
 int update_grid(int T, int tw, UpdBand band);
 

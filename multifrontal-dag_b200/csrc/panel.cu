@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(potrf_threads<NSB>(), 1) k_potrf(DevFronts F, 
 constexpr int kTrWarps = 4;
 template <typename T>
 __global__ void __launch_bounds__(32 * kTrWarps, 3) k_trsm(DevFronts F, const int32_t* list, int step, T* panel,
-                                                        const double* packed, float* q) {
+                                                        const double* packed, T* q) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* L = reinterpret_cast<double*>(smem_raw);
   const int f = list[blockIdx.y];
@@ -150,7 +150,18 @@ __global__ void __launch_bounds__(32 * kTrWarps, 3) k_trsm(DevFronts F, const in
     if (ok && c < w) P[(size_t)c * nf] = (T)acc[b].x;
     if (ok && c + 1 < w) P[(size_t)(c + 1) * nf] = (T)acc[b].y;
   }
-  if constexpr (sizeof(T) == 4) {
+  if constexpr (sizeof(T) == 8) {
+    if (q != nullptr) {     // the same rows as packed operands of the update
+      double* Qf = q + F.q_off[f];
+      const int r = rel + 8 * warp + g;
+#pragma unroll
+      for (int b = 0; b < 16; ++b) {
+        const int c = 8 * b + c2;
+        Qf[packed_dp_offset(r, c)] = ok && c < w ? acc[b].x : 0.0;
+        Qf[packed_dp_offset(r, c + 1)] = ok && c + 1 < w ? acc[b].y : 0.0;
+      }
+    }
+  } else {
     if (q != nullptr) {     // the same rows as packed TF32 hi / lo operands of the tensor-core update
       float* Qf = q + F.q_off[f];
 #pragma unroll
@@ -270,12 +281,12 @@ void launch_potrf(const DevFronts& F, const int32_t* list, int count, int step, 
 
 template <typename T>
 void launch_trsm(const DevFronts& F, const int32_t* list, int count, int step, int row_blocks, int max_w, T* panel,
-                 const double* packed, cudaStream_t st, bool pdl, float* q) {
+                 const double* packed, cudaStream_t st, bool pdl, T* q) {
   if (count <= 0 || row_blocks <= 0) return;
   // row_blocks counts 64-row blocks; shared memory for the widest block of the launch
   const size_t smem = (size_t)blk_count((max_w + 7) / 8) * kBlkElems * sizeof(double);
   launch_k(k_trsm<T>, dim3(row_blocks * (kTrRowsH / (8 * kTrWarps)), count), dim3(32 * kTrWarps), smem, st, pdl, F, list,
-           step, panel, packed, sizeof(T) == 4 ? q : nullptr);
+           step, panel, packed, q);
 }
 
 template <typename T>
@@ -290,7 +301,7 @@ void launch_invert(const DevFronts& F, const int32_t* list, int count, int steps
   template void launch_potrf<T>(const DevFronts&, const int32_t*, int, int, T*, double*, int32_t*, cudaStream_t, bool, \
                                 int, int32_t*, const int32_t*);                                                    \
   template void launch_trsm<T>(const DevFronts&, const int32_t*, int, int, int, int, T*, const double*, cudaStream_t,  \
-                               bool, float*);                                                                      \
+                               bool, T*);                                                                      \
   template void launch_invert<T>(const DevFronts&, const int32_t*, int, int, int, const T*, T*, cudaStream_t);
 
 MFD_INSTANTIATE_PANEL(double)

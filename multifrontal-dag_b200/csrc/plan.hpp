@@ -53,7 +53,7 @@ struct DevFronts {
   const int64_t* s_off;       // scratch offset (large-front solve partial sums)
   const int64_t* d_off;       // offset of f's inverted 128 x 128 diagonal blocks (one per panel step);
                               // null: the inverse of list slot i lives at linv + i * 128 * 128
-  const int64_t* q_off;       // FP32: offset of f's packed update operands (null when unused)
+  const int64_t* q_off;       // offset of f's packed update operands
 };
 
 struct HostFront {
@@ -82,6 +82,7 @@ struct LevelPlan {
   LaunchList fwd_tasks, bwd_tasks;
   int32_t large_max_nf = 0;
   int32_t defer = 1;                 // panel steps per deferred trailing update
+  bool packed = false;               // the trailing updates read operands that the TRSM packs
 };
 
 }  // namespace mfd

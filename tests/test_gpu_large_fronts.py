@@ -124,3 +124,30 @@ def test_small_front_sizes(n, precision):
         r = np.abs(b - a @ X).max()
         den = np.abs(a).sum(axis=1).max() * np.abs(X).max() + np.abs(b).max()
         assert r / den <= (1e-14 if precision == 0 else 1e-12)
+
+
+@pytest.mark.parametrize("n", [2049, 2190])
+def test_packed_fp64_update_bitwise(n):
+    """A dense front long enough for the packed-operand FP64 update (its trailing
+    triangle in 128 x 64 pieces fills the chip), full and partial last panel: the
+    factor is bit for bit the one of the whole-tile kernel that reads the panel
+    (reserved[0] = 3), with the lookahead on and off, and with either deferral
+    depth; its backward error is at most 1e-14."""
+    a = _spd(n, n)
+    col = np.concatenate([[1], 1 + np.cumsum(np.arange(n, 0, -1))]).astype(np.int32)
+    rows = np.concatenate([np.arange(j + 1, n + 1) for j in range(n)]).astype(np.int32)
+    vals = np.concatenate([a[j:, j] for j in range(n)])
+    b = np.random.default_rng(1).uniform(-1, 1, n)
+    panels = {}
+    for kind, lookahead_off, defer in ((0, 0, 0), (0, 1, 0), (3, 0, 0), (0, 0, 1)):
+        s = H.Solver.analyze(n, col, rows, None, max_zero=0, reserved=(kind, lookahead_off, 0, 0, 0, defer, 0))
+        assert s.factorize(vals) == 0
+        x = b.copy()
+        s.solve(x)
+        den = np.abs(a).sum(axis=1).max() * np.abs(x).max() + np.abs(b).max()
+        assert np.abs(b - a @ x).max() / den <= 1e-14
+        panels[kind, lookahead_off, defer] = np.tril(s.front_panel(1).reshape((n, n), order="F"))
+        s.close()
+    ref = panels.pop((3, 0, 0))
+    for key, p in panels.items():
+        assert np.array_equal(p, ref), key
