@@ -50,9 +50,11 @@ constexpr int kWarpFrontsAtOnce = 148 * 24;   // one-warp fronts the chip holds 
 // panel chain (elasticity 21^3, mixed, with it on every level: 6.00 -> 6.16 ms).
 constexpr int kDeferDefault = 2;
 constexpr double kDeferBytes = 64e6;
-// FP64: levels whose largest front has this many rows pack the update's operands (below, the updates
-// are a few partly filled tiles and the panel itself is read)
-constexpr int kPackedDpRows = 768;
+// FP64: levels whose largest front has this many rows pack the update's operands.  Lower is faster
+// while pieces fill the chip (64^3 Laplacian 29.9 / 29.45 / 29.25 ms from 1536 / 768 / 128 rows on,
+// 30^3 elasticity 14.82 / 14.68 / 14.61); below three blocks of rows the operands of a batch's
+// thousands of fronts would take more memory than their panels.
+constexpr int kPackedDpRows = 3 * kFactB;
 int64_t align_up(int64_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
 template <typename T>
@@ -244,7 +246,7 @@ struct mfd_handle {
   void* d_exch = nullptr;                           // single-RHS sweeps: n_total exchange entries of 2 sizeof(T)
   std::vector<int> small_bins;
   int64_t panel_elems = 0, upool_elems = 0, v_elems = 0, s_elems = 0, dinv_elems = 0;
-  int64_t q_elems = 0;                              // packed update operands of one step
+  int64_t q_elems = 0;                              // packed update operands (2 defer steps) of the level that needs most
   int32_t max_large_count = 0, max_nf = 0;
   int64_t cost = 0, nonzero = 0;
 
@@ -554,7 +556,8 @@ int build_plan(mfd_handle* h) {
         fr.q_off = q;
         q += (nrem + kFactB - 1) / kFactB * (h->fp32 ? kPackedBlockElems : (int64_t)kFactB * kFactB);
       }
-      h->q_elems = std::max(h->q_elems, q);
+      L.q_elems = q;
+      h->q_elems = std::max(h->q_elems, 2 * L.defer * q);
     }
     // panel steps: prefix of the nc-sorted list
     int steps = (max_nc + kFactB - 1) / kFactB;
@@ -875,7 +878,7 @@ int upload_plan(mfd_handle* h) {
   if (h->max_large_count > 0)
     CK(cudaMalloc(&h->d_packed, (size_t)h->max_large_count * kPackedPanelElems * sizeof(double)));
   if (h->q_elems > 0) {
-    const size_t bytes = (size_t)(2 * h->defer * h->q_elems) * esz;
+    const size_t bytes = (size_t)h->q_elems * esz;
     CK(cudaMalloc(&h->d_q, bytes));
     // rows past a front's last row are never written and only reach discarded outputs; zero keeps them finite
     CK(cudaMemsetAsync(h->d_q, 0, bytes, h->st));
@@ -1091,7 +1094,7 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
     // buffers taken in turn: the bulk update of a group reads its own D, and is complete before
     // the TRSM of the group after the next one starts
     const bool packed = L.packed && (kind == 0 || (sizeof(T) == 4 && kind == 2));
-    auto packed_rows = [&](size_t step) { return static_cast<T*>(h->d_q) + (step % (2 * D)) * h->q_elems; };
+    auto packed_rows = [&](size_t step) { return static_cast<T*>(h->d_q) + (step % (2 * D)) * L.q_elems; };
     int pend = -1;                            // step of the latest bulk on st2 not yet fully waited for
     for (size_t s = 0; s < L.steps.size(); ++s) {
       const LaunchList& p = L.steps[s];
@@ -1161,10 +1164,11 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
             }
           }
           if constexpr (sizeof(T) == 8) {
-            // where 128 x 64 pieces fill the chip; launch_update's smaller ones read the panel
-            if (packed && (int64_t)2 * update_grid(p.param2, kUpdTile, band) * p.count > kNumSms) {
+            // where 128 x 64 pieces reach half of the SMs or more; below, launch_update's smaller ones
+            // that read the panel (64^3 Laplacian 29.30 / 29.12 ms with the line at 148 / 64 pieces)
+            if (packed && (int64_t)2 * update_grid(p.param2, kUpdTile, band) * p.count > kNumSms / 2) {
               n += launch_update_dp(F, lists + p.off, p.count, (int)s, p.param2, static_cast<const double*>(h->d_q),
-                                    h->q_elems, 2 * D, reinterpret_cast<double*>(panel), reinterpret_cast<double*>(upool),
+                                    L.q_elems, 2 * D, reinterpret_cast<double*>(panel), reinterpret_cast<double*>(upool),
                                     h->d_info.p + 1, us, band, D, upd_pdl);
               return;
             }
@@ -1924,8 +1928,7 @@ int mfd_autotune(mfd_handle* h, const double* a, int32_t repeats, mfd_options* b
       mfd_options o = base;
       o.reserved[0] = kinds[ki];
       o.reserved[5] = d;
-      const int base_d = base.reserved[5] > 0 ? base.reserved[5] : kDeferDefault;
-      if (kinds[ki] == base.reserved[0] && d == base_d) continue;   // timed in stage 1
+      if (kinds[ki] == base.reserved[0] && d == base.reserved[5]) continue;   // timed in stage 1
       int rc = consider(o);
       if (rc) return rc;
     }

@@ -83,6 +83,7 @@ struct LevelPlan {
   int32_t large_max_nf = 0;
   int32_t defer = 1;                 // panel steps per deferred trailing update
   bool packed = false;               // the trailing updates read operands that the TRSM packs
+  int64_t q_elems = 0;               // of one panel step
 };
 
 }  // namespace mfd
