@@ -51,15 +51,16 @@ typedef struct {
   double ir_tol;           /* target normwise backward error, default 1e-12                   */
   int32_t use_graph;       /* 1: replay factor/solve as CUDA graphs (default 1)               */
   int32_t device;          /* CUDA device ordinal (default 0)                                 */
-  int32_t small_front_max; /* fronts up to this order run in the fused one-CTA kernel (0=auto)*/
+  int32_t small_front_max; /* fronts up to this order (at most 160) run in the fused kernels (0=auto) */
   int32_t panel_width;     /* column panel of the blocked large-front factorization (0=auto) */
   int32_t reserved[7];     /* schedule switches, 0 = default: [0] trailing-update kind (1 FFMA
                               tiles, 2 single-pass TF32, 3 FP64 DMMA in whole 128 x 128 tiles),
                               [1] = 1 lookahead off, [2] = 1 programmatic launch along the panel
                               chain, [3] = 1 no programmatic launch between solve steps, [4] = 1
                               no side streams per level, [5] = panel steps per deferred trailing
-                              update (1 = none), [6] = 1 single-RHS large-front solves one launch
-                              per panel step instead of one per level                           */
+                              update (1 = none; 0: two on levels whose fronts exceed 64 MB),
+                              [6] = 1 large-front solves one launch per panel step instead of
+                              one per level                                                     */
 } mfd_options;
 
 /* Symbolic data exactly as the reference holds it after hppllt_analyze
@@ -98,8 +99,9 @@ typedef struct {
   double time_info[7];      /* the reference's 7 phase timers (time_list_m.f90:3-10), seconds:
                                ordering, analyze, factorize, solve, forward, backward,
                                real_factorize                                                  */
-  int64_t pivot_fallbacks;  /* FP32 factorization: 32-column diagonal sub-blocks whose FP32 pivot
-                               chain met a small pivot and was redone in FP64 (last factorize) */
+  int64_t pivot_fallbacks;  /* FP32 factorization: 32-column diagonal sub-blocks with a pivot below
+                               2^-12 of its starting diagonal entry (factored in FP64, as all
+                               are; last factorize)                                            */
   double setup_s[4];        /* handle set-up, seconds: host symbolic analysis (mfd_analyze*),
                                level / memory plan, device index maps and their exports,
                                residual CSR and numeric storage                                */
@@ -248,12 +250,12 @@ int64_t mfd_get_front_panel(mfd_handle *h, int32_t system, int32_t node, double 
  * each class accumulates its launches, device time and algorithmic work
  * (flops and bytes of the algorithm, not hardware counters). */
 #define MFD_K_SMALL_FRONT 0   /* fused one-CTA fronts                         */
-#define MFD_K_ZERO 1          /* large-front zero fill                         */
+#define MFD_K_ZERO 1          /* no launches: the gather writes every entry    */
 #define MFD_K_ASSEMBLE 2      /* large-front assembly of A                     */
-#define MFD_K_EXTEND_ADD 3    /* large-front extend-add                        */
-#define MFD_K_PANEL 4         /* diagonal-block POTRF + inverse                */
+#define MFD_K_EXTEND_ADD 3    /* large fronts, gather of the children          */
+#define MFD_K_PANEL 4         /* diagonal-block POTRF; inverses for the solves */
 #define MFD_K_UPDATE 5        /* trailing SYRK/GEMM update                     */
-#define MFD_K_SOLVE_SMALL 6   /* one-CTA forward/backward solves               */
+#define MFD_K_SOLVE_SMALL 6   /* forward/backward solves of small fronts       */
 #define MFD_K_SOLVE_LARGE 7   /* blocked forward/backward solves               */
 #define MFD_K_OTHER 8         /* permutations, residuals, norms                */
 #define MFD_K_TRSM 9          /* panel TRSM (rows below the diagonal block)    */
@@ -274,8 +276,8 @@ int mfd_get_profile(mfd_handle *h, int32_t kind, mfd_kernel_profile *out);
  * next mfd_factorize returns MFD_E_TIMEOUT (no GPU fault: every wait is
  * bounded).  Disable it and the handle factors normally again.  FP64 handles
  * and fronts that use no tensor-core update factor normally.  While enabled,
- * the single-RHS large-front solve sweeps' device waits (one launch per level,
- * tasks waiting on other tasks' flags) likewise wait for a value nothing
+ * the large-front solve sweeps' device waits (one launch per level, tasks
+ * waiting on other tasks' values or flags) likewise wait for a value nothing
  * writes, with a ~1 ms limit: mfd_solve returns MFD_E_TIMEOUT, and solves
  * normally once the request is withdrawn. */
 int mfd_test_expire_waits(mfd_handle *h, int32_t enable);

@@ -4,8 +4,12 @@
 
 Sources: csrc/analysis.cpp (host symbolic analysis), csrc/ordering.cpp (nested
 dissection ordering), csrc/partition.cpp (subtree-to-GPU mapping),
-csrc/kernels.cu (device
-kernels), csrc/update_tc.cu (FP32 tcgen05 update), csrc/api.cu (C ABI, plan,
+csrc/kernels.cu (index
+maps, large-front assembly, panel-fed updates), csrc/small_front.cu and
+csrc/small_solve.cu (fronts up to 160 rows), csrc/panel.cu (POTRF, TRSM),
+csrc/solve_single.cu and csrc/solve_multi.cu (large-front sweeps),
+csrc/update_tc.cu (FP32 tcgen05 update), csrc/update_dp.cu (FP64 update from
+packed operands), csrc/api.cu (C ABI, plan,
 launch sequences), csrc/noalloc.cu (allocation-free fronts), csrc/input.cu
 (Matrix Market, COO -> CCS on the GPU, CSR input).  Output:
 multifrontal-dag_b200/mfdag/libmfdag.so, loaded by mfdag/hppllt.py.
@@ -19,8 +23,8 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "mfdag", "libmfdag.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-SOURCES = ["analysis.cpp", "ordering.cpp", "partition.cpp", "kernels.cu", "small_front.cu", "small_solve.cu", "panel.cu", "solve_single.cu", "solve_multi.cu", "update_tc.cu", "update_dp.cu", "api.cu", "noalloc.cu",
-           "input.cu"]
+SOURCES = ["analysis.cpp", "ordering.cpp", "partition.cpp", "kernels.cu", "small_front.cu", "small_solve.cu", "panel.cu",
+           "solve_single.cu", "solve_multi.cu", "update_tc.cu", "update_dp.cu", "api.cu", "noalloc.cu", "input.cu"]
 
 
 def build(debug: bool = False, verbose: bool = False) -> str:

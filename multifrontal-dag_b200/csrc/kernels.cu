@@ -2,18 +2,15 @@
 //
 // Index maps (built once):      local_index, supernodal_index + assembly map,
 //                               block_local_index (reference tiling, export only)
-// Factorization, per tree level: fused kernels for small fronts (assembly +
-//                               extend-add + partial Cholesky on chip: one warp
-//                               per front up to 32 rows, one CTA per front up to
-//                               128 with the trailing update on DMMA tiles);
-//                               blocked global-memory path for large fronts
-//                               (zero, assemble, extend-add per child rank, panel
-//                               POTRF+TRSM, trailing SYRK/GEMM on the FP64 tensor
-//                               pipe (DMMA), tcgen05 3xTF32 (update_tc.cu) or
-//                               FFMA tiles)
-// Solves:                       forward/backward per level with the same split
-//                               (one warp per small front; 128-column steps with
-//                               the kept inverted diagonal blocks for large ones)
+// Factorization, per tree level: large fronts in global memory (gather of the
+//                               children, assembly, trailing SYRK/GEMM on the FP64
+//                               tensor pipe (DMMA) or FFMA tiles; small fronts are
+//                               in small_front.cu, the panel steps' POTRF / TRSM in
+//                               panel.cu, the updates from packed operands in
+//                               update_dp.cu and update_tc.cu)
+// Solves:                       permutations and the large fronts' per-step form
+//                               (small_solve.cu, solve_single.cu and solve_multi.cu
+//                               hold the rest)
 // Residual / norms:             FP64 CSR SpMV for iterative refinement.
 #include <cuda_runtime.h>
 

@@ -22,7 +22,7 @@
 // any MMA, every CTA waits on an mbarrier that nothing arrives at, with a
 // ~1 ms limit, so the expiry path runs without any fault.
 //
-// k_update_tcq (deferral depth 1, the default schedule) takes its operands
+// k_update_tcq (deferral depth 1 and 2, the default schedule) takes its operands
 // already split: the step's TRSM writes the solved rows once as TF32 hi / lo
 // blocks in the UMMA layout (packed_offset), so the main loop does no SIMT
 // work per element.  Warp-specialised, one tile per CTA, two CTAs per SM:
