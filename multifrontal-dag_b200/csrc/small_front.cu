@@ -12,8 +12,11 @@
 // With the records, the block layout and two panels per update pass the whole
 // steps take: 100 x 100 Laplacian 975 -> 554 us, batch of 1000 2D systems 12.35
 // -> 8.37 ms (1.5 TFLOP/s, 0.9 TB/s).  160 rows is the line to the blocked path:
-// up to there a front fits one CTA's shared memory next to another's, and its two
-// panel steps there cost ~37 us each whatever their width.
+// up to there a front's blocks (105 KB) leave room for a second CTA on the SM, and
+// the blocked path's two panel steps cost ~37 us each whatever their width.  Line
+// at 128 / 160 rows: batch of 1000 8.90 / 8.39 ms, batch solve 802 / 774 us, 100 x
+// 100 Laplacian 598 / 573 us, 21^3 elasticity 5.90 / 5.88 ms, 37 x 41 x 43 solve
+// 798 / 810 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>

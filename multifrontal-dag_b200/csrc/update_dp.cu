@@ -16,8 +16,11 @@
 // the operands from the panel itself takes 12 8- or 16-byte cp.async per thread
 // and 32 columns with their addresses, and 8-byte fragment loads: 24.6 TFLOP/s on
 // a 43-tile trailing matrix with K = 256, of 36.9 of the pipe.  With packed
-// operands the 64^3 Laplacian's whole step goes from 33.0 to 29.4 ms, 30^3
-// elasticity with 64 right-hand sides from 15.7 to 14.7 ms.
+// operands the 64^3 Laplacian's whole step goes from 33.0 to 29.2 ms, 30^3
+// elasticity with 64 right-hand sides from 15.7 to 14.6 ms; the pipe is active in
+// 60-63 % of a bulk launch's cycles (50 before).  One barrier per chunk for the
+// whole CTA: refilling a stage on a barrier of its own, warp by warp, was no faster
+// (29.5 ms, more registers spilled).
 #include <cuda_runtime.h>
 
 #include <algorithm>
