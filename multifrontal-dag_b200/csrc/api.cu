@@ -21,6 +21,7 @@
 #include "analysis.hpp"
 #include "kernels.cuh"
 #include "plan.hpp"
+#include "small_bins.hpp"
 
 namespace mfd {
 namespace {
@@ -43,7 +44,6 @@ int fail(int code, const std::string& msg) {
 constexpr int64_t kAlign = 32;  // elements; keeps every front 256-byte aligned in FP64
 constexpr int kResMulti = 4;     // from this many right-hand sides on, one multi-column residual per IR sweep
 constexpr int kPotrfSplitMin = 148;   // fronts in a panel step above which POTRF launches per width class
-constexpr int kWarpFrontsAtOnce = 148 * 24;   // one-warp fronts the chip holds at once
 // panel steps per deferred trailing update: K = 256 per pass halves the update's C traffic, which
 // counts on levels whose trailing matrices pass through HBM, their lower triangles above half of the
 // 126 MB L2 (80^3 diffusion, mixed: 45.7 -> 40.7 ms).  Below, a deferred update only lengthens the
@@ -465,9 +465,7 @@ int build_plan(mfd_handle* h) {
     h->upool_elems = std::max<int64_t>(ff.top, kAlign);
   }
   // level launch lists
-  h->small_bins = std::vector<int>{16, 24, 32, 64, 96, 128, 160};
-  while (!h->small_bins.empty() && h->small_bins.back() > sfm) h->small_bins.pop_back();
-  if (h->small_bins.empty() || h->small_bins.back() < sfm) h->small_bins.push_back(sfm);
+  h->small_bins = small_bin_sizes(sfm);
   h->levels.assign(nlev, LevelPlan{});
   h->h_lists.clear();
   h->h_stasks.clear();
@@ -480,26 +478,13 @@ int build_plan(mfd_handle* h) {
     LevelPlan& L = h->levels[l];
     std::vector<std::vector<int32_t>> bins(h->small_bins.size());
     std::vector<int32_t> large;
-    // the one-warp fronts in one launch sized for the largest unless they fill the chip more than
-    // once: below that the launches' number counts, not their warps' registers and shared memory
-    int warp_fronts = 0, warp_max = 0;
-    for (int32_t g : lev_fronts[l]) {
-      const int nf = h->fronts[g].nc + h->fronts[g].nr;
-      if (nf > 32) continue;
-      ++warp_fronts;
-      warp_max = std::max(warp_max, nf);
-    }
-    const bool split_warp_bins = warp_fronts > kWarpFrontsAtOnce;
-    for (int32_t g : lev_fronts[l]) {
-      int nf = h->fronts[g].nc + h->fronts[g].nr;
-      if (nf <= sfm) {
-        const int fit = nf <= 32 && !split_warp_bins ? warp_max : nf;
-        size_t b = 0;
-        while (h->small_bins[b] < fit) ++b;
-        bins[b].push_back(g);
-      } else {
-        large.push_back(g);
-      }
+    std::vector<int> orders;
+    orders.reserve(lev_fronts[l].size());
+    for (int32_t g : lev_fronts[l]) orders.push_back(h->fronts[g].nc + h->fronts[g].nr);
+    const std::vector<int> bin_of = small_bins_of_level(h->small_bins, sfm, orders);
+    for (size_t k = 0; k < bin_of.size(); ++k) {
+      if (bin_of[k] >= 0) bins[bin_of[k]].push_back(lev_fronts[l][k]);
+      else large.push_back(lev_fronts[l][k]);
     }
     for (size_t b = 0; b < bins.size(); ++b) {
       if (bins[b].empty()) continue;
