@@ -1,6 +1,7 @@
 // Host side of the C ABI (include/mfdag.h): handle, static plan, graph-captured
 // launch sequences, iterative refinement, exports, and the reference-named
 // hppllt_* entry points.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -11,7 +12,6 @@
 #include <cstring>
 #include <map>
 #include <memory>
-#include <mutex>
 #include <set>
 #include <string>
 #include <thread>
@@ -21,6 +21,7 @@
 #include "analysis.hpp"
 #include "kernels.cuh"
 #include "plan.hpp"
+#include "slot_pool.hpp"
 #include "small_bins.hpp"
 
 namespace mfd {
@@ -151,49 +152,31 @@ struct HostStatus {
   int32_t ir_i[2];
   int32_t expired;
 };
-// One page-locked block for the process, cut into slots (a handle takes one and gives it back);
-// page-locking memory per handle would cost more than a small handle's set-up.
-class StatusPool {
- public:
-  HostStatus* take() {
-    std::lock_guard<std::mutex> lk(mu_);
-    if (!base_) {
-      void* p = nullptr;
-      if (cudaHostAlloc(&p, kSlots * kSlotBytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+struct StatusMemory {                       // what SlotPool takes its blocks from
+  // id of the current context; after a device reset the device's context has another one
+  static unsigned long long context() {
+    static const auto get_id = [] {
+      void* f = nullptr;
+      cudaDriverEntryPointQueryResult found;
+      if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &found) != cudaSuccess) {
         cudaGetLastError();
-        return nullptr;
+        f = nullptr;
       }
-      base_ = static_cast<char*>(p);
-      for (int i = kSlots; i-- > 0;) free_.push_back(i);
-    }
-    if (!free_.empty()) {
-      const int i = free_.back();
-      free_.pop_back();
-      return reinterpret_cast<HostStatus*>(base_ + i * kSlotBytes);
-    }
-    void* p = nullptr;                      // every slot in use: an allocation of its own
-    if (cudaHostAlloc(&p, kSlotBytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
-    return static_cast<HostStatus*>(p);
+      return reinterpret_cast<CUresult (*)(CUcontext, unsigned long long*)>(f);
+    }();
+    unsigned long long id = 0;
+    return get_id && get_id(nullptr, &id) == CUDA_SUCCESS ? id : 0;
   }
-  void give(HostStatus* s) {
-    if (!s) return;
-    std::lock_guard<std::mutex> lk(mu_);
-    char* p = reinterpret_cast<char*>(s);
-    if (base_ && p >= base_ && p < base_ + kSlots * kSlotBytes) free_.push_back((int)((p - base_) / kSlotBytes));
-    else cudaFreeHost(p);
+  static void* lock(size_t bytes) {
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
   }
-
- private:
-  static constexpr int kSlots = 256;
-  static constexpr size_t kSlotBytes = 256;
-  static_assert(sizeof(HostStatus) <= kSlotBytes, "slot size");
-  std::mutex mu_;
-  char* base_ = nullptr;
-  std::vector<int> free_;
+  static void unlock(void* p) { cudaFreeHost(p); }
 };
+using StatusPool = SlotPool<StatusMemory>;
+static_assert(sizeof(HostStatus) <= StatusPool::kSlotBytes, "slot size");
 StatusPool& status_pool() {
   static StatusPool* p = new StatusPool();  // never destroyed: handles may outlive static destruction
   return *p;
@@ -289,7 +272,8 @@ struct mfd_handle {
   bool factored = false;
   bool expire_waits = false;                        // test request (mfd_test_expire_waits)
   bool expire_on_device = false;                    // its value in d_info[2]
-  HostStatus* status = nullptr;
+  StatusPool::Slot status_slot;
+  HostStatus* status = nullptr;                     // in status_slot
   int64_t pivot_fallbacks = 0;                      // FP32 diagonal sub-blocks redone in FP64, last factorize
   int64_t launches_factor = 0, launches_solve = 0;
   double factor_ms = 0, solve_ms = 0, anorm = 0;
@@ -313,7 +297,7 @@ struct mfd_handle {
 
   ~mfd_handle() {
     if (st) cudaStreamSynchronize(st);
-    status_pool().give(status);
+    status_pool().give(status_slot);
     for (cudaEvent_t e : event_pool) cudaEventDestroy(e);
     if (g_factor) cudaGraphExecDestroy(g_factor);
     for (auto& kv : g_solve) cudaGraphExecDestroy(kv.second);
@@ -1650,7 +1634,8 @@ int create_common(mfd_handle** out, std::vector<Symbolic>&& syms, const mfd_opti
   h->sys = std::move(syms);
   CK(cudaSetDevice(h->device));
   CK(prepare_kernels());
-  h->status = status_pool().take();
+  h->status_slot = status_pool().take(h->device);
+  h->status = static_cast<HostStatus*>(h->status_slot.p);
   if (!h->status) return fail(MFD_E_NOMEM, "no page-locked memory for a handle's status");
   int prio_lo = 0, prio_hi = 0;
   CK(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi));
