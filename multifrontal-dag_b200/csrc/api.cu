@@ -37,9 +37,11 @@ int fail(int code, const std::string& msg) {
 #define CK(call)                                                                             \
   do {                                                                                       \
     cudaError_t e_ = (call);                                                                 \
-    if (e_ != cudaSuccess)                                                                   \
+    if (e_ != cudaSuccess) {                                                                 \
+      cudaGetLastError(); /* reported here: not again by the next look at the last error */  \
       return fail(e_ == cudaErrorMemoryAllocation ? MFD_E_NOMEM : MFD_E_CUDA,                \
                   std::string(#call) + ": " + cudaGetErrorString(e_));                       \
+    }                                                                                        \
   } while (0)
 
 constexpr int64_t kAlign = 32;  // elements; keeps every front 256-byte aligned in FP64
@@ -871,8 +873,11 @@ bool solve_fused(const mfd_handle* h, int nrhs) {
          (int64_t)h->h_stasks.size() / 4 * multi_tiles(nrhs) <= INT32_MAX;
 }
 
+// Storage for nrhs right-hand sides.  Until all of it is there the handle has none (nrhs_cap 0): the
+// solve after a failed one allocates again, as much as it needs itself.
 int ensure_rhs(mfd_handle* h, int nrhs) {
   if (nrhs <= h->nrhs_cap) return MFD_OK;
+  h->nrhs_cap = 0;
   for (auto& kv : h->g_solve) cudaGraphExecDestroy(kv.second);
   h->g_solve.clear();
   for (auto& kv : h->g_ir) cudaGraphExecDestroy(kv.second);
@@ -880,8 +885,8 @@ int ensure_rhs(mfd_handle* h, int nrhs) {
   size_t esz = h->fp32 ? sizeof(float) : sizeof(double);
   for (void** p : {&h->d_X, &h->d_V, &h->d_S, &h->d_bwpart})
     if (*p) { cudaFree(*p); *p = nullptr; }
-  if (!h->d_exch && solve_fused(h, 1)) {
-    CK(cudaMalloc(&h->d_exch, (size_t)h->n_total * 2 * esz));
+  if (!h->d_epoch.p && solve_fused(h, 1)) {
+    if (!h->d_exch) CK(cudaMalloc(&h->d_exch, (size_t)h->n_total * 2 * esz));
     CK(cudaMemsetAsync(h->d_exch, 0, (size_t)h->n_total * 2 * esz, h->st));
     CK(h->d_epoch.alloc(1));
     CK(cudaMemsetAsync(h->d_epoch.p, 0, sizeof(int32_t), h->st));
