@@ -231,6 +231,7 @@ struct mfd_handle {
   void* d_exch = nullptr;                           // single-RHS sweeps: n_total exchange entries of 2 sizeof(T)
   std::vector<int> small_bins;
   int64_t panel_elems = 0, upool_elems = 0, v_elems = 0, s_elems = 0, dinv_elems = 0;
+  int64_t g_elems = 0;                              // gathered vectors of the level's fronts of many children, largest level
   int64_t q_elems = 0;                              // packed update operands (2 defer steps) of the level that needs most
   int32_t max_large_count = 0, max_nf = 0;
   int64_t cost = 0, nonzero = 0;
@@ -246,7 +247,7 @@ struct mfd_handle {
   DBuf<int64_t> d_inv_off;
   DBuf<FrontRec> d_rec;
   DBuf<ChildRec> d_crec;
-  DBuf<int64_t> d_panel_off, d_u_off, d_v_off, d_s_off, d_d_off, d_q_off;
+  DBuf<int64_t> d_panel_off, d_u_off, d_v_off, d_s_off, d_d_off, d_q_off, d_g_off;
   DevFronts F{};
 
   // CSR of the permuted full matrix (residuals)
@@ -261,7 +262,7 @@ struct mfd_handle {
   void* d_diag = nullptr;
   double* d_packed = nullptr;                       // the current panel step's packed diagonal blocks, one per list slot
   void* d_q = nullptr;                              // T, packed update operands, 2 defer step buffers
-  DBuf<double> d_a, d_b, d_xp, d_bp, d_r, d_norms, d_cnorms, d_xt;
+  DBuf<double> d_a, d_b, d_xp, d_bp, d_r, d_norms, d_cnorms, d_xt, d_G;
   void* d_X = nullptr;   // T, n_total x nrhs
   void* d_V = nullptr;   // T
   void* d_S = nullptr;   // T
@@ -458,6 +459,7 @@ int build_plan(mfd_handle* h) {
   h->solve_flags = 0;
   h->bw_part_elems = 0;
   h->max_large_count = 0;
+  h->g_elems = 0;
   std::vector<std::vector<int32_t>> lev_fronts(nlev);
   for (int32_t g = 0; g < nfr; ++g) lev_fronts[h->fronts[g].level].push_back(g);
   for (int l = 0; l < nlev; ++l) {
@@ -507,6 +509,21 @@ int build_plan(mfd_handle* h) {
     }
     L.large.param = max_entries;
     L.large.param2 = max_nc;
+    {
+      std::vector<int32_t> many;
+      int64_t g_elems = 0;
+      for (int32_t g : large) {
+        HostFront& fr = h->fronts[g];
+        if (cnt[g] <= kManyChildren) continue;
+        many.push_back(g);
+        L.many_max_nf = std::max(L.many_max_nf, fr.nc + fr.nr);
+        fr.g_off = g_elems;
+        g_elems += fr.nc + fr.nr;
+      }
+      L.many.off = push_list(h, many);
+      L.many.count = (int32_t)many.size();
+      h->g_elems = std::max(h->g_elems, g_elems);
+    }
     // deferral depth: the caller's (reserved[5]) on every level, the default where it pays
     {
       double bytes = 0;
@@ -611,12 +628,13 @@ int upload_plan(mfd_handle* h) {
   cudaStream_t st = h->st;
   const int32_t nfr = h->num_front;
   std::vector<int32_t> nc(nfr), nr(nfr), first(nfr), parent(nfr);
-  std::vector<int64_t> poff(nfr), uoff(nfr), voff(nfr), soff(nfr), doff(nfr), qoff(nfr);
+  std::vector<int64_t> poff(nfr), uoff(nfr), voff(nfr), soff(nfr), doff(nfr), qoff(nfr), goff(nfr);
   for (int32_t g = 0; g < nfr; ++g) {
     const HostFront& f = h->fronts[g];
     nc[g] = f.nc; nr[g] = f.nr; first[g] = f.first; parent[g] = f.parent;
     poff[g] = f.panel_off; uoff[g] = f.u_off; voff[g] = f.v_off; soff[g] = f.s_off; doff[g] = f.d_off;
     qoff[g] = f.q_off;
+    goff[g] = f.g_off;
   }
   std::vector<int32_t> lrow_glob;
   lrow_glob.reserve(h->h_lrow_off[nfr]);
@@ -638,6 +656,7 @@ int upload_plan(mfd_handle* h) {
   CK(h->d_s_off.upload(soff, st));
   CK(h->d_d_off.upload(doff, st));
   CK(h->d_q_off.upload(qoff, st));
+  if (h->g_elems > 0) CK(h->d_g_off.upload(goff, st));
   CK(h->d_lists.upload(h->h_lists, st));
   // the fused sweeps' task entries hold 32-bit partial-sum bases and flag offsets: beyond that
   // range (far larger problems than one GPU holds) the per-step sweeps are used instead
@@ -664,7 +683,7 @@ int upload_plan(mfd_handle* h) {
   F.a_src = h->d_a_src.p; F.a_pos = h->d_a_pos.p; F.v_off = h->d_v_off.p; F.s_off = h->d_s_off.p;
   F.d_off = h->d_d_off.p;
   F.q_off = h->d_q_off.p;
-
+  F.g_off = h->d_g_off.p;
 
   // permuted global A structure, value sources, front of every column
   std::vector<int32_t> acol(h->n_total + 1), arow(h->nnz_total), src(h->nnz_total), colf(h->n_total),
@@ -786,7 +805,7 @@ int upload_plan(mfd_handle* h) {
     }
   }
 
-  // the children of large fronts: the inverse of their local index; the fronts' and children's records
+  // the children of large fronts, unless many: the inverse of their local index; the fronts' and children's records
   if (h->max_large_count > 0) {
     std::vector<int64_t> ioff(nfr, 0);
     std::vector<int32_t> kids;
@@ -795,6 +814,7 @@ int upload_plan(mfd_handle* h) {
     for (int32_t g = 0; g < nfr; ++g) {
       const int32_t p = h->fronts[g].parent;
       if (p < 0 || h->fronts[p].nc + h->fronts[p].nr <= sfm) continue;
+      if (h->h_child_ptr[p + 1] - h->h_child_ptr[p] > kManyChildren) continue;
       ioff[g] = len;
       len += h->fronts[p].nc + h->fronts[p].nr;
       kids.push_back(g);
@@ -900,6 +920,7 @@ int ensure_rhs(mfd_handle* h, int nrhs) {
   CK(cudaMalloc(&h->d_X, (size_t)std::max<int64_t>(h->n_total, 1) * nrhs * esz));
   CK(cudaMalloc(&h->d_V, (size_t)std::max<int64_t>(h->v_elems, 1) * nrhs * esz));
   CK(cudaMalloc(&h->d_S, (size_t)std::max<int64_t>(h->s_elems, 1) * nrhs * esz));
+  if (h->g_elems > 0) CK(h->d_G.alloc((size_t)h->g_elems * nrhs));
   CK(h->d_b.alloc((size_t)h->n_total * nrhs));
   CK(h->d_xp.alloc((size_t)h->n_total * nrhs));
   CK(h->d_bp.alloc((size_t)h->n_total * nrhs));
@@ -1048,6 +1069,11 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
     record(h, st, MFD_K_ASSEMBLE, 0, ab,
            [&] { launch_assemble_large<T>(F, lists + L.large.off, L.large.count, L.large.param, a, panel, upool, st); });
     n += 2;
+    if (L.many.count) {
+      record(h, st, MFD_K_EXTEND_ADD, 0, 0,
+             [&] { launch_add_children<T>(F, lists + L.many.off, L.many.count, L.many_max_nf, panel, upool, st); });
+      ++n;
+    }
     // Lookahead (on unless reserved[1] = 1; profiling runs the serial schedule so
     // that every kernel is timed alone) with deferred updates (groups of D =
     // h->defer panel steps, update_k_range): after the TRSM of step s the next
@@ -1237,16 +1263,20 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
   }
   // a level's fused sweep
   auto sweep = [&](const LevelPlan& L, bool backward) {
+    if (!backward && L.many.count) {
+      launch_gather_many<T>(F, lists + L.many.off, L.many.count, L.many_max_nf, X, ldx, V, h->d_G.p, nrhs, st);
+      ++n;
+    }
     const LaunchList& tl = backward ? L.bwd_tasks : L.fwd_tasks;
     int32_t* ticket = ssync + 1 + 2 * (&L - h->levels.data()) + (backward ? 1 : 0);
     int32_t* flags = backward ? bwd_flags : fwd_flags;
     T* part = static_cast<T*>(h->d_bwpart);
     if (nrhs == 1)
-      launch_large_fused<T>(F, stasks + tl.off, tl.count, backward, ticket, ssync, h->d_epoch.p, panel, dinv, X, V,
+      launch_large_fused<T>(F, stasks + tl.off, tl.count, backward, ticket, ssync, h->d_epoch.p, panel, dinv, X, V, h->d_G.p,
                             h->d_exch, st, h->d_info.p + 2, part, bwd_flags + nflags);
     else
-      launch_large_multi<T>(F, stasks + tl.off, tl.count, backward, ticket, flags, ssync, panel, dinv, X, ldx, V, nrhs, st,
-                            h->d_info.p + 2, part, bwd_flags + nflags);
+      launch_large_multi<T>(F, stasks + tl.off, tl.count, backward, ticket, flags, ssync, panel, dinv, X, ldx, V, h->d_G.p, nrhs,
+                            st, h->d_info.p + 2, part, bwd_flags + nflags);
     ++n;
   };
   // algorithmic work of one sweep over a list: read the panel once, 2 flops per entry per RHS

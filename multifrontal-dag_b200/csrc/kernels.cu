@@ -245,7 +245,8 @@ __global__ void __launch_bounds__(256) k_gather_children(DevFronts F, const int3
   const int nc = F.nc[f], nr = F.nr[f], nf = nc + nr;
   T* P = panel + F.panel_off[f];
   T* Uf = upool + F.u_off[f];
-  const int cb = F.child_ptr[f], ce = F.child_ptr[f + 1];
+  const int cb = F.child_ptr[f], nch = F.child_ptr[f + 1] - cb;
+  const int ce = nch > kManyChildren ? cb : cb + nch;    // many: zero only
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int pairs = (nf + 1) / 2;
   for (int q = blockIdx.x * nw + warp; q < pairs; q += gridDim.x * nw) {
@@ -303,7 +304,8 @@ template <typename T>
 __global__ void k_assemble_large(DevFronts F, const int32_t* list, const double* __restrict__ a, T* panel,
                                  const T* __restrict__ upool) {
   const int f = list[blockIdx.y];
-  const int nf = F.nc[f] + F.nr[f], cb = F.child_ptr[f], ce = F.child_ptr[f + 1];
+  const int nf = F.nc[f] + F.nr[f], cb = F.child_ptr[f], nch = F.child_ptr[f + 1] - cb;
+  const int ce = nch > kManyChildren ? cb : cb + nch;    // many: added afterwards (k_add_children)
   T* P = panel + F.panel_off[f];
   for (int k = F.a_beg[f] + blockIdx.x * blockDim.x + threadIdx.x; k < F.a_beg[f + 1]; k += gridDim.x * blockDim.x) {
     const int pos = F.a_pos[k], j = pos / nf, i = pos - j * nf;
@@ -316,6 +318,48 @@ __global__ void k_assemble_large(DevFronts F, const int32_t* list, const double*
     }
     P[pos] = v;
   }
+}
+
+// The children of a front with many of them, added in child order to what A's
+// entries and zeros left there: the same sums in the same order as above.  A warp
+// takes the columns j and nf - 1 - j; its lanes look column j up in 32 children at
+// a time and those that have it are added one after another, lanes over their rows.
+// Both sides are at kManyChildren.
+template <typename T>
+__global__ void __launch_bounds__(256) k_add_children(DevFronts F, const int32_t* list, T* panel, T* upool) {
+  const int f = list[blockIdx.y];
+  const int nc = F.nc[f], nr = F.nr[f], nf = nc + nr;
+  T* P = panel + F.panel_off[f];
+  T* Uf = upool + F.u_off[f];
+  const int cb = F.child_ptr[f], ce = F.child_ptr[f + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int pairs = (nf + 1) / 2;
+  for (int q = blockIdx.x * nw + warp; q < pairs; q += gridDim.x * nw)
+#pragma unroll 1
+    for (int hh = 0; hh < 2; ++hh) {
+      const int j = hh ? nf - 1 - q : q;
+      if (hh && j == q) break;
+      T* dst = j < nc ? P + (size_t)j * nf : Uf + (size_t)(j - nc) * nr - nc;   // entry (i, j) at dst[i]
+      for (int t0 = cb; t0 < ce; t0 += 32) {
+        int cnr = 0, clo = 0, cj = 0;
+        long long cuo = 0;
+        bool has = false;
+        if (t0 + lane < ce) {
+          const ChildRec c = F.crec[t0 + lane];
+          cnr = c.nr; clo = c.lrow_off; cuo = c.u_off;
+          cj = lower_bound_dev(F.local + clo, cnr, j + 1);
+          has = cj < cnr && F.local[clo + cj] == j + 1;
+        }
+        for (unsigned m = __ballot_sync(0xffffffffu, has); m; m &= m - 1) {
+          const int s = __ffs(m) - 1;
+          const int n = __shfl_sync(0xffffffffu, cnr, s), c = __shfl_sync(0xffffffffu, cj, s);
+          const int32_t* loc = F.local + __shfl_sync(0xffffffffu, clo, s);
+          const T* col = upool + __shfl_sync(0xffffffffu, cuo, s) + (size_t)c * n;
+          for (int r = c + lane; r < n; r += 32) dst[loc[r] - 1] += col[r];
+          __syncwarp();                                  // the next child's rows may be other lanes'
+        }
+      }
+    }
 }
 
 // Inverted diagonal block of panel step `step` of front f (k_invert writes them).
@@ -761,6 +805,73 @@ __device__ void fwd_diag_cta(const DevFronts& F, int f, int step, int slot, cons
       }
     }
   }
+}
+
+// The vectors of fronts with many children before their panel steps (sweep_sync.cuh
+// has the other fronts' form): own X entries plus the children's update vectors in
+// child order, in FP64.  A warp takes 32 rows of R right-hand sides in shared
+// memory; its lanes look for rows in their range in 32 children at a time, and the
+// entries of C of those that have some, at most one per lane and child, are in
+// flight together.  Front of 300 columns, 20,000 children of five rows: one
+// right-hand side 7.0 -> 2.2 ms a solve (each row looked up in every child before),
+// five 5.6 -> 3.3 (one child after another: 11.6).
+constexpr int kGatherRows = 32, kGatherWarps = 4;
+template <typename T, int R, int C>
+__global__ void __launch_bounds__(32 * kGatherWarps) k_gather_many(DevFronts F, const int32_t* list, const T* X, int64_t ldx,
+                                                                   const T* V, double* G, int nrhs) {
+  __shared__ double acc[kGatherWarps][R][kGatherRows];
+  const int f = list[blockIdx.y];
+  const int nc = F.nc[f], nf = nc + F.nr[f], first = F.first[f];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i0 = (blockIdx.x * kGatherWarps + warp) * kGatherRows, i1 = min(nf, i0 + kGatherRows);
+  const int r0 = blockIdx.z * R, rn = min(R, nrhs - r0);
+  if (i0 >= nf) return;
+  double (*a)[kGatherRows] = acc[warp];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    a[r][lane] = r < rn && i0 + lane < nc ? (double)X[first + i0 + lane + (int64_t)(r0 + r) * ldx] : 0.0;
+  __syncwarp();
+  const int cb = F.child_ptr[f], ce = F.child_ptr[f + 1];
+  for (int t0 = cb; t0 < ce; t0 += 32) {
+    int cnr = 0, cnc = 0, clo = 0, at = 0;
+    long long cvo = 0;
+    bool has = false;
+    if (t0 + lane < ce) {
+      const ChildRec c = F.crec[t0 + lane];
+      cnr = c.nr; cnc = c.nc; clo = c.lrow_off; cvo = c.v_off;
+      at = lower_bound_dev(F.local + clo, cnr, i0 + 1);
+      has = at < cnr && F.local[clo + at] <= i1;
+    }
+    unsigned m = __ballot_sync(0xffffffffu, has);
+    while (m) {
+      int i[C];
+      T v[C][R];
+#pragma unroll
+      for (int u = 0; u < C; ++u) {
+        const int s = m ? __ffs(m) - 1 : 0;
+        const int n = __shfl_sync(0xffffffffu, cnr, s), cols = __shfl_sync(0xffffffffu, cnc, s);
+        const int e = __shfl_sync(0xffffffffu, at, s) + lane;
+        const int32_t* loc = F.local + __shfl_sync(0xffffffffu, clo, s);
+        const T* vc = V + __shfl_sync(0xffffffffu, cvo, s) * nrhs + (int64_t)r0 * (cols + n) + cols;
+        i[u] = m && e < n ? loc[e] - 1 : i1;
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[u][r] = i[u] < i1 && r < rn ? vc[(int64_t)r * (cols + n) + e] : T(0);
+        m &= m - 1;                                      // stays 0
+      }
+#pragma unroll
+      for (int u = 0; u < C; ++u) {
+        if (i[u] < i1)
+#pragma unroll
+          for (int r = 0; r < R; ++r) a[r][i[u] - i0] += (double)v[u][r];
+        __syncwarp();
+      }
+    }
+  }
+  double* g = G + F.g_off[f] * nrhs + (int64_t)r0 * nf + i0 + lane;
+  if (i0 + lane < nf)
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (r < rn) g[(int64_t)r * nf] = a[r][lane];
 }
 
 // gather v (own X entries + the children's update vectors), then y_0
@@ -1243,6 +1354,23 @@ void launch_assemble_large(const DevFronts& F, const int32_t* list, int count, i
   dim3 grid(clamp_grid(ceil_div(max_entries, 256), 256), count);
   k_assemble_large<T><<<grid, 256, 0, st>>>(F, list, a, panel, upool);
 }
+template <typename T>
+void launch_add_children(const DevFronts& F, const int32_t* many, int count, int max_nf, T* panel, T* upool,
+                         cudaStream_t st) {
+  if (count <= 0) return;
+  const int gx = std::max(1, std::min(ceil_div((max_nf + 1) / 2, 8), 1024));
+  k_add_children<T><<<dim3(gx, count), 256, 0, st>>>(F, many, panel, upool);
+}
+template <typename T>
+void launch_gather_many(const DevFronts& F, const int32_t* many, int count, int max_nf, const T* X, int64_t ldx, const T* V,
+                        double* G, int nrhs, cudaStream_t st) {
+  if (count <= 0) return;
+  const int gx = ceil_div(max_nf, kGatherWarps * kGatherRows);
+  if (nrhs == 1)
+    k_gather_many<T, 1, 8><<<dim3(gx, count), 32 * kGatherWarps, 0, st>>>(F, many, X, ldx, V, G, nrhs);
+  else
+    k_gather_many<T, 8, 4><<<dim3(gx, count, ceil_div(nrhs, 8)), 32 * kGatherWarps, 0, st>>>(F, many, X, ldx, V, G, nrhs);
+}
 int update_grid(int T, int tw, UpdBand band) {
   const int c1 = kFactB / tw, jlo = band.blo * c1;
   if (T <= 0 || jlo >= T) return 0;
@@ -1439,6 +1567,9 @@ void launch_remap_int(const int32_t* map, int32_t* a, int64_t n, cudaStream_t st
   template void launch_build_large<T>(const DevFronts&, const int32_t*, int, int, T*, T*, cudaStream_t);            \
   template void launch_assemble_large<T>(const DevFronts&, const int32_t*, int, int, const double*, T*, const T*,   \
                                          cudaStream_t);                                                            \
+  template void launch_add_children<T>(const DevFronts&, const int32_t*, int, int, T*, T*, cudaStream_t);           \
+  template void launch_gather_many<T>(const DevFronts&, const int32_t*, int, int, const T*, int64_t, const T*,      \
+                                      double*, int, cudaStream_t);                                                 \
   template int launch_update<T>(const DevFronts&, const int32_t*, int, int, int, int, T*, T*, int, cudaStream_t,    \
                                  UpdBand, int, bool);                                                              \
   template void launch_fwd_large<T>(const DevFronts&, const int32_t*, int, int, int, const T*, const T*, T*,       \

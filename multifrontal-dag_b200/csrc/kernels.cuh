@@ -130,7 +130,8 @@ template <typename T>
 void launch_small_fronts(const DevFronts& F, const FrontRec* rec, int count, int nf_max, const double* a, T* panel,
                          T* upool, int32_t* info, cudaStream_t st);
 // A level's large fronts before their panel steps: build writes every lower entry as the sum of
-// the children's (max_nf: the largest front), assemble then sets A's entries on top.
+// the children's (max_nf: the largest front), assemble then sets A's entries on top.  Fronts of
+// more than kManyChildren are zeroed, given A's entries, and add their children after that.
 void launch_inverse_index(const DevFronts& F, const int32_t* kids, int count, int32_t* inv, cudaStream_t st);
 template <typename T>
 void launch_build_large(const DevFronts& F, const int32_t* list, int count, int max_nf, T* panel, T* upool,
@@ -138,6 +139,9 @@ void launch_build_large(const DevFronts& F, const int32_t* list, int count, int 
 template <typename T>
 void launch_assemble_large(const DevFronts& F, const int32_t* list, int count, int max_entries, const double* a,
                            T* panel, const T* upool, cudaStream_t st);
+template <typename T>
+void launch_add_children(const DevFronts& F, const int32_t* many, int count, int max_nf, T* panel, T* upool,
+                         cudaStream_t st);
 // Panel step s of the blocked large-front factorization (columns s*kFactB ..), panel.cu:
 //   potrf  : one CTA per front; L11 into the panel and, in packed 8 x 8 blocks with the diagonal
 //            ones inverted, into list slot i's kPackedPanelElems doubles of `packed`
@@ -229,6 +233,11 @@ template <typename T>
 void launch_bwd_small(const DevFronts& F, const FrontRec* rec, int count, int nf_max, int panel_elems, const T* panel,
                       T* X, int64_t ldx, int nrhs, cudaStream_t st);
 // Large fronts: dinv holds the inverted 128 x 128 diagonal blocks the factorization kept (DevFronts::d_off).
+// Fronts of more than kManyChildren (max_nf: the largest): x plus the children's update vectors, in
+// FP64, for every right-hand side, into G (F.g_off; nrhs columns of nf) before their sweep's tasks.
+template <typename T>
+void launch_gather_many(const DevFronts& F, const int32_t* many, int count, int max_nf, const T* X, int64_t ldx, const T* V,
+                        double* G, int nrhs, cudaStream_t st);
 // One launch per panel step (the fallback of launch_large_fused / launch_large_multi).
 template <typename T>
 void launch_fwd_large(const DevFronts& F, const int32_t* list, int count, int max_nc, int max_nf, const T* panel,
@@ -253,14 +262,15 @@ cudaError_t prepare_solve_single();
 void launch_solve_begin(int32_t* sync, int64_t n, int32_t* epoch, cudaStream_t st);
 template <typename T>
 void launch_large_fused(const DevFronts& F, const int4* tasks, int ntask, bool backward, int32_t* ticket,
-                        int32_t* expired, const int32_t* epoch, const T* panel, const T* dinv, T* X, T* V, void* exch,
-                        cudaStream_t st, const int32_t* test_req, T* part = nullptr, int32_t* counters = nullptr);
+                        int32_t* expired, const int32_t* epoch, const T* panel, const T* dinv, T* X, T* V, const double* G,
+                        void* exch, cudaStream_t st, const int32_t* test_req, T* part = nullptr,
+                        int32_t* counters = nullptr);
 // The same sweep for several right-hand sides (solve_multi.cu), each task split into
 // multi_tiles(nrhs) tiles: flags and counters hold as many entries per front and panel
 // step, part multi_part(nrhs) times the single-RHS size.
 template <typename T>
 void launch_large_multi(const DevFronts& F, const int4* tasks, int ntask, bool backward, int32_t* ticket, int32_t* flags,
-                        int32_t* expired, const T* panel, const T* dinv, T* X, int64_t ldx, T* V, int nrhs,
+                        int32_t* expired, const T* panel, const T* dinv, T* X, int64_t ldx, T* V, const double* G, int nrhs,
                         cudaStream_t st, const int32_t* test_req, T* part = nullptr, int32_t* counters = nullptr);
 // pdl: the step kernels go out with programmatic dependent launch
 // (each waits for its predecessor before reading the sweep's vectors)

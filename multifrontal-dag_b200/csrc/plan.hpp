@@ -30,6 +30,14 @@ struct alignas(16) ChildRec {
   int64_t inv_off, pad2;
 };
 
+// A large front of more children than this adds them from the children's side (k_add_children,
+// k_gather_many).  The other form looks every row of the front up in every child: it moves least
+// where each child covers much of the front, the two or three children of a nested dissection, and
+// costs the front's rows times its children where there are many.  Factorization of a front of 2,000
+// columns, the other form / this one: 33 children of 5 rows 1.21 / 0.91 ms, of 1,000 rows 1.76 /
+// 1.41, 200 of 5 rows 2.20 / 0.91, 20,000 of 5 rows 207 / 2.0, 100,000 1,092 / 6.5.
+constexpr int kManyChildren = 32;
+
 // Pointers into the device copies of the per-front tables (all 0-based).
 struct DevFronts {
   const int32_t* nc;          // supernode columns
@@ -44,8 +52,10 @@ struct DevFronts {
   const int32_t* lrow_off;    // offset of f's L rows in lrow / local
   const int32_t* lrow;        // L rows, global permuted 0-based
   const int32_t* local;       // reference local_index values (1-based positions in the parent front)
-  const int32_t* inv;         // children of large fronts: the child's row at every position of the parent, or -1
+  const int32_t* inv;         // children of large fronts of at most kManyChildren: the child's row at every position
+                              // of the parent, or -1
   const int64_t* inv_off;     // offset of a child's part of inv
+  const int64_t* g_off;       // large fronts of more: offset of the front's gathered vector (solves)
   const int32_t* a_beg;       // entries of A assembled into f: [a_beg[f], a_beg[f+1])
   const int32_t* a_src;       // per A entry: index into the caller's value array
   const int32_t* a_pos;       // per A entry: row + col*nf inside the front
@@ -58,7 +68,7 @@ struct DevFronts {
 
 struct HostFront {
   int32_t nc, nr, first, parent, level, sys, node;
-  int64_t panel_off, u_off, v_off, s_off, d_off, q_off;
+  int64_t panel_off, u_off, v_off, s_off, d_off, q_off, g_off;
 };
 
 struct LaunchList {          // a list of front ids in the device list pool
@@ -72,6 +82,8 @@ struct LevelPlan {
   std::vector<LaunchList> small;     // fused one-warp or one-CTA fronts, one list per size bin
   std::vector<LaunchList> small_solve;   // the same for the solves: bins up to 32 rows in one list
   LaunchList large;                  // blocked fronts (sorted by nc descending)
+  LaunchList many;                   // those of more than kManyChildren children
+  int32_t many_max_nf = 0;
   std::vector<LaunchList> steps;     // per panel step: prefix of `large`; param = TRSM row blocks,
                                      // param2 = 128-tiles, param3 = 64-tiles of the trailing triangle
   // per panel step: how many fronts of the step's list (in order) need 4, 3, 2, 1

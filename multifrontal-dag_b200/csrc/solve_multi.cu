@@ -114,8 +114,19 @@ __device__ __forceinline__ void zero(double2 (&v)[2][NB]) {
 
 // gather_row (sweep_sync.cuh) for right-hand sides rc + 8 n and rc + 8 n + 1, n < NB, below re; row i < 0: zeros
 template <int NB, typename T>
-__device__ __forceinline__ void gather_rows(double2 (&v)[NB], const DevFronts& F, int f, int i, int nc, const T* Xf,
-                                            int64_t ldx, const T* V, int nrhs, int rc, int re) {
+__device__ __forceinline__ void gather_rows(double2 (&v)[NB], const DevFronts& F, int f, int i, int nf, int nc, const T* Xf,
+                                            int64_t ldx, const T* V, const double* G, int nrhs, int rc, int re) {
+  const int cb = F.child_ptr[f], ce = F.child_ptr[f + 1];
+  if (ce - cb > kManyChildren) {
+    const double* g = G + F.g_off[f] * nrhs + i;
+#pragma unroll
+    for (int n = 0; n < NB; ++n) {
+      const int r = rc + 8 * n;
+      v[n].x = i >= 0 && r < re ? g[(int64_t)r * nf] : 0.0;
+      v[n].y = i >= 0 && r + 1 < re ? g[(int64_t)(r + 1) * nf] : 0.0;
+    }
+    return;
+  }
 #pragma unroll
   for (int n = 0; n < NB; ++n) {
     const int r = rc + 8 * n;
@@ -123,7 +134,7 @@ __device__ __forceinline__ void gather_rows(double2 (&v)[NB], const DevFronts& F
     v[n].y = i >= 0 && i < nc && r + 1 < re ? (double)Xf[i + (int64_t)(r + 1) * ldx] : 0.0;
   }
   if (i < 0) return;
-  for (int t = F.child_ptr[f], ce = F.child_ptr[f + 1]; t < ce; ++t) {
+  for (int t = cb; t < ce; ++t) {
     const ChildRec c = F.crec[t];
     const int ci = F.inv[c.inv_off + i];
     if (ci < 0) continue;
@@ -144,7 +155,7 @@ template <typename T, int NB>
 __global__ void __launch_bounds__(256, 2)
     k_fwd_multi(DevFronts F, const int4* __restrict__ tasks, int ntask, int tiles, int stride, int32_t* ticket, int32_t* flags,
                 int32_t* expired, const T* __restrict__ panel, const T* __restrict__ dinv, T* X, int64_t ldx, T* V,
-                int nrhs, const int32_t* test_req) {
+                const double* __restrict__ G, int nrhs, const int32_t* test_req) {
   __shared__ int sh_t, sh_ok;
   __shared__ __align__(16) double Y[NB * 1024];
   if (threadIdx.x == 0) sh_t = atomicAdd(ticket, 1);
@@ -172,7 +183,7 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
   for (int m = 0; m < 2; ++m) {
     const int r = r0 + ri + 8 * m;
-    gather_rows<NB>(v[m], F, f, r < r1 ? r : -1, nc, X + first, ldx, V, nrhs, c0r + q2, c0r + cols);
+    gather_rows<NB>(v[m], F, f, r < r1 ? r : -1, nf, nc, X + first, ldx, V, G, nrhs, c0r + q2, c0r + cols);
   }
   T a[2][kHalf][2];
   for (int s = 0; s < nsteps; ++s) {
@@ -384,7 +395,7 @@ __global__ void __launch_bounds__(256, 2)
 
 template <typename T>
 void launch_large_multi(const DevFronts& F, const int4* tasks, int ntask, bool backward, int32_t* ticket, int32_t* flags,
-                        int32_t* expired, const T* panel, const T* dinv, T* X, int64_t ldx, T* V, int nrhs,
+                        int32_t* expired, const T* panel, const T* dinv, T* X, int64_t ldx, T* V, const double* G, int nrhs,
                         cudaStream_t st, const int32_t* test_req, T* part, int32_t* counters) {
   if (ntask <= 0) return;
   const int stride = multi_tiles(nrhs);
@@ -395,7 +406,7 @@ void launch_large_multi(const DevFronts& F, const int4* tasks, int ntask, bool b
                                          nrhs, part, counters, test_req);
     else
       fwd<<<ntask * tiles, 256, 0, st>>>(F, tasks, ntask, tiles, stride, ticket, flags, expired, panel, dinv, X, ldx, V,
-                                         nrhs, test_req);
+                                         G, nrhs, test_req);
   };
   // Sixteen columns per task where the level has more tasks than the chip holds: there the tasks'
   // number counts.  Where all run at once the chain of steps counts, and eight columns have half
@@ -408,8 +419,8 @@ void launch_large_multi(const DevFronts& F, const int4* tasks, int ntask, bool b
 
 #define MFD_INSTANTIATE_MULTI(T)                                                                                     \
   template void launch_large_multi<T>(const DevFronts&, const int4*, int, bool, int32_t*, int32_t*, int32_t*,        \
-                                      const T*, const T*, T*, int64_t, T*, int, cudaStream_t, const int32_t*, T*,    \
-                                      int32_t*);
+                                      const T*, const T*, T*, int64_t, T*, const double*, int, cudaStream_t,         \
+                                      const int32_t*, T*, int32_t*);
 MFD_INSTANTIATE_MULTI(double)
 MFD_INSTANTIATE_MULTI(float)
 

@@ -109,7 +109,8 @@ template <typename T, int N>
 __global__ void __launch_bounds__(256, N == 64 && sizeof(T) == 8 ? 1 : 2) k_fwd_single(DevFronts F, const int4* __restrict__ tasks, int ntask,
                                                     int32_t* ticket, int32_t* expired, const int32_t* epoch,
                                                     const T* __restrict__ panel, const T* __restrict__ dinv, T* X, T* V,
-                                                    typename Exchange<T>::Word* E, const int32_t* test_req) {
+                                                    const double* __restrict__ G, typename Exchange<T>::Word* E,
+                                                    const int32_t* test_req) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* Ls = reinterpret_cast<T*>(smem_raw);
   __shared__ int sh_t;
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(256, N == 64 && sizeof(T) == 8 ? 1 : 2) k_fwd_
   const bool valid = i < r1;
   if (code >= 0) stage_inverse(Ls, dinv + F.d_off[f] + (size_t)code * kSolveB * kSolveB, r1 - r0);
   T v = T(0);
-  if (h == 0 && valid) v = gather_row(F, f, i, nc, X + first, V, 1, 0);
+  if (h == 0 && valid) v = gather_row(F, f, i, nf, nc, X + first, V, G, 1, 0);
   T acc[4] = {T(0), T(0), T(0), T(0)};
   for (int s = 0; s < nsteps; ++s) {
     const int c0 = s * kSolveB, w = min(kSolveB, nc - c0);
@@ -358,8 +359,8 @@ void launch_solve_begin(int32_t* sync, int64_t n, int32_t* epoch, cudaStream_t s
 
 template <typename T>
 void launch_large_fused(const DevFronts& F, const int4* tasks, int ntask, bool backward, int32_t* ticket,
-                        int32_t* expired, const int32_t* epoch, const T* panel, const T* dinv, T* X, T* V, void* exch,
-                        cudaStream_t st, const int32_t* test_req, T* part, int32_t* counters) {
+                        int32_t* expired, const int32_t* epoch, const T* panel, const T* dinv, T* X, T* V, const double* G,
+                        void* exch, cudaStream_t st, const int32_t* test_req, T* part, int32_t* counters) {
   if (ntask <= 0) return;
   auto* E = static_cast<typename Exchange<T>::Word*>(exch);
   const size_t sm = kFoldElems * sizeof(T);
@@ -367,7 +368,7 @@ void launch_large_fused(const DevFronts& F, const int4* tasks, int ntask, bool b
     k<<<ntask, 256, sm, st>>>(F, tasks, ntask, ticket, expired, epoch, panel, dinv, X, E, part, counters, test_req);
   };
   auto fwd = [&](auto k) {
-    k<<<ntask, 256, sm, st>>>(F, tasks, ntask, ticket, expired, epoch, panel, dinv, X, V, E, test_req);
+    k<<<ntask, 256, sm, st>>>(F, tasks, ntask, ticket, expired, epoch, panel, dinv, X, V, G, E, test_req);
   };
   if constexpr (sizeof(T) == 8) {
     if (ntask > 148) {
@@ -382,7 +383,8 @@ void launch_large_fused(const DevFronts& F, const int4* tasks, int ntask, bool b
 
 #define MFD_INSTANTIATE_SINGLE(T)                                                                                  \
   template void launch_large_fused<T>(const DevFronts&, const int4*, int, bool, int32_t*, int32_t*, const int32_t*, \
-                                      const T*, const T*, T*, T*, void*, cudaStream_t, const int32_t*, T*, int32_t*);
+                                      const T*, const T*, T*, T*, const double*, void*, cudaStream_t, const int32_t*,  \
+                                      T*, int32_t*);
 MFD_INSTANTIATE_SINGLE(double)
 MFD_INSTANTIATE_SINGLE(float)
 

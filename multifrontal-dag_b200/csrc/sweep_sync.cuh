@@ -49,13 +49,15 @@ __device__ __forceinline__ bool cta_wait_flag(const int32_t* flag, int32_t* expi
 
 // Entry i of front f's vector before its panel steps: its own right-hand side
 // (Xf: the front's first column) plus the children's update vectors in child
-// order (V: nrhs columns per front, column r), two children's loads in flight.
+// order (V: nrhs columns per front, column r), two children's loads in flight;
+// with many children the sum is in G already (launch_gather_many).
 template <typename T>
-__device__ __forceinline__ T gather_row(const DevFronts& F, int f, int i, int nc, const T* Xf, const T* V, int nrhs,
-                                        int r) {
+__device__ __forceinline__ T gather_row(const DevFronts& F, int f, int i, int nf, int nc, const T* Xf, const T* V,
+                                        const double* G, int nrhs, int r) {
+  const int cb = F.child_ptr[f], ce = F.child_ptr[f + 1];
+  if (ce - cb > kManyChildren) return (T)G[F.g_off[f] * nrhs + (int64_t)r * nf + i];
   T v = i < nc ? Xf[i] : T(0);
-  const int ce = F.child_ptr[f + 1];
-  for (int t = F.child_ptr[f]; t < ce; t += 2) {
+  for (int t = cb; t < ce; t += 2) {
     T x[2];
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
