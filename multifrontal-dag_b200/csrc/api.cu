@@ -674,8 +674,6 @@ int upload_plan(mfd_handle* h) {
   // [3] FP32 diagonal sub-blocks redone in FP64 (small pivot)
   CK(h->d_info.alloc(4));
   CK(cudaMemsetAsync(h->d_info.p, 0, 4 * sizeof(int32_t), h->st));
-  CK(h->d_cnt.alloc(std::max(1, h->max_large_count)));   // backward-solve tickets, one per list slot
-  CK(cudaMemsetAsync(h->d_cnt.p, 0, sizeof(int32_t) * std::max(1, h->max_large_count), h->st));
   DevFronts& F = h->F;
   F.nc = h->d_nc.p; F.nr = h->d_nr.p; F.first = h->d_first.p; F.parent = h->d_parent.p;
   F.child_ptr = h->d_child_ptr.p; F.child = h->d_child.p; F.panel_off = h->d_panel_off.p; F.u_off = h->d_u_off.p;
@@ -921,6 +919,10 @@ int ensure_rhs(mfd_handle* h, int nrhs) {
   CK(cudaMalloc(&h->d_V, (size_t)std::max<int64_t>(h->v_elems, 1) * nrhs * esz));
   CK(cudaMalloc(&h->d_S, (size_t)std::max<int64_t>(h->s_elems, 1) * nrhs * esz));
   if (h->g_elems > 0) CK(h->d_G.alloc((size_t)h->g_elems * nrhs));
+  if (h->max_large_count > 0 && !solve_fused(h, nrhs)) {   // tickets of the sweeps of one launch per step
+    CK(h->d_cnt.alloc((size_t)h->max_large_count * ((nrhs + kRhsG - 1) / kRhsG)));
+    CK(cudaMemsetAsync(h->d_cnt.p, 0, sizeof(int32_t) * h->d_cnt.n, h->st));
+  }
   CK(h->d_b.alloc((size_t)h->n_total * nrhs));
   CK(h->d_xp.alloc((size_t)h->n_total * nrhs));
   CK(h->d_bp.alloc((size_t)h->n_total * nrhs));

@@ -753,8 +753,9 @@ __global__ void __launch_bounds__(256) k_update_simt(DevFronts F, const int32_t*
 //   backward: t_s = v_s - L_rest,s^T x_rest, partial sums per 64-row chunk;
 //             the last CTA sums them in chunk order (deterministic) and forms
 //             x_s = Li^T t_s (k_bwd_large_step)
-// The diagonal solves write the front's own entries of X directly.
-constexpr int kRhsG = 8;      // right-hand sides per pass
+// The diagonal solves write the front's own entries of X directly.  Grid z takes kRhsG right-hand
+// sides, with a ticket of its own: one group after another in the same CTAs, 64 right-hand sides on
+// the 64^3 Laplacian took 91.9 ms (FP64) and 130 ms (FP32 + refinement), side by side 38 and 53.
 constexpr int kFwdRows = 32;  // rows per CTA of k_fwd_large_rest
 
 // y_s = Li v_s by one CTA of 256 threads: thread (row i, half h) sums k in
@@ -764,15 +765,15 @@ constexpr int kFwdRows = 32;  // rows per CTA of k_fwd_large_rest
 // CTAs wrote it.
 template <typename T>
 __device__ void fwd_diag_cta(const DevFronts& F, int f, int step, int slot, const T* __restrict__ dinv, T* X,
-                             int64_t ldx, T* Vf, int nf, int nrhs, T* vs, T* hs) {
+                             int64_t ldx, T* Vf, int nf, int rb, int re, T* vs, T* hs) {
   const int nc = F.nc[f];
   const int c0 = step * kSolveB;
   const int w = min(kSolveB, nc - c0);
   const T* Li = inv_block(F, dinv, f, step);
   const int first = F.first[f];
   const int tid = threadIdx.x, i = tid & (kSolveB - 1), h = tid >> 7;
-  for (int r0 = 0; r0 < nrhs; r0 += kRhsG) {
-    const int g = min(kRhsG, nrhs - r0);
+  for (int r0 = rb; r0 < re; r0 += kRhsG) {
+    const int g = min(kRhsG, re - r0);
     __syncthreads();
     for (int e = tid; e < kSolveB * kRhsG; e += blockDim.x) {
       const int k = e % kSolveB, r = e / kSolveB;
@@ -884,11 +885,12 @@ __global__ void __launch_bounds__(256) k_fwd_large_gather(DevFronts F, const int
   const int f = list[blockIdx.x];
   const int nc = F.nc[f], nf = nc + F.nr[f], first = F.first[f];
   T* Vbase = V + F.v_off[f] * nrhs;
+  const int rb = blockIdx.z * kRhsG, re = min(nrhs, rb + kRhsG);
   // loads batched kGU per thread (in flight together); each entry takes one
   // add per child, children in order
   constexpr int kGU = 4;
   const int nt = blockDim.x;
-  for (int r = 0; r < nrhs; ++r) {
+  for (int r = rb; r < re; ++r) {
     T* Vf = Vbase + (int64_t)r * nf;
     for (int i0 = threadIdx.x; i0 < nf; i0 += kGU * nt) {
       T xv[kGU];
@@ -926,7 +928,7 @@ __global__ void __launch_bounds__(256) k_fwd_large_gather(DevFronts F, const int
     }
   }
   __threadfence_block();
-  fwd_diag_cta(F, f, 0, blockIdx.x, dinv, X, ldx, Vbase, nf, nrhs, vs, hs);
+  fwd_diag_cta(F, f, 0, blockIdx.x, dinv, X, ldx, Vbase, nf, rb, re, vs, hs);
 }
 
 // v_rest -= L_rest,s y_s: 32 rows per CTA (lane = row), warp q takes panel
@@ -962,40 +964,38 @@ __global__ void __launch_bounds__(256) k_fwd_large_rest(DevFronts F, const int32
     const int col = warp * 16 + k;
     lr[k] = (valid && col < w) ? P[i + (size_t)(c0 + col) * nf] : T(0);
   }
-  for (int r0 = 0; r0 < nrhs; r0 += kRhsG) {
-    const int g = min(kRhsG, nrhs - r0);
+  const int r0 = blockIdx.z * kRhsG, g = min(kRhsG, nrhs - r0);
 #pragma unroll
-    for (int u = 0; u < kRhsG; ++u) {
-      T s = T(0);
-      if (u < g) {
-        const T* y = Vf + (int64_t)(r0 + u) * nf + c0 + warp * 16;
+  for (int u = 0; u < kRhsG; ++u) {
+    T s = T(0);
+    if (u < g) {
+      const T* y = Vf + (int64_t)(r0 + u) * nf + c0 + warp * 16;
 #pragma unroll
-        for (int k = 0; k < 16; ++k)
-          if (warp * 16 + k < w) s += lr[k] * y[k];
-      }
-      part[warp][u][lane] = s;
+      for (int k = 0; k < 16; ++k)
+        if (warp * 16 + k < w) s += lr[k] * y[k];
     }
-    __syncthreads();
-    {
-      const int u = threadIdx.x >> 5;
-      if (u < g && valid) {
-        T s = T(0);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) s += part[q][u][lane];
-        Vf[(int64_t)(r0 + u) * nf + i] -= s;
-      }
-    }
-    __syncthreads();
+    part[warp][u][lane] = s;
   }
+  __syncthreads();
+  {
+    const int u = threadIdx.x >> 5;
+    if (u < g && valid) {
+      T s = T(0);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) s += part[q][u][lane];
+      Vf[(int64_t)(r0 + u) * nf + i] -= s;
+    }
+  }
+  int32_t* ticket = cnt + blockIdx.y * gridDim.z + blockIdx.z;
   if (rs0 >= nc) return;                                 // no next step for this front
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&cnt[blockIdx.y], 1) == nchunks - 1;
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1) == nchunks - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
-  fwd_diag_cta(F, f, step + 1, blockIdx.y, dinv, X, ldx, Vf, nf, nrhs, vs, hs);
-  if (threadIdx.x == 0) cnt[blockIdx.y] = 0;
+  fwd_diag_cta(F, f, step + 1, blockIdx.y, dinv, X, ldx, Vf, nf, r0, r0 + g, vs, hs);
+  if (threadIdx.x == 0) *ticket = 0;
 }
 
 template <typename T>
@@ -1005,7 +1005,7 @@ __global__ void k_bwd_large_gather(DevFronts F, const int32_t* list, const T* X,
   const int32_t* lr = F.lrow + F.lrow_off[f];
   constexpr int kGU = 4;                     // loads in flight per thread
   const int nt = blockDim.x;
-  for (int r = 0; r < nrhs; ++r) {
+  for (int r = blockIdx.z * kRhsG; r < min(nrhs, (int)(blockIdx.z + 1) * kRhsG); ++r) {
     T* Vf = V + F.v_off[f] * nrhs + (int64_t)r * nf;
     for (int i0 = threadIdx.x; i0 < nf; i0 += kGU * nt) {
       int gi[kGU];
@@ -1031,7 +1031,7 @@ constexpr int kBwdG = 4;   // right-hand sides per pass of the backward partial 
 // partial sums (64 rows; warp (g, q) takes rows 32g .. 32g+31 against the
 // block's columns 32q .. 32q+31, lane = row, coalesced column reads, 16
 // columns at a time, then a butterfly transpose-reduce leaves column kb +
-// (l mod 16)'s sum in lane l); the last CTA of the front to finish (ticket on cnt[slot])
+// (l mod 16)'s sum in lane l); the last CTA of the front to finish (its group's ticket)
 // sums them in chunk order (deterministic), forms x_s = Li^T t_s, writes V_s
 // and X, and resets the ticket.  A front without rows below the block is
 // finished by CTA 0 alone.  The finish reads Li straight from memory rather
@@ -1060,12 +1060,14 @@ __global__ void __launch_bounds__(256, 3) k_bwd_large_step(DevFronts F, const in
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const T* P = panel + F.panel_off[f];
   T* Vf = V + F.v_off[f] * nrhs;
+  const int rb = blockIdx.z * kRhsG, re = min(nrhs, rb + kRhsG);
+  int32_t* ticket = cnt + blockIdx.y * gridDim.z + blockIdx.z;
   if (nchunks > 0) {
     const int rg = warp & 1, cq = warp >> 1;
     const int i = rbase + rg * 32 + lane;
     const bool valid = i < nf;
-    for (int r0 = 0; r0 < nrhs; r0 += kBwdG) {
-      const int g = min(kBwdG, nrhs - r0);
+    for (int r0 = rb; r0 < re; r0 += kBwdG) {
+      const int g = min(kBwdG, re - r0);
       T xi[kBwdG];
 #pragma unroll
       for (int u = 0; u < kBwdG; ++u) xi[u] = (valid && u < g) ? Vf[(int64_t)(r0 + u) * nf + i] : T(0);
@@ -1104,7 +1106,7 @@ __global__ void __launch_bounds__(256, 3) k_bwd_large_step(DevFronts F, const in
     }
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(&cnt[blockIdx.y], 1) == nchunks - 1;
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1) == nchunks - 1;
     __syncthreads();
     if (!last) return;
     __threadfence();
@@ -1112,7 +1114,7 @@ __global__ void __launch_bounds__(256, 3) k_bwd_large_step(DevFronts F, const in
   // finish: x_s = Li^T (v_s - sum of partials)
   const T* Li = inv_block(F, dinv, f, step);
   const int first = F.first[f];
-  for (int r = 0; r < nrhs; ++r) {
+  for (int r = rb; r < re; ++r) {
     __syncthreads();
     if (threadIdx.x < kSolveB) {
       T s = T(0);
@@ -1148,7 +1150,7 @@ __global__ void __launch_bounds__(256, 3) k_bwd_large_step(DevFronts F, const in
       }
     }
   }
-  if (nchunks > 0 && threadIdx.x == 0) cnt[blockIdx.y] = 0;
+  if (nchunks > 0 && threadIdx.x == 0) *ticket = 0;
 }
 
 // ============================================================================
@@ -1418,11 +1420,12 @@ void launch_fwd_large(const DevFronts& F, const int32_t* list, int count, int ma
                       const T* dinv, T* X, int64_t ldx, T* V, int32_t* cnt, int nrhs, cudaStream_t st,
                       int64_t* launches, bool pdl) {
   if (count <= 0) return;
-  k_fwd_large_gather<T><<<count, 256, 0, st>>>(F, list, dinv, X, ldx, V, nrhs);
+  const int gz = ceil_div(nrhs, kRhsG);
+  k_fwd_large_gather<T><<<dim3(count, 1, gz), 256, 0, st>>>(F, list, dinv, X, ldx, V, nrhs);
   const int steps = ceil_div(max_nc, kSolveB);
   const int chunks = std::max(1, ceil_div(max_nf, kFwdRows));
   for (int s = 0; s < steps; ++s)
-    launch_k(k_fwd_large_rest<T>, dim3(chunks, count), dim3(256), 0, st, pdl, F, list, s, panel, dinv, X, ldx, V, cnt,
+    launch_k(k_fwd_large_rest<T>, dim3(chunks, count, gz), dim3(256), 0, st, pdl, F, list, s, panel, dinv, X, ldx, V, cnt,
              nrhs);
   if (launches) *launches += 1 + steps;
 }
@@ -1431,11 +1434,12 @@ void launch_bwd_large(const DevFronts& F, const int32_t* list, int count, int ma
                       const T* dinv, T* X, int64_t ldx, T* V, T* scratch, int32_t* cnt, int nrhs, cudaStream_t st,
                       int64_t* launches, bool pdl) {
   if (count <= 0) return;
-  k_bwd_large_gather<T><<<count, 256, 0, st>>>(F, list, X, ldx, V, nrhs);
+  const int gz = ceil_div(nrhs, kRhsG);
+  k_bwd_large_gather<T><<<dim3(count, 1, gz), 256, 0, st>>>(F, list, X, ldx, V, nrhs);
   const int steps = ceil_div(max_nc, kSolveB);
   const int chunks = std::max(1, ceil_div(max_nf, kSolveRows));
   for (int s = steps - 1; s >= 0; --s)
-    launch_k(k_bwd_large_step<T>, dim3(chunks, count), dim3(256), 0, st, pdl, F, list, s, panel, dinv, X, ldx, V,
+    launch_k(k_bwd_large_step<T>, dim3(chunks, count, gz), dim3(256), 0, st, pdl, F, list, s, panel, dinv, X, ldx, V,
              scratch, cnt, nrhs);
   if (launches) *launches += 1 + steps;
 }

@@ -238,12 +238,13 @@ void launch_bwd_small(const DevFronts& F, const FrontRec* rec, int count, int nf
 template <typename T>
 void launch_gather_many(const DevFronts& F, const int32_t* many, int count, int max_nf, const T* X, int64_t ldx, const T* V,
                         double* G, int nrhs, cudaStream_t st);
-// One launch per panel step (the fallback of launch_large_fused / launch_large_multi).
+// One launch per panel step (the fallback of launch_large_fused / launch_large_multi).  cnt: a
+// zero-initialised ticket per list slot and kRhsG right-hand sides (left zero again on exit).
+constexpr int kRhsG = 8;
 template <typename T>
 void launch_fwd_large(const DevFronts& F, const int32_t* list, int count, int max_nc, int max_nf, const T* panel,
                       const T* dinv, T* X, int64_t ldx, T* V, int32_t* cnt, int nrhs, cudaStream_t st,
                       int64_t* launches, bool pdl);
-// cnt: one zero-initialised ticket per list slot (left zero again on exit)
 template <typename T>
 void launch_bwd_large(const DevFronts& F, const int32_t* list, int count, int max_nc, int max_nf, const T* panel,
                       const T* dinv, T* X, int64_t ldx, T* V, T* scratch, int32_t* cnt, int nrhs, cudaStream_t st,
