@@ -282,6 +282,11 @@ int mfd_get_profile(mfd_handle *h, int32_t kind, mfd_kernel_profile *out);
  * normally once the request is withdrawn. */
 int mfd_test_expire_waits(mfd_handle *h, int32_t enable);
 
+/* Test of the out-of-memory path: the calling thread's nth device allocation
+ * for a handle from now on is refused as if there were no memory for it (0:
+ * none); returns how many the thread has made since the last call. */
+int64_t mfd_test_fail_alloc(int64_t nth);
+
 int mfd_destroy(mfd_handle *h);
 
 /* ---- dense fronts without allocation ------------------------------------------

@@ -58,7 +58,19 @@ constexpr double kDeferBytes = 64e6;
 // 30^3 elasticity 14.82 / 14.68 / 14.61); below three blocks of rows the operands of a batch's
 // thousands of fronts would take more memory than their panels.
 constexpr int kPackedDpRows = 3 * kFactB;
+// ... and launches whose 128 x 64 pieces reach half of the SMs or more; below, launch_update's smaller
+// ones that read the panel (64^3 Laplacian 29.30 / 29.12 ms with the line at 148 / 64 pieces)
+bool packed_dp_pays(int tiles, int count, UpdBand band) {
+  return (int64_t)2 * update_grid(tiles, kUpdTile, band) * count > kNumSms / 2;
+}
 int64_t align_up(int64_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
+
+// Every device allocation of a handle; the test request (mfd_test_fail_alloc) refuses the thread's t_fail_at-th.
+thread_local int64_t t_allocs = 0, t_fail_at = 0;
+cudaError_t dev_alloc(void** p, size_t bytes) {
+  if (++t_allocs == t_fail_at) return cudaErrorMemoryAllocation;
+  return cudaMalloc(p, bytes);
+}
 
 template <typename T>
 struct DBuf {
@@ -76,7 +88,7 @@ struct DBuf {
   cudaError_t alloc(size_t count) {
     release();
     n = count;
-    return cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T));
+    return dev_alloc(reinterpret_cast<void**>(&p), std::max<size_t>(count, 1) * sizeof(T));
   }
   cudaError_t upload(const std::vector<T>& v, cudaStream_t st) {
     cudaError_t e = alloc(v.size());
@@ -232,7 +244,7 @@ struct mfd_handle {
   std::vector<int> small_bins;
   int64_t panel_elems = 0, upool_elems = 0, v_elems = 0, s_elems = 0, dinv_elems = 0;
   int64_t g_elems = 0;                              // gathered vectors of the level's fronts of many children, largest level
-  int64_t q_elems = 0;                              // packed update operands (2 defer steps) of the level that needs most
+  int64_t q_elems = 0, packed_elems = 0;            // packed update operands / diagonal blocks of the level that needs most
   int32_t max_large_count = 0, max_nf = 0;
   int64_t cost = 0, nonzero = 0;
 
@@ -459,7 +471,7 @@ int build_plan(mfd_handle* h) {
   h->solve_flags = 0;
   h->bw_part_elems = 0;
   h->max_large_count = 0;
-  h->g_elems = 0;
+  h->g_elems = h->packed_elems = 0;
   std::vector<std::vector<int32_t>> lev_fronts(nlev);
   for (int32_t g = 0; g < nfr; ++g) lev_fronts[h->fronts[g].level].push_back(g);
   for (int l = 0; l < nlev; ++l) {
@@ -533,20 +545,6 @@ int build_plan(mfd_handle* h) {
       }
       L.defer = h->opt.reserved[5] > 0 || bytes > kDeferBytes ? h->defer : 1;
     }
-    // packed operands of the trailing update: the level's large fronts side by side, each with the
-    // 128-row blocks of its largest step (step 0); reused level after level
-    L.packed = h->defer <= kPackedDefer && (h->fp32 || L.large_max_nf >= kPackedDpRows);
-    if (L.packed) {
-      int64_t q = 0;
-      for (int32_t g : large) {
-        HostFront& fr = h->fronts[g];
-        const int64_t nrem = (int64_t)fr.nc + fr.nr - std::min(kFactB, fr.nc);
-        fr.q_off = q;
-        q += (nrem + kFactB - 1) / kFactB * (h->fp32 ? kPackedBlockElems : (int64_t)kFactB * kFactB);
-      }
-      L.q_elems = q;
-      h->q_elems = std::max(h->q_elems, 2 * L.defer * q);
-    }
     // panel steps: prefix of the nc-sorted list
     int steps = (max_nc + kFactB - 1) / kFactB;
     for (int s = 0; s < steps; ++s) {
@@ -575,6 +573,32 @@ int build_plan(mfd_handle* h) {
       }
       L.potrf_cls.push_back(cls);
     }
+    // Packed operands of the trailing update: the fronts side by side, each with the 128-row blocks of
+    // its first step.  The TRSM of step s writes to buffer s mod 2 defer (enqueue_factor); only the steps
+    // that some launch reads packed have one, for their fronts (a prefix of the list): on the 64^3
+    // Laplacian 153 MB, where 2 defer buffers for all fronts took 611.
+    const int kind = h->opt.reserved[0];
+    if (h->defer <= kPackedDefer && (h->fp32 ? kind == 0 || kind == 2 : kind == 0 && L.large_max_nf >= kPackedDpRows)) {
+      for (const LaunchList& ll : L.steps) {
+        if (!h->fp32 && !packed_dp_pays(ll.param2, ll.count, UpdBand{})) break;   // nor any later one: they shrink
+        ++L.packed_steps;
+      }
+      std::vector<int64_t> upto(1, 0);
+      for (int32_t g : large) {
+        HostFront& fr = h->fronts[g];
+        const int64_t nrem = (int64_t)fr.nc + fr.nr - std::min(kFactB, fr.nc);
+        fr.q_off = upto.back();
+        upto.push_back(upto.back() + (nrem + kFactB - 1) / kFactB * (h->fp32 ? kPackedBlockElems : (int64_t)kFactB * kFactB));
+      }
+      int64_t q = 0;
+      for (int s = 0; s < std::min(L.packed_steps, 2 * L.defer); ++s) {
+        L.q_base.push_back(q);
+        q += upto[L.steps[s].count];
+      }
+      h->q_elems = std::max(h->q_elems, q);
+    }
+    L.packed_slot = packed_panel_elems(std::min(kFactB, max_nc));
+    h->packed_elems = std::max(h->packed_elems, (int64_t)L.large.count * L.packed_slot);
     // single-RHS solve tasks of the level, in dependency order (see launch_large_fused)
     {
       auto push_task = [&](int32_t g, int32_t code, int32_t flag) {
@@ -621,6 +645,20 @@ int build_plan(mfd_handle* h) {
     }
   }
   return MFD_OK;
+}
+
+// The packed update operands are for speed: where there is no memory for them the updates read the panels
+// (FP64: the same bits; FP32: the same products, summed in another order).
+void drop_packed(mfd_handle* h) {
+  if (h->d_q) cudaFree(h->d_q);
+  h->d_q = nullptr;
+  h->q_elems = 0;
+  for (LevelPlan& L : h->levels) {
+    L.packed_steps = 0;
+    L.q_base.clear();
+  }
+  if (h->g_factor) cudaGraphExecDestroy(h->g_factor);
+  h->g_factor = nullptr;
 }
 
 int upload_plan(mfd_handle* h) {
@@ -861,22 +899,28 @@ int upload_plan(mfd_handle* h) {
   size_t esz = h->fp32 ? sizeof(float) : sizeof(double);
   // 32 elements of slack: the FP32 tensor-core update copies column segments
   // in 16-byte chunks and may read up to 3 elements past the last panel
-  CK(cudaMalloc(&h->d_panel, (std::max<int64_t>(h->panel_elems, 1) + 32) * esz));
-  CK(cudaMalloc(&h->d_upool, std::max<int64_t>(h->upool_elems, 1) * esz));
-  CK(cudaMalloc(&h->d_diag, (size_t)std::max<int64_t>(h->dinv_elems, 1) * esz));
+  CK(dev_alloc(&h->d_panel, (std::max<int64_t>(h->panel_elems, 1) + 32) * esz));
+  CK(dev_alloc(&h->d_upool, std::max<int64_t>(h->upool_elems, 1) * esz));
+  CK(dev_alloc(&h->d_diag, (size_t)std::max<int64_t>(h->dinv_elems, 1) * esz));
   if (h->max_large_count > 0)
-    CK(cudaMalloc(&h->d_packed, (size_t)h->max_large_count * kPackedPanelElems * sizeof(double)));
-  if (h->q_elems > 0) {
-    const size_t bytes = (size_t)h->q_elems * esz;
-    CK(cudaMalloc(&h->d_q, bytes));
-    // rows past a front's last row are never written and only reach discarded outputs; zero keeps them finite
-    CK(cudaMemsetAsync(h->d_q, 0, bytes, h->st));
-  }
+    CK(dev_alloc(reinterpret_cast<void**>(&h->d_packed), (size_t)h->packed_elems * sizeof(double)));
   // the inverted diagonal blocks are written on their lower w x w part only: the rest stays zero
   CK(cudaMemsetAsync(h->d_diag, 0, (size_t)std::max<int64_t>(h->dinv_elems, 1) * esz, h->st));
   h->a_len = h->nnz_total;
   CK(h->d_a.alloc(h->a_len));
   CK(h->d_norms.alloc(8));
+  if (h->q_elems > 0) {
+    const size_t bytes = (size_t)h->q_elems * esz;
+    const cudaError_t e = dev_alloc(&h->d_q, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      drop_packed(h);
+    } else {
+      CK(e);
+      // rows past a front's last row are never written and only reach discarded outputs; zero keeps them finite
+      CK(cudaMemsetAsync(h->d_q, 0, bytes, h->st));
+    }
+  }
   h->setup_s[3] = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   return MFD_OK;
 }
@@ -891,10 +935,7 @@ bool solve_fused(const mfd_handle* h, int nrhs) {
          (int64_t)h->h_stasks.size() / 4 * multi_tiles(nrhs) <= INT32_MAX;
 }
 
-// Storage for nrhs right-hand sides.  Until all of it is there the handle has none (nrhs_cap 0): the
-// solve after a failed one allocates again, as much as it needs itself.
-int ensure_rhs(mfd_handle* h, int nrhs) {
-  if (nrhs <= h->nrhs_cap) return MFD_OK;
+int rhs_storage(mfd_handle* h, int nrhs) {
   h->nrhs_cap = 0;
   for (auto& kv : h->g_solve) cudaGraphExecDestroy(kv.second);
   h->g_solve.clear();
@@ -904,7 +945,7 @@ int ensure_rhs(mfd_handle* h, int nrhs) {
   for (void** p : {&h->d_X, &h->d_V, &h->d_S, &h->d_bwpart})
     if (*p) { cudaFree(*p); *p = nullptr; }
   if (!h->d_epoch.p && solve_fused(h, 1)) {
-    if (!h->d_exch) CK(cudaMalloc(&h->d_exch, (size_t)h->n_total * 2 * esz));
+    if (!h->d_exch) CK(dev_alloc(&h->d_exch, (size_t)h->n_total * 2 * esz));
     CK(cudaMemsetAsync(h->d_exch, 0, (size_t)h->n_total * 2 * esz, h->st));
     CK(h->d_epoch.alloc(1));
     CK(cudaMemsetAsync(h->d_epoch.p, 0, sizeof(int32_t), h->st));
@@ -913,15 +954,15 @@ int ensure_rhs(mfd_handle* h, int nrhs) {
   while (widest > 1 && !solve_fused(h, widest)) --widest;
   CK(h->d_ssync.alloc(solve_sync_ints(h, solve_fused(h, widest) ? widest : 1)));
   CK(cudaMemsetAsync(h->d_ssync.p, 0, sizeof(int32_t) * h->d_ssync.n, h->st));
-  CK(cudaMalloc(&h->d_bwpart, (size_t)std::max<int64_t>(h->bw_part_elems, 1) * esz *
+  CK(dev_alloc(&h->d_bwpart, (size_t)std::max<int64_t>(h->bw_part_elems, 1) * esz *
                                   multi_part(widest)));
-  CK(cudaMalloc(&h->d_X, (size_t)std::max<int64_t>(h->n_total, 1) * nrhs * esz));
-  CK(cudaMalloc(&h->d_V, (size_t)std::max<int64_t>(h->v_elems, 1) * nrhs * esz));
-  CK(cudaMalloc(&h->d_S, (size_t)std::max<int64_t>(h->s_elems, 1) * nrhs * esz));
+  CK(dev_alloc(&h->d_X, (size_t)std::max<int64_t>(h->n_total, 1) * nrhs * esz));
+  CK(dev_alloc(&h->d_V, (size_t)std::max<int64_t>(h->v_elems, 1) * nrhs * esz));
   if (h->g_elems > 0) CK(h->d_G.alloc((size_t)h->g_elems * nrhs));
   if (h->max_large_count > 0 && !solve_fused(h, nrhs)) {   // tickets of the sweeps of one launch per step
     CK(h->d_cnt.alloc((size_t)h->max_large_count * ((nrhs + kRhsG - 1) / kRhsG)));
     CK(cudaMemsetAsync(h->d_cnt.p, 0, sizeof(int32_t) * h->d_cnt.n, h->st));
+    CK(dev_alloc(&h->d_S, (size_t)std::max<int64_t>(h->s_elems, 1) * nrhs * esz));   // and their partial sums
   }
   CK(h->d_b.alloc((size_t)h->n_total * nrhs));
   CK(h->d_xp.alloc((size_t)h->n_total * nrhs));
@@ -936,6 +977,18 @@ int ensure_rhs(mfd_handle* h, int nrhs) {
   }
   h->nrhs_cap = nrhs;
   return MFD_OK;
+}
+
+// Storage for nrhs right-hand sides.  Until all of it is there the handle has none (nrhs_cap 0): the
+// solve after a failed one allocates again, as much as it needs itself.
+int ensure_rhs(mfd_handle* h, int nrhs) {
+  if (nrhs <= h->nrhs_cap) return MFD_OK;
+  int rc = rhs_storage(h, nrhs);
+  if (rc == MFD_E_NOMEM && h->d_q) {
+    drop_packed(h);
+    rc = rhs_storage(h, nrhs);
+  }
+  return rc;
 }
 
 // ---- per-launch profiling ----------------------------------------------------------
@@ -1095,8 +1148,8 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
     // packed operands: the TRSM also writes the step's rows for k_update_tcq / k_update_dp, in 2 D
     // buffers taken in turn: the bulk update of a group reads its own D, and is complete before
     // the TRSM of the group after the next one starts
-    const bool packed = L.packed && (kind == 0 || (sizeof(T) == 4 && kind == 2));
-    auto packed_rows = [&](size_t step) { return static_cast<T*>(h->d_q) + (step % (2 * D)) * L.q_elems; };
+    auto packed = [&](size_t step) { return (int)step < L.packed_steps; };
+    auto packed_rows = [&](size_t step) { return static_cast<T*>(h->d_q) + L.q_base[step % L.q_base.size()]; };
     int pend = -1;                            // step of the latest bulk on st2 not yet fully waited for
     for (size_t s = 0; s < L.steps.size(); ++s) {
       const LaunchList& p = L.steps[s];
@@ -1137,12 +1190,12 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
              [&] {
                // many fronts: one launch per sub-block class (narrow blocks fit many CTAs per SM);
                // a few: one launch (measured: the extra launches on the panel chain cost more)
-               launch_potrf<T>(F, lists + p.off, p.count, (int)s, panel, h->d_packed, h->d_info.p, st, pdl, 0,
-                               h->d_info.p + 3, p.count > kPotrfSplitMin ? L.potrf_cls[s].data() : nullptr);
+               launch_potrf<T>(F, lists + p.off, p.count, (int)s, panel, h->d_packed, L.packed_slot, h->d_info.p, st,
+                               pdl, 0, h->d_info.p + 3, p.count > kPotrfSplitMin ? L.potrf_cls[s].data() : nullptr);
              });
       record(h, st, MFD_K_TRSM, tf, tb, [&] {
         launch_trsm<T>(F, lists + p.off, p.count, (int)s, p.param, std::min(kFactB, L.large.param2 - (int)s * kFactB),
-                       panel, h->d_packed, st, pdl, packed ? packed_rows(s) : nullptr);
+                       panel, h->d_packed, L.packed_slot, st, pdl, packed(s) ? packed_rows(s) : nullptr);
       });
       n += 2;
       auto update = [&](cudaStream_t us, UpdBand band) {
@@ -1151,7 +1204,7 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
         const bool upd_pdl = pdl && us == st;        // right behind the TRSM on the main stream
         record(h, us, MFD_K_UPDATE, fl, by, [&] {
           if constexpr (sizeof(T) == 4) {
-            if (packed) {
+            if (packed(s)) {
               n += launch_update_tcq(F, lists + p.off, p.count, (int)s, p.param2, packed_rows(s),
                                      s > 0 ? packed_rows(s - 1) : nullptr, reinterpret_cast<float*>(panel),
                                      reinterpret_cast<float*>(upool), kind == 0 ? 1 : 0, h->d_info.p + 1, us, band, D,
@@ -1166,12 +1219,10 @@ int64_t enqueue_factor(mfd_handle* h, cudaStream_t st) {
             }
           }
           if constexpr (sizeof(T) == 8) {
-            // where 128 x 64 pieces reach half of the SMs or more; below, launch_update's smaller ones
-            // that read the panel (64^3 Laplacian 29.30 / 29.12 ms with the line at 148 / 64 pieces)
-            if (packed && (int64_t)2 * update_grid(p.param2, kUpdTile, band) * p.count > kNumSms / 2) {
-              n += launch_update_dp(F, lists + p.off, p.count, (int)s, p.param2, static_cast<const double*>(h->d_q),
-                                    L.q_elems, 2 * D, reinterpret_cast<double*>(panel), reinterpret_cast<double*>(upool),
-                                    h->d_info.p + 1, us, band, D, upd_pdl);
+            if (packed(s) && packed_dp_pays(p.param2, p.count, band)) {
+              n += launch_update_dp(F, lists + p.off, p.count, (int)s, p.param2, packed_rows(s),
+                                    s > 0 ? packed_rows(s - 1) : nullptr, reinterpret_cast<double*>(panel),
+                                    reinterpret_cast<double*>(upool), h->d_info.p + 1, us, band, D, upd_pdl);
               return;
             }
           }
@@ -2046,6 +2097,13 @@ int mfd_get_profile(mfd_handle* h, int32_t kind, mfd_kernel_profile* out) {
   if (!h || !out || kind < 0 || kind >= MFD_K_COUNT) return fail(MFD_E_ARG, "bad argument");
   *out = h->prof[kind];
   return MFD_OK;
+}
+
+int64_t mfd_test_fail_alloc(int64_t nth) {
+  const int64_t made = t_allocs;
+  t_allocs = 0;
+  t_fail_at = nth;
+  return made;
 }
 
 int mfd_destroy(mfd_handle* h) {

@@ -22,7 +22,7 @@ constexpr int kSolveRows = 64;       // rows per CTA of the backward large-front
 // tiles of the several-RHS fused large-front sweeps: eight right-hand sides each (a level may take
 // them sixteen at a time, launch_large_multi)
 constexpr int multi_tiles(int nrhs) { return (nrhs + 7) / 8; }
-constexpr int multi_part(int nrhs) { return nrhs == 1 ? 1 : 16 * ((nrhs + 15) / 16); }
+constexpr int multi_part(int nrhs) { return nrhs == 1 ? 1 : nrhs <= 8 ? 8 : 16 * ((nrhs + 15) / 16); }
 
 // Trailing-update work of panel step s of a front (columns c0 = s * kFactB
 // .. c0 + w, base = c0 + w): the lower triangle of the trailing matrix (rows
@@ -144,7 +144,8 @@ void launch_add_children(const DevFronts& F, const int32_t* many, int count, int
                          cudaStream_t st);
 // Panel step s of the blocked large-front factorization (columns s*kFactB ..), panel.cu:
 //   potrf  : one CTA per front; L11 into the panel and, in packed 8 x 8 blocks with the diagonal
-//            ones inverted, into list slot i's kPackedPanelElems doubles of `packed`
+//            ones inverted, into list slot i's slot_elems doubles of `packed` (packed_panel_elems
+//            of the widest block of the list, or more)
 //   trsm   : rows below the diagonal block, X <- X L11^{-T}, from the packed slots
 //   invert : L11^{-1} of the first `steps` panel steps of every front into linv (DevFronts::d_off)
 //   update : trailing lower triangle -= P P^T
@@ -153,17 +154,18 @@ void launch_add_children(const DevFronts& F, const int32_t* many, int count, int
 // cls (may be null: one launch): four counts splitting the list, in order, into fronts whose
 // block needs 4, 3, 2, 1 groups of 32 columns, each class launched with its own (smaller)
 // shared memory and thread count.
-constexpr int kPackedPanelElems = 136 * 64;   // 16 x 17 / 2 blocks
+constexpr int packed_panel_elems(int w) { return (w + 7) / 8 * ((w + 7) / 8 + 1) / 2 * 64; }
+constexpr int kPackedPanelElems = packed_panel_elems(kFactB);
 cudaError_t prepare_panel();
 template <typename T>
-void launch_potrf(const DevFronts& F, const int32_t* list, int count, int step, T* panel, double* packed, int32_t* info,
-                  cudaStream_t st, bool pdl = false, int info_stride = 0, int32_t* fallbacks = nullptr,
+void launch_potrf(const DevFronts& F, const int32_t* list, int count, int step, T* panel, double* packed, int slot_elems,
+                  int32_t* info, cudaStream_t st, bool pdl = false, int info_stride = 0, int32_t* fallbacks = nullptr,
                   const int32_t* cls = nullptr);
 // max_w: the widest diagonal block of the step.  q (may be null): also write the solved rows as packed
 // operands of the update (FP32: TF32 hi / lo, packed_offset; FP64: packed_dp_offset), at q + F.q_off[f].
 template <typename T>
 void launch_trsm(const DevFronts& F, const int32_t* list, int count, int step, int row_blocks, int max_w, T* panel,
-                 const double* packed, cudaStream_t st, bool pdl = false, T* q = nullptr);
+                 const double* packed, int slot_elems, cudaStream_t st, bool pdl = false, T* q = nullptr);
 template <typename T>
 void launch_invert(const DevFronts& F, const int32_t* list, int count, int steps, int max_w, const T* panel, T* linv,
                    cudaStream_t st);
@@ -207,8 +209,7 @@ int launch_update_tcq(const DevFronts& F, const int32_t* list, int count, int st
                       UpdBand band = {}, int defer = 1, bool pdl = false);
 // The same for FP64 (update_dp.cu): 128-row blocks of 128 columns, kFactB * kFactB doubles each, in
 // chunks of 16 columns, [row][16] with column k at position 4 (k % 4) + (k % 16) / 4 and the
-// row's 16-byte pairs XORed by (row & 1).  Step t's rows at q + (t % nbuf) * buf; err[0] is raised
-// if a bounded wait expires.
+// row's 16-byte pairs XORed by (row & 1).  err[0] is raised if a bounded wait expires.
 constexpr int kPackedDefer = 2;       // the deepest deferral the packed-operand updates take
 #ifdef __CUDACC__
 __device__ __forceinline__ int64_t packed_dp_offset(int row, int k) {   // row, k: 0-based within the step
@@ -217,9 +218,9 @@ __device__ __forceinline__ int64_t packed_dp_offset(int row, int k) {   // row, 
 }
 #endif
 cudaError_t prepare_update_dp();
-int launch_update_dp(const DevFronts& F, const int32_t* list, int count, int step, int T128, const double* q, int64_t buf,
-                     int nbuf, double* panel, double* upool, int32_t* err, cudaStream_t st, UpdBand band, int defer,
-                     bool pdl);
+int launch_update_dp(const DevFronts& F, const int32_t* list, int count, int step, int T128, const double* q,
+                     const double* qprev, double* panel, double* upool, int32_t* err, cudaStream_t st, UpdBand band,
+                     int defer, bool pdl);
 // grid size of an update launch over a band of the T x T lower tiles of width tw
 int update_grid(int T, int tw, UpdBand band);
 

@@ -146,9 +146,9 @@ extern "C" __attribute__((visibility("default"))) int mfd_factor_fronts_noalloc(
       tiles = T > tiles ? T : tiles;
     }
     // fronts whose columns are exhausted return at once inside the kernels
-    launch_potrf<double>(F, list, count, s, fronts, scratch, dinfo, st, false, 1);
+    launch_potrf<double>(F, list, count, s, fronts, scratch, kPackedPanelElems, dinfo, st, false, 1);
     launch_trsm<double>(F, list, count, s, rows, maxnc - s * kFactB < kFactB ? maxnc - s * kFactB : kFactB, fronts,
-                        scratch, st);
+                        scratch, kPackedPanelElems, st);
     launch_update<double>(F, list, count, s, tiles, 0, fronts, fronts, 0, st);
   }
   e = cudaGetLastError();

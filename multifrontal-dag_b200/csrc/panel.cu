@@ -71,8 +71,8 @@ __device__ __forceinline__ void load_block(const T* P, size_t ld, int w, int nb,
 // fallbacks (may be null; counted for FP32 storage): 32-column groups with a small pivot.
 template <typename T, int NSB>
 __global__ void __launch_bounds__(potrf_threads<NSB>(), 1) k_potrf(DevFronts F, const int32_t* list, int slot0,
-                                                                   int step, T* panel, double* packed, int32_t* info,
-                                                                   int info_stride, int32_t* fallbacks) {
+                                                                   int step, T* panel, double* packed, int slot_elems,
+                                                                   int32_t* info, int info_stride, int32_t* fallbacks) {
   constexpr int NW = potrf_warps<NSB>(), NT = 32 * NW;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* S = reinterpret_cast<double*>(smem_raw);
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(potrf_threads<NSB>(), 1) k_potrf(DevFronts F, 
       });
   invert_diagonal_blocks(S, scratch + kCholRq, Dinv, nb, nb);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  double2* Q = reinterpret_cast<double2*>(packed + (size_t)slot * kPackedPanelElems);
+  double2* Q = reinterpret_cast<double2*>(packed + (size_t)slot * slot_elems);
   for (int e = tid; e < blk_count(nb) * 32; e += NT) Q[e] = reinterpret_cast<const double2*>(S)[e];
   __syncthreads();        // the diagonal blocks of the slot are rewritten below
   for (int e = tid; e < nb * 32; e += NT)
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(potrf_threads<NSB>(), 1) k_potrf(DevFronts F, 
 constexpr int kTrWarps = 4;
 template <typename T>
 __global__ void __launch_bounds__(32 * kTrWarps, 3) k_trsm(DevFronts F, const int32_t* list, int step, T* panel,
-                                                        const double* packed, T* q) {
+                                                        const double* packed, int slot_elems, T* q) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* L = reinterpret_cast<double*>(smem_raw);
   const int f = list[blockIdx.y];
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(32 * kTrWarps, 3) k_trsm(DevFronts F, const in
   }
   pdl_wait();
   pdl_trigger();
-  const double* Q = packed + (size_t)blockIdx.y * kPackedPanelElems;
+  const double* Q = packed + (size_t)blockIdx.y * slot_elems;
   for (int e = threadIdx.x; e < blk_count(nb) * 32; e += 32 * kTrWarps) {
     const unsigned sa = (unsigned)__cvta_generic_to_shared(L + 2 * e);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(Q + 2 * e));
@@ -265,13 +265,14 @@ cudaError_t prepare_panel() {
 }
 
 template <typename T>
-void launch_potrf(const DevFronts& F, const int32_t* list, int count, int step, T* panel, double* packed, int32_t* info,
-                  cudaStream_t st, bool pdl, int info_stride, int32_t* fallbacks, const int32_t* cls) {
+void launch_potrf(const DevFronts& F, const int32_t* list, int count, int step, T* panel, double* packed, int slot_elems,
+                  int32_t* info, cudaStream_t st, bool pdl, int info_stride, int32_t* fallbacks, const int32_t* cls) {
   if (count <= 0) return;
   int off = 0;
   auto go = [&](auto kern, int nt, size_t smem, int cnt) {
     if (cnt > 0)
-      launch_k(kern, dim3(cnt), dim3(nt), smem, st, pdl, F, list, off, step, panel, packed, info, info_stride, fallbacks);
+      launch_k(kern, dim3(cnt), dim3(nt), smem, st, pdl, F, list, off, step, panel, packed, slot_elems, info,
+               info_stride, fallbacks);
     off += cnt;
   };
   if (cls == nullptr) {                   // one launch, any block width
@@ -287,12 +288,12 @@ void launch_potrf(const DevFronts& F, const int32_t* list, int count, int step, 
 
 template <typename T>
 void launch_trsm(const DevFronts& F, const int32_t* list, int count, int step, int row_blocks, int max_w, T* panel,
-                 const double* packed, cudaStream_t st, bool pdl, T* q) {
+                 const double* packed, int slot_elems, cudaStream_t st, bool pdl, T* q) {
   if (count <= 0 || row_blocks <= 0) return;
   // row_blocks counts 64-row blocks; shared memory for the widest block of the launch
   const size_t smem = (size_t)blk_count((max_w + 7) / 8) * kBlkElems * sizeof(double);
   launch_k(k_trsm<T>, dim3(row_blocks * (kTrRowsH / (8 * kTrWarps)), count), dim3(32 * kTrWarps), smem, st, pdl, F, list,
-           step, panel, packed, q);
+           step, panel, packed, slot_elems, q);
 }
 
 template <typename T>
@@ -304,10 +305,10 @@ void launch_invert(const DevFronts& F, const int32_t* list, int count, int steps
 }
 
 #define MFD_INSTANTIATE_PANEL(T)                                                                                   \
-  template void launch_potrf<T>(const DevFronts&, const int32_t*, int, int, T*, double*, int32_t*, cudaStream_t, bool, \
-                                int, int32_t*, const int32_t*);                                                    \
-  template void launch_trsm<T>(const DevFronts&, const int32_t*, int, int, int, int, T*, const double*, cudaStream_t,  \
-                               bool, T*);                                                                      \
+  template void launch_potrf<T>(const DevFronts&, const int32_t*, int, int, T*, double*, int, int32_t*, cudaStream_t,  \
+                                bool, int, int32_t*, const int32_t*);                                              \
+  template void launch_trsm<T>(const DevFronts&, const int32_t*, int, int, int, int, T*, const double*, int,           \
+                               cudaStream_t, bool, T*);                                                        \
   template void launch_invert<T>(const DevFronts&, const int32_t*, int, int, int, const T*, T*, cudaStream_t);
 
 MFD_INSTANTIATE_PANEL(double)

@@ -94,8 +94,9 @@ struct LevelPlan {
   LaunchList fwd_tasks, bwd_tasks;
   int32_t large_max_nf = 0;
   int32_t defer = 1;                 // panel steps per deferred trailing update
-  bool packed = false;               // the trailing updates read operands that the TRSM packs
-  int64_t q_elems = 0;               // of one panel step
+  int packed_steps = 0;              // the first panel steps, whose rows the TRSM also writes as packed update operands
+  std::vector<int64_t> q_base;       // their buffers: step s in number s mod the count
+  int packed_slot = 0;               // doubles of one front's packed diagonal block
 };
 
 }  // namespace mfd

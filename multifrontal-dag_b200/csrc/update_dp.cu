@@ -38,6 +38,7 @@ constexpr size_t kSmem = kStages * (size_t)kStageBytes;       // 96 KB: two CTAs
 constexpr long long kWait = 1ll << 31;                        // cycles (~1.1 s)
 constexpr int kChunks = kFactB / kKc;                         // of one step's block
 constexpr int kMaxGroup = kPackedDefer;
+static_assert(kMaxGroup == 2, "q and qprev");
 
 __device__ __forceinline__ void dmma16(double (&d)[4], const double (&a)[8], const double (&b)[4]) {
   asm volatile(
@@ -71,10 +72,10 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const double* src, uint3
                : "memory");
 }
 
-// q: the packed rows of the step's and the earlier steps' of its group, step t at
-// q + (t % nbuf) * buf; err[0] is raised if a wait expires.
+// q, qprev: the packed rows of the step and of the one before (read where its group has two);
+// err[0] is raised if a wait expires.
 __global__ void __launch_bounds__(kThreads, 2) k_update_dp(DevFronts F, const int32_t* list, int step, const double* q,
-                                                           int64_t buf, int nbuf, double* panel, double* upool,
+                                                           const double* qprev, double* panel, double* upool,
                                                            int32_t* err, int blo, int bhi, int defer) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long full[kStages];
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_update_dp(DevFronts F, const in
     // a 128-row block relative to `base` lies (step - s) blocks further down in the rows of step s
     // (every step of a group but its last is 128 wide)
     for (int s = g0; s <= step; ++s) {
-      const double* b = q + (s % nbuf) * buf + F.q_off[f] + (int64_t)(step - s) * (kFactB * kFactB);
+      const double* b = (s == step ? q : qprev) + F.q_off[f] + (int64_t)(step - s) * (kFactB * kFactB);
       src[0][s - g0] = b + (int64_t)ti * (kFactB * kFactB);
       src[1][s - g0] = b + (int64_t)tj * (kFactB * kFactB) + hf * kN * kKc;
     }
@@ -203,12 +204,12 @@ cudaError_t prepare_update_dp() {
   return cudaFuncSetAttribute(k_update_dp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
 }
 
-int launch_update_dp(const DevFronts& F, const int32_t* list, int count, int step, int T128, const double* q, int64_t buf,
-                     int nbuf, double* panel, double* upool, int32_t* err, cudaStream_t st, UpdBand band, int defer,
-                     bool pdl) {
+int launch_update_dp(const DevFronts& F, const int32_t* list, int count, int step, int T128, const double* q,
+                     const double* qprev, double* panel, double* upool, int32_t* err, cudaStream_t st, UpdBand band,
+                     int defer, bool pdl) {
   const int g = update_grid(T128, kUpdTile, band);
   if (count <= 0 || g <= 0) return 0;
-  launch_k(k_update_dp, dim3(2 * g, count), dim3(kThreads), kSmem, st, pdl, F, list, step, q, buf, nbuf, panel, upool, err,
+  launch_k(k_update_dp, dim3(2 * g, count), dim3(kThreads), kSmem, st, pdl, F, list, step, q, qprev, panel, upool, err,
            band.blo, band.bhi, defer);
   return 1;
 }

@@ -72,7 +72,7 @@ EXPORTS = [
     "mfd_autotune",
     "mfd_solve", "mfd_factorize_solve", "mfd_get_stats", "mfd_get_index", "mfd_get_symbolic", "mfd_get_front_panel",
     "mfd_destroy", "mfd_last_error", "mfd_set_profiling", "mfd_get_profile", "mfd_test_expire_waits",
-    "mfd_factor_fronts_noalloc",
+    "mfd_test_fail_alloc", "mfd_factor_fronts_noalloc",
     "mfd_noalloc_last_error", "mfd_symbolic_analyze", "mfd_symbolic_view", "mfd_symbolic_free", "mfd_mm_read",
     "mfd_coo_free", "mfd_coo_to_ccs", "mfd_analyze_csr", "mfd_order", "mfd_subtree_partition", "hppllt_init", "hppllt_set_precision", "hppllt_analyze",
     "hppllt_set_ordering",
@@ -124,6 +124,8 @@ def load(build_if_missing: bool = True):
     L.mfd_set_profiling.argtypes = [vp, i32]
     L.mfd_get_profile.argtypes = [vp, i32, C.POINTER(KernelProfile)]
     L.mfd_test_expire_waits.argtypes = [vp, i32]
+    L.mfd_test_fail_alloc.argtypes = [i64]
+    L.mfd_test_fail_alloc.restype = i64
     L.mfd_symbolic_analyze.argtypes = [C.POINTER(vp), i32, vp, vp, vp, i32]
     L.mfd_symbolic_view.argtypes = [vp, C.POINTER(Symbolic)]
     L.mfd_symbolic_free.argtypes = [vp]
