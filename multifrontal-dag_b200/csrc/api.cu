@@ -239,8 +239,6 @@ struct mfd_handle {
   std::vector<int32_t> h_stasks;                    // fused single-RHS solve tasks, 4 ints each
   int32_t solve_flags = 0;                          // per front and panel step, one sweep's worth
   int64_t bw_part_elems = 0;                        // backward sweep partial sums, largest level
-  void* d_bwpart = nullptr;                         // T, the backward sweep's partial sums
-  void* d_exch = nullptr;                           // single-RHS sweeps: n_total exchange entries of 2 sizeof(T)
   std::vector<int> small_bins;
   int64_t panel_elems = 0, upool_elems = 0, v_elems = 0, s_elems = 0, dinv_elems = 0;
   int64_t g_elems = 0;                              // gathered vectors of the level's fronts of many children, largest level
@@ -250,11 +248,11 @@ struct mfd_handle {
 
   // device tables
   DBuf<int32_t> d_nc, d_nr, d_first, d_parent, d_child_ptr, d_child, d_lrow_off, d_lrow, d_local, d_a_beg, d_a_src,
-      d_a_pos, d_sidx, d_lists, d_perm, d_info, d_cnt;
-  // fused solve: the tasks, and [0] expiry flag, [1 + 2 l] / [2 + 2 l] level l's forward /
+      d_a_pos, d_sidx, d_lists, d_perm, d_info;
+  // fused solve: the tasks, and (d_ssync) [0] expiry flag, [1 + 2 l] / [2 + 2 l] level l's forward /
   // backward tickets, then forward flags, backward flags and backward update-row counters,
   // one per front, panel step and RHS tile (zeroed before every solve)
-  DBuf<int32_t> d_stasks, d_ssync, d_epoch;
+  DBuf<int32_t> d_stasks;
   DBuf<int32_t> d_inv;
   DBuf<int64_t> d_inv_off;
   DBuf<FrontRec> d_rec;
@@ -274,11 +272,19 @@ struct mfd_handle {
   void* d_diag = nullptr;
   double* d_packed = nullptr;                       // the current panel step's packed diagonal blocks, one per list slot
   void* d_q = nullptr;                              // T, packed update operands, 2 defer step buffers
-  DBuf<double> d_a, d_b, d_xp, d_bp, d_r, d_norms, d_cnorms, d_xt, d_G;
-  void* d_X = nullptr;   // T, n_total x nrhs
-  void* d_V = nullptr;   // T
-  void* d_S = nullptr;   // T
+  DBuf<double> d_a, d_norms;
+
+  // storage of the solves for up to nrhs_cap right-hand sides, one allocation cut into parts (rhs_storage)
+  void* d_rhs = nullptr;
   int nrhs_cap = 0;
+  void *d_X = nullptr, *d_V = nullptr;              // T: n_total x nrhs; the fronts' vectors
+  void *d_S = nullptr, *d_bwpart = nullptr;         // T: partial sums of the backward sweeps, per step / fused
+  void* d_exch = nullptr;                           // single-RHS sweeps: n_total exchange entries of 2 sizeof(T)
+  double* d_G = nullptr;                            // gathered vectors of fronts with many children
+  double *d_b = nullptr, *d_bp = nullptr, *d_xp = nullptr, *d_r = nullptr, *d_xt = nullptr, *d_cnorms = nullptr;
+  int32_t *d_ssync = nullptr, *d_epoch = nullptr, *d_cnt = nullptr;
+  int32_t* d_ir_i = nullptr;                        // refinement state (launch_ir_init / launch_ir_check)
+  double *d_ir_d = nullptr, *d_ir_prev = nullptr;
 
   // block-local index export (per system)
   std::vector<std::vector<int32_t>> bli_node_ptr, bli_block_ptr, bli_pnum, bli_cnum, bli_off, bli_val, local_sys,
@@ -297,11 +303,11 @@ struct mfd_handle {
   cudaGraphExec_t g_factor = nullptr;
   std::map<int, cudaGraphExec_t> g_solve;
   std::map<int, cudaGraphExec_t> g_ir;              // FP32 + FP64 refinement, whole loop per RHS count
+  bool factor_ran = false;                          // a first factorization, first solves by graph key: without a graph
+  std::set<int> solve_ran;
   // captures the refinement loop's body; in other graphs what runs next to the main chain for a
   // whole factorization or solve (inverted diagonal blocks, the residual's matrix and right-hand side)
   cudaStream_t bst = nullptr;
-  DBuf<int32_t> d_ir_i;                             // refinement state (launch_ir_init / launch_ir_check)
-  DBuf<double> d_ir_d, d_ir_prev;
 
   // per-kernel-class profiling (graphs off while enabled)
   bool profiling = false;
@@ -318,7 +324,7 @@ struct mfd_handle {
     for (auto& kv : g_solve) cudaGraphExecDestroy(kv.second);
     for (auto& kv : g_ir) cudaGraphExecDestroy(kv.second);
     if (bst) cudaStreamDestroy(bst);
-    for (void* p : {d_panel, d_upool, d_diag, d_X, d_V, d_S, d_q, static_cast<void*>(d_packed), d_bwpart, d_exch})
+    for (void* p : {d_panel, d_upool, d_diag, d_q, static_cast<void*>(d_packed), d_rhs})
       if (p) cudaFree(p);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
@@ -941,40 +947,44 @@ int rhs_storage(mfd_handle* h, int nrhs) {
   h->g_solve.clear();
   for (auto& kv : h->g_ir) cudaGraphExecDestroy(kv.second);
   h->g_ir.clear();
-  size_t esz = h->fp32 ? sizeof(float) : sizeof(double);
-  for (void** p : {&h->d_X, &h->d_V, &h->d_S, &h->d_bwpart})
-    if (*p) { cudaFree(*p); *p = nullptr; }
-  if (!h->d_epoch.p && solve_fused(h, 1)) {
-    if (!h->d_exch) CK(dev_alloc(&h->d_exch, (size_t)h->n_total * 2 * esz));
-    CK(cudaMemsetAsync(h->d_exch, 0, (size_t)h->n_total * 2 * esz, h->st));
-    CK(h->d_epoch.alloc(1));
-    CK(cudaMemsetAsync(h->d_epoch.p, 0, sizeof(int32_t), h->st));
-  }
+  h->solve_ran.clear();
+  if (h->d_rhs) cudaFree(h->d_rhs);
+  h->d_rhs = nullptr;
+  const size_t esz = h->fp32 ? sizeof(float) : sizeof(double), n = h->n_total, k = nrhs;
+  const bool one_fused = solve_fused(h, 1), all_fused = solve_fused(h, nrhs), any_large = h->max_large_count > 0;
   int widest = nrhs;                        // the most right-hand sides up to nrhs that take the fused sweeps
   while (widest > 1 && !solve_fused(h, widest)) --widest;
-  CK(h->d_ssync.alloc(solve_sync_ints(h, solve_fused(h, widest) ? widest : 1)));
-  CK(cudaMemsetAsync(h->d_ssync.p, 0, sizeof(int32_t) * h->d_ssync.n, h->st));
-  CK(dev_alloc(&h->d_bwpart, (size_t)std::max<int64_t>(h->bw_part_elems, 1) * esz *
-                                  multi_part(widest)));
-  CK(dev_alloc(&h->d_X, (size_t)std::max<int64_t>(h->n_total, 1) * nrhs * esz));
-  CK(dev_alloc(&h->d_V, (size_t)std::max<int64_t>(h->v_elems, 1) * nrhs * esz));
-  if (h->g_elems > 0) CK(h->d_G.alloc((size_t)h->g_elems * nrhs));
-  if (h->max_large_count > 0 && !solve_fused(h, nrhs)) {   // tickets of the sweeps of one launch per step
-    CK(h->d_cnt.alloc((size_t)h->max_large_count * ((nrhs + kRhsG - 1) / kRhsG)));
-    CK(cudaMemsetAsync(h->d_cnt.p, 0, sizeof(int32_t) * h->d_cnt.n, h->st));
-    CK(dev_alloc(&h->d_S, (size_t)std::max<int64_t>(h->s_elems, 1) * nrhs * esz));   // and their partial sums
-  }
-  CK(h->d_b.alloc((size_t)h->n_total * nrhs));
-  CK(h->d_xp.alloc((size_t)h->n_total * nrhs));
-  CK(h->d_bp.alloc((size_t)h->n_total * nrhs));
-  CK(h->d_r.alloc((size_t)h->n_total * nrhs));
-  CK(h->d_cnorms.alloc((size_t)8 * nrhs));
-  if (h->fp32 && nrhs >= kResMulti) CK(h->d_xt.alloc((size_t)h->n_total * nrhs));
-  if (h->fp32) {
-    CK(h->d_ir_i.alloc(2));
-    CK(h->d_ir_d.alloc(2));
-    CK(h->d_ir_prev.alloc(nrhs));
-  }
+  size_t at = 0;
+  std::vector<std::pair<void**, size_t>> parts;
+  auto part = [&](auto*& p, size_t count, size_t size, bool used) {
+    p = nullptr;
+    if (!used) return;
+    parts.push_back({reinterpret_cast<void**>(&p), at});
+    at += (count * size + 255) / 256 * 256;
+  };
+  // zero at allocation: the exchange words (their tags) and the sweep's number, the flags, the tickets
+  part(h->d_exch, 2 * n, esz, one_fused);
+  part(h->d_epoch, 1, 4, one_fused);
+  part(h->d_ssync, solve_sync_ints(h, solve_fused(h, widest) ? widest : 1), 4, one_fused);
+  part(h->d_cnt, (size_t)h->max_large_count * ((k + kRhsG - 1) / kRhsG), 4, any_large && !all_fused);
+  const size_t zero = at;
+  part(h->d_X, n * k, esz, true);
+  part(h->d_V, h->v_elems * k, esz, true);
+  part(h->d_S, h->s_elems * k, esz, any_large && !all_fused);
+  part(h->d_bwpart, h->bw_part_elems * multi_part(widest), esz, one_fused);
+  part(h->d_G, h->g_elems * k, 8, h->g_elems > 0);
+  part(h->d_b, n * k, 8, true);
+  part(h->d_bp, h->fp32 ? n * k : n, 8, true);
+  part(h->d_r, h->fp32 ? n * k : n, 8, true);
+  part(h->d_xp, n * k, 8, h->fp32);
+  part(h->d_xt, n * k, 8, h->fp32 && nrhs >= kResMulti);
+  part(h->d_cnorms, 8 * k, 8, h->fp32);
+  part(h->d_ir_i, 2, 4, h->fp32);
+  part(h->d_ir_d, 2, 8, h->fp32);
+  part(h->d_ir_prev, k, 8, h->fp32);
+  CK(dev_alloc(&h->d_rhs, at));
+  for (auto& q : parts) *q.first = static_cast<char*>(h->d_rhs) + q.second;
+  if (zero) CK(cudaMemsetAsync(h->d_rhs, 0, zero, h->st));
   h->nrhs_cap = nrhs;
   return MFD_OK;
 }
@@ -1306,18 +1316,18 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
   const bool solve_pdl = h->opt.reserved[3] != 1 && !prof;
   const bool fused = solve_fused(h, nrhs);
   const int4* stasks = reinterpret_cast<const int4*>(h->d_stasks.p);
-  int32_t* ssync = h->d_ssync.p;
+  int32_t* ssync = h->d_ssync;
   int32_t* fwd_flags = ssync + 1 + 2 * h->levels.size();
   const int64_t nflags = h->solve_flags * multi_tiles(nrhs);
   int32_t* bwd_flags = fwd_flags + nflags;
   if (fused) {                              // a kernel, not a memset node: this also runs in the refinement loop's body
-    launch_solve_begin(ssync, solve_sync_ints(h, nrhs), h->d_epoch.p, st);
+    launch_solve_begin(ssync, solve_sync_ints(h, nrhs), h->d_epoch, st);
     ++n;
   }
   // a level's fused sweep
   auto sweep = [&](const LevelPlan& L, bool backward) {
     if (!backward && L.many.count) {
-      launch_gather_many<T>(F, lists + L.many.off, L.many.count, L.many_max_nf, X, ldx, V, h->d_G.p, nrhs, st);
+      launch_gather_many<T>(F, lists + L.many.off, L.many.count, L.many_max_nf, X, ldx, V, h->d_G, nrhs, st);
       ++n;
     }
     const LaunchList& tl = backward ? L.bwd_tasks : L.fwd_tasks;
@@ -1325,10 +1335,10 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
     int32_t* flags = backward ? bwd_flags : fwd_flags;
     T* part = static_cast<T*>(h->d_bwpart);
     if (nrhs == 1)
-      launch_large_fused<T>(F, stasks + tl.off, tl.count, backward, ticket, ssync, h->d_epoch.p, panel, dinv, X, V, h->d_G.p,
+      launch_large_fused<T>(F, stasks + tl.off, tl.count, backward, ticket, ssync, h->d_epoch, panel, dinv, X, V, h->d_G,
                             h->d_exch, st, h->d_info.p + 2, part, bwd_flags + nflags);
     else
-      launch_large_multi<T>(F, stasks + tl.off, tl.count, backward, ticket, flags, ssync, panel, dinv, X, ldx, V, h->d_G.p, nrhs,
+      launch_large_multi<T>(F, stasks + tl.off, tl.count, backward, ticket, flags, ssync, panel, dinv, X, ldx, V, h->d_G, nrhs,
                             st, h->d_info.p + 2, part, bwd_flags + nflags);
     ++n;
   };
@@ -1368,7 +1378,7 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
         if (fused) sweep(L, false);
         else
           launch_fwd_large<T>(F, lists + L.large.off, L.large.count, L.large.param2, L.large_max_nf, panel, dinv, X, ldx,
-                              V, h->d_cnt.p, nrhs, st, &n, solve_pdl);
+                              V, h->d_cnt, nrhs, st, &n, solve_pdl);
       });
     }
     if (nside) side_join(h, st, nside);
@@ -1393,7 +1403,7 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
         if (fused) sweep(L, true);
         else
           launch_bwd_large<T>(F, lists + L.large.off, L.large.count, L.large.param2, L.large_max_nf, panel, dinv, X, ldx,
-                              V, S, h->d_cnt.p, nrhs, st, &n, solve_pdl);
+                              V, S, h->d_cnt, nrhs, st, &n, solve_pdl);
       });
     }
     if (nside) side_join(h, st, nside);
@@ -1401,9 +1411,18 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
   return n;
 }
 
+// Whether this factorization or solve goes out as a graph: from the second one of its kind on (`ran`).
+// Building one takes 5 us a node along a chain and 20-25 with branches, more than the launches it
+// saves one call, which overlap with the kernels.  First factorization / solve of a new handle, as
+// graphs and now: 17 x 19 Laplacian 0.32 / 0.37 and 0.15 / 0.17 ms, batch of 200 systems 3.9 / 6.1 and
+// 1.7 / 1.3, 30 x 33 x 35 diffusion with five right-hand sides 4.7 / 4.7 and 2.2 / 1.4 (for the solves
+// also one allocation in place of up to seventeen).
+bool use_graph(const mfd_handle* h, bool ran) { return h->opt.use_graph && !h->profiling && ran; }
+
 template <typename Fn>
-int run_graph(mfd_handle* h, cudaGraphExec_t* exec, Fn&& fn) {
-  if (!h->opt.use_graph || h->profiling) {
+int run_graph(mfd_handle* h, bool graph, cudaGraphExec_t* exec, Fn&& fn) {
+  if (!graph) {
+    CK(cudaEventRecord(h->ev0, h->st));
     fn(h->st);
     CK(cudaGetLastError());
     return MFD_OK;
@@ -1420,6 +1439,7 @@ int run_graph(mfd_handle* h, cudaGraphExec_t* exec, Fn&& fn) {
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return fail(MFD_E_CUDA, std::string("instantiate: ") + cudaGetErrorString(e));
   }
+  CK(cudaEventRecord(h->ev0, h->st));
   CK(cudaGraphLaunch(*exec, h->st));
   return MFD_OK;
 }
@@ -1446,10 +1466,12 @@ int do_factorize(mfd_handle* h, const double* a) {
   cudaMemcpyKind kind = is_device_ptr(a) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   CK(cudaMemcpyAsync(h->d_a.p, a, sizeof(double) * h->a_len, kind, h->st));
   set_test_request(h);
-  CK(cudaEventRecord(h->ev0, h->st));
-  int rc = h->fp32 ? run_graph(h, &h->g_factor, [&](cudaStream_t s) { h->launches_factor = enqueue_factor<float>(h, s); })
-                   : run_graph(h, &h->g_factor, [&](cudaStream_t s) { h->launches_factor = enqueue_factor<double>(h, s); });
+  const bool graph = use_graph(h, h->factor_ran);
+  int rc = run_graph(h, graph, &h->g_factor, [&](cudaStream_t s) {
+    h->launches_factor = h->fp32 ? enqueue_factor<float>(h, s) : enqueue_factor<double>(h, s);
+  });
   if (rc) return rc;
+  h->factor_ran = true;
   CK(cudaEventRecord(h->ev1, h->st));
   CK(cudaStreamSynchronize(h->st));
   const int32_t* infos = h->status->info;
@@ -1485,29 +1507,30 @@ int fp64_solve(mfd_handle* h, int nrhs, bool report) {
   const int key = 2 * nrhs + (report ? 1 : 0);
   auto it = h->g_solve.find(key);
   cudaGraphExec_t exec = it == h->g_solve.end() ? nullptr : it->second;
-  const bool graph = h->opt.use_graph && !h->profiling, side = report && side_streams(h);
-  int rc = run_graph(h, &exec, [&](cudaStream_t s) {
+  const bool graph = use_graph(h, h->solve_ran.count(key) > 0), side = report && side_streams(h);
+  int rc = run_graph(h, graph, &exec, [&](cudaStream_t s) {
     if (report) {                                    // next to the sweeps: d_b stands until the end
       if (side) {
         cudaEventRecord(h->ev_inv, s);
         cudaStreamWaitEvent(h->bst, h->ev_inv, 0);
       }
-      launch_permute_in<double>(h->d_b.p, n, h->d_perm.p, h->d_bp.p, n, n, 1, side ? h->bst : s);
+      launch_permute_in<double>(h->d_b, n, h->d_perm.p, h->d_bp, n, n, 1, side ? h->bst : s);
       if (side) cudaEventRecord(h->ev_inv, h->bst);
     }
-    launch_permute_in<double>(h->d_b.p, n, h->d_perm.p, X, n, n, nrhs, s);
+    launch_permute_in<double>(h->d_b, n, h->d_perm.p, X, n, n, nrhs, s);
     h->launches_solve = enqueue_solve_core<double>(h, nrhs, s);
     cudaEventRecordWithFlags(h->ev1, s, graph ? cudaEventRecordExternal : cudaEventRecordDefault);
     if (report) {
       if (side) cudaStreamWaitEvent(s, h->ev_inv, 0);
-      launch_residual(h->d_csr_ptr.p, h->d_csr_col.p, h->d_csr_val.p, X, h->d_bp.p, h->d_r.p, n, s);
-      launch_norms(h->d_r.p, X, h->d_bp.p, n, h->d_norms.p, s);
+      launch_residual(h->d_csr_ptr.p, h->d_csr_col.p, h->d_csr_val.p, X, h->d_bp, h->d_r, n, s);
+      launch_norms(h->d_r, X, h->d_bp, n, h->d_norms.p, s);
     }
-    launch_permute_out<double>(X, n, h->d_perm.p, h->d_b.p, n, n, nrhs, s);
-    launch_solve_report(report ? h->d_norms.p : nullptr, nullptr, nullptr, solve_fused(h, nrhs) ? h->d_ssync.p : nullptr,
+    launch_permute_out<double>(X, n, h->d_perm.p, h->d_b, n, n, nrhs, s);
+    launch_solve_report(report ? h->d_norms.p : nullptr, nullptr, nullptr, solve_fused(h, nrhs) ? h->d_ssync : nullptr,
                         h->status->norms, nullptr, nullptr, &h->status->expired, s);
   });
   if (exec) h->g_solve[key] = exec;
+  if (rc == MFD_OK) h->solve_ran.insert(key);
   return rc;
 }
 
@@ -1515,18 +1538,18 @@ int fp64_solve(mfd_handle* h, int nrhs, bool report) {
 // in FP64, r = b - A x and the per-column norms (launch_norms layout) in FP64.
 int ir_sweep(mfd_handle* h, int nrhs, cudaStream_t st) {
   const int64_t n = h->n_total;
-  launch_to_t<float>(h->d_r.p, static_cast<float*>(h->d_X), n * nrhs, st);
+  launch_to_t<float>(h->d_r, static_cast<float*>(h->d_X), n * nrhs, st);
   h->launches_solve = enqueue_solve_core<float>(h, nrhs, st);
-  launch_axpy_from_t<float>(static_cast<float*>(h->d_X), h->d_xp.p, n * nrhs, st);
+  launch_axpy_from_t<float>(static_cast<float*>(h->d_X), h->d_xp, n * nrhs, st);
   if (nrhs >= kResMulti) {               // A read once for all columns
-    launch_residual_multi(h->d_csr_ptr.p, h->d_csr_col.p, h->d_csr_val.p, h->d_xp.p, h->d_xt.p, h->d_bp.p,
-                          h->d_r.p, n, nrhs, h->d_cnorms.p, st);
+    launch_residual_multi(h->d_csr_ptr.p, h->d_csr_col.p, h->d_csr_val.p, h->d_xp, h->d_xt, h->d_bp,
+                          h->d_r, n, nrhs, h->d_cnorms, st);
   } else {
     for (int r = 0; r < nrhs; ++r) {
       const int64_t o = (int64_t)r * n;
-      launch_residual(h->d_csr_ptr.p, h->d_csr_col.p, h->d_csr_val.p, h->d_xp.p + o, h->d_bp.p + o, h->d_r.p + o, n,
+      launch_residual(h->d_csr_ptr.p, h->d_csr_col.p, h->d_csr_val.p, h->d_xp + o, h->d_bp + o, h->d_r + o, n,
                       st);
-      launch_norms(h->d_r.p + o, h->d_xp.p + o, h->d_bp.p + o, n, h->d_cnorms.p + 8 * r, st);
+      launch_norms(h->d_r + o, h->d_xp + o, h->d_bp + o, n, h->d_cnorms + 8 * r, st);
     }
   }
   CK(cudaGetLastError());
@@ -1544,10 +1567,10 @@ int ir_graph(mfd_handle* h, int nrhs) {
     const int maxit = h->opt.ir_max_iter > 0 ? h->opt.ir_max_iter : 20;
     cudaStream_t st = h->st;
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    launch_permute_in<double>(h->d_b.p, n, h->d_perm.p, h->d_bp.p, n, n, nrhs, st);
-    cudaMemsetAsync(h->d_xp.p, 0, sizeof(double) * n * nrhs, st);
-    cudaMemcpyAsync(h->d_r.p, h->d_bp.p, sizeof(double) * n * nrhs, cudaMemcpyDeviceToDevice, st);
-    launch_ir_init(h->d_ir_i.p, h->d_ir_d.p, h->d_ir_prev.p, nrhs, st);
+    launch_permute_in<double>(h->d_b, n, h->d_perm.p, h->d_bp, n, n, nrhs, st);
+    cudaMemsetAsync(h->d_xp, 0, sizeof(double) * n * nrhs, st);
+    cudaMemcpyAsync(h->d_r, h->d_bp, sizeof(double) * n * nrhs, cudaMemcpyDeviceToDevice, st);
+    launch_ir_init(h->d_ir_i, h->d_ir_d, h->d_ir_prev, nrhs, st);
     cudaStreamCaptureStatus cs;
     cudaGraph_t g = nullptr;
     const cudaGraphNode_t* deps = nullptr;
@@ -1568,16 +1591,16 @@ int ir_graph(mfd_handle* h, int nrhs) {
       e = cudaStreamBeginCaptureToGraph(h->bst, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
       if (e == cudaSuccess) {
         int rc = ir_sweep(h, nrhs, h->bst);
-        launch_ir_check(h->d_cnorms.p, h->d_norms.p + 7, nrhs, h->opt.ir_tol, maxit, h->d_ir_prev.p, h->d_ir_i.p,
-                        h->d_ir_d.p, cond, h->bst);
+        launch_ir_check(h->d_cnorms, h->d_norms.p + 7, nrhs, h->opt.ir_tol, maxit, h->d_ir_prev, h->d_ir_i,
+                        h->d_ir_d, cond, h->bst);
         cudaGraph_t got = nullptr;
         cudaError_t e2 = cudaStreamEndCapture(h->bst, &got);
         if (rc != MFD_OK) e = cudaErrorUnknown;
         else if (e2 != cudaSuccess) e = e2;
       }
     }
-    launch_permute_out<double>(h->d_xp.p, n, h->d_perm.p, h->d_b.p, n, n, nrhs, st);
-    launch_solve_report(nullptr, h->d_ir_i.p, h->d_ir_d.p, solve_fused(h, nrhs) ? h->d_ssync.p : nullptr, nullptr,
+    launch_permute_out<double>(h->d_xp, n, h->d_perm.p, h->d_b, n, n, nrhs, st);
+    launch_solve_report(nullptr, h->d_ir_i, h->d_ir_d, solve_fused(h, nrhs) ? h->d_ssync : nullptr, nullptr,
                         h->status->ir_i, h->status->ir_d, &h->status->expired, st);
     cudaGraph_t outer = nullptr;
     cudaError_t e3 = cudaStreamEndCapture(st, &outer);
@@ -1590,6 +1613,7 @@ int ir_graph(mfd_handle* h, int nrhs) {
       return fail(MFD_E_CUDA, std::string("refinement graph: ") + cudaGetErrorString(e));
     }
   }
+  CK(cudaEventRecord(h->ev0, h->st));
   CK(cudaGraphLaunch(exec, h->st));
   return MFD_OK;
 }
@@ -1604,16 +1628,15 @@ int do_solve(mfd_handle* h, double* b, int nrhs, int64_t ldb, mfd_report* rep) {
   const int64_t n = h->n_total;
   cudaStream_t st = h->st;
   if (ldb == n) {
-    CK(cudaMemcpyAsync(h->d_b.p, b, sizeof(double) * n * nrhs, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(h->d_b, b, sizeof(double) * n * nrhs, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
   } else {
-    CK(cudaMemcpy2DAsync(h->d_b.p, sizeof(double) * n, b, sizeof(double) * ldb, sizeof(double) * n, nrhs,
+    CK(cudaMemcpy2DAsync(h->d_b, sizeof(double) * n, b, sizeof(double) * ldb, sizeof(double) * n, nrhs,
                          dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
   }
   set_test_request(h);
-  CK(cudaEventRecord(h->ev0, st));
   int iters = 0;
   double bwd = 0;
-  const bool ir_graphed = h->fp32 && h->opt.use_graph && !h->profiling;
+  const bool ir_graphed = h->fp32 && use_graph(h, h->solve_ran.count(nrhs) > 0);
   h->status->expired = 0;
   if (!h->fp32) {
     rc = fp64_solve(h, nrhs, rep != nullptr);
@@ -1628,10 +1651,11 @@ int do_solve(mfd_handle* h, double* b, int nrhs, int64_t ldb, mfd_report* rep) {
   } else {
     // FP32 factor + FP64 iterative refinement, all right-hand sides together,
     // the convergence test on the host after every sweep (schedule without
-    // graphs, and the per-kernel profiling runs)
-    launch_permute_in<double>(h->d_b.p, n, h->d_perm.p, h->d_bp.p, n, n, nrhs, st);
-    CK(cudaMemsetAsync(h->d_xp.p, 0, sizeof(double) * n * nrhs, st));
-    CK(cudaMemcpyAsync(h->d_r.p, h->d_bp.p, sizeof(double) * n * nrhs, cudaMemcpyDeviceToDevice, st));
+    // graphs, first solves, and the per-kernel profiling runs)
+    CK(cudaEventRecord(h->ev0, st));
+    launch_permute_in<double>(h->d_b, n, h->d_perm.p, h->d_bp, n, n, nrhs, st);
+    CK(cudaMemsetAsync(h->d_xp, 0, sizeof(double) * n * nrhs, st));
+    CK(cudaMemcpyAsync(h->d_r, h->d_bp, sizeof(double) * n * nrhs, cudaMemcpyDeviceToDevice, st));
     const int maxit = h->opt.ir_max_iter > 0 ? h->opt.ir_max_iter : 20;
     std::vector<double> prev(nrhs, 1e300), cur(nrhs, 1e300), nv((size_t)8 * nrhs);
     double worst_ref = 0;
@@ -1639,7 +1663,7 @@ int do_solve(mfd_handle* h, double* b, int nrhs, int64_t ldb, mfd_report* rep) {
     for (; it < maxit; ++it) {
       rc = ir_sweep(h, nrhs, st);
       if (rc) return rc;
-      CK(cudaMemcpyAsync(nv.data(), h->d_cnorms.p, sizeof(double) * 8 * nrhs, cudaMemcpyDeviceToHost, st));
+      CK(cudaMemcpyAsync(nv.data(), h->d_cnorms, sizeof(double) * 8 * nrhs, cudaMemcpyDeviceToHost, st));
       CK(cudaStreamSynchronize(st));
       bool all_ok = true, all_stalled = it > 2;
       bwd = 0;
@@ -1665,18 +1689,19 @@ int do_solve(mfd_handle* h, double* b, int nrhs, int64_t ldb, mfd_report* rep) {
       rep->backward_error = bwd;
       rep->residual_ref = worst_ref;
     }
-    launch_permute_out<double>(h->d_xp.p, n, h->d_perm.p, h->d_b.p, n, n, nrhs, st);
+    launch_permute_out<double>(h->d_xp, n, h->d_perm.p, h->d_b, n, n, nrhs, st);
     CK(cudaEventRecord(h->ev1, st));
+    h->solve_ran.insert(nrhs);
     if (!converged) rc = MFD_E_NOCONV;
   }
   if (ldb == n) {
-    CK(cudaMemcpyAsync(b, h->d_b.p, sizeof(double) * n * nrhs, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(b, h->d_b, sizeof(double) * n * nrhs, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
   } else {
-    CK(cudaMemcpy2DAsync(b, sizeof(double) * ldb, h->d_b.p, sizeof(double) * n, sizeof(double) * n, nrhs,
+    CK(cudaMemcpy2DAsync(b, sizeof(double) * ldb, h->d_b, sizeof(double) * n, sizeof(double) * n, nrhs,
                          dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
   }
   if (h->fp32 && !ir_graphed)
-    launch_solve_report(nullptr, nullptr, nullptr, solve_fused(h, nrhs) ? h->d_ssync.p : nullptr, nullptr, nullptr, nullptr,
+    launch_solve_report(nullptr, nullptr, nullptr, solve_fused(h, nrhs) ? h->d_ssync : nullptr, nullptr, nullptr, nullptr,
                         &h->status->expired, st);
   CK(cudaStreamSynchronize(st));
   const HostStatus& hs = *h->status;
@@ -1935,20 +1960,18 @@ int mfd_autotune(mfd_handle* h, const double* a, int32_t repeats, mfd_options* b
   if (!h || !a || !best || repeats < 1) return fail(MFD_E_ARG, "autotune: null handle, values or output");
   double best_t = 1e300;
   mfd_options best_o = h->opt;
-  // one candidate: a temporary handle on h's symbolic data, one warm-up
-  // factorization (graph capture), then the median of `repeats`
+  // one candidate: a temporary handle on h's symbolic data, two warm-up
+  // factorizations (the second one captures the graph), then the median of `repeats`
   auto trial = [&](const mfd_options& o, int* err) -> double {
     std::vector<Symbolic> syms = h->sys;
     mfd_handle* t = nullptr;
     if (create_common(&t, std::move(syms), &o) != MFD_OK) return 1e300;   // e.g. out of memory: skip it
     std::unique_ptr<mfd_handle> guard(t);
-    int rc = do_factorize(t, a);
-    if (rc != MFD_OK) { *err = rc; return 1e300; }
     std::vector<double> ms;
-    for (int r = 0; r < repeats; ++r) {
-      rc = do_factorize(t, a);
+    for (int r = -2; r < repeats; ++r) {
+      const int rc = do_factorize(t, a);
       if (rc != MFD_OK) { *err = rc; return 1e300; }
-      ms.push_back(t->factor_ms);
+      if (r >= 0) ms.push_back(t->factor_ms);
     }
     std::sort(ms.begin(), ms.end());
     return ms[ms.size() / 2];

@@ -89,7 +89,7 @@ def test_every_allocation_refused_once(which, precision):
         ref = solve(s)
         in_solve = L.mfd_test_fail_alloc(0)
         s.close()
-        assert in_setup > 20 and in_solve > 5
+        assert in_setup > 20 and in_solve >= 1
         without = 0
         for k in range(1, in_setup + 1):
             L.mfd_test_fail_alloc(k)
