@@ -1980,14 +1980,14 @@ int mfd_autotune(mfd_handle* h, const double* a, int32_t repeats, mfd_options* b
     int err = MFD_OK;
     const double t = trial(o, &err);
     if (err != MFD_OK) return err;
-    if (t < best_t) {
+    if (t < 0.97 * best_t) {                // within the noise of a small system's times the earlier one stands
       best_t = t;
       best_o = o;
     }
     return MFD_OK;
   };
   // stage 1: the schedule -- small-front / blocked split x lookahead
-  const int sfms[] = {32, 64, 96, 128};   // small-front split (at most kSmallFrontMax)
+  const int sfms[] = {32, 64, 96, 128, kSmallFrontMax};   // small-front split; the last one is the default
   for (int sfm : sfms)
     for (int lookahead_off = 0; lookahead_off <= 1; ++lookahead_off) {
       mfd_options o = h->opt;
