@@ -271,12 +271,13 @@ int mfd_set_profiling(mfd_handle *h, int32_t enable);
 int mfd_get_profile(mfd_handle *h, int32_t kind, mfd_kernel_profile *out);
 
 /* Test of the failure path (no counterpart in the reference).  While enabled,
- * every CTA of the FP32 tensor-core trailing update first waits on an mbarrier
- * that nothing arrives at, with a ~1 ms limit, before issuing any MMA; the
- * expired wait raises the handle's error flag and the kernel returns, so the
- * next mfd_factorize returns MFD_E_TIMEOUT (no GPU fault: every wait is
- * bounded).  Disable it and the handle factors normally again.  FP64 handles
- * and fronts that use no tensor-core update factor normally.  While enabled,
+ * every CTA of the trailing updates that have device waits (FP32: tensor cores;
+ * FP64: packed operands, fronts of 384 rows and more) waits on an mbarrier that
+ * nothing arrives at, with a ~1 ms limit; the expired wait raises the handle's
+ * error flag and the kernel returns, so the next mfd_factorize returns
+ * MFD_E_TIMEOUT (no GPU fault: every wait is bounded).  Disable it and the
+ * handle factors normally again.  Handles whose updates have no such wait factor
+ * normally.  While enabled,
  * the large-front solve sweeps' device waits (one launch per level, tasks
  * waiting on other tasks' values or flags) likewise wait for a value nothing
  * writes, with a ~1 ms limit: mfd_solve returns MFD_E_TIMEOUT, and solves

@@ -36,6 +36,7 @@ constexpr int kThreads = 256, kN = 64, kKc = 16, kStages = 4;
 constexpr uint32_t kABytes = kFactB * kKc * 8, kBBytes = kN * kKc * 8, kStageBytes = kABytes + kBBytes;   // 16 + 8 KB
 constexpr size_t kSmem = kStages * (size_t)kStageBytes;       // 96 KB: two CTAs per SM
 constexpr long long kWait = 1ll << 31;                        // cycles (~1.1 s)
+constexpr long long kProbeWait = 1ll << 21;                   // the test request's (~1 ms)
 constexpr int kChunks = kFactB / kKc;                         // of one step's block
 constexpr int kMaxGroup = kPackedDefer;
 static_assert(kMaxGroup == 2, "q and qprev");
@@ -48,8 +49,8 @@ __device__ __forceinline__ void dmma16(double (&d)[4], const double (&a)[8], con
       : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]), "d"(b[0]), "d"(b[1]),
         "d"(b[2]), "d"(b[3]));
 }
-// completion of the barrier's phase `parity`, bounded
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
+// completion of the barrier's phase `parity`, bounded by the cycles at `limit`
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, const volatile long long* limit) {
   const long long t0 = clock64();
   while (true) {
     uint32_t done;
@@ -63,7 +64,7 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
         : "r"(bar), "r"(parity)
         : "memory");
     if (done) return true;
-    if (clock64() - t0 > kWait) return false;
+    if (clock64() - t0 > *limit) return false;
   }
 }
 __device__ __forceinline__ void bulk_copy(uint32_t dst, const double* src, uint32_t bytes, uint32_t bar) {
@@ -73,13 +74,16 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const double* src, uint3
 }
 
 // q, qprev: the packed rows of the step and of the one before (read where its group has two);
-// err[0] is raised if a wait expires.
+// err[0] is raised if a wait expires; err[1] != 0 (a test of that path): the first chunk's barrier
+// expects one arrival more than it gets, and the limit is short.
 __global__ void __launch_bounds__(kThreads, 2) k_update_dp(DevFronts F, const int32_t* list, int step, const double* q,
                                                            const double* qprev, double* panel, double* upool,
                                                            int32_t* err, int blo, int bhi, int defer) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long full[kStages];
+  __shared__ long long limit;
   __shared__ const double* src[2][kMaxGroup];            // thread 0's: operand (A, B) rows in each step of the group
+  const bool probe = threadIdx.x == 0 && err[1] != 0;    // in flight with the front's sizes
   const int f = list[blockIdx.y];
   const int nc = F.nc[f], nr = F.nr[f], nf = nc + nr;
   const int c0 = step * kFactB;
@@ -97,7 +101,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_update_dp(DevFronts F, const in
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t sb = (uint32_t)__cvta_generic_to_shared(smem_raw), fb = (uint32_t)__cvta_generic_to_shared(full);
   if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(fb + 8 * s));
+    limit = probe ? kProbeWait : kWait;
+    for (int s = 0; s < kStages; ++s)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(fb + 8 * s), "r"(probe && s == 0 ? 2 : 1));
     // a 128-row block relative to `base` lies (step - s) blocks further down in the rows of step s
     // (every step of a group but its last is 128 wide)
     for (int s = g0; s <= step; ++s) {
@@ -160,7 +166,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_update_dp(DevFronts F, const in
   int c = 0;
   for (; c < nchunk; ++c) {
     const int s = c % kStages;
-    ok = bar_wait(fb + 8 * s, (c / kStages) & 1);
+    ok = bar_wait(fb + 8 * s, (c / kStages) & 1, &limit);
     if (!idle && ok) {
       const double* As = reinterpret_cast<const double*>(smem_raw + s * kStageBytes);
       const double* Bs = diag ? As + hf * kN * kKc : As + kABytes / 8;
@@ -191,7 +197,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_update_dp(DevFronts F, const in
   if (c < nchunk) {                                      // a wait expired: leave C alone, let the copies land
     if (tid == 0) {
       atomicExch(err, 1);
-      for (int d = c; d < min(nchunk, c + kStages); ++d) bar_wait(fb + 8 * (d % kStages), (d / kStages) & 1);
+      if (err[1] != 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(fb) : "memory");   // the arrival held back
+      for (int d = c; d < min(nchunk, c + kStages); ++d) bar_wait(fb + 8 * (d % kStages), (d / kStages) & 1, &limit);
     }
     return;
   }

@@ -153,3 +153,36 @@ def test_packed_fp64_update_bitwise(n):
     ref = panels.pop((3, 0, 2))
     for key, p in panels.items():
         assert np.array_equal(p, ref), key
+
+
+@pytest.mark.parametrize("use_graph", [0, 1])
+@pytest.mark.parametrize("n,lookahead_off", [(1153, 1), (2049, 0)])
+def test_packed_fp64_update_expired_wait(n, lookahead_off, use_graph):
+    """The packed-operand FP64 update's bounded wait runs out with its copies in flight (the request makes it wait
+    on a barrier of its own): the factorization ends with MFD_E_TIMEOUT, there is no factor to solve with, and the
+    handle factors as before, bit for bit, once the request is withdrawn.  1153 rows: 90 pieces in the first step as
+    one launch, too few for packed operands where the lookahead splits it; 2049 rows: 240 in its second part.  Not
+    packed (reserved[0] = 3): no wait."""
+    a = _spd(n, n)
+    col = np.concatenate([[1], 1 + np.cumsum(np.arange(n, 0, -1))]).astype(np.int32)
+    rows = np.concatenate([np.arange(j + 1, n + 1) for j in range(n)]).astype(np.int32)
+    vals = np.concatenate([a[j:, j] for j in range(n)])
+    s = H.Solver.analyze(n, col, rows, None, max_zero=0, use_graph=use_graph, reserved=(0, lookahead_off, 0, 0, 0, 0, 0))
+    assert s.factorize(vals) == 0
+    ref = s.front_panel(1).copy()
+    for _ in range(2):
+        s.test_expire_waits(True)
+        with pytest.raises(H.MfdError) as e:
+            s.factorize(vals)
+        assert e.value.code == -4
+        with pytest.raises(H.MfdError) as e:
+            s.solve(np.ones(n))
+        assert e.value.code == -6
+        s.test_expire_waits(False)
+        assert s.factorize(vals) == 0
+        assert np.array_equal(s.front_panel(1), ref)
+    s.close()
+    s = H.Solver.analyze(n, col, rows, None, max_zero=0, use_graph=use_graph, reserved=(3, 0, 0, 0, 0, 0, 0))
+    s.test_expire_waits(True)
+    assert s.factorize(vals) == 0
+    s.close()
