@@ -11,6 +11,7 @@
 import numpy as np
 import pytest
 
+from helpers import lower_panel
 from mfdag import hppllt as H
 from mfdag import problems as P
 
@@ -186,3 +187,70 @@ def test_packed_fp64_update_expired_wait(n, lookahead_off, use_graph):
     s.test_expire_waits(True)
     assert s.factorize(vals) == 0
     s.close()
+
+
+def _dense_ccs(n):
+    a = _spd(n, n)
+    col = np.concatenate([[1], 1 + np.cumsum(np.arange(n, 0, -1))]).astype(np.int32)
+    rows = np.concatenate([np.arange(j + 1, n + 1) for j in range(n)]).astype(np.int32)
+    return a, col, rows, np.concatenate([a[j:, j] for j in range(n)])
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("sizes", [(161, 384, 641, 1153), (1537, 1500, 129 * 9, 512, 385, 200), (2049, 1025, 1024, 1023)])
+def test_packed_updates_of_fronts_that_end_at_different_steps(sizes, precision):
+    """Dense systems of different orders in one handle: one level of fronts that leave the panel steps one after
+    another, so that a step's packed rows hold fewer fronts than the one's before and the deferred groups end at
+    different steps.  FP64: bit for bit the factor of the whole-tile kernel that reads the panel; FP32 + refinement:
+    a backward error of 1e-12, with the number of sweeps of the unpacked form (deferral 4) or one more."""
+    parts = [_dense_ccs(n) for n in sizes]
+    systems = [(n, p[1], p[2], None) for n, p in zip(sizes, parts)]
+    vals = np.concatenate([p[3] for p in parts])
+    b = np.random.default_rng(2).uniform(-1, 1, sum(sizes))
+    schedules = [(0, 0, 0), (0, 1, 0), (0, 0, 1), (0, 0, 2), (0, 1, 2), (3, 0, 0)] if precision == 0 else [(0, 0, 1), (0, 0, 2), (0, 1, 2), (0, 0, 4)]
+    got = {}
+    for kind, lookahead_off, defer in schedules:
+        s = H.Solver.analyze_batch(systems, max_zero=0, precision=precision,
+                                   reserved=(kind, lookahead_off, 0, 0, 0, defer, 0))
+        for _ in range(2):                               # launched, then as a graph
+            assert s.factorize(vals) == 0
+        x = b.copy()
+        rep, rc = s.solve(x)
+        assert rc == 0
+        at = 0
+        for n, p in zip(sizes, parts):
+            xs, bs = x[at:at + n], b[at:at + n]
+            den = np.abs(p[0]).sum(axis=1).max() * np.abs(xs).max() + np.abs(bs).max()
+            assert np.abs(bs - p[0] @ xs).max() / den <= (1e-14 if precision == 0 else 1e-12)
+            at += n
+        panels = [np.tril(s.front_panel(1, system=k).reshape((n, n), order="F")) for k, n in enumerate(sizes)]
+        got[kind, lookahead_off, defer] = (panels, rep.iterations)
+        s.close()
+    if precision == 0:
+        for key, (panels, _) in got.items():
+            for p, q in zip(panels, got[3, 0, 0][0]):
+                assert np.array_equal(p, q), key
+    else:
+        for key, (_, sweeps) in got.items():
+            assert sweeps <= got[0, 0, 4][1] + 1, key
+
+
+def test_packed_fp64_update_in_a_tree():
+    """A 3D Laplacian whose upper levels pack their operands (fronts of up to 1,296 columns, with update rows, several
+    to a level) and whose lower ones do not: the same bits as with the whole-tile kernel that reads the panel."""
+    p = P.laplace3d(36)
+    sym = H.symbolic_analyze(p.n, p.col, p.row, p.order, 1000)
+    nc, nr = np.diff(sym["node_ptr"]), np.diff(sym["lptr"])
+    b = np.random.default_rng(4).uniform(-1, 1, p.n)
+    got = []
+    for kind, lookahead_off, defer in ((3, 0, 0), (0, 0, 0), (0, 1, 2), (0, 0, 1)):
+        s = H.Solver.analyze(p.n, p.col, p.row, p.order, max_zero=1000, reserved=(kind, lookahead_off, 0, 0, 0, defer, 0))
+        assert s.factorize(p.val) == 0
+        x = b.copy()
+        s.solve(x)
+        assert s.stats().num_front == nc.size
+        got.append([x] + [lower_panel(s.front_panel(f + 1), int(nc[f] + nr[f]), int(nc[f])) for f in range(nc.size - 40, nc.size)])
+        s.close()
+    for other in got[1:]:
+        for u, v in zip(got[0], other):
+            assert np.array_equal(u, v)
