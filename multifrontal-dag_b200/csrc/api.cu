@@ -46,7 +46,7 @@ int fail(int code, const std::string& msg) {
 
 constexpr int64_t kAlign = 32;  // elements; keeps every front 256-byte aligned in FP64
 constexpr int kResMulti = 4;     // from this many right-hand sides on, one multi-column residual per IR sweep
-constexpr int kPotrfSplitMin = 148;   // fronts in a panel step above which POTRF launches per width class
+constexpr int kPotrfSplitMin = kNumSms;   // fronts in a panel step above which POTRF launches per width class
 // panel steps per deferred trailing update: K = 256 per pass halves the update's C traffic, which
 // counts on levels whose trailing matrices pass through HBM, their lower triangles above half of the
 // 126 MB L2 (80^3 diffusion, mixed: 45.7 -> 40.7 ms).  Below, a deferred update only lengthens the

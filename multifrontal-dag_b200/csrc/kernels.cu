@@ -48,16 +48,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-template <typename T>
-__device__ __forceinline__ void cp_async_t(T* dst, const T* src, bool valid) {
-  unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
-  const int sz = valid ? (int)sizeof(T) : 0;
-  if constexpr (sizeof(T) == 8)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(src), "r"(sz));
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sa), "l"(src), "r"(sz));
-}
-
 // Strided element loop (e = threadIdx.x, += blockDim.x, e < total) whose
 // global loads are issued kBatch at a time before the matching stores, so a
 // thread keeps kBatch independent loads in flight instead of one.
@@ -1279,7 +1269,7 @@ __global__ void k_fill_int(int32_t* p, int32_t v, int64_t n) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) p[i] = v;
 }
 
-inline int grid_1d(int64_t n, int threads = 256) { return clamp_grid(ceil_div(n, threads), 148 * 16); }
+inline int grid_1d(int64_t n, int threads = 256) { return clamp_grid(ceil_div(n, threads), kNumSms * 16); }
 
 // Dynamic shared memory above 48 KB is opted into once per kernel at handle
 // creation (prepare_kernels), never inside a stream capture.
@@ -1288,8 +1278,6 @@ template <typename KernelT>
 cudaError_t opt_in(KernelT k) {
   return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
 }
-template <typename KernelT>
-void set_smem(KernelT, size_t) {}
 
 }  // namespace
 

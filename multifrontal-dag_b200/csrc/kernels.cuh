@@ -11,7 +11,6 @@
 
 namespace mfd {
 
-constexpr int kNumSms = 148;
 constexpr int kSmallFrontMax = 160;   // widest front of the one-CTA / one-warp small-front kernels
 constexpr int kFactB = 128;          // column panel of the blocked large-front factorization
 constexpr int kTrRowsH = 64;         // rows per CTA of the panel TRSM

@@ -16,6 +16,8 @@
 
 namespace mfd {
 
+constexpr int kNumSms = 148;
+
 // A front as the small-front kernels read it: one 64-byte record per entry of the launch lists.
 struct alignas(16) FrontRec {
   int32_t nc, nr, first, lrow_off;

@@ -3,9 +3,11 @@
 #include <algorithm>
 #include <vector>
 
+#include "plan.hpp"
+
 namespace mfd {
 
-constexpr int kWarpFrontsAtOnce = 148 * 24;   // one-warp fronts the chip holds at once
+constexpr int kWarpFrontsAtOnce = kNumSms * 24;   // one-warp fronts the chip holds at once
 
 // The bins' largest orders, ascending, of a handle whose small fronts have at most sfm rows.
 inline std::vector<int> small_bin_sizes(int sfm) {

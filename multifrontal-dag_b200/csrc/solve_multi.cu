@@ -413,7 +413,7 @@ void launch_large_multi(const DevFronts& F, const int4* tasks, int ntask, bool b
   // its MMAs (elasticity 30^3, 64 right-hand sides, root front of 2,883 columns: forward sweep
   // 207 us with 8, 360 us with 16; its level of 928 fronts: 268 us with 16, 716 us with 8 and
   // whole blocks in registers).
-  if (nrhs <= 8 || (int64_t)ntask * stride <= 4 * 148) go(k_fwd_multi<T, 1>, k_bwd_multi<T, 1>, 8);
+  if (nrhs <= 8 || (int64_t)ntask * stride <= 4 * kNumSms) go(k_fwd_multi<T, 1>, k_bwd_multi<T, 1>, 8);
   else go(k_fwd_multi<T, 2>, k_bwd_multi<T, 2>, 16);
 }
 

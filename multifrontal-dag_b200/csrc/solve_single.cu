@@ -354,7 +354,7 @@ cudaError_t prepare_solve_single() {
 }
 
 void launch_solve_begin(int32_t* sync, int64_t n, int32_t* epoch, cudaStream_t st) {
-  k_solve_begin<<<(int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 148 * 4)), 256, 0, st>>>(sync, n, epoch);
+  k_solve_begin<<<(int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, kNumSms * 4)), 256, 0, st>>>(sync, n, epoch);
 }
 
 template <typename T>
@@ -371,7 +371,7 @@ void launch_large_fused(const DevFronts& F, const int4* tasks, int ntask, bool b
     k<<<ntask, 256, sm, st>>>(F, tasks, ntask, ticket, expired, epoch, panel, dinv, X, V, G, E, test_req);
   };
   if constexpr (sizeof(T) == 8) {
-    if (ntask > 148) {
+    if (ntask > kNumSms) {
       if (backward) bwd(k_bwd_single<T, 2>);
       else fwd(k_fwd_single<T, 32>);
       return;
