@@ -608,7 +608,7 @@ int build_plan(mfd_handle* h) {
     // single-RHS solve tasks of the level, in dependency order (see launch_large_fused)
     {
       auto push_task = [&](int32_t g, int32_t code, int32_t flag) {
-        h->h_stasks.insert(h->h_stasks.end(), {g, code, flag, 0});
+        h->h_stasks.insert(h->h_stasks.end(), {g, code, flag, cnt[g] > kManyChildren ? 1 : 0});
       };
       std::vector<int32_t> fbase(large.size());
       for (size_t k = 0; k < large.size(); ++k) {
@@ -1326,6 +1326,7 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
   }
   // a level's fused sweep
   auto sweep = [&](const LevelPlan& L, bool backward) {
+    const double* G = L.many.count ? h->d_G : nullptr;
     if (!backward && L.many.count) {
       launch_gather_many<T>(F, lists + L.many.off, L.many.count, L.many_max_nf, X, ldx, V, h->d_G, nrhs, st);
       ++n;
@@ -1335,10 +1336,10 @@ int64_t enqueue_solve_core(mfd_handle* h, int nrhs, cudaStream_t st) {
     int32_t* flags = backward ? bwd_flags : fwd_flags;
     T* part = static_cast<T*>(h->d_bwpart);
     if (nrhs == 1)
-      launch_large_fused<T>(F, stasks + tl.off, tl.count, backward, ticket, ssync, h->d_epoch, panel, dinv, X, V, h->d_G,
+      launch_large_fused<T>(F, stasks + tl.off, tl.count, backward, ticket, ssync, h->d_epoch, panel, dinv, X, V, G,
                             h->d_exch, st, h->d_info.p + 2, part, bwd_flags + nflags);
     else
-      launch_large_multi<T>(F, stasks + tl.off, tl.count, backward, ticket, flags, ssync, panel, dinv, X, ldx, V, h->d_G, nrhs,
+      launch_large_multi<T>(F, stasks + tl.off, tl.count, backward, ticket, flags, ssync, panel, dinv, X, ldx, V, G, nrhs,
                             st, h->d_info.p + 2, part, bwd_flags + nflags);
     ++n;
   };

@@ -250,13 +250,15 @@ void launch_bwd_large(const DevFronts& F, const int32_t* list, int count, int ma
                       const T* dinv, T* X, int64_t ldx, T* V, T* scratch, int32_t* cnt, int nrhs, cudaStream_t st,
                       int64_t* launches, bool pdl);
 // A level's single-RHS large-front sweep as one launch over its task list (4 ints per task:
-// front, code, flag base, partial-sum base; solve_single.cu).  Forward code >= 0: diagonal block,
+// front, code, flag base, backward partial-sum base / forward 1 with more than kManyChildren
+// children; solve_single.cu).  Forward code >= 0: diagonal block,
 // < 0: rest rows chunk -1 - code.  Backward code < 0: partial sums of update-row chunk j
 // (kBwdRestRows rows) against column block s (code = -1 - (s << 16 | j)), written to part and
 // counted in counters (one per front and step); code >= 0: column block, which adds its chunks'
 // partials in chunk order.  ticket and counters: zero before the launch; expired: raised when a
 // bounded wait gives up; epoch: the sweep's number (launch_solve_begin); exch: n_total exchange
-// entries of 2 sizeof(T), zero at allocation.  test_req (read once per CTA): nonzero makes every
+// entries of 2 sizeof(T), zero at allocation; G: null on levels without fronts of many children.
+// test_req (read once per CTA): nonzero makes every
 // wait run out after ~1 ms (a test of the expiry path).
 constexpr int kBwdRestRows = 256;
 cudaError_t prepare_solve_single();

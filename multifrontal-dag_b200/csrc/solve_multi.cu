@@ -113,11 +113,10 @@ __device__ __forceinline__ void zero(double2 (&v)[2][NB]) {
 }
 
 // gather_row (sweep_sync.cuh) for right-hand sides rc + 8 n and rc + 8 n + 1, n < NB, below re; row i < 0: zeros
-template <int NB, typename T>
-__device__ __forceinline__ void gather_rows(double2 (&v)[NB], const DevFronts& F, int f, int i, int nf, int nc, const T* Xf,
+template <int NB, bool kMany, typename T>
+__device__ __forceinline__ void gather_rows(double2 (&v)[NB], const DevFronts& F, int f, bool many, int i, int nf, int nc, const T* Xf,
                                             int64_t ldx, const T* V, const double* G, int nrhs, int rc, int re) {
-  const int cb = F.child_ptr[f], ce = F.child_ptr[f + 1];
-  if (ce - cb > kManyChildren) {
+  if (kMany && many) {
     const double* g = G + F.g_off[f] * nrhs + i;
 #pragma unroll
     for (int n = 0; n < NB; ++n) {
@@ -134,7 +133,7 @@ __device__ __forceinline__ void gather_rows(double2 (&v)[NB], const DevFronts& F
     v[n].y = i >= 0 && i < nc && r + 1 < re ? (double)Xf[i + (int64_t)(r + 1) * ldx] : 0.0;
   }
   if (i < 0) return;
-  for (int t = cb; t < ce; ++t) {
+  for (int t = F.child_ptr[f], ce = F.child_ptr[f + 1]; t < ce; ++t) {
     const ChildRec c = F.crec[t];
     const int ci = F.inv[c.inv_off + i];
     if (ci < 0) continue;
@@ -151,7 +150,7 @@ __device__ __forceinline__ void gather_rows(double2 (&v)[NB], const DevFronts& F
 // Forward: task (f, s, tile): y_s = Li (v_s - sum_{t<s} L_st y_t); rest tasks
 // (128 rows below the columns): v -= sum_t L_rest,t y_t.  Warp w has rows
 // 16 w .. 16 w + 15 of the task.
-template <typename T, int NB>
+template <typename T, int NB, bool kMany>
 __global__ void __launch_bounds__(256, 2)
     k_fwd_multi(DevFronts F, const int4* __restrict__ tasks, int ntask, int tiles, int stride, int32_t* ticket, int32_t* flags,
                 int32_t* expired, const T* __restrict__ panel, const T* __restrict__ dinv, T* X, int64_t ldx, T* V,
@@ -183,7 +182,7 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
   for (int m = 0; m < 2; ++m) {
     const int r = r0 + ri + 8 * m;
-    gather_rows<NB>(v[m], F, f, r < r1 ? r : -1, nf, nc, X + first, ldx, V, G, nrhs, c0r + q2, c0r + cols);
+    gather_rows<NB, kMany>(v[m], F, f, tk.w != 0, r < r1 ? r : -1, nf, nc, X + first, ldx, V, G, nrhs, c0r + q2, c0r + cols);
   }
   T a[2][kHalf][2];
   for (int s = 0; s < nsteps; ++s) {
@@ -413,8 +412,13 @@ void launch_large_multi(const DevFronts& F, const int4* tasks, int ntask, bool b
   // its MMAs (elasticity 30^3, 64 right-hand sides, root front of 2,883 columns: forward sweep
   // 207 us with 8, 360 us with 16; its level of 928 fronts: 268 us with 16, 716 us with 8 and
   // whole blocks in registers).
-  if (nrhs <= 8 || (int64_t)ntask * stride <= 4 * kNumSms) go(k_fwd_multi<T, 1>, k_bwd_multi<T, 1>, 8);
-  else go(k_fwd_multi<T, 2>, k_bwd_multi<T, 2>, 16);
+  if (nrhs <= 8 || (int64_t)ntask * stride <= 4 * kNumSms) {
+    if (G) go(k_fwd_multi<T, 1, true>, k_bwd_multi<T, 1>, 8);
+    else go(k_fwd_multi<T, 1, false>, k_bwd_multi<T, 1>, 8);
+  } else {
+    if (G) go(k_fwd_multi<T, 2, true>, k_bwd_multi<T, 2>, 16);
+    else go(k_fwd_multi<T, 2, false>, k_bwd_multi<T, 2>, 16);
+  }
 }
 
 #define MFD_INSTANTIATE_MULTI(T)                                                                                     \

@@ -105,7 +105,7 @@ __device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_grou
 // N: columns per half step in flight: 64, all of them, before the wait; in FP64 32
 // where the level has more tasks than SMs, so that two CTAs share an SM (in FP32
 // two do with 64).
-template <typename T, int N>
+template <typename T, int N, bool kMany>
 __global__ void __launch_bounds__(256, N == 64 && sizeof(T) == 8 ? 1 : 2) k_fwd_single(DevFronts F, const int4* __restrict__ tasks, int ntask,
                                                     int32_t* ticket, int32_t* expired, const int32_t* epoch,
                                                     const T* __restrict__ panel, const T* __restrict__ dinv, T* X, T* V,
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(256, N == 64 && sizeof(T) == 8 ? 1 : 2) k_fwd_
   const bool valid = i < r1;
   if (code >= 0) stage_inverse(Ls, dinv + F.d_off[f] + (size_t)code * kSolveB * kSolveB, r1 - r0);
   T v = T(0);
-  if (h == 0 && valid) v = gather_row(F, f, i, nf, nc, X + first, V, G, 1, 0);
+  if (h == 0 && valid) v = gather_row<kMany>(F, f, tk.w != 0, i, nf, nc, X + first, V, G, 1, 0);
   T acc[4] = {T(0), T(0), T(0), T(0)};
   for (int s = 0; s < nsteps; ++s) {
     const int c0 = s * kSolveB, w = min(kSolveB, nc - c0);
@@ -347,9 +347,10 @@ cudaError_t prepare_solve_single() {
     cudaError_t r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (r != cudaSuccess && e == cudaSuccess) e = r;
   };
-  chk(k_fwd_single<double, 64>, kFoldElems * sizeof(double)); chk(k_bwd_single<double, 4>, kFoldElems * sizeof(double));
-  chk(k_fwd_single<double, 32>, kFoldElems * sizeof(double)); chk(k_bwd_single<double, 2>, kFoldElems * sizeof(double));
-  chk(k_fwd_single<float, 64>, kFoldElems * sizeof(float)); chk(k_bwd_single<float, 4>, kFoldElems * sizeof(float));
+  auto fwd = [&](auto k, auto k_many, size_t bytes) { chk(k, bytes); chk(k_many, bytes); };
+  fwd(k_fwd_single<double, 64, false>, k_fwd_single<double, 64, true>, kFoldElems * sizeof(double)); chk(k_bwd_single<double, 4>, kFoldElems * sizeof(double));
+  fwd(k_fwd_single<double, 32, false>, k_fwd_single<double, 32, true>, kFoldElems * sizeof(double)); chk(k_bwd_single<double, 2>, kFoldElems * sizeof(double));
+  fwd(k_fwd_single<float, 64, false>, k_fwd_single<float, 64, true>, kFoldElems * sizeof(float)); chk(k_bwd_single<float, 4>, kFoldElems * sizeof(float));
   return e;
 }
 
@@ -373,12 +374,14 @@ void launch_large_fused(const DevFronts& F, const int4* tasks, int ntask, bool b
   if constexpr (sizeof(T) == 8) {
     if (ntask > kNumSms) {
       if (backward) bwd(k_bwd_single<T, 2>);
-      else fwd(k_fwd_single<T, 32>);
+      else if (G) fwd(k_fwd_single<T, 32, true>);
+      else fwd(k_fwd_single<T, 32, false>);
       return;
     }
   }
   if (backward) bwd(k_bwd_single<T, 4>);
-  else fwd(k_fwd_single<T, 64>);
+  else if (G) fwd(k_fwd_single<T, 64, true>);
+  else fwd(k_fwd_single<T, 64, false>);
 }
 
 #define MFD_INSTANTIATE_SINGLE(T)                                                                                  \

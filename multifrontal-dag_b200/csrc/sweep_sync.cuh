@@ -50,14 +50,16 @@ __device__ __forceinline__ bool cta_wait_flag(const int32_t* flag, int32_t* expi
 // Entry i of front f's vector before its panel steps: its own right-hand side
 // (Xf: the front's first column) plus the children's update vectors in child
 // order (V: nrhs columns per front, column r), two children's loads in flight;
-// with many children the sum is in G already (launch_gather_many).
-template <typename T>
-__device__ __forceinline__ T gather_row(const DevFronts& F, int f, int i, int nf, int nc, const T* Xf, const T* V,
+// with many children (`many`, said by the task) the sum is in G already (launch_gather_many).
+// kMany: the level has such fronts; the others' sweeps are compiled without (37 x 41 x 43 solve
+// 801 us, 805 with the branch).
+template <bool kMany, typename T>
+__device__ __forceinline__ T gather_row(const DevFronts& F, int f, bool many, int i, int nf, int nc, const T* Xf, const T* V,
                                         const double* G, int nrhs, int r) {
-  const int cb = F.child_ptr[f], ce = F.child_ptr[f + 1];
-  if (ce - cb > kManyChildren) return (T)G[F.g_off[f] * nrhs + (int64_t)r * nf + i];
+  if (kMany && many) return (T)G[F.g_off[f] * nrhs + (int64_t)r * nf + i];
   T v = i < nc ? Xf[i] : T(0);
-  for (int t = cb; t < ce; t += 2) {
+  const int ce = F.child_ptr[f + 1];
+  for (int t = F.child_ptr[f]; t < ce; t += 2) {
     T x[2];
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
