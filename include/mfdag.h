@@ -49,7 +49,8 @@ typedef struct {
   int32_t precision;       /* MFD_PREC_*                                                      */
   int32_t ir_max_iter;     /* refinement iterations (precision FP32_IR), default 20           */
   double ir_tol;           /* target normwise backward error, default 1e-12                   */
-  int32_t use_graph;       /* 1: replay factor/solve as CUDA graphs (default 1)               */
+  int32_t use_graph;       /* 1: CUDA graphs, captured at the second factorization / solve of a
+                              kind and replayed from then on (default 1)                     */
   int32_t device;          /* CUDA device ordinal (default 0)                                 */
   int32_t small_front_max; /* fronts up to this order (at most 160) run in the fused kernels (0=auto) */
   int32_t panel_width;     /* column panel of the blocked large-front factorization (0=auto) */
@@ -58,7 +59,8 @@ typedef struct {
                               [1] = 1 lookahead off, [2] = 1 programmatic launch along the panel
                               chain, [3] = 1 no programmatic launch between solve steps, [4] = 1
                               no side streams per level, [5] = panel steps per deferred trailing
-                              update (1 = none; 0: two on levels whose fronts exceed 64 MB),
+                              update (1 = none; 0: two on levels whose lower triangles exceed
+                              64 MB),
                               [6] = 1 large-front solves one launch per panel step instead of
                               one per level                                                     */
 } mfd_options;

@@ -46,8 +46,9 @@ def test_expired_wait_reports_timeout_and_handle_recovers():
 
 
 def test_expire_request_leaves_fp64_factor_alone():
-    """In the factorization the request only concerns the FP32 tensor-core
-    update: an FP64 handle factors normally with it set."""
+    """In the factorization the request concerns the updates that have device
+    waits: an FP64 handle whose fronts are below the packed-operand update's
+    (test_gpu_large_fronts.py has that one) factors normally with it set."""
     p = P.laplace3d(12)
     s = H.Solver.analyze(p.n, p.col, p.row, p.order, max_zero=10, small_front_max=48)
     s.test_expire_waits(True)
