@@ -66,3 +66,42 @@ def test_device_times_leave_the_capture_out():
         t.append(rep.time_ms)
     assert f[1] <= 3 * np.median(f[2:]) + 0.2 and t[1] <= 3 * np.median(t[2:]) + 0.2
     s.close()
+
+
+def test_handles_on_several_threads():
+    """Four threads, each with handles of its own coming and going: direct first calls, captures, replays, set-ups and
+    frees of one thread run while the others capture.  Every solution has the bits of a handle used alone."""
+    import threading
+    kinds = [("laplace", 0), ("batch", 0), ("laplace", 1), ("batch", 1)]
+    alone = {}
+    for kind, precision in kinds:
+        s, val = _handle(kind, precision=precision)
+        b = np.random.default_rng(9).uniform(-1, 1, s.n)
+        assert s.factorize(val) == 0
+        x = b.copy()
+        s.solve(x)
+        alone[kind, precision] = x
+        s.close()
+    errors = []
+
+    def work(first):
+        try:
+            for turn in range(6):
+                kind, precision = kinds[(first + turn) % 4]
+                s, val = _handle(kind, precision=precision)
+                b = np.random.default_rng(9).uniform(-1, 1, s.n)
+                for _ in range(4):
+                    assert s.factorize(val) == 0
+                    x = b.copy()
+                    rep, rc = s.solve(x)
+                    assert rc == 0 and np.array_equal(x, alone[kind, precision])
+                s.close()
+        except BaseException as e:                       # noqa: BLE001 - reported by the main thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(300)
+    assert not errors and not any(t.is_alive() for t in threads), errors
